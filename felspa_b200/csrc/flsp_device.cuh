@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace flsp {
 
 constexpr int kMaxP = 3;
@@ -50,6 +52,94 @@ static __constant__ Tab1D<float> c_tab_f[kMaxP + 1];
 template <typename T> __device__ __forceinline__ const Tab1D<T>& tab(int p);
 template <> __device__ __forceinline__ const Tab1D<double>& tab<double>(int p) { return c_tab_d[p]; }
 template <> __device__ __forceinline__ const Tab1D<float>& tab<float>(int p) { return c_tab_f[p]; }
+
+// ---------------------------------------------------------------------
+// 1D Legendre sums by parity.  About the interval's centre L_a and the
+// Gauss rule are even / odd (L_a(1 - x) = (-1)^a L_a(x), L_0 = 1, L_1'
+// constant), so the points q and NQ-1-q share the even and the odd part of
+// a sum: 3 modes to 4 points take 6 instructions instead of 12, their
+// derivatives 5 instead of 12, 4 modes to 5 points 11 instead of 20.
+// ---------------------------------------------------------------------
+// v[q] = sum_a c[a S] L_a(x_q)
+template <int N1, int NQ, int S, typename T>
+__device__ __forceinline__ void gauss_values(const Tab1D<T>& tb, const T* c, T* v) {
+  constexpr int H = NQ / 2;
+#pragma unroll
+  for (int q = 0; q < H; ++q) {
+    T e = c[0];
+    if constexpr (N1 > 2) e += c[2 * S] * tb.Lq[2][q];
+    if constexpr (N1 > 3) {
+      const T o = c[S] * tb.Lq[1][q] + c[3 * S] * tb.Lq[3][q];
+      v[q] = e + o;
+      v[NQ - 1 - q] = e - o;
+    } else {
+      v[q] = e + c[S] * tb.Lq[1][q];
+      v[NQ - 1 - q] = e - c[S] * tb.Lq[1][q];
+    }
+  }
+  if constexpr (NQ % 2) {
+    T e = c[0];
+    if constexpr (N1 > 2) e += c[2 * S] * tb.Lq[2][H];
+    v[H] = e;
+  }
+}
+// v[q] = sum_a c[a S] L_a'(x_q); c[0] is not read
+template <int N1, int NQ, int S, typename T>
+__device__ __forceinline__ void gauss_derivatives(const Tab1D<T>& tb, const T* c, T* v) {
+  constexpr int H = NQ / 2;
+  const T c1 = c[S] * tb.Dq[1][0];
+#pragma unroll
+  for (int q = 0; q < H; ++q) {
+    T e = c1;
+    if constexpr (N1 > 3) e += c[3 * S] * tb.Dq[3][q];
+    if constexpr (N1 > 2) {
+      v[q] = e + c[2 * S] * tb.Dq[2][q];
+      v[NQ - 1 - q] = e - c[2 * S] * tb.Dq[2][q];
+    } else {
+      v[q] = e;
+      v[NQ - 1 - q] = e;
+    }
+  }
+  if constexpr (NQ % 2) {
+    T e = c1;
+    if constexpr (N1 > 3) e += c[3 * S] * tb.Dq[3][H];
+    v[H] = e;
+  }
+}
+// X[a S] += sum_q f[q] L_a(x_q), a < NA
+template <int NA, int NQ, int S, typename T>
+__device__ __forceinline__ void gauss_project(const Tab1D<T>& tb, const T* f, T* X) {
+  constexpr int H = NQ / 2;
+#pragma unroll
+  for (int q = 0; q < H; ++q) {
+    const T s = f[q] + f[NQ - 1 - q];
+    X[0] += s;
+    if constexpr (NA > 1) {
+      const T d = f[q] - f[NQ - 1 - q];
+      X[S] += d * tb.Lq[1][q];
+      if constexpr (NA > 3) X[3 * S] += d * tb.Lq[3][q];
+    }
+    if constexpr (NA > 2) X[2 * S] += s * tb.Lq[2][q];
+  }
+  if constexpr (NQ % 2) {
+    X[0] += f[H];
+    if constexpr (NA > 2) X[2 * S] += f[H] * tb.Lq[2][H];
+  }
+}
+// the values at the interval's ends 0 and 1
+template <int N1, int S, typename T>
+__device__ __forceinline__ void end_values(const Tab1D<T>& tb, const T* c, T& lo, T& hi) {
+  T e = c[0], o = T(0);
+  if constexpr (N1 > 2) e += c[2 * S] * tb.L1[2];
+  if constexpr (N1 > 3) {
+    o = c[S] * tb.L1[1] + c[3 * S] * tb.L1[3];
+    lo = e - o;
+    hi = e + o;
+  } else {
+    lo = e - c[S] * tb.L1[1];
+    hi = e + c[S] * tb.L1[1];
+  }
+}
 
 // ---------------------------------------------------------------------
 // device clock: simulation time and CFL state live on the GPU so that a
@@ -118,6 +208,14 @@ __device__ __forceinline__ void atomic_max_pos(unsigned long long* slot, double 
   atomicMax(slot, (unsigned long long)__double_as_longlong(v));
 }
 
+// rsqrtf of a normal number (rsqrtf's own instruction without the scaling
+// around it for subnormal inputs)
+__device__ __forceinline__ float rsqrt_normal(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 template <typename T>
 __device__ __forceinline__ T warp_max(T v) {
 #pragma unroll
@@ -130,6 +228,23 @@ __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+
+// max of a non-negative value over a warp, NaN counting as zero; into the
+// shared slot of the block (atomics on the bit patterns), which starts at 0
+__device__ __forceinline__ void slot_max(unsigned int* slot, float v) {
+  const unsigned int u = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(v, 0.f)));
+  if ((threadIdx.x & 31) == 0) atomicMax(slot, u);
+}
+__device__ __forceinline__ void slot_max(unsigned long long* slot, double v) {
+  v = warp_max(fmax(v, 0.0));
+  if ((threadIdx.x & 31) == 0) atomicMax(slot, (unsigned long long)__double_as_longlong(v));
+}
+__device__ __forceinline__ double slot_value(const unsigned int* slot) { return (double)__uint_as_float(*slot); }
+__device__ __forceinline__ double slot_value(const unsigned long long* slot) {
+  return __longlong_as_double((long long)*slot);
+}
+template <typename T>
+using MaxSlot = std::conditional_t<sizeof(T) == 4, unsigned int, unsigned long long>;
 
 // block-wide max of a non-negative double, result valid in thread 0
 __device__ __forceinline__ double block_max(double v, double* red) {
@@ -299,6 +414,11 @@ __device__ __forceinline__ void cp_async_elem(T* smem, const T* gmem) {
   else
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
 }
+// 16 bytes, both addresses 16-byte aligned (past the L1: read once per CTA)
+__device__ __forceinline__ void cp_async_16(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // Load of the tile and its face halo (no edges/corners) from a cell-major
@@ -405,6 +525,33 @@ __device__ __forceinline__ void store_tile(const MeshArgs& m, const T* __restric
         dst[e] = src[(size_t)cx * NM + m.g2q[k]];
       }
     }
+  }
+}
+
+// Halo box of the TX x TY x TZ tile at (ox, oy, oz) as rows of cells along x:
+// row (ly, lz) holds cells [max(ox - 1, 0), min(ox + TX + 1, n)) of NMB bytes
+// from the 16-byte aligned address at or below the first, in slot
+// (ly + 1) + BY (lz + 1) of SLOT bytes; rows outside the mesh and edge rows
+// are left out.  One warp per row, 16 bytes per lane: against one bulk copy
+// per row (36 rows of 0.7 KB for a 4x4x4 tile) it spreads the requests over
+// the load units.  Completes with cp_async_wait_all() and a barrier.
+template <int DIM, int TX, int TY, int TZ, int NMB, int SLOT>
+__device__ __forceinline__ void load_box_rows(const MeshArgs& m, const void* g, unsigned char* box, int ox, int oy,
+                                              int oz, int warp, int nw) {
+  constexpr int BY = TY + 2, NROWS = BY * (DIM > 2 ? TZ + 2 : 1);
+  const int lane = threadIdx.x & 31;
+  const char* src = reinterpret_cast<const char*>(g);
+  const int hx0 = max(ox - 1, 0), hx1 = min(ox + TX + 1, m.n[0]);
+  for (int rr = warp; rr < NROWS; rr += nw) {
+    const int ly = rr % BY - 1, lz = DIM > 2 ? rr / BY - 1 : 0;
+    const bool yout = ly < 0 || ly >= TY, zout = DIM > 2 && (lz < 0 || lz >= TZ);
+    if (yout && zout) continue;
+    const int gy = oy + ly, gz = oz + lz;
+    if (gy < 0 || gy >= m.n[1] || (DIM > 2 && (gz < 0 || gz >= m.n[2]))) continue;
+    const long long rowcell = (long long)m.n[0] * (gy + (long long)m.n[1] * (DIM > 2 ? gz : 0));
+    const long long a0 = ((rowcell + hx0) * NMB) & ~15LL;
+    const int n16 = (int)(((rowcell + hx1) * NMB + 15 - a0) >> 4);
+    for (int c = lane; c < n16; c += 32) cp_async_16(box + (size_t)rr * SLOT + 16 * c, src + a0 + 16 * c);
   }
 }
 

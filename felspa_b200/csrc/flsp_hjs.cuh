@@ -55,18 +55,26 @@ struct HjsPlan {
   static constexpr int BY = TL::Y + 2, BZ = DIM > 2 ? TL::Z + 2 : 1, NROWS = BY * BZ;
   static constexpr int NMB = NM * (int)sizeof(T);   // bytes per cell
   static constexpr int SLOT = (((TL::X + 2) * NMB + 30) + 15) / 16 * 16;
-  static constexpr size_t OFF_BOX = 16;
+  static constexpr size_t OFF_BOX = 32;   // mbarrier, CFL maximum
   static constexpr size_t OFF_JN = OFF_BOX + (size_t)NROWS * SLOT;
   static constexpr size_t OFF_JV = OFF_JN + (size_t)2 * DIM * NQF * TL::N * sizeof(T);
-  // the tile's slice of the sign table (pseudo-steps: staged with the box),
-  // then, once every thread has read its entries, the plane projections
+  // the tile's slice of the sign table (pseudo-steps: staged with the box);
+  // a thread's plane projections overwrite the entries of its own plane
   static constexpr int NS = ipow(NQ, DIM) + (1 << DIM);
   static constexpr size_t TAB_BYTES = (size_t)NS * TL::N * sizeof(T);
   static constexpr size_t UB_BYTES = (size_t)NQ * NU * TL::N * sizeof(T);
   static constexpr size_t OFF_UB = (OFF_JV + (size_t)2 * DIM * NC * TL::N * sizeof(T) + 15) / 16 * 16;
-  static constexpr size_t OFF_RED = (OFF_UB + (TAB_BYTES > UB_BYTES ? TAB_BYTES : UB_BYTES) + 15) / 16 * 16;
-  static constexpr size_t BYTES = OFF_RED + 64 * sizeof(double);
+  static constexpr size_t BYTES = OFF_UB + (TAB_BYTES > UB_BYTES ? TAB_BYTES : UB_BYTES);
 };
+
+// CTAs per SM the registers are held to: FP32 3D, as many as the shared
+// memory admits (80 registers, 24 warps: left to itself the compiler takes
+// 105 and two CTAs, and the kernel is no faster than before it lost a third
+// of its instructions)
+template <int DIM, int P, typename T>
+constexpr int hjs_min_blocks() {
+  return DIM == 3 && sizeof(T) == 4 ? (P == 1 ? 4 : 3) : 1;
+}
 
 template <int DIM, int P, typename T>
 __host__ __device__ inline size_t hjs_smem_bytes(const int*) {
@@ -139,13 +147,10 @@ __device__ __forceinline__ void hjs_face(const MeshArgs& m, const CellP& cellp, 
     for (int mf = 0; mf < NF; ++mf) {
       const int m0 = mf % N1, m1 = mf / N1;
       const int base = m0 * st[t0] + (DIM > 2 ? m1 * st[t1] : 0);
-      T tup = T(0), tdn = T(0);
+      T j = cu[base] - cd[base];   // L_0 = 1
 #pragma unroll
-      for (int b = 0; b < N1; ++b) {
-        tup += tb.L0[b] * cu[base + b * st[E]];
-        tdn += tb.L1[b] * cd[base + b * st[E]];
-      }
-      J[mf] = tup - tdn;
+      for (int b = 1; b < N1; ++b) j += tb.L0[b] * cu[base + b * st[E]] - tb.L1[b] * cd[base + b * st[E]];
+      J[mf] = j;
     }
   } else {
 #pragma unroll
@@ -156,136 +161,113 @@ __device__ __forceinline__ void hjs_face(const MeshArgs& m, const CellP& cellp, 
   const int cu_l = f < tl[E] ? lu[0] + tl[0] * (lu[1] + tl[1] * lu[2]) : -1;
   const int cd_l = f >= 1 ? ll[0] + tl[0] * (ll[1] + tl[1] * ll[2]) : -1;
   const T ihE = T(1.0 / m.h[E]);
+#pragma unroll
+  for (int mf = 0; mf < NF; ++mf) J[mf] *= ihE;
   auto put = [&](int q, T v, bool corner) {
     const int base = corner ? 2 * E * NC : 2 * E * NQF, stride = corner ? NC : NQF;
     T* dst = corner ? jv : jn;
-    v *= ihE;
     if (cu_l >= 0) dst[(size_t)(base + q) * nt + cu_l] = v;
     if (cd_l >= 0) dst[(size_t)(base + stride + q) * nt + cd_l] = v;
   };
   if constexpr (DIM == 2) {
+    T v[NQ], lo, hi;
+    gauss_values<N1, NQ, 1, T>(tb, J, v);
+#pragma unroll
+    for (int q0 = 0; q0 < NQ; ++q0) put(q0, v[q0], false);
+    end_values<N1, 1, T>(tb, J, lo, hi);
+    put(0, lo, true);
+    put(1, hi, true);
+  } else {
+    T Pq[N1][NQ], Pl[N1], Ph[N1];   // [m1][q0], and at the ends of axis t0
+#pragma unroll
+    for (int m1 = 0; m1 < N1; ++m1) {
+      gauss_values<N1, NQ, 1, T>(tb, J + N1 * m1, Pq[m1]);
+      end_values<N1, 1, T>(tb, J + N1 * m1, Pl[m1], Ph[m1]);
+    }
 #pragma unroll
     for (int q0 = 0; q0 < NQ; ++q0) {
-      T s = T(0);
+      T v[NQ];
+      gauss_values<N1, NQ, NQ, T>(tb, &Pq[0][q0], v);
 #pragma unroll
-      for (int m0 = 0; m0 < N1; ++m0) s += J[m0] * tb.Lq[m0][q0];
-      put(q0, s, false);
+      for (int q1 = 0; q1 < NQ; ++q1) put(q0 + NQ * q1, v[q1], false);
     }
-#pragma unroll
-    for (int cr = 0; cr < 2; ++cr) {
-      T s = T(0);
-#pragma unroll
-      for (int m0 = 0; m0 < N1; ++m0) s += J[m0] * (cr ? tb.L1[m0] : tb.L0[m0]);
-      put(cr, s, true);
-    }
-  } else {
-    T Pq[NQ][N1];
-#pragma unroll
-    for (int q0 = 0; q0 < NQ; ++q0)
-#pragma unroll
-      for (int m1 = 0; m1 < N1; ++m1) {
-        T s = T(0);
-#pragma unroll
-        for (int m0 = 0; m0 < N1; ++m0) s += J[m0 + N1 * m1] * tb.Lq[m0][q0];
-        Pq[q0][m1] = s;
-      }
-#pragma unroll
-    for (int q1 = 0; q1 < NQ; ++q1)
-#pragma unroll
-      for (int q0 = 0; q0 < NQ; ++q0) {
-        T s = T(0);
-#pragma unroll
-        for (int m1 = 0; m1 < N1; ++m1) s += Pq[q0][m1] * tb.Lq[m1][q1];
-        put(q0 + NQ * q1, s, false);
-      }
-#pragma unroll
-    for (int cr = 0; cr < 4; ++cr) {
-      T s = T(0);
-#pragma unroll
-      for (int mf = 0; mf < NF; ++mf) {
-        const int m0 = mf % N1, m1 = mf / N1;
-        s += J[mf] * ((cr & 1) ? tb.L1[m0] : tb.L0[m0]) * ((cr & 2) ? tb.L1[m1] : tb.L0[m1]);
-      }
-      put(cr, s, true);
-    }
+    T c0, c1, c2, c3;
+    end_values<N1, 1, T>(tb, Pl, c0, c2);
+    end_values<N1, 1, T>(tb, Ph, c1, c3);
+    put(0, c0, true);
+    put(1, c1, true);
+    put(2, c2, true);
+    put(3, c3, true);
   }
 }
 
 // values and gradients (reference-cell derivatives) of the modal field c
 // at the two vertices (vx = 0, 1) of the x-line with corner bits (vy, vz):
-// the y/z reductions are shared by both ends of the line
+// the y/z reductions are shared by both ends of the line.  The odd modes
+// change sign between the two ends of an axis, L_0 = 1, D_0 = 0.
 template <int DIM, int N1, typename T>
 __device__ __forceinline__ void hjs_line(const T* c, const Tab1D<T>& tb, int vy, int vz, T* val, T (*gr)[3]) {
-  T Y[N1], Yd[N1];
+  T Y[N1], Yd[N1], Z[N1], Zd[N1];
 #pragma unroll
-  for (int b = 0; b < N1; ++b) {
+  for (int b = 1; b < N1; ++b) {
     Y[b] = vy ? tb.L1[b] : tb.L0[b];
     Yd[b] = vy ? tb.D1[b] : tb.D0[b];
+    Z[b] = vz ? tb.L1[b] : tb.L0[b];
+    Zd[b] = vz ? tb.D1[b] : tb.D0[b];
   }
   T V[N1], Vy[N1], Vz[N1];
-  if constexpr (DIM == 2) {
 #pragma unroll
-    for (int a = 0; a < N1; ++a) {
-      T s0 = T(0), s1 = T(0);
-#pragma unroll
-      for (int b = 0; b < N1; ++b) {
-        s0 += c[a + N1 * b] * Y[b];
-        s1 += c[a + N1 * b] * Yd[b];
-      }
-      V[a] = s0;
-      Vy[a] = s1;
-      Vz[a] = T(0);
-    }
-  } else {
-    T Z[N1], Zd[N1];
+  for (int a = 0; a < N1; ++a) {
+    T W[N1], Wd[N1];
 #pragma unroll
     for (int b = 0; b < N1; ++b) {
-      Z[b] = vz ? tb.L1[b] : tb.L0[b];
-      Zd[b] = vz ? tb.D1[b] : tb.D0[b];
-    }
+      W[b] = c[a + N1 * b];
+      Wd[b] = T(0);
+      if constexpr (DIM > 2) {
 #pragma unroll
-    for (int a = 0; a < N1; ++a) {
-      T W[N1], Wd[N1];
-#pragma unroll
-      for (int b = 0; b < N1; ++b) {
-        T s0 = T(0), s1 = T(0);
-#pragma unroll
-        for (int cc = 0; cc < N1; ++cc) {
-          s0 += c[a + N1 * (b + N1 * cc)] * Z[cc];
-          s1 += c[a + N1 * (b + N1 * cc)] * Zd[cc];
+        for (int cc = 1; cc < N1; ++cc) {
+          W[b] += c[a + N1 * (b + N1 * cc)] * Z[cc];
+          Wd[b] += c[a + N1 * (b + N1 * cc)] * Zd[cc];
         }
-        W[b] = s0;
-        Wd[b] = s1;
       }
-      T s0 = T(0), s1 = T(0), s2 = T(0);
-#pragma unroll
-      for (int b = 0; b < N1; ++b) {
-        s0 += W[b] * Y[b];
-        s1 += W[b] * Yd[b];
-        s2 += Wd[b] * Y[b];
-      }
-      V[a] = s0;
-      Vy[a] = s1;
-      Vz[a] = s2;
     }
-  }
+    T s0 = W[0], s1 = T(0), s2 = Wd[0];
 #pragma unroll
-  for (int vx = 0; vx < 2; ++vx) {
-    const T* X = vx ? tb.L1 : tb.L0;
-    const T* Xd = vx ? tb.D1 : tb.D0;
-    T v = T(0), gx = T(0), gy = T(0), gz = T(0);
-#pragma unroll
-    for (int a = 0; a < N1; ++a) {
-      v += V[a] * X[a];
-      gx += V[a] * Xd[a];
-      gy += Vy[a] * X[a];
-      gz += Vz[a] * X[a];
+    for (int b = 1; b < N1; ++b) {
+      s0 += W[b] * Y[b];
+      s1 += W[b] * Yd[b];
+      if constexpr (DIM > 2) s2 += Wd[b] * Y[b];
     }
-    val[vx] = v;
-    gr[vx][0] = gx;
-    gr[vx][1] = gy;
-    gr[vx][2] = gz;
+    V[a] = s0;
+    Vy[a] = s1;
+    Vz[a] = s2;
   }
+  end_values<N1, 1, T>(tb, V, val[0], val[1]);
+  end_values<N1, 1, T>(tb, Vy, gr[0][1], gr[1][1]);
+  if constexpr (DIM > 2) end_values<N1, 1, T>(tb, Vz, gr[0][2], gr[1][2]);
+  T ge = V[1] * tb.D1[1], go = T(0);   // L_a' is even for odd a
+  if constexpr (N1 > 3) ge += V[3] * tb.D1[3];
+  if constexpr (N1 > 2) go = V[2] * tb.D1[2];
+  gr[0][0] = ge - go;
+  gr[1][0] = ge + go;
+}
+
+// the characteristic speed at a vertex (ReinitOperator::
+// characteristic_velocity, reinit.cc:235-264) from the upwind parts of the
+// one-sided gradients: their unit vector times S, i.e. |S| unless every
+// part vanishes (then the vanishing norm itself).  A norm that overflows
+// or is NaN gives NaN, which the maxima ignore.
+template <int DIM, typename T>
+__device__ __forceinline__ T hjs_speed(T S, const T* left, const T* right) {
+  T n2 = T(0);
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    const T l = S >= T(0) ? left[d] : -left[d], r = S >= T(0) ? -right[d] : right[d];
+    const T g = fmax(fmax(l, T(0)), fmax(r, T(0)));
+    n2 += g * g;
+  }
+  constexpr T eps2 = T(2.220446049250313e-16) * T(2.220446049250313e-16);
+  return n2 > eps2 ? fabs(S) + (n2 - n2) : sqrt(n2);
 }
 
 // One block serves one HjsTile of cells (launch slot blockIdx.x) with NQ
@@ -294,7 +276,7 @@ __device__ __forceinline__ void hjs_line(const T* c, const Tab1D<T>& tb, int vy,
 // table, CFL estimate of the first pseudo-step) and kHJStep (one pseudo-
 // step from the table, CFL estimate of the next).
 template <int DIM, int P, typename T>
-__global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2)) hjs_kernel(const HJArgs<T> a) {
+__global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjs_min_blocks<DIM, P, T>()) hjs_kernel(const HJArgs<T> a) {
   using PL = HjsPlan<DIM, P, T>;
   constexpr int N1 = P + 1, NQ = P + 2, NM = ipow(N1, DIM), NV = 1 << DIM;
   constexpr int NQF = ipow(NQ, DIM - 1), NC = 1 << (DIM - 1);
@@ -302,14 +284,15 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2)) hjs_kernel(const HJ
   using TL = HjsTile<DIM>;
   constexpr int TX = TL::X, TY = TL::Y, TZ = TL::Z, NT = TL::N, NMB = PL::NMB;
   static_assert(NM <= 2 * DIM * NQF, "the store staging reuses the face-jump area");
+  static_assert(NU <= NQF, "a plane's projection fits its table entries");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem_raw);
   unsigned char* boxb = smem_raw + PL::OFF_BOX;
   T* jn = reinterpret_cast<T*>(smem_raw + PL::OFF_JN);   // [2*DIM*NQF][NT]
   T* jv = reinterpret_cast<T*>(smem_raw + PL::OFF_JV);   // [2*DIM*NC][NT]
-  T* ub = reinterpret_cast<T*>(smem_raw + PL::OFF_UB);   // [NQ][NU][NT], after the table slice
-  T* stl = ub;                                            // table slice [NS][NT] (pseudo-steps)
-  double* red = reinterpret_cast<double*>(smem_raw + PL::OFF_RED);
+  MaxSlot<T>* cfl = reinterpret_cast<MaxSlot<T>*>(smem_raw + 16);
+  T* stl = reinterpret_cast<T*>(smem_raw + PL::OFF_UB);   // table slice [NS][NT] (pseudo-steps)
+  T* ub = stl;                                            // plane projections [NQ][NQF][NT] (u < NU used)
   const MeshArgs& m = a.m;
   const Tab1D<T>& tb = tab<T>(P);
   const int slot = (int)blockIdx.x;
@@ -323,44 +306,6 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2)) hjs_kernel(const HJ
     o[2] = DIM > 2 ? (b / m.ntile[1]) * TZ : 0;
   };
   const bool step = a.mode == kHJStep;
-  // halo box of the tile in launch slot `slot`: rows (ly, lz) of cells
-  // [max(ox - 1, 0), min(ox + TX + 1, n)) by bulk copies (warp 0); for a
-  // pseudo-step also the tile's slice of the sign table (one copy)
-  auto issue = [&](int slot) {
-    int so[3];
-    origin(slot, so);
-    const int hx0 = max(so[0] - 1, 0), hx1 = min(so[0] + TX + 1, m.n[0]);
-    const int lane = threadIdx.x;
-    const char* gsrc = reinterpret_cast<const char*>(a.phi);
-    unsigned bytes = 0;
-    // pass 0 counts the bytes, pass 1 issues the copies
-    for (int pass = 0; pass < 2; ++pass) {
-      if (pass == 1) {
-#pragma unroll
-        for (int w = 16; w > 0; w >>= 1) bytes += __shfl_xor_sync(0xffffffffu, bytes, w);
-        if (lane == 0) mbar_arrive_expect_tx(bar, bytes);
-        __syncwarp();
-      }
-      for (int rr = lane; rr < PL::NROWS; rr += 32) {
-        const int ly = rr % PL::BY - 1, lz = DIM > 2 ? rr / PL::BY - 1 : 0;
-        const bool yout = ly < 0 || ly >= TY, zout = DIM > 2 && (lz < 0 || lz >= TZ);
-        if (yout && zout) continue;
-        const int gy = so[1] + ly, gz = so[2] + lz;
-        if (gy < 0 || gy >= m.n[1] || (DIM > 2 && (gz < 0 || gz >= m.n[2]))) continue;
-        const long long rowcell = (long long)m.n[0] * (gy + (long long)m.n[1] * (DIM > 2 ? gz : 0));
-        const long long s0 = (rowcell + hx0) * NMB, s1 = (rowcell + hx1) * NMB;
-        const long long a0 = s0 & ~15LL, a1 = (s1 + 15) & ~15LL;
-        if (pass == 0) bytes += (unsigned)(a1 - a0);
-        else bulk_g2s(boxb + (size_t)rr * PL::SLOT, gsrc + a0, (unsigned)(a1 - a0), bar);
-      }
-      if (step && lane == 0) {
-        const int tl = m.tiles ? m.tiles[slot] : slot;
-        if (pass == 0) bytes += (unsigned)PL::TAB_BYTES;
-        else bulk_g2s(stl, a.stab + (size_t)tl * NS * NT, (unsigned)PL::TAB_BYTES, bar);
-      }
-    }
-  };
-
   const int cl = (int)threadIdx.x % NT, k = (int)threadIdx.x / NT;   // cell, Gauss plane
   const int l[3] = {cl % TX, (cl / TX) % TY, DIM > 2 ? cl / (TX * TY) : 0};
   const T ih[3] = {T(1.0 / m.h[0]), T(1.0 / m.h[1]), T(DIM > 2 ? 1.0 / m.h[2] : 1.0)};
@@ -372,17 +317,26 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2)) hjs_kernel(const HJ
   for (int b = 0; b < N1; ++b) {
     Lk[b] = tb.Lq[b][k];
     Dk[b] = tb.Dq[b][k];
+    if (step) Dk[b] *= ih[DIM - 1];   // the pseudo-steps' plane derivative, per unit length
   }
   const T dt = a.clk ? T(a.clk->hj_dt) : T(a.dt_explicit);
-  double vmax = 0.0;
-
-  if (threadIdx.x == 0) mbar_init(bar, 1);
-  __syncthreads();
-  if (threadIdx.x < 32) issue(slot);
+  T vmax = T(0);
 
   int o[3];
   origin(slot, o);
   const int tile = m.tiles ? m.tiles[slot] : slot;
+  // the tile's slice of the sign table by one bulk copy, the halo box by
+  // 16-byte copies of every warp
+  if (threadIdx.x == 0) {
+    mbar_init(bar, 1);
+    *cfl = 0;
+    if (step) {
+      mbar_arrive_expect_tx(bar, (unsigned)PL::TAB_BYTES);
+      bulk_g2s(stl, a.stab + (size_t)tile * NS * NT, (unsigned)PL::TAB_BYTES, bar);
+    }
+  }
+  load_box_rows<DIM, TX, TY, TZ, NMB, PL::SLOT>(m, a.phi, boxb, o[0], o[1], o[2], (int)threadIdx.x >> 5,
+                                                NT * NQ / 32);
   const int g[3] = {o[0] + l[0], o[1] + l[1], o[2] + l[2]};
   const bool valid = g[0] < m.n[0] && g[1] < m.n[1] && (DIM < 3 || g[2] < m.n[2]);
   const int gx0 = max(o[0] - 1, 0);
@@ -393,19 +347,27 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2)) hjs_kernel(const HJ
     const unsigned phase = ((rowcell + (unsigned)gx0) * (unsigned)NMB) & 15u;
     return reinterpret_cast<const T*>(boxb + (size_t)rr * PL::SLOT + phase + (o[0] + lx - gx0) * NMB);
   };
-  if (!mbar_wait(bar, 0u, 1 << 22)) {
-    if (threadIdx.x == 0 && a.err) atomicOr(a.err, kErrCopyTimeout);
-  }
+  cp_async_wait_all();
+  __syncthreads();
 
   // -------- face jumps, one work item per face of the tile
   {
     constexpr int C0 = (TX + 1) * (NT / TX), C1 = (TY + 1) * (NT / TY);
     constexpr int C2 = DIM > 2 ? (TZ + 1) * (NT / TZ) : 0;
-    for (int i = threadIdx.x; i < C0 + C1 + C2; i += NT * NQ) {
-      if (i < C0) hjs_face<DIM, P, 0, T>(m, cellp, jn, jv, o, i);
-      else if (i < C0 + C1) hjs_face<DIM, P, 1, T>(m, cellp, jn, jv, o, i - C0);
-      else if constexpr (DIM > 2) hjs_face<DIM, P, 2, T>(m, cellp, jn, jv, o, i - C0 - C1);
+    // each axis' items start on a warp boundary: no warp runs two axes' code
+    constexpr int W0 = (C0 + 31) / 32 * 32, W1 = W0 + (C1 + 31) / 32 * 32;
+    for (int i = threadIdx.x; i < W1 + C2; i += NT * NQ) {
+      if (i < W0) {
+        if (i < C0) hjs_face<DIM, P, 0, T>(m, cellp, jn, jv, o, i);
+      } else if (i < W1) {
+        if (i < W0 + C1) hjs_face<DIM, P, 1, T>(m, cellp, jn, jv, o, i - W0);
+      } else if constexpr (DIM > 2) {
+        hjs_face<DIM, P, 2, T>(m, cellp, jn, jv, o, i - W1);
+      }
     }
+  }
+  if (step && !mbar_wait(bar, 0u, 1 << 22)) {
+    if (threadIdx.x == 0 && a.err) atomicOr(a.err, kErrCopyTimeout);
   }
   __syncthreads();
 
@@ -525,45 +487,24 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2)) hjs_kernel(const HJ
       } else {
         S = stl[(size_t)(NQV + v) * NT + cl];
       }
-      T gs[DIM];
+      T lft[DIM], rgt[DIM];
 #pragma unroll
       for (int d = 0; d < DIM; ++d) {
         const int t0 = d == 0 ? 1 : 0, t1 = d == 2 ? 1 : 2;
         const int cr = vb[t0] + (DIM > 2 ? 2 * vb[t1] : 0);
         const T gd = dphi[d] * ih[d];
-        const T L = gd + tb.K0v[vb[d]] * jv[(size_t)(2 * d * NC + cr) * NT + cl];
-        const T Rr = gd + tb.K1v[vb[d]] * jv[(size_t)((2 * d + 1) * NC + cr) * NT + cl];
-        if (S >= T(0)) {
-          const T lp = max(L, T(0)), rm = -min(Rr, T(0));
-          gs[d] = fabs(lp) > fabs(rm) ? lp : rm;
-        } else {
-          const T lm = -min(L, T(0)), rp = max(Rr, T(0));
-          gs[d] = fabs(lm) > fabs(rp) ? lm : rp;
-        }
+        lft[d] = gd + tb.K0v[vb[d]] * jv[(size_t)(2 * d * NC + cr) * NT + cl];
+        rgt[d] = gd + tb.K1v[vb[d]] * jv[(size_t)((2 * d + 1) * NC + cr) * NT + cl];
       }
-      T n2 = T(0);
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) n2 += gs[d] * gs[d];
-      const T nrm = sqrt(n2);
-      if (!(fabs((double)nrm) <= 2.220446049250313e-16)) {
-        const T inv = T(1) / nrm;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) gs[d] *= inv;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) gs[d] *= S;
-      }
-      T s2 = T(0);
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) s2 += gs[d] * gs[d];
-      vmax = fmax(vmax, (double)sqrt(s2));
+      vmax = fmax(vmax, hjs_speed<DIM, T>(S, lft, rgt));
       }
     }
     if (!fill) {
 #pragma unroll
       for (int u = 0; u < NU; ++u) {
-        T s1 = T(0), s2 = T(0);
+        T s1 = cr[u], s2 = T(0);
 #pragma unroll
-        for (int cc = 0; cc < N1; ++cc) {
+        for (int cc = 1; cc < N1; ++cc) {
           const T cv = cr[u + NU * cc];
           s1 += cv * Lk[cc];
           s2 += cv * Dk[cc];
@@ -573,130 +514,154 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2)) hjs_kernel(const HJ
       }
     }
   }
-  vmax = vmax / m.diam;
-  const double bm = block_max(vmax, red);
-  if (threadIdx.x == 0 && a.clk) atomic_max_pos(&a.clk->hj_vd_bits, bm);
-  if (a.mode != kHJStep) return;
+  slot_max(cfl, vmax);
+  if (!step) {
+    __syncthreads();
+    if (threadIdx.x == 0 && a.clk) atomic_max_pos(&a.clk->hj_vd_bits, slot_value(cfl) / m.diam);
+    return;
+  }
 
   // -------- pseudo-step: H at this plane's Gauss points, projected onto
-  // the modes of the other axes
+  // the modes of the other axes.  With the half jumps p = K0 jl / 2 and
+  // q = K1 jh / 2 of an axis the one-sided gradients are g + 2 p and
+  // g + 2 q: their mean is g + p + q, half their difference p - q.
   auto jnv = [&](int d, int side, int qf) -> T { return jn[(size_t)((2 * d + side) * NQF + qf) * NT + cl]; };
-  auto hfun = [&](T S, const T* lft, const T* rgt) -> T {
+  auto hfun = [&](T S, const T* avg, T dif) -> T {
     T avg2 = T(0);
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) { const T av = T(0.5) * (lft[d] + rgt[d]); avg2 += av * av; }
+    for (int d = 0; d < DIM; ++d) avg2 += avg[d] * avg[d];
     T nrm;
-    if constexpr (sizeof(T) == 4) nrm = avg2 * rsqrtf(fmaxf(avg2, 1e-30f));
+    if constexpr (sizeof(T) == 4) nrm = avg2 * rsqrt_normal(fmaxf(avg2, 1e-30f));
     else nrm = sqrt(avg2);
-    T H = S * (nrm - T(1));
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) H += T(0.5) * fabs(S) * (lft[d] - rgt[d]);
-    return H;
+    return S * (nrm - T(1)) + fabs(S) * dif;
   };
-  T Sq[NQF];
   if (valid) {
-#pragma unroll
-    for (int j = 0; j < NQF; ++j) Sq[j] = stl[(size_t)(k * NQF + j) * NT + cl];
-  }
-  __syncthreads();   // the table slice is consumed: its region takes the plane projections
-  if (valid) {
-    const T K0k = tb.K0q[k], K1k = tb.K1q[k];
+    const T hK0k = T(0.5) * tb.K0q[k], hK1k = T(0.5) * tb.K1q[k];
+    // PL1 already carries 1/h of the plane's axis (Dk)
     if constexpr (DIM == 2) {
       const int qy = k;
-      const T* Py = PL0;
-      const T* Pdy = PL1;
-      const T jlx = jnv(0, 0, qy), jhx = jnv(0, 1, qy);
-      T X[N1];
+      const T jlx = T(0.5) * jnv(0, 0, qy), jhx = T(0.5) * jnv(0, 1, qy);
+      T gx[NQ], gy[NQ], f[NQ], X[N1];
 #pragma unroll
-      for (int aa = 0; aa < N1; ++aa) X[aa] = T(0);
+      for (int aa = 1; aa < N1; ++aa) PL0[aa] *= ih[0];
+      gauss_derivatives<N1, NQ, 1, T>(tb, PL0, gx);
+      gauss_values<N1, NQ, 1, T>(tb, PL1, gy);
 #pragma unroll
       for (int qx = 0; qx < NQ; ++qx) {
-        T gx = T(0), gy = T(0);
-#pragma unroll
-        for (int aa = 0; aa < N1; ++aa) {
-          gx += Py[aa] * tb.Dq[aa][qx];
-          gy += Pdy[aa] * tb.Lq[aa][qx];
-        }
-        gx *= ih[0];
-        gy *= ih[1];
         const T jly = jnv(1, 0, qx), jhy = jnv(1, 1, qx);
-        const T lft[2] = {gx + tb.K0q[qx] * jlx, gy + K0k * jly};
-        const T rgt[2] = {gx + tb.K1q[qx] * jhx, gy + K1k * jhy};
-        const T wH = hfun(Sq[qx], lft, rgt);   // weighted sign: w_q H
-#pragma unroll
-        for (int aa = 0; aa < N1; ++aa) X[aa] += wH * tb.Lq[aa][qx];
+        const T avg[2] = {gx[qx] + tb.K0q[qx] * jlx + tb.K1q[qx] * jhx, gy[qx] + hK0k * jly + hK1k * jhy};
+        T dif = tb.K0q[qx] * jlx;
+        dif += hK0k * jly;
+        dif -= tb.K1q[qx] * jhx;
+        dif -= hK1k * jhy;
+        f[qx] = hfun(stl[(size_t)(k * NQF + qx) * NT + cl], avg, dif);   // w_q H
       }
 #pragma unroll
-      for (int aa = 0; aa < N1; ++aa) ub[(size_t)(k * NU + aa) * NT + cl] = X[aa];
+      for (int aa = 0; aa < N1; ++aa) X[aa] = T(0);
+      gauss_project<N1, NQ, 1, T>(tb, f, X);
+#pragma unroll
+      for (int aa = 0; aa < N1; ++aa) ub[(size_t)(k * NQF + aa) * NT + cl] = X[aa];
     } else {
+      T PLy[N1][N1];   // [aa][b >= 1], for the y derivative
+#pragma unroll
+      for (int aa = 0; aa < N1; ++aa)
+#pragma unroll
+        for (int b = 1; b < N1; ++b) PLy[aa][b] = PL0[aa + N1 * b] * ih[1];
+#pragma unroll
+      for (int aa = 1; aa < N1; ++aa)
+#pragma unroll
+        for (int b = 0; b < N1; ++b) PL0[aa + N1 * b] *= ih[0];
+      T jly[NQ], jhy[NQ];
+#pragma unroll
+      for (int qx = 0; qx < NQ; ++qx) {
+        jly[qx] = T(0.5) * jnv(1, 0, qx + NQ * k);
+        jhy[qx] = T(0.5) * jnv(1, 1, qx + NQ * k);
+      }
       T U[N1][N1];
 #pragma unroll
       for (int aa = 0; aa < N1; ++aa)
 #pragma unroll
         for (int b = 0; b < N1; ++b) U[aa][b] = T(0);
-#pragma unroll
-      for (int qy = 0; qy < NQ; ++qy) {
-        T Py[N1], Pdy[N1], Dzy[N1];
-#pragma unroll
-        for (int aa = 0; aa < N1; ++aa) {
-          T s1 = T(0), s2 = T(0), s3 = T(0);
-#pragma unroll
-          for (int b = 0; b < N1; ++b) {
-            s1 += PL0[aa + N1 * b] * tb.Lq[b][qy];
-            s2 += PL0[aa + N1 * b] * tb.Dq[b][qy];
-            s3 += PL1[aa + N1 * b] * tb.Lq[b][qy];
-          }
-          Py[aa] = s1 * ih[0];
-          Pdy[aa] = s2 * ih[1];
-          Dzy[aa] = s3 * ih[2];
-        }
-        const T jlx = jnv(0, 0, qy + NQ * k), jhx = jnv(0, 1, qy + NQ * k);
-        T X[N1];
-#pragma unroll
-        for (int aa = 0; aa < N1; ++aa) X[aa] = T(0);
+      auto line = [&](int qy, const T* Py, const T* Pdy, const T* Dzy) {
+        T gx[NQ], gy[NQ], gz[NQ], f[NQ], X[N1];
+        gauss_derivatives<N1, NQ, 1, T>(tb, Py, gx);
+        gauss_values<N1, NQ, 1, T>(tb, Pdy, gy);
+        gauss_values<N1, NQ, 1, T>(tb, Dzy, gz);
+        const T jlx = T(0.5) * jnv(0, 0, qy + NQ * k), jhx = T(0.5) * jnv(0, 1, qy + NQ * k);
 #pragma unroll
         for (int qx = 0; qx < NQ; ++qx) {
-          T gx = T(0), gy = T(0), gz = T(0);
-#pragma unroll
-          for (int aa = 0; aa < N1; ++aa) {
-            gx += Py[aa] * tb.Dq[aa][qx];
-            gy += Pdy[aa] * tb.Lq[aa][qx];
-            gz += Dzy[aa] * tb.Lq[aa][qx];
-          }
-          const T jly = jnv(1, 0, qx + NQ * k), jhy = jnv(1, 1, qx + NQ * k);
           const T jlz = jnv(2, 0, qx + NQ * qy), jhz = jnv(2, 1, qx + NQ * qy);
-          const T lft[3] = {gx + tb.K0q[qx] * jlx, gy + tb.K0q[qy] * jly, gz + K0k * jlz};
-          const T rgt[3] = {gx + tb.K1q[qx] * jhx, gy + tb.K1q[qy] * jhy, gz + K1k * jhz};
-          const T wH = hfun(Sq[qx + NQ * qy], lft, rgt);   // weighted sign: w_q H
-#pragma unroll
-          for (int aa = 0; aa < N1; ++aa) X[aa] += wH * tb.Lq[aa][qx];
+          const T avg[3] = {gx[qx] + tb.K0q[qx] * jlx + tb.K1q[qx] * jhx,
+                            gy[qx] + tb.K0q[qy] * jly[qx] + tb.K1q[qy] * jhy[qx], gz[qx] + hK0k * jlz + hK1k * jhz};
+          T dif = tb.K0q[qx] * jlx;
+          dif += tb.K0q[qy] * jly[qx];
+          dif += hK0k * jlz;
+          dif -= tb.K1q[qx] * jhx;
+          dif -= tb.K1q[qy] * jhy[qx];
+          dif -= hK1k * jhz;
+          f[qx] = hfun(stl[(size_t)(k * NQF + qx + NQ * qy) * NT + cl], avg, dif);   // w_q H
         }
 #pragma unroll
-        for (int b = 0; b < N1; ++b)
+        for (int aa = 0; aa < N1; ++aa) X[aa] = T(0);
+        gauss_project<N1, NQ, 1, T>(tb, f, X);
 #pragma unroll
-          for (int aa = 0; aa < N1; ++aa) U[aa][b] += X[aa] * tb.Lq[b][qy];
+        for (int aa = 0; aa < N1; ++aa) {
+          U[aa][0] += X[aa];
+#pragma unroll
+          for (int b = 1; b < N1; ++b) U[aa][b] += X[aa] * tb.Lq[b][qy];
+        }
+      };
+      T Py[N1][NQ], Pdy[N1][NQ], Dzy[N1][NQ];
+#pragma unroll
+      for (int aa = 0; aa < N1; ++aa) {
+        if (aa > 0) gauss_values<N1, NQ, N1, T>(tb, PL0 + aa, Py[aa]);
+        gauss_derivatives<N1, NQ, 1, T>(tb, PLy[aa], Pdy[aa]);
+        gauss_values<N1, NQ, N1, T>(tb, PL1 + aa, Dzy[aa]);
+      }
+#pragma unroll
+      for (int qy = 0; qy < NQ; ++qy) {
+        T py[N1], pdy[N1], dzy[N1];
+#pragma unroll
+        for (int aa = 0; aa < N1; ++aa) {
+          py[aa] = aa > 0 ? Py[aa][qy] : T(0);
+          pdy[aa] = Pdy[aa][qy];
+          dzy[aa] = Dzy[aa][qy];
+        }
+        line(qy, py, pdy, dzy);
       }
 #pragma unroll
       for (int b = 0; b < N1; ++b)
 #pragma unroll
-        for (int aa = 0; aa < N1; ++aa) ub[(size_t)(k * NU + aa + N1 * b) * NT + cl] = U[aa][b];
+        for (int aa = 0; aa < N1; ++aa) ub[(size_t)(k * NQF + aa + N1 * b) * NT + cl] = U[aa][b];
     }
   }
   __syncthreads();   // planes done: the face-jump area becomes the store staging
+  if (threadIdx.x == 0 && a.clk) atomic_max_pos(&a.clk->hj_vd_bits, slot_value(cfl) / m.diam);
 
-  // -------- modes q = k, k + NQ, ...: sum over the planes, update, stage
+  // -------- columns u = k, k + NQ, ... of modes: project over the planes,
+  // update, stage
   {
   T* sb = jn;   // [NT][NM]
   if (valid) {
     const long long cell = (long long)g[0] + (long long)m.n[0] * (g[1] + (long long)m.n[1] * g[2]);
-#pragma unroll 1
-    for (int q = k; q < NM; q += NQ) {
-      const int u = q % NU, cz = q / NU;   // (aa, b) of the plane projection, last-axis mode
-      T R = T(0);
 #pragma unroll
-      for (int kk = 0; kk < NQ; ++kk) R -= ub[(size_t)(kk * NU + u) * NT + cl] * tb.Lq[cz][kk];
-      if (a.rdiff) R += a.rdiff[cell * m.nb + m.q2g[q]];
-      sb[(size_t)cl * NM + q] = hj_combine<T>(a.rk, c[q], R, dt);
+    for (int u0 = 0; u0 < NU; u0 += NQ) {
+      const int u = u0 + k;
+      if (u < NU) {
+        T f[NQ], R[N1];
+#pragma unroll
+        for (int kk = 0; kk < NQ; ++kk) f[kk] = ub[(size_t)(kk * NQF + u) * NT + cl];
+#pragma unroll
+        for (int cz = 0; cz < N1; ++cz) R[cz] = T(0);
+        gauss_project<N1, NQ, 1, T>(tb, f, R);
+#pragma unroll
+        for (int cz = 0; cz < N1; ++cz) {
+          const int q = u + NU * cz;
+          T r = -R[cz];
+          if (a.rdiff) r += a.rdiff[cell * NM + q];
+          sb[(size_t)cl * NM + q] = hj_combine<T>(a.rk, c[q], r, dt);
+        }
+      }
     }
   }
   __syncthreads();
