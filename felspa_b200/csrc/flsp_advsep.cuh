@@ -69,21 +69,6 @@ struct AdvSepArgs {
   double dt_explicit;
 };
 
-// In-cell DoF index (HBM order) of Q-layout mode q for FE_DGP
-// (PolynomialSpace order: c outer, b, a inner with a + b + c <= P), -1 for a
-// mode outside P-space
-template <int DIM, int P>
-__host__ __device__ constexpr int q2g_ct(int q) {
-  const int N1 = P + 1;
-  const int a = q % N1, b = (q / N1) % N1, c = DIM > 2 ? q / (N1 * N1) : 0;
-  if (a + b + c > P) return -1;
-  int idx = 0;
-  for (int cc = 0; cc < c; ++cc)
-    for (int bb = 0; bb <= P - cc; ++bb) idx += P - bb - cc + 1;
-  for (int bb = 0; bb < b; ++bb) idx += P - bb - c + 1;
-  return idx + a;
-}
-
 // Shared-memory plan of the separable stage kernel for a compile-time tile
 // TX x TY x TZ (TZ = 1 in 2D): mbarrier | halo box rows | operator rows |
 // face fluxes (reused for the tile's R).  Box rows: (TY+2)(TZ+2) slots of

@@ -302,16 +302,14 @@ int prepare_kernels(flsp_handle* h) {
   ST(adv_prepare(c, h->veldev(), h->adv_tile));
   ST(hj_default_tile(c, h->hj_tile));
   ST(hj_prepare(c, h->hj_tile));
-  if (h->basis == FLSP_BASIS_Q) {
-    size_t bytes = 0;
-    ST(hj_table_bytes(c, h->hj_tile, &bytes));
-    if (bytes != h->hj_stab_bytes) {
-      if (h->hj_stab) cudaFree(h->hj_stab);
-      h->hj_stab = nullptr;
-      h->hj_stab_bytes = 0;
-      CU(cudaMalloc(&h->hj_stab, bytes));
-      h->hj_stab_bytes = bytes;
-    }
+  size_t bytes = 0;
+  ST(hj_table_bytes(c, h->hj_tile, &bytes));
+  if (bytes != h->hj_stab_bytes) {
+    if (h->hj_stab) cudaFree(h->hj_stab);
+    h->hj_stab = nullptr;
+    h->hj_stab_bytes = 0;
+    CU(cudaMalloc(&h->hj_stab, bytes));
+    h->hj_stab_bytes = bytes;
   }
   ST(ldg_prepare(c));
   if (h->dim == 2) ST(weno_prepare(c));

@@ -24,6 +24,21 @@ constexpr int kMaxFeVel = 3;        // largest degree of an FE velocity field
 
 __host__ __device__ constexpr int ipow(int b, int e) { return e == 0 ? 1 : b * ipow(b, e - 1); }
 
+// In-cell DoF index (HBM order) of Q-layout mode q for FE_DGP
+// (PolynomialSpace order: c outer, b, a inner with a + b + c <= P), -1 for a
+// mode outside P-space
+template <int DIM, int P>
+__host__ __device__ constexpr int q2g_ct(int q) {
+  const int N1 = P + 1;
+  const int a = q % N1, b = (q / N1) % N1, c = DIM > 2 ? q / (N1 * N1) : 0;
+  if (a + b + c > P) return -1;
+  int idx = 0;
+  for (int cc = 0; cc < c; ++cc)
+    for (int bb = 0; bb <= P - cc; ++bb) idx += P - bb - cc + 1;
+  for (int bb = 0; bb < b; ++bb) idx += P - bb - c + 1;
+  return idx + a;
+}
+
 // 1D tables for one polynomial degree p (entries beyond p unused)
 template <typename T>
 struct Tab1D {
@@ -401,6 +416,24 @@ __device__ __forceinline__ int box_cells(const MeshArgs& m, int dim) {
   return (m.tile[0] + 2) * (dim > 1 ? m.tile[1] + 2 : 1) * (dim > 2 ? m.tile[2] + 2 : 1);
 }
 
+// Store of a compile-time tile's cells from [cell][NE] smem to NE DoFs per
+// cell in HBM, one warp per row of cells.
+template <int DIM, int TX, int TY, int TZ, int NE, typename T>
+__device__ __forceinline__ void store_cells(const MeshArgs& m, const T* __restrict__ sm, T* __restrict__ g, int ox,
+                                            int oy, int oz) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int n = min(TX, m.n[0] - ox) * NE;
+  for (int r = warp; r < TY * TZ; r += nw) {
+    const int gy = oy + r % TY, gz = oz + r / TY;
+    if (gy >= m.n[1] || gz >= m.n[2]) continue;
+    T* dst = g + ((long long)m.n[0] * (gy + (long long)m.n[1] * gz) + ox) * NE;
+    const T* src = sm + (size_t)TX * r * NE;
+#pragma unroll
+    for (int e = lane; e < TX * NE; e += 32)
+      if (e < n) dst[e] = src[e];
+  }
+}
+
 // ---------------------------------------------------------------------
 // asynchronous global -> shared copies (cp.async, one element each): a
 // thread issues all of its copies before waiting, so the latency of every
@@ -583,6 +616,28 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
           smem_u32(dst)),
       "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
+}
+// The rows of load_box_rows by one bulk copy each, issued by the lanes of one
+// warp: 32 arrivals on the barrier, each announcing its lane's bytes.
+template <int DIM, int TX, int TY, int TZ, int NMB, int SLOT>
+__device__ __forceinline__ void bulk_box_rows(const MeshArgs& m, const void* g, unsigned char* box, int ox, int oy,
+                                              int oz, unsigned long long* bar) {
+  constexpr int BY = TY + 2, NROWS = BY * (DIM > 2 ? TZ + 2 : 1);
+  const char* src = reinterpret_cast<const char*>(g);
+  const int hx0 = max(ox - 1, 0), hx1 = min(ox + TX + 1, m.n[0]);
+  unsigned bytes = 0;
+  for (int rr = threadIdx.x & 31; rr < NROWS; rr += 32) {
+    const int ly = rr % BY - 1, lz = DIM > 2 ? rr / BY - 1 : 0;
+    const bool yout = ly < 0 || ly >= TY, zout = DIM > 2 && (lz < 0 || lz >= TZ);
+    if (yout && zout) continue;
+    const int gy = oy + ly, gz = oz + lz;
+    if (gy < 0 || gy >= m.n[1] || (DIM > 2 && (gz < 0 || gz >= m.n[2]))) continue;
+    const long long rowcell = (long long)m.n[0] * (gy + (long long)m.n[1] * (DIM > 2 ? gz : 0));
+    const long long a0 = ((rowcell + hx0) * NMB) & ~15LL, a1 = ((rowcell + hx1) * NMB + 15) & ~15LL;
+    bulk_g2s(box + (size_t)rr * SLOT, src + a0, (unsigned)(a1 - a0), bar);
+    bytes += (unsigned)(a1 - a0);
+  }
+  mbar_arrive_expect_tx(bar, bytes);
 }
 // Wait for phase `parity` of the barrier, at most max_iter polls (each
 // try_wait may itself suspend for a while); false when it ran out.

@@ -15,7 +15,16 @@
 //    last axis (z in 3D, y in 2D).  Its partial projection onto the modes
 //    goes through shared memory, and each thread finishes every NQ-th mode
 //    of the cell (the sums over planes keep their order);
-//  * the face jumps are formed once per face, not once per cell side.
+//  * the face jumps are formed once per face, not once per cell side;
+//  * the sums over modes and points go by parity (gauss_values and its
+//    neighbours), the Hamiltonian takes the mean and half the difference of
+//    the one-sided gradients, and the plane projections overwrite the sign
+//    table entries of the thread's own plane.
+// What bounds it: issue and latency (64^3 Q2 FP32: 68 M warp instructions,
+// 57 % issue active, 24 warps per SM; the loads, barriers and store alone take
+// 47 us).  64^3 Q2 FP32 135 -> 98 us, 128^3 996 -> 708, 45x37x50 Q2 FP64
+// 129 -> 101, 256^2 Q2 FP32 14.4 -> 10.3 against the kernel with plain sums
+// and a two-pass copy issue.
 //
 // Table layout: stab[(tile * NS + j) * nt + c], c the cell within the tile;
 // j < NQ^dim: the Gauss point qx + NQ (qy + NQ qz), holding w_q S (the
@@ -74,11 +83,6 @@ struct HjsPlan {
 template <int DIM, int P, typename T>
 constexpr int hjs_min_blocks() {
   return DIM == 3 && sizeof(T) == 4 ? (P == 1 ? 4 : 3) : 1;
-}
-
-template <int DIM, int P, typename T>
-__host__ __device__ inline size_t hjs_smem_bytes(const int*) {
-  return HjsPlan<DIM, P, T>::BYTES;
 }
 
 // smooth sign from phi0's value and (scaled) gradient at a point, with the
@@ -328,15 +332,17 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjs_min_blocks<DIM,
   // the tile's slice of the sign table by one bulk copy, the halo box by
   // 16-byte copies of every warp
   if (threadIdx.x == 0) {
-    mbar_init(bar, 1);
+    mbar_init(bar, 32 + (step ? 1 : 0));
     *cfl = 0;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
     if (step) {
       mbar_arrive_expect_tx(bar, (unsigned)PL::TAB_BYTES);
       bulk_g2s(stl, a.stab + (size_t)tile * NS * NT, (unsigned)PL::TAB_BYTES, bar);
     }
   }
-  load_box_rows<DIM, TX, TY, TZ, NMB, PL::SLOT>(m, a.phi, boxb, o[0], o[1], o[2], (int)threadIdx.x >> 5,
-                                                NT * NQ / 32);
+  if (threadIdx.x < 32) bulk_box_rows<DIM, TX, TY, TZ, NMB, PL::SLOT>(m, a.phi, boxb, o[0], o[1], o[2], bar);
   const int g[3] = {o[0] + l[0], o[1] + l[1], o[2] + l[2]};
   const bool valid = g[0] < m.n[0] && g[1] < m.n[1] && (DIM < 3 || g[2] < m.n[2]);
   const int gx0 = max(o[0] - 1, 0);
@@ -347,8 +353,9 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjs_min_blocks<DIM,
     const unsigned phase = ((rowcell + (unsigned)gx0) * (unsigned)NMB) & 15u;
     return reinterpret_cast<const T*>(boxb + (size_t)rr * PL::SLOT + phase + (o[0] + lx - gx0) * NMB);
   };
-  cp_async_wait_all();
-  __syncthreads();
+  if (!mbar_wait(bar, 0u, 1 << 22)) {
+    if (threadIdx.x == 0 && a.err) atomicOr(a.err, kErrCopyTimeout);
+  }
 
   // -------- face jumps, one work item per face of the tile
   {
@@ -365,9 +372,6 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjs_min_blocks<DIM,
         hjs_face<DIM, P, 2, T>(m, cellp, jn, jv, o, i - W1);
       }
     }
-  }
-  if (step && !mbar_wait(bar, 0u, 1 << 22)) {
-    if (threadIdx.x == 0 && a.err) atomicOr(a.err, kErrCopyTimeout);
   }
   __syncthreads();
 
@@ -665,7 +669,7 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjs_min_blocks<DIM,
     }
   }
   __syncthreads();
-  store_tile<DIM, NM>(m, sb, a.out, o[0], o[1], o[2]);
+  store_cells<DIM, TX, TY, TZ, NM, T>(m, sb, a.out, o[0], o[1], o[2]);
   }
 }
 

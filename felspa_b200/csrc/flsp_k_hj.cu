@@ -3,6 +3,7 @@
 #include <cstring>
 
 #include "flsp_hj.cuh"
+#include "flsp_hjp.cuh"
 #include "flsp_hjs.cuh"
 #include "flsp_ldg.cuh"
 #include "flsp_launch.h"
@@ -16,25 +17,20 @@ int upload_tables_hj() {
   return FLSP_OK;
 }
 
+// tile of the reinitialisation launches: the kernels' block of cells; in the
+// P basis several blocks together (the unit the narrow band lists: a sweep's
+// frozen margin, and with it its result, depends on it)
 int hj_default_tile(const Ctx& c, int* tile) {
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
     constexpr int DIM = decltype(D)::value, P = decltype(PP)::value;
     using T = decltype(tz);
-    static const int c2[][3] = {{16, 16, 1}, {16, 8, 1}, {8, 8, 1}, {8, 4, 1}};
-    static const int c3[][3] = {{8, 8, 4}, {8, 4, 4}, {4, 4, 4}, {4, 4, 2}};
-    if (c.basis == FLSP_BASIS_Q) {   // the tensor-product kernel's fixed tile
-      tile[0] = HjsTile<DIM>::X;
-      tile[1] = HjsTile<DIM>::Y;
-      tile[2] = HjsTile<DIM>::Z;
-      return FLSP_OK;
-    }
-    const int(*cand)[3] = DIM == 2 ? c2 : c3;
-    int i = 0;
-    for (; i < 3; ++i)
-      if (hj_smem_bytes<DIM, P, T>(cand[i]) <= 200 * 1024) break;
-    tile[0] = cand[i][0];
-    tile[1] = cand[i][1];
-    tile[2] = cand[i][2];
+    tile[0] = HjsTile<DIM>::X;
+    tile[1] = HjsTile<DIM>::Y;
+    tile[2] = HjsTile<DIM>::Z;
+    if (c.basis == FLSP_BASIS_Q) return FLSP_OK;
+    if (DIM == 2) tile[0] = tile[1] = 16;
+    else if (P == 1) tile[0] = tile[1] = 8;
+    else if (sizeof(T) == 4) tile[0] = 8;
     return FLSP_OK;
   });
 }
@@ -43,16 +39,21 @@ int hj_prepare(const Ctx& c, const int* tile) {
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
     constexpr int DIM = decltype(D)::value, P = decltype(PP)::value;
     using T = decltype(tz);
+    using TL = HjsTile<DIM>;
     const bool tq = c.basis == FLSP_BASIS_Q;
-    const size_t smem = tq ? hjs_smem_bytes<DIM, P, T>(tile) : hj_smem_bytes<DIM, P, T>(tile);
-    if (smem > 227 * 1024) return set_error(FLSP_ERR_BAD_ARG, "reinit tile too large for shared memory");
-    if (tq && (tile[0] != HjsTile<DIM>::X || tile[1] != HjsTile<DIM>::Y || (DIM > 2 && tile[2] != HjsTile<DIM>::Z)))
-      return set_error(FLSP_ERR_BAD_ARG, "the tensor-product reinit kernel has a fixed tile");
-    cudaError_t e = cudaFuncSetAttribute(tq ? hjs_kernel<DIM, P, T> : hj_kernel<DIM, P, T>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tq ? hjs_kernel<DIM, P, T> : hj_kernel<DIM, P, T>,
-                               cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    if (tile[0] % TL::X || tile[1] % TL::Y || (DIM > 2 && tile[2] % TL::Z) ||
+        (tq && (tile[0] != TL::X || tile[1] != TL::Y || (DIM > 2 && tile[2] != TL::Z))))
+      return set_error(FLSP_ERR_BAD_ARG, "the reinit kernels have a fixed tile");
+    constexpr size_t bytes[2] = {HjsPlan<DIM, P, T>::BYTES, HjpPlan<DIM, P, T>::BYTES};
+    static_assert(bytes[0] <= 227 * 1024 && bytes[1] <= 227 * 1024, "reinit tile too large for shared memory");
+    cudaError_t e = cudaSuccess;
+    auto attr = [&](auto k, size_t smem) {
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    };
+    if (tq) attr(hjs_kernel<DIM, P, T>, bytes[0]);
+    else attr(hjp_kernel<DIM, P, T>, bytes[1]);
+    attr(hj_gradient_kernel<DIM, P, T>, hjg_smem_bytes<DIM, P, T>());
     if (e != cudaSuccess) return set_error(FLSP_ERR_CUDA, std::string("hj attr: ") + cudaGetErrorString(e));
     return FLSP_OK;
   });
@@ -123,44 +124,34 @@ int launch_hj(const Ctx& c, const void* phi, const void* phi0, void* out, DevClo
     a.dt_explicit = dt_explicit;
     a.block = block;
     a.rdiff = reinterpret_cast<const T*>(rdiff);
-    // the gradient export mode uses the modal kernel for both bases
-    if (mode != kHJGradients) apply_band(c, kNbHJ, a.m);   // the gradient export uses no band
-    if (c.basis == FLSP_BASIS_Q && mode != kHJGradients) {
-      // the smooth-sign table is filled by the sweep's kHJCflOnly launch,
-      // which evaluates phi0 as phi
-      if (!c.hj_stab) return set_error(FLSP_ERR_BAD_ARG, "reinit sign table not allocated");
-      if (mode == kHJCflOnly && phi != phi0)
-        return set_error(FLSP_ERR_BAD_ARG, "the sign-table launch needs phi == phi0");
-      if (a.m.tile[0] != HjsTile<DIM>::X || a.m.tile[1] != HjsTile<DIM>::Y || a.m.tile[2] != HjsTile<DIM>::Z)
-        return set_error(FLSP_ERR_BAD_ARG, "the tensor-product reinit kernel has a fixed tile");
-      a.stab = reinterpret_cast<T*>(c.hj_stab);
-      a.err = clk ? &clk->err : nullptr;
-      const size_t smem = hjs_smem_bytes<DIM, P, T>(a.m.tile);
-      const int threads = HjsTile<DIM>::N * (P + 2);
-      hjs_kernel<DIM, P, T><<<(unsigned)nblocks(a.m), threads, smem, c.stream>>>(a);
+    if (mode == kHJGradients) {   // the export, every cell
+      static const int tg[3] = {HjgTile<DIM>::X, HjgTile<DIM>::Y, HjgTile<DIM>::Z};
+      set_tile(a.m, DIM, tg);
+      hj_gradient_kernel<DIM, P, T>
+          <<<(unsigned)nblocks(a.m), tg[0] * tg[1] * tg[2], hjg_smem_bytes<DIM, P, T>(), c.stream>>>(a);
+      return launch_status("hj_gradient_kernel");
+    }
+    apply_band(c, kNbHJ, a.m);
+    // the smooth-sign table is filled by the sweep's kHJCflOnly launch,
+    // which evaluates phi0 as phi
+    if (!c.hj_stab) return set_error(FLSP_ERR_BAD_ARG, "reinit sign table not allocated");
+    if (mode == kHJCflOnly && phi != phi0)
+      return set_error(FLSP_ERR_BAD_ARG, "the sign-table launch needs phi == phi0");
+    using TL = HjsTile<DIM>;
+    if (a.m.tile[0] % TL::X || a.m.tile[1] % TL::Y || a.m.tile[2] % TL::Z ||
+        (c.basis == FLSP_BASIS_Q && (a.m.tile[0] != TL::X || a.m.tile[1] != TL::Y || a.m.tile[2] != TL::Z)))
+      return set_error(FLSP_ERR_BAD_ARG, "the reinit kernels have a fixed tile");
+    a.stab = reinterpret_cast<T*>(c.hj_stab);
+    a.err = clk ? &clk->err : nullptr;
+    const int threads = TL::N * (P + 2);
+    if (c.basis == FLSP_BASIS_Q) {
+      hjs_kernel<DIM, P, T><<<(unsigned)nblocks(a.m), threads, HjsPlan<DIM, P, T>::BYTES, c.stream>>>(a);
       return launch_status("hjs_kernel");
     }
-    int tm[3];
-    if (c.basis == FLSP_BASIS_Q) {  // modal kernel with its own tile
-      a.m.tiles = nullptr;
-      a.m.n_tiles = nullptr;
-      Ctx cp = c;
-      cp.basis = FLSP_BASIS_P;
-      hj_default_tile(cp, tm);
-      set_tile(a.m, DIM, tm);
-      const size_t sm2 = hj_smem_bytes<DIM, P, T>(a.m.tile);
-      static bool attr_done[2][4][4] = {};
-      bool& done = attr_done[sizeof(T) == 8][DIM][P];
-      if (!done) {
-        cudaFuncSetAttribute(hj_kernel<DIM, P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2);
-        done = true;
-      }
-      hj_kernel<DIM, P, T><<<(unsigned)nblocks(a.m), tm[0] * tm[1] * tm[2], sm2, c.stream>>>(a);
-      return launch_status("hj_kernel");
-    }
-    const size_t smem = hj_smem_bytes<DIM, P, T>(a.m.tile);
-    hj_kernel<DIM, P, T><<<(unsigned)nblocks(a.m), t[0] * t[1] * t[2], smem, c.stream>>>(a);
-    return launch_status("hj_kernel");
+    const long long parts = (long long)(a.m.tile[0] / TL::X) * (a.m.tile[1] / TL::Y) * (a.m.tile[2] / TL::Z);
+    hjp_kernel<DIM, P, T>
+        <<<(unsigned)(nblocks(a.m) * parts), threads, HjpPlan<DIM, P, T>::BYTES, c.stream>>>(a);
+    return launch_status("hjp_kernel");
   });
 }
 
