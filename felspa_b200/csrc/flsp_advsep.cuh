@@ -76,7 +76,8 @@ struct AdvSepArgs {
 // 16-byte-aligned address at or below the first one.
 template <int DIM, int P, bool PB, int TX, int TY, int TZ, typename T>
 struct SepPlan {
-  static constexpr int N1 = P + 1, NM = ipow(N1, DIM), NF = ipow(N1, DIM - 1);
+  static constexpr int N1 = P + 1, NM = ipow(N1, DIM);
+  static constexpr int NF = PB ? (DIM == 2 ? N1 : (P + 1) * (P + 2) / 2) : ipow(N1, DIM - 1);   // face modes
   static constexpr int NBG = PB ? (DIM == 2 ? (P + 1) * (P + 2) / 2 : (P + 1) * (P + 2) * (P + 3) / 6) : NM;
   static constexpr int OPW = sep_opw<P>();
   static constexpr int NT = TX * TY * TZ;
@@ -88,7 +89,7 @@ struct SepPlan {
   static constexpr int SL0 = (TX + 1) * TY * TZ, SL1 = TX * (TY + 1) * TZ,
                        SL2 = DIM > 2 ? TX * TY * (TZ + 1) : 0;
   static constexpr int FLN = NF * (SL0 + SL1 + SL2);
-  static constexpr int FLE = FLN > NT * NM ? FLN : NT * NM;  // elements
+  static constexpr int FLE = FLN > NT * NBG ? FLN : NT * NBG;  // elements
   static constexpr size_t OFF_BOX = 16;
   static constexpr size_t OFF_OPS = OFF_BOX + (size_t)NROWS * SLOT;
   static constexpr size_t OFF_FL = OFF_OPS + (size_t)DIM * SPAN * OPW * sizeof(T);
@@ -123,135 +124,148 @@ __device__ __forceinline__ void load_op(const T* __restrict__ src, T (&M)[N1][N1
     for (int b = 0; b < N1; ++b) M[a][b] = v[a * N1 + b];
 }
 
-// F = s1 (A0 (x) A1) S + s2 (B0 (x) B1) D on the face modes (m0 + N1 m1);
+// Modes in use: every (a, b, c) of the Q layout, or with PB those of the P
+// space, a + b + c <= P; sums and results outside it are left out at compile
+// time (3D degree 2: 10 of 27 modes).
+template <int P, bool PB>
+__host__ __device__ constexpr bool mode_in(int sum) {
+  return !PB || sum <= P;
+}
+// index of the face mode (m0, m1) among those in use
+template <int P, bool PB>
+__host__ __device__ constexpr int face_index(int m0, int m1) {
+  int i = m0;
+  for (int k = 0; k < m1; ++k) i += PB ? P + 1 - k : P + 1;
+  return i;
+}
+// index of mode (a, b, c) in a cell's HBM order
+template <int DIM, int P, bool PB>
+__host__ __device__ constexpr int cell_index(int q) {
+  return PB ? q2g_ct<DIM, P>(q) : q;
+}
+
+// F = s1 (A0 (x) A1) S + s2 (B0 (x) B1) D on the face modes in use;
 // in 2D only A0 / B0; the B blocks start BOFF elements after the A blocks
-template <int DIM, int N1, int BOFF, typename T>
+template <int DIM, int P, bool PB, int BOFF, typename T>
 __device__ __forceinline__ void face_apply(const T* __restrict__ rowA0, const T* __restrict__ rowA1,
                                            const T* S, const T* D, T s1, T s2, bool upwind, T* F) {
-  constexpr int NF = DIM > 2 ? N1 * N1 : N1;
-  T M0[N1][N1];
-  load_op<N1, T>(rowA0, M0);
-  if constexpr (DIM == 2) {
+  constexpr int N1 = P + 1, NH = DIM > 2 ? N1 : 1;
+  auto apply = [&](const T* r0, const T* r1, const T* x, T s, bool acc_into) {
+    T M0[N1][N1], u[N1][NH];   // u: [a0][b1]
+    load_op<N1, T>(r0, M0);
 #pragma unroll
-    for (int a0 = 0; a0 < N1; ++a0) {
-      T acc = T(0);
+    for (int a0 = 0; a0 < N1; ++a0)
 #pragma unroll
-      for (int b0 = 0; b0 < N1; ++b0) acc += M0[a0][b0] * S[b0];
-      F[a0] = s1 * acc;
-    }
-    if (upwind) {
-      load_op<N1, T>(rowA0 + BOFF, M0);
-#pragma unroll
-      for (int a0 = 0; a0 < N1; ++a0) {
+      for (int b1 = 0; b1 < NH; ++b1) {
         T acc = T(0);
 #pragma unroll
-        for (int b0 = 0; b0 < N1; ++b0) acc += M0[a0][b0] * D[b0];
-        F[a0] += s2 * acc;
+        for (int b0 = 0; b0 < N1; ++b0)
+          if (mode_in<P, PB>(b0 + b1)) acc += M0[a0][b0] * x[face_index<P, PB>(b0, b1)];
+        u[a0][b1] = acc;
       }
-    }
-  } else {
     T M1[N1][N1];
-    load_op<N1, T>(rowA1, M1);
-    auto apply2 = [&](const T* x, T s, bool acc_into) {
-      T u[N1][N1];   // [a0][b1]
+    if constexpr (DIM > 2) load_op<N1, T>(r1, M1);
 #pragma unroll
-      for (int a0 = 0; a0 < N1; ++a0)
+    for (int a1 = 0; a1 < NH; ++a1)
 #pragma unroll
-        for (int b1 = 0; b1 < N1; ++b1) {
-          T acc = T(0);
-#pragma unroll
-          for (int b0 = 0; b0 < N1; ++b0) acc += M0[a0][b0] * x[b0 + N1 * b1];
-          u[a0][b1] = acc;
-        }
-#pragma unroll
-      for (int a1 = 0; a1 < N1; ++a1)
-#pragma unroll
-        for (int a0 = 0; a0 < N1; ++a0) {
-          T acc = T(0);
+      for (int a0 = 0; a0 < N1; ++a0) {
+        if (!mode_in<P, PB>(a0 + a1)) continue;
+        T acc = T(0);
+        if constexpr (DIM > 2) {
 #pragma unroll
           for (int b1 = 0; b1 < N1; ++b1) acc += M1[a1][b1] * u[a0][b1];
-          if (acc_into) F[a0 + N1 * a1] += s * acc;
-          else F[a0 + N1 * a1] = s * acc;
+        } else {
+          acc = u[a0][0];
         }
-    };
-    apply2(S, s1, false);
-    if (upwind) {
-      load_op<N1, T>(rowA0 + BOFF, M0);
-      load_op<N1, T>(rowA1 + BOFF, M1);
-      apply2(D, s2, true);
-    }
-  }
-  (void)NF;
+        const int f = face_index<P, PB>(a0, a1);
+        F[f] = acc_into ? F[f] + s * acc : s * acc;
+      }
+  };
+  apply(rowA0, rowA1, S, s1, false);
+  if (upwind) apply(rowA0 + BOFF, rowA1 + BOFF, D, s2, true);
 }
 
 // trace of a box cell (HBM order) on its face normal to E, in face modes
-// (side values Ls = L(0) or L(1)); the P basis reads its modes through the
-// Q-layout map
+// (side values Ls = L(0) or L(1); L_0 = 1)
 template <int DIM, int P, bool PB, int E, typename T>
 __device__ __forceinline__ void face_trace_ct(const T* __restrict__ src, const T* Ls, T* tr) {
-  constexpr int N1 = P + 1, NF = DIM > 2 ? N1 * N1 : N1;
+  constexpr int N1 = P + 1;
   constexpr int t0 = E == 0 ? 1 : 0, t1 = E == 2 ? 1 : 2;
   constexpr int st[3] = {1, N1, N1 * N1};
 #pragma unroll
-  for (int mf = 0; mf < NF; ++mf) {
-    const int m0 = mf % N1, m1 = mf / N1;
-    const int base = m0 * st[t0] + (DIM > 2 ? m1 * st[t1] : 0);
-    T s = T(0);
+  for (int m1 = 0; m1 < (DIM > 2 ? N1 : 1); ++m1)
 #pragma unroll
-    for (int aa = 0; aa < N1; ++aa) {
-      const int q = base + aa * st[E];
-      if constexpr (PB) {
-        const int gi = q2g_ct<DIM, P>(q);
-        if (gi >= 0) s += Ls[aa] * src[gi];
-      } else {
-        s += Ls[aa] * src[q];
-      }
+    for (int m0 = 0; m0 < N1; ++m0) {
+      if (!mode_in<P, PB>(m0 + m1)) continue;
+      const int base = m0 * st[t0] + (DIM > 2 ? m1 * st[t1] : 0);
+      T s = src[cell_index<DIM, P, PB>(base)];
+#pragma unroll
+      for (int aa = 1; aa < N1; ++aa)
+        if (mode_in<P, PB>(m0 + m1 + aa)) s += Ls[aa] * src[cell_index<DIM, P, PB>(base + aa * st[E])];
+      tr[face_index<P, PB>(m0, m1)] = s;
     }
-    tr[mf] = s;
-  }
 }
 
-// R += s (M0 (x) M1 (x) M2) c (Q layout, index a0 + N1 a1 + N1^2 a2),
-// contracted one z-slab of c at a time; M2 read from its shared-memory row
-template <int DIM, int P, typename T>
-__device__ __forceinline__ void apply_sep_reg(const T (&M0)[P + 1][P + 1], const T (&M1)[P + 1][P + 1],
+// R += s (M0 (x) M1 (x) M2) c for component D (Q layout, index a0 + N1 a1 +
+// N1^2 a2), contracted one z-slab of c at a time; M2 read from its
+// shared-memory row.  The operator of axis D holds L_a', so its row a = 0
+// vanishes and the modes a_D = 0 get nothing.
+template <int DIM, int P, bool PB, int D, typename T>
+__device__ __forceinline__ void apply_sep_reg(const T* __restrict__ m0row, const T* __restrict__ m1row,
                                               const T* __restrict__ m2row, const T* c, T* R, T s) {
   constexpr int N1 = P + 1, NZ = DIM > 2 ? N1 : 1;
+  T M0[N1][N1], M1[N1][N1];
+  load_op<N1, T>(m0row, M0);
+  load_op<N1, T>(m1row, M1);
+#pragma unroll
+  for (int a0 = D == 0 ? 1 : 0; a0 < N1; ++a0)
+#pragma unroll
+    for (int b0 = 0; b0 < N1; ++b0) M0[a0][b0] *= s;
 #pragma unroll
   for (int b2 = 0; b2 < NZ; ++b2) {
     T u[N1][N1];   // [a0][b1]
 #pragma unroll
-    for (int a0 = 0; a0 < N1; ++a0)
+    for (int a0 = D == 0 ? 1 : 0; a0 < N1; ++a0)
 #pragma unroll
       for (int b1 = 0; b1 < N1; ++b1) {
+        if (!mode_in<P, PB>(b1 + b2)) continue;
         T acc = T(0);
 #pragma unroll
-        for (int b0 = 0; b0 < N1; ++b0) acc += M0[a0][b0] * c[b0 + N1 * (b1 + N1 * b2)];
+        for (int b0 = 0; b0 < N1; ++b0)
+          if (mode_in<P, PB>(b0 + b1 + b2)) acc += M0[a0][b0] * c[b0 + N1 * (b1 + N1 * b2)];
         u[a0][b1] = acc;
       }
     T m2c[N1];   // column b2 of M2
     if constexpr (DIM > 2) {
 #pragma unroll
-      for (int a2 = 0; a2 < N1; ++a2) m2c[a2] = m2row[a2 * N1 + b2];
+      for (int a2 = D == 2 ? 1 : 0; a2 < N1; ++a2) m2c[a2] = m2row[a2 * N1 + b2];
     }
 #pragma unroll
-    for (int a1 = 0; a1 < N1; ++a1)
+    for (int a1 = D == 1 ? 1 : 0; a1 < N1; ++a1)
 #pragma unroll
-      for (int a0 = 0; a0 < N1; ++a0) {
-        T acc = T(0);
+      for (int a0 = D == 0 ? 1 : 0; a0 < N1; ++a0) {
+        if (!mode_in<P, PB>(a0 + a1)) continue;
+        T v = T(0);
 #pragma unroll
-        for (int b1 = 0; b1 < N1; ++b1) acc += M1[a1][b1] * u[a0][b1];
-        const T v = s * acc;
+        for (int b1 = 0; b1 < N1; ++b1)
+          if (mode_in<P, PB>(b1 + b2)) v += M1[a1][b1] * u[a0][b1];
         if constexpr (DIM == 2) {
           R[a0 + N1 * a1] += v;
         } else {
 #pragma unroll
-          for (int a2 = 0; a2 < N1; ++a2) R[a0 + N1 * (a1 + N1 * a2)] += m2c[a2] * v;
+          for (int a2 = D == 2 ? 1 : 0; a2 < N1; ++a2)
+            if (mode_in<P, PB>(a0 + a1 + a2)) R[a0 + N1 * (a1 + N1 * a2)] += m2c[a2] * v;
         }
       }
   }
 }
 
+// What bounds it: issue and latency, 16 warps per SM at Q2 3D (128 registers).
+// 64^3 Q2 FP32 51.4 -> 39.5 us, 128^3 372 -> 290, 60^3 P2 FP32 48.9 -> 22.4,
+// FP64 72 -> 36, 45x37x50 Q2 FP64 43.8 -> 38.3 against the version with the
+// zero rows, the padded modes, a mode switch per stored value and 8 instead
+// of 5 instructions per lifted face mode.
+//
 // FP32 tiles fit two CTAs per SM (<= 128 registers); an FP64 tile takes most
 // of an SM's shared memory, so FP64 gets the full register file.
 //
@@ -269,7 +283,6 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(T) == 4 ? 2 : 1)
   constexpr int N1 = PL::N1, NM = PL::NM, NF = PL::NF, OPW = PL::OPW, BOFF = sep_boff<P>();
   constexpr int NBG = PL::NBG;
   constexpr int NT = PL::NT, NMB = PL::NMB, SPAN = PL::SPAN;
-  constexpr int TL[3] = {TX, TY, TZ};
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem_raw);
   unsigned char* boxb = smem_raw + PL::OFF_BOX;
@@ -302,42 +315,22 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(T) == 4 ? 2 : 1)
     return ops + (size_t)(d * SPAN + roff + le) * OPW;
   };
 
-  // ---- staging: box rows and operator rows by bulk copies (warp 0)
-  if (threadIdx.x == 0) mbar_init(bar, 1);
+  // ---- staging on one mbarrier: the box rows by bulk copies issued by the
+  // lanes of warp 0, the operator rows by thread 0
+  if (threadIdx.x == 0) mbar_init(bar, 33);
   __syncthreads();
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    const char* gsrc = reinterpret_cast<const char*>(a.phi_s);
-    // pass 0 counts the bytes, pass 1 issues the copies
-    unsigned bytes = 0;
-    for (int pass = 0; pass < 2; ++pass) {
-      if (pass == 1) {
+  if (threadIdx.x == 0) {
+    constexpr unsigned kRowBytes = OPW * sizeof(T);
+    mbar_arrive_expect_tx(bar, DIM * SPAN * kRowBytes);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) bytes += __shfl_xor_sync(0xffffffffu, bytes, o);
-        if (lane == 0) mbar_arrive_expect_tx(bar, bytes);
-        __syncwarp();
-      }
-      for (int rr = lane; rr < PL::NROWS; rr += 32) {
-        const int ly = (DIM > 1 ? rr % PL::BY : 0) - 1, lz = DIM > 2 ? rr / PL::BY - 1 : 0;
-        const bool yout = ly < 0 || ly >= TY, zout = DIM > 2 && (lz < 0 || lz >= TZ);
-        if (yout && zout) continue;
-        const int gy = oy + ly, gz = oz + lz;
-        if (gy < 0 || gy >= m.n[1] || (DIM > 2 && (gz < 0 || gz >= m.n[2]))) continue;
-        const long long rowcell = (long long)m.n[0] * (gy + (long long)m.n[1] * (DIM > 2 ? gz : 0));
-        const long long s0 = (rowcell + gx0) * NMB, s1 = (rowcell + gx1) * NMB;
-        const long long a0 = s0 & ~15LL, a1 = (s1 + 15) & ~15LL;
-        if (pass == 0) bytes += (unsigned)(a1 - a0);
-        else bulk_g2s(boxb + (size_t)rr * PL::SLOT, gsrc + a0, (unsigned)(a1 - a0), bar);
-      }
-      for (int k = lane; k < DIM * DIM; k += 32) {
-        const int d = k / DIM, e = k % DIM;
-        const int o = e == 0 ? ox : (e == 1 ? oy : oz);
-        const unsigned nbytes = (unsigned)(TL[e] * OPW * sizeof(T));
-        if (pass == 0) bytes += nbytes;
-        else bulk_g2s(const_cast<T*>(rowp(d, e, 0)), a.optab + ((size_t)(d * 3 + e) * a.nmax + o) * OPW, nbytes, bar);
-      }
-    }
+    for (int d = 0; d < DIM; ++d)
+#pragma unroll
+      for (int e = 0; e < DIM; ++e)
+        bulk_g2s(const_cast<T*>(rowp(d, e, 0)),
+                 a.optab + ((size_t)(d * 3 + e) * a.nmax + (e == 0 ? ox : (e == 1 ? oy : oz))) * OPW,
+                 (e == 0 ? TX : (e == 1 ? TY : TZ)) * kRowBytes, bar);
   }
+  if (threadIdx.x < 32) bulk_box_rows<DIM, TX, TY, TZ, NMB, PL::SLOT>(m, a.phi_s, boxb, ox, oy, oz, bar);
   if (!mbar_wait(bar, 0, 1 << 22)) {
     if (threadIdx.x == 0 && a.err) atomicOr(a.err, kErrCopyTimeout);
     mbar_wait(bar, 0, 1 << 22);   // give copies in flight a last chance to land
@@ -385,8 +378,8 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(T) == 4 ? 2 : 1)
     // one expression; rows past the mesh hold no face values)
     const T* r0 = rowp(E, t0, lc[t0]);
     const T* r1 = DIM > 2 ? rowp(E, t1, lc[t1]) : nullptr;
-    const T fe = (f < TL[E] && has_p) ? rowp(E, E, f)[BOFF] : rowp(E, E, f - 1)[BOFF + 1];
-    const T s1 = ct * fe;
+    const T fe = (f < (E == 0 ? TX : (E == 1 ? TY : TZ)) && has_p) ? rowp(E, E, f)[BOFF] : rowp(E, E, f - 1)[BOFF + 1];
+    const T s1 = ct * fe * ih[E];   // the flux is kept per unit length
     T F[NF];
     // tangential factors of one sign over the face: |u_E| = sigma u_E, so
     // the flux is u_E times the upwind trace alone
@@ -401,7 +394,7 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(T) == 4 ? 2 : 1)
         const bool up_m = flow_up ? has_m : !has_p;
         face_trace_ct<DIM, P, PB, E, T>(up_m ? cm : cp, up_m ? tb.L1 : tb.L0, W);
       }
-      face_apply<DIM, N1, BOFF, T>(r0, r1, W, W, s1, T(0), false, F);
+      face_apply<DIM, P, PB, BOFF, T>(r0, r1, W, W, s1, T(0), false, F);
     } else {
       T S[NF], D[NF];   // traces Tm / Tp, then their mean / half jump in place
       if (has_m) face_trace_ct<DIM, P, PB, E, T>(cm, tb.L1, S);
@@ -413,7 +406,7 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(T) == 4 ? 2 : 1)
         S[mf] = T(0.5) * (tm + tp);
         D[mf] = T(0.5) * (tm - tp);
       }
-      face_apply<DIM, N1, BOFF, T>(r0, r1, S, D, s1, s1 < T(0) ? -s1 : s1, (has_m && has_p) || dir, F);
+      face_apply<DIM, P, PB, BOFF, T>(r0, r1, S, D, s1, s1 < T(0) ? -s1 : s1, (has_m && has_p) || dir, F);
     }
     const int sl = lx + EX * (ly + EY * lz);
 #pragma unroll
@@ -440,62 +433,78 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(T) == 4 ? 2 : 1)
       const T* cme = cellp(l[0], l[1], l[2]);
 #pragma unroll
       for (int q = 0; q < NM; ++q) {
-        if constexpr (PB) {
-          const int gi = m.q2g[q];
-          c[q] = gi >= 0 ? cme[gi] : T(0);
-        } else {
-          c[q] = cme[q];
-        }
+        constexpr int kOut = -1;
+        const int gi = cell_index<DIM, P, PB>(q);
+        c[q] = gi != kOut ? cme[gi] : T(0);
       }
     }
-#pragma unroll 1
-    for (int d = 0; d < DIM; ++d) {
-      T M0[N1][N1], M1[N1][N1];
-      load_op<N1, T>(rowp(d, 0, l[0]), M0);
-      load_op<N1, T>(rowp(d, 1, l[1]), M1);
-      const T ihd = d == 0 ? ih[0] : (d == 1 ? ih[1] : ih[2]);
-      apply_sep_reg<DIM, P, T>(M0, M1, DIM > 2 ? rowp(d, 2, l[2]) : nullptr, c, R, ct * ihd);
+    const T* m2[3] = {nullptr, nullptr, nullptr};
+    if constexpr (DIM > 2) {
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) m2[d] = rowp(d, 2, l[2]);
     }
+    apply_sep_reg<DIM, P, PB, 0, T>(rowp(0, 0, l[0]), rowp(0, 1, l[1]), m2[0], c, R, ct * ih[0]);
+    apply_sep_reg<DIM, P, PB, 1, T>(rowp(1, 0, l[0]), rowp(1, 1, l[1]), m2[1], c, R, ct * ih[1]);
+    if constexpr (DIM > 2) apply_sep_reg<DIM, P, PB, 2, T>(rowp(2, 0, l[0]), rowp(2, 1, l[1]), m2[2], c, R, ct * ih[2]);
+    // R += L(0) F_lower - L(1) F_upper: by parity (L_a(0) = (-1)^a L_a(1)) the
+    // even modes along E take L_a(1) times the difference, the odd ones
+    // minus L_a(1) times the sum
     auto lift = [&](auto EC) {
       constexpr int E = decltype(EC)::value;
+      constexpr int t0 = E == 0 ? 1 : 0, t1 = E == 2 ? 1 : 2;
+      constexpr int st[3] = {1, N1, N1 * N1};
       const int slo = l[0] + (TX + (E == 0)) * (l[1] + (TY + (E == 1)) * l[2]);
       const int sup = slo + (E == 0 ? 1 : (E == 1 ? TX : (TX * (TY + 0)) ));
-      T F[NF];
 #pragma unroll
-      for (int mf = 0; mf < NF; ++mf) F[mf] = fl[FLO[E] + mf * SL[E] + slo];
-      scatter_face<DIM, P, E, T>(R, tb.L0, F, ih[E]);
+      for (int m1 = 0; m1 < (DIM > 2 ? N1 : 1); ++m1)
 #pragma unroll
-      for (int mf = 0; mf < NF; ++mf) F[mf] = fl[FLO[E] + mf * SL[E] + sup];
-      scatter_face<DIM, P, E, T>(R, tb.L1, F, -ih[E]);
+        for (int m0 = 0; m0 < N1; ++m0) {
+          if (!mode_in<P, PB>(m0 + m1)) continue;
+          const int f = FLO[E] + face_index<P, PB>(m0, m1) * SL[E];
+          const T flo = fl[f + slo], fup = fl[f + sup];
+          const T dif = flo - fup, sum = flo + fup;
+          const int base = m0 * st[t0] + (DIM > 2 ? m1 * st[t1] : 0);
+          R[base] += dif;
+#pragma unroll
+          for (int a = 1; a < N1; ++a) {
+            if (!mode_in<P, PB>(m0 + m1 + a)) continue;
+            if (a % 2) R[base + a * st[E]] -= tb.L1[a] * sum;
+            else R[base + a * st[E]] += tb.L1[a] * dif;
+          }
+        }
     };
     lift(std::integral_constant<int, 0>());
     lift(std::integral_constant<int, 1>());
     if constexpr (DIM == 3) lift(std::integral_constant<int, 2>());
   }
-  __syncthreads();   // face fluxes consumed: the region now holds R [cell][NM]
+  __syncthreads();   // face fluxes consumed: the region now holds R [cell][NBG], HBM order
   T* rbuf = fl;
   if (work) {
 #pragma unroll
-    for (int q = 0; q < NM; ++q) rbuf[(size_t)cl * NM + q] = R[q];
+    for (int q = 0; q < NM; ++q) {
+      const int gi = cell_index<DIM, P, PB>(q);
+      if (gi >= 0) rbuf[(size_t)cl * NBG + gi] = R[q];
+    }
   }
   __syncthreads();
 
   // ---- RK combination fused into the coalesced store: one warp per row of
   // cells along x; stage input from the box, phi^n from HBM, all of a
   // lane's phi^n loads issued before the first use
+  const Combine<T> comb(a.combine, dt);
   const bool need_n = a.combine == kRK2b || a.combine == kRK3b || a.combine == kRK3c;
   constexpr int NW = NT / 32, NROW = TY * TZ, ROWE = TX * NBG;
   constexpr int RPW = (NROW + NW - 1) / NW, KPR = (ROWE + 31) / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nx = min(TX, m.n[0] - ox);
   // FP32 rows of whole tiles start on 16-byte boundaries in HBM, in the box
-  // copy (same 16-byte phase) and in the R buffer when TX * NM and the row
+  // copy (same 16-byte phase) and in the R buffer when TX * NBG and the row
   // pitch n[0] * NM are multiples of 4: float4 loads and stores
-  constexpr bool VEC = !PB && sizeof(T) == 4 && (TX * NM) % 4 == 0;
-  const bool vec_ok = VEC && nx == TX && ((long long)m.n[0] * NM) % 4 == 0 &&
+  constexpr bool VEC = sizeof(T) == 4 && (TX * NBG) % 4 == 0;
+  const bool vec_ok = VEC && nx == TX && ((long long)m.n[0] * NBG) % 4 == 0 &&
                       ((reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.phi_n)) & 15) == 0;
   if (VEC && vec_ok) {
-    constexpr int RV = TX * NM / 4, KV = (RV + 31) / 32;   // float4 per row, per lane
+    constexpr int RV = TX * NBG / 4, KV = (RV + 31) / 32;   // float4 per row, per lane
     constexpr int CV = RPW;                                 // rows with loads in flight together
 #pragma unroll
     for (int j0 = 0; j0 < RPW; j0 += CV) {
@@ -506,7 +515,7 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(T) == 4 ? 2 : 1)
         const int ly = r % TY, lz = r / TY;
         const bool rok = j0 + jj < RPW && r < NROW && oy + ly < m.n[1] && (DIM < 3 || oz + lz < m.n[2]);
         const long long gbase =
-            ((long long)m.n[0] * ((oy + ly) + (long long)m.n[1] * (DIM > 2 ? oz + lz : 0)) + ox) * NM;
+            ((long long)m.n[0] * ((oy + ly) + (long long)m.n[1] * (DIM > 2 ? oz + lz : 0)) + ox) * NBG;
         const float4* src = reinterpret_cast<const float4*>(a.phi_n + (rok ? gbase : 0));
 #pragma unroll
         for (int k = 0; k < KV; ++k) {
@@ -520,9 +529,9 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(T) == 4 ? 2 : 1)
         const int ly = r % TY, lz = r / TY;
         if (!(j0 + jj < RPW && r < NROW && oy + ly < m.n[1] && (DIM < 3 || oz + lz < m.n[2]))) continue;
         const long long gbase =
-            ((long long)m.n[0] * ((oy + ly) + (long long)m.n[1] * (DIM > 2 ? oz + lz : 0)) + ox) * NM;
+            ((long long)m.n[0] * ((oy + ly) + (long long)m.n[1] * (DIM > 2 ? oz + lz : 0)) + ox) * NBG;
         const float4* cs = reinterpret_cast<const float4*>(cellp(0, ly, lz));
-        const float4* rs = reinterpret_cast<const float4*>(rbuf + (size_t)TX * r * NM);
+        const float4* rs = reinterpret_cast<const float4*>(rbuf + (size_t)TX * r * NBG);
         float4* dst = reinterpret_cast<float4*>(a.out + gbase);
 #pragma unroll
         for (int k = 0; k < KV; ++k) {
@@ -532,16 +541,16 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(T) == 4 ? 2 : 1)
           float4 o = cv;
           if (active) {
             const float4 rv = rs[e], nv = pn[jj][k];
-            o.x = combine_value<float>(a.combine, cv.x, nv.x, rv.x, (float)dt);
-            o.y = combine_value<float>(a.combine, cv.y, nv.y, rv.y, (float)dt);
-            o.z = combine_value<float>(a.combine, cv.z, nv.z, rv.z, (float)dt);
-            o.w = combine_value<float>(a.combine, cv.w, nv.w, rv.w, (float)dt);
+            o.x = comb(cv.x, nv.x, rv.x);
+            o.y = comb(cv.y, nv.y, rv.y);
+            o.z = comb(cv.z, nv.z, rv.z);
+            o.w = comb(cv.w, nv.w, rv.w);
           }
           dst[e] = o;
         }
       }
     }
-  } else if constexpr (!PB) {
+  } else {
     // rows in chunks of CH, a chunk's phi^n loads all in flight together
     constexpr int CH = RPW * KPR > 16 ? (RPW > 2 ? 2 : RPW) : RPW;
 #pragma unroll
@@ -553,11 +562,11 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(T) == 4 ? 2 : 1)
         const int ly = r % TY, lz = r / TY;
         const bool rok = j0 + jj < RPW && r < NROW && oy + ly < m.n[1] && (DIM < 3 || oz + lz < m.n[2]);
         const long long gbase =
-            ((long long)m.n[0] * ((oy + ly) + (long long)m.n[1] * (DIM > 2 ? oz + lz : 0)) + ox) * NM;
+            ((long long)m.n[0] * ((oy + ly) + (long long)m.n[1] * (DIM > 2 ? oz + lz : 0)) + ox) * NBG;
 #pragma unroll
         for (int k = 0; k < KPR; ++k) {
           const int e = lane + 32 * k;
-          pn[jj][k] = (need_n && active && rok && e < nx * NM) ? __ldg(a.phi_n + gbase + e) : T(0);
+          pn[jj][k] = (need_n && active && rok && e < nx * NBG) ? __ldg(a.phi_n + gbase + e) : T(0);
         }
       }
 #pragma unroll
@@ -566,36 +575,16 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(T) == 4 ? 2 : 1)
         const int ly = r % TY, lz = r / TY;
         if (!(j0 + jj < RPW && r < NROW && oy + ly < m.n[1] && (DIM < 3 || oz + lz < m.n[2]))) continue;
         const long long gbase =
-            ((long long)m.n[0] * ((oy + ly) + (long long)m.n[1] * (DIM > 2 ? oz + lz : 0)) + ox) * NM;
+            ((long long)m.n[0] * ((oy + ly) + (long long)m.n[1] * (DIM > 2 ? oz + lz : 0)) + ox) * NBG;
         const T* cs = cellp(0, ly, lz);
-        const T* rs = rbuf + (size_t)TX * r * NM;
+        const T* rs = rbuf + (size_t)TX * r * NBG;
 #pragma unroll
         for (int k = 0; k < KPR; ++k) {
           const int e = lane + 32 * k;
-          if (e >= nx * NM) continue;
+          if (e >= nx * NBG) continue;
           const T cv = cs[e];
-          a.out[gbase + e] = active ? combine_value<T>(a.combine, cv, pn[jj][k], rs[e], dt) : cv;
+          a.out[gbase + e] = active ? comb(cv, pn[jj][k], rs[e]) : cv;
         }
-      }
-    }
-  } else {
-    for (int r = warp; r < NROW; r += NW) {
-      const int ly = r % TY, lz = r / TY;
-      const int gy = oy + ly, gz = oz + lz;
-      if (gy >= m.n[1] || (DIM > 2 && gz >= m.n[2]) || nx <= 0) continue;
-      const long long gbase = ((long long)m.n[0] * (gy + (long long)m.n[1] * (DIM > 2 ? gz : 0)) + ox) * NBG;
-      const T* cs = cellp(0, ly, lz);
-      const T* rs = rbuf + (size_t)TX * r * NM;
-      for (int e = lane; e < nx * NBG; e += 32) {
-        const int cx = e / NBG, kk = e - cx * NBG;
-        const int q = cx * NM + m.g2q[kk];
-        const T cv = cs[e];
-        T res = cv;
-        if (active) {
-          const T pnv = need_n ? __ldg(a.phi_n + gbase + e) : T(0);
-          res = combine_value<T>(a.combine, cv, pnv, rs[q], dt);
-        }
-        a.out[gbase + e] = res;
       }
     }
   }

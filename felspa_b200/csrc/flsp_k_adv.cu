@@ -22,25 +22,30 @@ static int sep_unit(int what, const Ctx& c, const VelDev* v, const int* tile, si
 }
 
 int adv_default_tile(const Ctx& c, const VelDev& v, int* tile) {
-  static const int c2[][3] = {{32, 8, 1}, {16, 16, 1}, {16, 8, 1}, {8, 8, 1}};
-  static const int c3[][3] = {{8, 8, 4}, {8, 4, 4}, {4, 4, 4}, {4, 4, 2}};
-  const int(*cand)[3] = c.dim == 2 ? c2 : c3;
-  const int ncand = c.dim == 2 ? 4 : 3;   // 4x4x2 only for the quadrature kernel
   if (use_sep_kernel(v)) {
-    // separable kernel: the first shape with two CTAs per SM, else the
-    // first that fits
-    int pick = -1;
-    for (int pass = 0; pass < 2 && pick < 0; ++pass)
-      for (int i = 0; i < ncand && pick < 0; ++i) {
-        size_t b = 0;
-        const int st = sep_unit(0, c, &v, cand[i], &b);
-        if (st) return st;
-        if (b <= (pass == 0 ? 113u * 1024u : 227u * 1024u)) pick = i;
-      }
-    if (pick < 0) return set_error(FLSP_ERR_UNSUPPORTED, "no separable tile fits in shared memory");
-    for (int d = 0; d < 3; ++d) tile[d] = cand[pick][d];
+    // the tiles that measured fastest, or within 1.5 % of it (us a stage):
+    // 2D FP32 16x8 (1200x1193 Q2: 54.0; 32x8 58.1, 8x8 60.8), FP64 8x8
+    // (1200x1193 Q3: 341, 32x8 422; 233x190 Q3: 14.7, 32x8 22.8: few tiles);
+    // 3D Q2 8x8x4 (128^3 FP32: 290; 8x4x4 314, 4x4x4 328; 96^3 FP64: 313;
+    // 329 with 4x4x4, which takes over when the larger tiles are fewer than
+    // the SMs: 24^3 12.2 against 14.4), otherwise FP32 8x4x4 (112^3 P2: 110;
+    // 8x8x4 139) and FP64 4x4x4 (128^3 Q1: 254; 8x8x4 329), P1 8x4x4 (191; 207)
+    const bool f32 = c.prec == FLSP_FP32, q = c.basis == FLSP_BASIS_Q;
+    static const int t2[2][3] = {{8, 8, 1}, {16, 8, 1}};
+    static const int t3[3][3] = {{4, 4, 4}, {8, 4, 4}, {8, 8, 4}};
+    int k = f32 ? 1 : 0;
+    if (c.dim == 3) {
+      MeshArgs m = c.m;
+      set_tile(m, 3, t3[2]);
+      if (q && c.p == 2 && (f32 || nblocks(m) >= 148)) k = 2;
+      else if (!q && c.p == 1) k = 1;
+    }
+    const int* t = c.dim == 2 ? t2[k] : t3[k];
+    for (int d = 0; d < 3; ++d) tile[d] = t[d];
     return FLSP_OK;
   }
+  static const int c2[][3] = {{32, 8, 1}, {16, 16, 1}, {16, 8, 1}, {8, 8, 1}};
+  static const int c3[][3] = {{8, 8, 4}, {8, 4, 4}, {4, 4, 4}, {4, 4, 2}};
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
     constexpr int DIM = decltype(D)::value, P = decltype(PP)::value;
     using T = decltype(tz);
