@@ -14,7 +14,7 @@
 #pragma once
 #include <type_traits>
 
-#include "flsp_device.cuh"
+#include "flsp_stage.cuh"
 
 namespace flsp {
 
@@ -33,24 +33,6 @@ struct AdvArgs {
   double dt_explicit;
 };
 
-// stage combination: v = phi + dt L (L itself for kRhsOnly), then
-// v + w (phi^n - v), w the weight of phi^n.  Written with the difference:
-// 1/3 is not representable, and a weighted sum of v and phi^n would scale
-// the field by 1 + 3e-8 (FP32) every step.
-template <typename T>
-struct Combine {
-  T dt, w;
-  bool rhs;
-  __device__ __forceinline__ Combine(int mode, T step)
-      : dt(mode == kRhsOnly ? T(1) : step),
-        w(mode == kRK2b ? T(0.5) : mode == kRK3b ? T(0.75) : mode == kRK3c ? T(1) / T(3) : T(0)),
-        rhs(mode == kRhsOnly) {}
-  __device__ __forceinline__ T operator()(T phi, T phin, T L) const {
-    const T v = (rhs ? T(0) : phi) + dt * L;
-    return w != T(0) ? v + w * (phin - v) : v;
-  }
-};
-
 // velocity term value at table columns (jx, jy, jz) in the order the
 // separable descriptor defines it: ((coeff f0) f1) f2
 template <int DIM, typename T>
@@ -64,15 +46,13 @@ __device__ __forceinline__ T term_val(const T* __restrict__ vx, const T* __restr
 // shared-memory footprint of the stage kernel: tile box with face halo,
 // velocity-table rows of the tile, upper-face fluxes shared with the
 // upper neighbours
-// tab: the velocity is read from the velocity tables (VelArgs::tab_q /
-// tab_f), no velocity rows in shared memory
 template <int DIM, int P, typename T>
-__host__ __device__ inline size_t adv_smem_bytes(const int* tile, int n_terms, bool tab = false) {
+__host__ __device__ inline size_t adv_smem_bytes(const int* tile, int n_terms) {
   constexpr int N1 = P + 1, NQ = P + 2, NM = ipow(N1, DIM), NPT = NQ + 2, NF = ipow(N1, DIM - 1);
   const int bx = tile[0] + 2, by = DIM > 1 ? tile[1] + 2 : 1, bz = DIM > 2 ? tile[2] + 2 : 1;
   const int nt = tile[0] * tile[1] * (DIM > 2 ? tile[2] : 1);
   size_t box = (size_t)bx * by * bz * NM * sizeof(T);
-  size_t vt = tab ? 0 : (size_t)n_terms * (tile[0] + tile[1] + (DIM > 2 ? tile[2] : 0)) * NPT * sizeof(T);
+  size_t vt = (size_t)n_terms * (tile[0] + tile[1] + (DIM > 2 ? tile[2] : 0)) * NPT * sizeof(T);
   size_t fl = (size_t)DIM * NF * nt * sizeof(T);
   return box + vt + fl;
 }
@@ -187,16 +167,13 @@ __device__ __forceinline__ void scatter_face(T* R, const T* Ls, const T* Fm, T c
   }
 }
 
-// General velocity: a runtime sum of separable terms per component.  (A
-// velocity whose components are single terms takes adv_sep_kernel.)  TAB:
-// the velocity's spatial part read from tables made once per field update
-// at every cell's quadrature points and, single-valued, at every face's
-// (vel_tabulate_* for a sum of terms, fe_tabulate_* for the velocity of a
-// coupled FE simulator, advection.implement.h:891-905), times the time
-// factor.
-// one tile of a stage (launch slot `slot`); a plain launch serves slot blockIdx.x
-template <int DIM, int P, typename T, bool TAB = false>
-__device__ __forceinline__ void adv_stage_tile(const AdvArgs<T>& a, int slot) {
+// A runtime sum of separable terms per component, evaluated at every point:
+// the form of a velocity of several terms whose tables (adv_tab_kernel) do not
+// fit in device memory.  (A velocity whose components are single terms takes
+// adv_sep_kernel.)
+template <int DIM, int P, typename T>
+__global__ void __launch_bounds__(256, 2) adv_stage_kernel(const AdvArgs<T> a) {
+  const int slot = (int)blockIdx.x;
   constexpr int N1 = P + 1, NQ = P + 2, NM = ipow(N1, DIM), NPT = NQ + 2, NF = ipow(N1, DIM - 1);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* box = reinterpret_cast<T*>(smem_raw);
@@ -207,26 +184,24 @@ __device__ __forceinline__ void adv_stage_tile(const AdvArgs<T>& a, int slot) {
   const int nterm = a.v.n_terms;
   const int span = tx + ty + (DIM > 2 ? tz : 0);
   T* vt = box + (size_t)nboxc * NM;
-  T* fl = vt + (TAB ? 0 : (size_t)max(nterm, 1) * span * NPT);   // [DIM][NF][nt]
+  T* fl = vt + (size_t)max(nterm, 1) * span * NPT;   // [DIM][NF][nt]
   const Tab1D<T>& tb = tab<T>(P);
   const TileCoord tc = tile_coord(m, DIM, slot);
 
-  if constexpr (!TAB) {
-    // ---- stage velocity-table rows of this tile: vt[(k*span + li)*NPT + j]
-    const int total = nterm * span * NPT;
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-      const int j = e % NPT;
-      const int r = e / NPT;
-      const int li = r % span;
-      const int k = r / span;
-      int axis, gi;
-      if (li < tx) { axis = 0; gi = tc.ox + li; }
-      else if (li < tx + ty) { axis = 1; gi = tc.oy + (li - tx); }
-      else { axis = 2; gi = tc.oz + (li - tx - ty); }
-      gi = min(gi, m.n[axis] - 1);
-      vt[(size_t)(k * span + li) * NPT + j] =
-          a.v.vtab[((size_t)(k * 3 + axis) * a.v.nmax + gi) * a.v.npt + j];
-    }
+  // ---- stage velocity-table rows of this tile: vt[(k*span + li)*NPT + j]
+  const int total = nterm * span * NPT;
+  for (int e = threadIdx.x; e < total; e += blockDim.x) {
+    const int j = e % NPT;
+    const int r = e / NPT;
+    const int li = r % span;
+    const int k = r / span;
+    int axis, gi;
+    if (li < tx) { axis = 0; gi = tc.ox + li; }
+    else if (li < tx + ty) { axis = 1; gi = tc.oy + (li - tx); }
+    else { axis = 2; gi = tc.oz + (li - tx - ty); }
+    gi = min(gi, m.n[axis] - 1);
+    vt[(size_t)(k * span + li) * NPT + j] =
+        a.v.vtab[((size_t)(k * 3 + axis) * a.v.nmax + gi) * a.v.npt + j];
   }
   load_box<DIM, NM>(m, a.phi_s, box, tc.ox, tc.oy, tc.oz, true);
   cp_async_wait_all();
@@ -255,24 +230,6 @@ __device__ __forceinline__ void adv_stage_tile(const AdvArgs<T>& a, int slot) {
   auto vrow = [&](int k, int axis) -> const T* {
     const int li = axis == 0 ? tc.lx : (axis == 1 ? tx + tc.ly : tx + ty + tc.lz);
     return vt + (size_t)(k * span + li) * NPT;
-  };
-  // TAB: the tables at this cell's quadrature points ([comp][point][cell],
-  // cell lexicographic) and at its faces ([E][point][face], face index
-  // lexicographic over n + e_E faces)
-  const long long tab_cell = tc.gx + (long long)m.n[0] * (tc.gy + (long long)m.n[1] * tc.gz);
-  auto tab_point = [&](int qx, int qy, int qz, T* u) {
-    constexpr int NQD = ipow(NQ, DIM);
-    const int q = qx + NQ * (qy + NQ * qz);
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) u[d] = a.v.tab_q[((size_t)d * NQD + q) * m.ncell + tab_cell] * ct;
-  };
-  auto tab_face = [&](auto EC, int S, int q0, int q1) -> T {
-    constexpr int E = decltype(EC)::value;
-    int f[3] = {tc.gx, tc.gy, tc.gz};
-    f[E] += S;
-    const long long nf0 = m.n[0] + (E == 0), nf1 = m.n[1] + (E == 1);
-    const long long face = f[0] + nf0 * (f[1] + nf1 * f[2]);
-    return a.v.tab_f[a.v.tab_foff[E] + (size_t)(q0 + NQ * q1) * a.v.tab_nf[E] + face] * ct;
   };
   // velocity component `comp` (times the time factor) at table columns
   auto vel = [&](int comp, int jx, int jy, int jz) -> T {
@@ -305,10 +262,7 @@ __device__ __forceinline__ void adv_stage_tile(const AdvArgs<T>& a, int slot) {
           T phi = T(0);
 #pragma unroll
           for (int aa = 0; aa < N1; ++aa) phi += Py[aa] * tb.Lq[aa][qx];
-          T uq[2];
-          if constexpr (TAB) tab_point(qx, qy, 0, uq);
-          else { uq[0] = vel(0, qx, qy, 0); uq[1] = vel(1, qx, qy, 0); }
-          const T u0 = uq[0], u1 = uq[1];
+          const T u0 = vel(0, qx, qy, 0), u1 = vel(1, qx, qy, 0);
           const T w = tb.wq[qx] * tb.wq[qy] * phi;
           const T fx = w * u0 * ih[0];
           const T fy = w * u1 * ih[1];
@@ -362,10 +316,7 @@ __device__ __forceinline__ void adv_stage_tile(const AdvArgs<T>& a, int slot) {
             T phi = T(0);
 #pragma unroll
             for (int aa = 0; aa < N1; ++aa) phi += Py[aa] * tb.Lq[aa][qx];
-            T uq[3];
-            if constexpr (TAB) tab_point(qx, qy, qz, uq);
-            else { uq[0] = vel(0, qx, qy, qz); uq[1] = vel(1, qx, qy, qz); uq[2] = vel(2, qx, qy, qz); }
-            const T u0 = uq[0], u1 = uq[1], u2 = uq[2];
+            const T u0 = vel(0, qx, qy, qz), u1 = vel(1, qx, qy, qz), u2 = vel(2, qx, qy, qz);
             const T w = tb.wq[qx] * tb.wq[qy] * tb.wq[qz] * phi;
             const T fx = w * u0 * ih[0];
             const T fy = w * u1 * ih[1];
@@ -408,8 +359,7 @@ __device__ __forceinline__ void adv_stage_tile(const AdvArgs<T>& a, int slot) {
       if (DIM > 2) j[t1] = q1;
       T w = tb.wq[q0];
       if constexpr (DIM > 2) w = w * tb.wq[q1];
-      if constexpr (TAB) return tab_face(std::integral_constant<int, E>(), S, q0, q1) * w;
-      else return vel(E, j[0], j[1], j[2]) * w;
+      return vel(E, j[0], j[1], j[2]) * w;
     };
   };
 
@@ -486,11 +436,6 @@ __device__ __forceinline__ void adv_stage_tile(const AdvArgs<T>& a, int slot) {
   }
   __syncthreads();
   store_tile<DIM, NM>(m, stage_buf, a.out, tc.ox, tc.oy, tc.oz);
-}
-
-template <int DIM, int P, typename T, bool TAB>
-__global__ void __launch_bounds__(256, 2) adv_stage_kernel(const AdvArgs<T> a) {
-  adv_stage_tile<DIM, P, T, TAB>(a, (int)blockIdx.x);
 }
 
 }  // namespace flsp

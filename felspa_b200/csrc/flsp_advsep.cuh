@@ -34,7 +34,9 @@
 // g_dd(1)).  Per cell that
 // is ~1.5k FMA for Q2 in 3D instead of the ~4k of point-wise quadrature.
 #pragma once
-#include "flsp_advect.cuh"
+#include <type_traits>
+
+#include "flsp_stage.cuh"
 
 namespace flsp {
 
@@ -124,26 +126,6 @@ __device__ __forceinline__ void load_op(const T* __restrict__ src, T (&M)[N1][N1
     for (int b = 0; b < N1; ++b) M[a][b] = v[a * N1 + b];
 }
 
-// Modes in use: every (a, b, c) of the Q layout, or with PB those of the P
-// space, a + b + c <= P; sums and results outside it are left out at compile
-// time (3D degree 2: 10 of 27 modes).
-template <int P, bool PB>
-__host__ __device__ constexpr bool mode_in(int sum) {
-  return !PB || sum <= P;
-}
-// index of the face mode (m0, m1) among those in use
-template <int P, bool PB>
-__host__ __device__ constexpr int face_index(int m0, int m1) {
-  int i = m0;
-  for (int k = 0; k < m1; ++k) i += PB ? P + 1 - k : P + 1;
-  return i;
-}
-// index of mode (a, b, c) in a cell's HBM order
-template <int DIM, int P, bool PB>
-__host__ __device__ constexpr int cell_index(int q) {
-  return PB ? q2g_ct<DIM, P>(q) : q;
-}
-
 // F = s1 (A0 (x) A1) S + s2 (B0 (x) B1) D on the face modes in use;
 // in 2D only A0 / B0; the B blocks start BOFF elements after the A blocks
 template <int DIM, int P, bool PB, int BOFF, typename T>
@@ -183,27 +165,6 @@ __device__ __forceinline__ void face_apply(const T* __restrict__ rowA0, const T*
   };
   apply(rowA0, rowA1, S, s1, false);
   if (upwind) apply(rowA0 + BOFF, rowA1 + BOFF, D, s2, true);
-}
-
-// trace of a box cell (HBM order) on its face normal to E, in face modes
-// (side values Ls = L(0) or L(1); L_0 = 1)
-template <int DIM, int P, bool PB, int E, typename T>
-__device__ __forceinline__ void face_trace_ct(const T* __restrict__ src, const T* Ls, T* tr) {
-  constexpr int N1 = P + 1;
-  constexpr int t0 = E == 0 ? 1 : 0, t1 = E == 2 ? 1 : 2;
-  constexpr int st[3] = {1, N1, N1 * N1};
-#pragma unroll
-  for (int m1 = 0; m1 < (DIM > 2 ? N1 : 1); ++m1)
-#pragma unroll
-    for (int m0 = 0; m0 < N1; ++m0) {
-      if (!mode_in<P, PB>(m0 + m1)) continue;
-      const int base = m0 * st[t0] + (DIM > 2 ? m1 * st[t1] : 0);
-      T s = src[cell_index<DIM, P, PB>(base)];
-#pragma unroll
-      for (int aa = 1; aa < N1; ++aa)
-        if (mode_in<P, PB>(m0 + m1 + aa)) s += Ls[aa] * src[cell_index<DIM, P, PB>(base + aa * st[E])];
-      tr[face_index<P, PB>(m0, m1)] = s;
-    }
 }
 
 // R += s (M0 (x) M1 (x) M2) c for component D (Q layout, index a0 + N1 a1 +
@@ -488,106 +449,7 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(T) == 4 ? 2 : 1)
   }
   __syncthreads();
 
-  // ---- RK combination fused into the coalesced store: one warp per row of
-  // cells along x; stage input from the box, phi^n from HBM, all of a
-  // lane's phi^n loads issued before the first use
-  const Combine<T> comb(a.combine, dt);
-  const bool need_n = a.combine == kRK2b || a.combine == kRK3b || a.combine == kRK3c;
-  constexpr int NW = NT / 32, NROW = TY * TZ, ROWE = TX * NBG;
-  constexpr int RPW = (NROW + NW - 1) / NW, KPR = (ROWE + 31) / 32;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nx = min(TX, m.n[0] - ox);
-  // FP32 rows of whole tiles start on 16-byte boundaries in HBM, in the box
-  // copy (same 16-byte phase) and in the R buffer when TX * NBG and the row
-  // pitch n[0] * NM are multiples of 4: float4 loads and stores
-  constexpr bool VEC = sizeof(T) == 4 && (TX * NBG) % 4 == 0;
-  const bool vec_ok = VEC && nx == TX && ((long long)m.n[0] * NBG) % 4 == 0 &&
-                      ((reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.phi_n)) & 15) == 0;
-  if (VEC && vec_ok) {
-    constexpr int RV = TX * NBG / 4, KV = (RV + 31) / 32;   // float4 per row, per lane
-    constexpr int CV = RPW;                                 // rows with loads in flight together
-#pragma unroll
-    for (int j0 = 0; j0 < RPW; j0 += CV) {
-      float4 pn[CV][KV];
-#pragma unroll
-      for (int jj = 0; jj < CV; ++jj) {
-        const int r = warp + NW * (j0 + jj);
-        const int ly = r % TY, lz = r / TY;
-        const bool rok = j0 + jj < RPW && r < NROW && oy + ly < m.n[1] && (DIM < 3 || oz + lz < m.n[2]);
-        const long long gbase =
-            ((long long)m.n[0] * ((oy + ly) + (long long)m.n[1] * (DIM > 2 ? oz + lz : 0)) + ox) * NBG;
-        const float4* src = reinterpret_cast<const float4*>(a.phi_n + (rok ? gbase : 0));
-#pragma unroll
-        for (int k = 0; k < KV; ++k) {
-          const int e = lane + 32 * k;
-          pn[jj][k] = (need_n && active && rok && e < RV) ? __ldg(src + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-      }
-#pragma unroll
-      for (int jj = 0; jj < CV; ++jj) {
-        const int r = warp + NW * (j0 + jj);
-        const int ly = r % TY, lz = r / TY;
-        if (!(j0 + jj < RPW && r < NROW && oy + ly < m.n[1] && (DIM < 3 || oz + lz < m.n[2]))) continue;
-        const long long gbase =
-            ((long long)m.n[0] * ((oy + ly) + (long long)m.n[1] * (DIM > 2 ? oz + lz : 0)) + ox) * NBG;
-        const float4* cs = reinterpret_cast<const float4*>(cellp(0, ly, lz));
-        const float4* rs = reinterpret_cast<const float4*>(rbuf + (size_t)TX * r * NBG);
-        float4* dst = reinterpret_cast<float4*>(a.out + gbase);
-#pragma unroll
-        for (int k = 0; k < KV; ++k) {
-          const int e = lane + 32 * k;
-          if (e >= RV) continue;
-          const float4 cv = cs[e];
-          float4 o = cv;
-          if (active) {
-            const float4 rv = rs[e], nv = pn[jj][k];
-            o.x = comb(cv.x, nv.x, rv.x);
-            o.y = comb(cv.y, nv.y, rv.y);
-            o.z = comb(cv.z, nv.z, rv.z);
-            o.w = comb(cv.w, nv.w, rv.w);
-          }
-          dst[e] = o;
-        }
-      }
-    }
-  } else {
-    // rows in chunks of CH, a chunk's phi^n loads all in flight together
-    constexpr int CH = RPW * KPR > 16 ? (RPW > 2 ? 2 : RPW) : RPW;
-#pragma unroll
-    for (int j0 = 0; j0 < RPW; j0 += CH) {
-      T pn[CH][KPR];
-#pragma unroll
-      for (int jj = 0; jj < CH; ++jj) {
-        const int r = warp + NW * (j0 + jj);
-        const int ly = r % TY, lz = r / TY;
-        const bool rok = j0 + jj < RPW && r < NROW && oy + ly < m.n[1] && (DIM < 3 || oz + lz < m.n[2]);
-        const long long gbase =
-            ((long long)m.n[0] * ((oy + ly) + (long long)m.n[1] * (DIM > 2 ? oz + lz : 0)) + ox) * NBG;
-#pragma unroll
-        for (int k = 0; k < KPR; ++k) {
-          const int e = lane + 32 * k;
-          pn[jj][k] = (need_n && active && rok && e < nx * NBG) ? __ldg(a.phi_n + gbase + e) : T(0);
-        }
-      }
-#pragma unroll
-      for (int jj = 0; jj < CH; ++jj) {
-        const int r = warp + NW * (j0 + jj);
-        const int ly = r % TY, lz = r / TY;
-        if (!(j0 + jj < RPW && r < NROW && oy + ly < m.n[1] && (DIM < 3 || oz + lz < m.n[2]))) continue;
-        const long long gbase =
-            ((long long)m.n[0] * ((oy + ly) + (long long)m.n[1] * (DIM > 2 ? oz + lz : 0)) + ox) * NBG;
-        const T* cs = cellp(0, ly, lz);
-        const T* rs = rbuf + (size_t)TX * r * NBG;
-#pragma unroll
-        for (int k = 0; k < KPR; ++k) {
-          const int e = lane + 32 * k;
-          if (e >= nx * NBG) continue;
-          const T cv = cs[e];
-          a.out[gbase + e] = active ? comb(cv, pn[jj][k], rs[e]) : cv;
-        }
-      }
-    }
-  }
+  combine_rows<DIM, TX, TY, TZ, NBG, NT / 32, T>(m, cellp, rbuf, a.phi_n, a.out, a.combine, dt, active, ox, oy, oz);
 }
 
 }  // namespace flsp

@@ -39,6 +39,34 @@ __host__ __device__ constexpr int q2g_ct(int q) {
   return idx + a;
 }
 
+// block of cells of the kernels that give a cell NQ threads (one per Gauss
+// plane): fixed per dimension so that every shared-memory and table offset is
+// a compile-time constant; a multiple of 32 cells keeps each warp on one plane
+template <int DIM>
+struct HjsTile {
+  static constexpr int X = DIM == 2 ? 8 : 4, Y = DIM == 2 ? 8 : 4, Z = DIM == 2 ? 1 : 4;
+  static constexpr int N = X * Y * Z;
+};
+
+// Velocity table of a problem (adv_tab_tile, flsp_advtab.cuh): per HjsTile,
+// w_q u_d / h_d at the cells' QGauss(p+2) points, entry (d NQ^DIM + q) N +
+// cell, then w_q u_E / h_E at the tile's faces' points, entry q NFT + off(E) +
+// slot; faces normal to E in slots lx + EX (ly + EY lz) of a block with one
+// more face than cells along E.
+template <int DIM>
+struct VelTabLayout {
+  using TL = HjsTile<DIM>;
+  static constexpr int S0 = (TL::X + 1) * TL::Y * TL::Z, S1 = TL::X * (TL::Y + 1) * TL::Z;
+  static constexpr int S2 = DIM > 2 ? TL::X * TL::Y * (TL::Z + 1) : 0, NFT = S0 + S1 + S2;
+  __host__ __device__ static constexpr int off(int E) { return E == 0 ? 0 : (E == 1 ? S0 : S0 + S1); }
+  // entries of a tile
+  __host__ __device__ static constexpr int entries(int nq) {
+    return DIM * ipow(nq, DIM) * TL::N + ipow(nq, DIM - 1) * NFT;
+  }
+  template <int NQ>
+  __host__ __device__ static constexpr int entries() { return entries(NQ); }
+};
+
 // 1D tables for one polynomial degree p (entries beyond p unused)
 template <typename T>
 struct Tab1D {
@@ -140,6 +168,24 @@ __device__ __forceinline__ void gauss_project(const Tab1D<T>& tb, const T* f, T*
     X[0] += f[H];
     if constexpr (NA > 2) X[2 * S] += f[H] * tb.Lq[2][H];
   }
+}
+// X[a] += sum_q f[q] L_a'(x_q), 1 <= a < NA
+template <int NA, int NQ, typename T>
+__device__ __forceinline__ void gauss_project_derivative(const Tab1D<T>& tb, const T* f, T* X) {
+  constexpr int H = NQ / 2;
+  T s1 = T(0);
+#pragma unroll
+  for (int q = 0; q < H; ++q) {
+    const T s = f[q] + f[NQ - 1 - q];
+    s1 += s;
+    if constexpr (NA > 3) X[3] += s * tb.Dq[3][q];
+    if constexpr (NA > 2) X[2] += (f[q] - f[NQ - 1 - q]) * tb.Dq[2][q];
+  }
+  if constexpr (NQ % 2) {
+    s1 += f[H];
+    if constexpr (NA > 3) X[3] += f[H] * tb.Dq[3][H];
+  }
+  X[1] += s1 * tb.Dq[1][0];
 }
 // the values at the interval's ends 0 and 1
 template <int N1, int S, typename T>
@@ -340,14 +386,6 @@ struct VelArgs {
   int npt;
   int comp[kMaxTerms];
   int cstart[4];   // terms of component c: [cstart[c], cstart[c+1]) (terms sorted by component)
-  // velocity tables (the point-wise kernel's TAB form): the spatial part
-  // at the cells' quadrature points, tab_q[comp][point][cell], and its
-  // normal component at the faces' points, tab_f[E][point][face] (block E
-  // at tab_foff[E], tab_nf[E] faces normal to E)
-  const T* tab_q;
-  const T* tab_f;
-  long long tab_foff[3];
-  long long tab_nf[3];
 };
 
 // first term of each component in a component-sorted term list

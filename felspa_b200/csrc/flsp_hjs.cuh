@@ -37,15 +37,6 @@
 
 namespace flsp {
 
-// the kernel's tile (cells), fixed per dimension so that every shared-
-// memory and table offset is a compile-time constant; a multiple of 32
-// cells keeps each warp on one Gauss plane
-template <int DIM>
-struct HjsTile {
-  static constexpr int X = DIM == 2 ? 8 : 4, Y = DIM == 2 ? 8 : 4, Z = DIM == 2 ? 1 : 4;
-  static constexpr int N = X * Y * Z;
-};
-
 // table entries per cell
 template <int DIM, int P>
 __host__ __device__ constexpr int hjs_ns() {
@@ -280,7 +271,7 @@ __device__ __forceinline__ T hjs_speed(T S, const T* left, const T* right) {
 // table, CFL estimate of the first pseudo-step) and kHJStep (one pseudo-
 // step from the table, CFL estimate of the next).
 template <int DIM, int P, typename T>
-__global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjs_min_blocks<DIM, P, T>()) hjs_kernel(const HJArgs<T> a) {
+__device__ __forceinline__ void hjs_tile(const HJArgs<T>& a, int slot) {
   using PL = HjsPlan<DIM, P, T>;
   constexpr int N1 = P + 1, NQ = P + 2, NM = ipow(N1, DIM), NV = 1 << DIM;
   constexpr int NQF = ipow(NQ, DIM - 1), NC = 1 << (DIM - 1);
@@ -299,7 +290,6 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjs_min_blocks<DIM,
   T* ub = stl;                                            // plane projections [NQ][NQF][NT] (u < NU used)
   const MeshArgs& m = a.m;
   const Tab1D<T>& tb = tab<T>(P);
-  const int slot = (int)blockIdx.x;
   if (tile_inactive(m, slot)) return;
 
   auto origin = [&](int slot, int* o) {
@@ -671,6 +661,12 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjs_min_blocks<DIM,
   __syncthreads();
   store_cells<DIM, TX, TY, TZ, NM, T>(m, sb, a.out, o[0], o[1], o[2]);
   }
+}
+
+template <int DIM, int P, typename T>
+__global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjs_min_blocks<DIM, P, T>())
+    hjs_kernel(const HJArgs<T> a) {
+  hjs_tile<DIM, P, T>(a, (int)blockIdx.x);
 }
 
 }  // namespace flsp

@@ -3,6 +3,7 @@
 #include <cstring>
 
 #include "flsp_advect.cuh"
+#include "flsp_advtab.cuh"
 #include "flsp_launch.h"
 #include "flsp_tables.h"
 
@@ -19,6 +20,13 @@ static int sep_unit(int what, const Ctx& c, const VelDev* v, const int* tile, si
                     const DevClock* clk = nullptr, int stage = 0, int combine = 0, double ct = 0.0) {
   if (c.dim == 2) return sep2_call(what, c, v, tile, bytes, in, phin, out, clk, stage, combine, ct);
   return sep3_call(what, c, v, tile, bytes, in, phin, out, clk, stage, combine, ct);
+}
+
+// the table kernel's fixed tile
+static void tab_tile(const Ctx& c, int* tile) {
+  tile[0] = c.dim == 2 ? HjsTile<2>::X : HjsTile<3>::X;
+  tile[1] = c.dim == 2 ? HjsTile<2>::Y : HjsTile<3>::Y;
+  tile[2] = c.dim == 2 ? HjsTile<2>::Z : HjsTile<3>::Z;
 }
 
 int adv_default_tile(const Ctx& c, const VelDev& v, int* tile) {
@@ -44,6 +52,10 @@ int adv_default_tile(const Ctx& c, const VelDev& v, int* tile) {
     for (int d = 0; d < 3; ++d) tile[d] = t[d];
     return FLSP_OK;
   }
+  if (v.tab) {
+    tab_tile(c, tile);
+    return FLSP_OK;
+  }
   static const int c2[][3] = {{32, 8, 1}, {16, 16, 1}, {16, 8, 1}, {8, 8, 1}};
   static const int c3[][3] = {{8, 8, 4}, {8, 4, 4}, {4, 4, 4}, {4, 4, 2}};
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
@@ -52,7 +64,7 @@ int adv_default_tile(const Ctx& c, const VelDev& v, int* tile) {
     const int(*cq)[3] = DIM == 2 ? c2 : c3;
     int i = 0;
     for (; i < 3; ++i)
-      if (adv_smem_bytes<DIM, P, T>(cq[i], std::max(v.n_terms, 1), v.tab) <= 200 * 1024) break;
+      if (adv_smem_bytes<DIM, P, T>(cq[i], std::max(v.n_terms, 1)) <= 200 * 1024) break;
     tile[0] = cq[i][0];
     tile[1] = cq[i][1];
     tile[2] = cq[i][2];
@@ -61,6 +73,11 @@ int adv_default_tile(const Ctx& c, const VelDev& v, int* tile) {
 }
 
 int adv_tile_candidates(const Ctx& c, const VelDev& v, int (*out)[3], int* n) {
+  if (!use_sep_kernel(v) && v.tab) {
+    tab_tile(c, out[0]);
+    *n = 1;
+    return FLSP_OK;
+  }
   static const int c2[][3] = {{32, 8, 1}, {16, 16, 1}, {16, 8, 1}, {8, 8, 1}};
   static const int c3s[][3] = {{8, 8, 4}, {8, 4, 4}, {4, 4, 4}};
   static const int c3q[][3] = {{8, 8, 4}, {8, 4, 4}, {4, 4, 4}, {4, 4, 2}};
@@ -76,9 +93,24 @@ int adv_prepare(const Ctx& c, const VelDev& v, const int* tile) {
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
     constexpr int DIM = decltype(D)::value, P = decltype(PP)::value;
     using T = decltype(tz);
-    const size_t smem = adv_smem_bytes<DIM, P, T>(tile, std::max(v.n_terms, 1), v.tab);
+    if (v.tab) {
+      int t[3];
+      tab_tile(c, t);
+      if (t[0] != tile[0] || t[1] != tile[1] || (DIM > 2 && t[2] != tile[2]))
+        return set_error(FLSP_ERR_BAD_ARG, "the velocity-table stage kernel has a fixed tile");
+      cudaError_t e = cudaSuccess;
+      auto attr = [&](auto kern, size_t smem) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+      };
+      if (c.basis == FLSP_BASIS_Q) attr(adv_tab_kernel<DIM, P, false, T>, AdvTabPlan<DIM, P, false, T>::BYTES);
+      else attr(adv_tab_kernel<DIM, P, true, T>, AdvTabPlan<DIM, P, true, T>::BYTES);
+      if (e != cudaSuccess) return set_error(FLSP_ERR_CUDA, std::string("adv attr: ") + cudaGetErrorString(e));
+      return FLSP_OK;
+    }
+    const size_t smem = adv_smem_bytes<DIM, P, T>(tile, std::max(v.n_terms, 1));
     if (smem > 227 * 1024) return set_error(FLSP_ERR_BAD_ARG, "advection tile too large for shared memory");
-    auto kern = v.tab ? adv_stage_kernel<DIM, P, T, true> : adv_stage_kernel<DIM, P, T, false>;
+    auto kern = adv_stage_kernel<DIM, P, T>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e != cudaSuccess) return set_error(FLSP_ERR_CUDA, std::string("adv attr: ") + cudaGetErrorString(e));
@@ -101,6 +133,31 @@ int launch_adv_stage(const Ctx& c, const VelDev& v, const void* in, const void* 
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
     constexpr int DIM = decltype(D)::value, P = decltype(PP)::value;
     using T = decltype(tz);
+    if (v.tab) {
+      AdvTabArgs<T> a;
+      std::memset(&a, 0, sizeof(a));
+      a.m = c.m;
+      int t[3];
+      tab_tile(c, t);
+      set_tile(a.m, DIM, t);
+      a.tab = reinterpret_cast<const T*>(v.tab);
+      a.phi_s = reinterpret_cast<const T*>(in);
+      a.phi_n = reinterpret_cast<const T*>(phin);
+      a.out = reinterpret_cast<T*>(out);
+      a.clk = clk;
+      a.stage = stage;
+      a.combine = combine;
+      a.ct_explicit = ct_explicit;
+      a.err = v.err;
+      const int threads = HjsTile<DIM>::N * (P + 2);
+      if (c.basis == FLSP_BASIS_Q)
+        adv_tab_kernel<DIM, P, false, T>
+            <<<(unsigned)nblocks(a.m), threads, AdvTabPlan<DIM, P, false, T>::BYTES, c.stream>>>(a);
+      else
+        adv_tab_kernel<DIM, P, true, T>
+            <<<(unsigned)nblocks(a.m), threads, AdvTabPlan<DIM, P, true, T>::BYTES, c.stream>>>(a);
+      return launch_status("adv_tab_kernel");
+    }
     AdvArgs<T> a;
     std::memset(&a, 0, sizeof(a));
     a.m = c.m;
@@ -114,14 +171,6 @@ int launch_adv_stage(const Ctx& c, const VelDev& v, const void* in, const void* 
     a.v.npt = v.npt;
     for (int k = 0; k < v.n_terms; ++k) a.v.comp[k] = v.comp[k];
     term_ranges(a.v.comp, v.n_terms, a.v.cstart);
-    if (v.tab) {
-      a.v.tab_q = reinterpret_cast<const T*>(v.tab_q);
-      a.v.tab_f = reinterpret_cast<const T*>(v.tab_f);
-      for (int e = 0; e < 3; ++e) {
-        a.v.tab_foff[e] = v.tab_foff[e];
-        a.v.tab_nf[e] = v.tab_nf[e];
-      }
-    }
     a.phi_s = reinterpret_cast<const T*>(in);
     a.phi_n = reinterpret_cast<const T*>(phin);
     a.out = reinterpret_cast<T*>(out);
@@ -129,11 +178,8 @@ int launch_adv_stage(const Ctx& c, const VelDev& v, const void* in, const void* 
     a.stage = stage;
     a.combine = combine;
     a.ct_explicit = ct_explicit;
-    const size_t smem = adv_smem_bytes<DIM, P, T>(a.m.tile, std::max(v.n_terms, 1), v.tab);
-    if (v.tab)
-      adv_stage_kernel<DIM, P, T, true><<<(unsigned)nblocks(a.m), t[0] * t[1] * t[2], smem, c.stream>>>(a);
-    else
-      adv_stage_kernel<DIM, P, T, false><<<(unsigned)nblocks(a.m), t[0] * t[1] * t[2], smem, c.stream>>>(a);
+    const size_t smem = adv_smem_bytes<DIM, P, T>(a.m.tile, std::max(v.n_terms, 1));
+    adv_stage_kernel<DIM, P, T><<<(unsigned)nblocks(a.m), t[0] * t[1] * t[2], smem, c.stream>>>(a);
     return launch_status("adv_stage_kernel");
   });
 }

@@ -1,20 +1,19 @@
 // flsp_k_batch.cu — batched problems: many independent 2D level-set
 // problems (their own meshes, degrees 1..3, velocities and clocks) advance
-// in ONE persistent launch per RK stage (and one per reinit pseudo-step and
-// limiter pass) per degree.  A block walks a list of work items (problem,
-// tile) of one degree and runs the same per-tile bodies as the
-// single-problem kernels (adv_stage_tile, hjq_tile, weno_tile); each degree
-// has its own instantiation, so its registers, shared memory and occupancy
-// are its own, not those of the most demanding degree in the batch.  The
-// tile shapes are launch parameters picked by the batch autotuner.
+// in ONE launch per RK stage (and one per reinit pseudo-step and limiter pass)
+// per degree.  A block serves a work item (problem, tile) of one degree with
+// the same per-tile bodies as the single-problem kernels (adv_tab_tile,
+// hjs_tile; the limiter's detection, weno_tile, walks its items persistently);
+// each degree has its own instantiation, so its registers, shared memory and
+// occupancy are its own, not those of the most demanding degree in the batch.
 #include <algorithm>
 #include <cstring>
 #include <string>
 #include <type_traits>
 
-#include "flsp_advect.cuh"
+#include "flsp_advtab.cuh"
 #include "flsp_clock.cuh"
-#include "flsp_hjq.cuh"
+#include "flsp_hjs.cuh"
 #include "flsp_launch.h"
 #include "flsp_tables.h"
 #include "flsp_weno.cuh"
@@ -29,76 +28,59 @@ int upload_tables_batch() {
 
 namespace {
 
-// per-item argument structs are assembled (in shared memory, by one
-// thread) from the problem's descriptor and the launch's buffer roles
-template <typename T>
-__device__ __forceinline__ void make_adv_args(const BatchProb& pr, int ix, int in_n, int iout, int stage, int combine,
-                                              AdvArgs<T>& a) {
-  a.m = pr.m_adv;
-  a.v.vtab = reinterpret_cast<const T*>(pr.vtab);
-  a.v.n_terms = pr.n_terms;
-  a.v.nmax = pr.nmax;
-  a.v.npt = pr.npt;
-#pragma unroll 1
-  for (int k = 0; k < kMaxTerms; ++k) a.v.comp[k] = pr.comp[k];
-  term_ranges(pr.comp, pr.n_terms, a.v.cstart);
-  a.v.tab_q = reinterpret_cast<const T*>(pr.tab_q);
-  a.v.tab_f = reinterpret_cast<const T*>(pr.tab_f);
-#pragma unroll
-  for (int e = 0; e < 3; ++e) {
-    a.v.tab_foff[e] = pr.tab_foff[e];
-    a.v.tab_nf[e] = pr.tab_nf[e];
+// an item's mesh, copied from the problem's descriptor by the whole block
+// (every thread reads it, like a plain launch's kernel parameters)
+__device__ __forceinline__ void copy_mesh(MeshArgs* dst, const MeshArgs& src) {
+  static_assert(sizeof(MeshArgs) % 4 == 0, "copied in words");
+  for (int i = threadIdx.x; i < (int)(sizeof(MeshArgs) / 4); i += blockDim.x)
+    reinterpret_cast<int*>(dst)[i] = reinterpret_cast<const int*>(&src)[i];
+}
+
+// one block per (problem, tile): the stage of the problem's own velocity table
+template <typename T, int P>
+__global__ void __launch_bounds__(HjsTile<2>::N * (P + 2), advtab_min_blocks<2, P, T>())
+    batch_adv_kernel(const BatchProb* __restrict__ probs, const int2* __restrict__ items, int ix, int in_n, int iout,
+                     int stage, int combine) {
+  __shared__ AdvTabArgs<T> a;
+  const int2 w = items[blockIdx.x];
+  const BatchProb& pr = probs[w.x];
+  copy_mesh(&a.m, pr.m_adv);
+  if (threadIdx.x == 0) {
+    a.tab = reinterpret_cast<const T*>(pr.tab);
+    a.phi_s = reinterpret_cast<const T*>(pr.buf[ix]);
+    a.phi_n = reinterpret_cast<const T*>(pr.buf[in_n]);
+    a.out = reinterpret_cast<T*>(pr.buf[iout]);
+    a.clk = pr.clk;
+    a.stage = stage;
+    a.combine = combine;
+    a.err = &pr.clk->err;
   }
-  a.phi_s = reinterpret_cast<const T*>(pr.buf[ix]);
-  a.phi_n = reinterpret_cast<const T*>(pr.buf[in_n]);
-  a.out = reinterpret_cast<T*>(pr.buf[iout]);
-  a.clk = pr.clk;
-  a.stage = stage;
-  a.combine = combine;
-  a.ct_explicit = 0.0;
-  a.dt_explicit = 0.0;
+  __syncthreads();
+  adv_tab_tile<2, P, false, T>(a, w.y);
 }
 
 template <typename T, int P>
-__global__ void __launch_bounds__(256, 2)
-    batch_adv_kernel(const BatchProb* __restrict__ probs, const int2* __restrict__ items, int n_items, int ix,
-                     int in_n, int iout, int stage, int combine) {
-  // the item's arguments are assembled once per block in shared memory
-  // (every thread reads them, like a plain launch's kernel parameters)
-  __shared__ AdvArgs<T> a;
-  for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-    const int2 w = items[it];
-    if (threadIdx.x == 0) make_adv_args<T>(probs[w.x], ix, in_n, iout, stage, combine, a);
-    __syncthreads();
-    adv_stage_tile<2, P, T, true>(a, w.y);   // velocity from the problem's tables
-    __syncthreads();   // shared memory is reused by the next item
-  }
-}
-
-template <typename T, int P>
-__global__ void __launch_bounds__(128)
-    batch_hj_kernel(const BatchProb* __restrict__ probs, const int2* __restrict__ items, int n_items, int isrc,
-                    int iphi0, int idst, int mode, int rk) {
+__global__ void __launch_bounds__(HjsTile<2>::N * (P + 2), hjs_min_blocks<2, P, T>())
+    batch_hj_kernel(const BatchProb* __restrict__ probs, const int2* __restrict__ items, int isrc, int iphi0, int idst,
+                    int mode, int rk) {
   __shared__ HJArgs<T> a;
-  for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-    const int2 w = items[it];
-    if (threadIdx.x == 0) {
-      const BatchProb& pr = probs[w.x];
-      a.m = pr.m_hj;
-      a.phi = reinterpret_cast<const T*>(pr.buf[isrc]);
-      a.phi0 = reinterpret_cast<const T*>(pr.buf[iphi0]);
-      a.out = idst >= 0 ? reinterpret_cast<T*>(pr.buf[idst]) : nullptr;
-      a.clk = pr.clk;
-      a.mode = mode;
-      a.rk = rk;
-      a.dt_explicit = 0.0;
-      a.block = pr.m_hj.ncell * pr.m_hj.nb;
-      a.rdiff = nullptr;
-    }
-    __syncthreads();
-    hjq_tile<2, P, T>(a, w.y);
-    __syncthreads();
+  const int2 w = items[blockIdx.x];
+  const BatchProb& pr = probs[w.x];
+  copy_mesh(&a.m, pr.m_hj);
+  if (threadIdx.x == 0) {
+    a.phi = reinterpret_cast<const T*>(pr.buf[isrc]);
+    a.phi0 = reinterpret_cast<const T*>(pr.buf[iphi0]);
+    a.out = idst >= 0 ? reinterpret_cast<T*>(pr.buf[idst]) : nullptr;
+    a.clk = pr.clk;
+    a.mode = mode;
+    a.rk = rk;
+    a.dt_explicit = 0.0;
+    a.rdiff = nullptr;
+    a.stab = reinterpret_cast<T*>(pr.stab);
+    a.err = &pr.clk->err;
   }
+  __syncthreads();
+  hjs_tile<2, P, T>(a, w.y);
 }
 
 template <typename T, int P>
@@ -169,32 +151,6 @@ int persistent_grid(K kern, int threads, size_t smem, int n_items) {
 
 }  // namespace
 
-int batch_smem(int kind, int p, int prec, const int* tile, int n_terms, size_t* bytes) {
-  auto go = [&](auto tz) -> size_t {
-    using T = decltype(tz);
-    if (kind == kBatchKindAdv) {
-      switch (p) {
-        case 1: return adv_smem_bytes<2, 1, T>(tile, std::max(n_terms, 1), true);
-        case 2: return adv_smem_bytes<2, 2, T>(tile, std::max(n_terms, 1), true);
-        default: return adv_smem_bytes<2, 3, T>(tile, std::max(n_terms, 1), true);
-      }
-    } else if (kind == kBatchKindHJ) {
-      switch (p) {
-        case 1: return hjq_smem_bytes<2, 1, T>(tile);
-        case 2: return hjq_smem_bytes<2, 2, T>(tile);
-        default: return hjq_smem_bytes<2, 3, T>(tile);
-      }
-    }
-    switch (p) {
-      case 1: return weno_smem_bytes<1, T>(tile);
-      case 2: return weno_smem_bytes<2, T>(tile);
-      default: return weno_smem_bytes<3, T>(tile);
-    }
-  };
-  *bytes = prec == FLSP_FP64 ? go((double)0) : go((float)0);
-  return FLSP_OK;
-}
-
 int launch_batch_clock(cudaStream_t s, const BatchProb* probs, int n, int what, double cfl_max) {
   batch_clock_kernel<<<(n + 127) / 128, 128, 0, s>>>(probs, n, what, cfl_max);
   return launch_status("batch_clock_kernel");
@@ -211,30 +167,34 @@ int with_degree(int p, F&& f) {
   return set_error(FLSP_ERR_UNSUPPORTED, "batched problems: degree 1..3");
 }
 
-template <typename T, int P>
-static int batch_attr(int kind, size_t smem) {
-  cudaError_t e = cudaSuccess;
-  const int s = (int)smem;
-  if (kind == kBatchKindAdv) e = cudaFuncSetAttribute(batch_adv_kernel<T, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, s);
-  else if (kind == kBatchKindHJ) e = cudaFuncSetAttribute(batch_hj_kernel<T, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, s);
-  else e = cudaFuncSetAttribute(batch_weno_kernel<T, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, s);
-  if (e != cudaSuccess) return set_error(FLSP_ERR_CUDA, std::string("batch attr: ") + cudaGetErrorString(e));
-  return FLSP_OK;
-}
-
-int batch_prepare(int kind, int prec, int p, size_t smem, int threads, int n_items, int* grid) {
-  if (smem > 227 * 1024) return set_error(FLSP_ERR_BAD_ARG, "batch tile too large for shared memory");
+int batch_prepare(int kind, int prec, int p, int n_items, size_t* smem, int* threads, int* grid) {
   return with_degree(p, [&](auto PC) -> int {
     constexpr int P = decltype(PC)::value;
-    int st = prec == FLSP_FP64 ? batch_attr<double, P>(kind, smem) : batch_attr<float, P>(kind, smem);
-    if (st) return st;
-    auto g = [&](auto tz) -> int {
+    cudaError_t e = cudaSuccess;
+    auto go = [&](auto tz) {
       using T = decltype(tz);
-      if (kind == kBatchKindAdv) return persistent_grid(batch_adv_kernel<T, P>, threads, smem, n_items);
-      if (kind == kBatchKindHJ) return persistent_grid(batch_hj_kernel<T, P>, threads, smem, n_items);
-      return persistent_grid(batch_weno_kernel<T, P>, threads, smem, n_items);
+      auto attr = [&](auto kern) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+      };
+      *threads = HjsTile<2>::N * (P + 2);
+      *grid = n_items;   // a block per item
+      if (kind == kBatchKindAdv) {
+        *smem = AdvTabPlan<2, P, false, T>::BYTES;
+        attr(batch_adv_kernel<T, P>);
+      } else if (kind == kBatchKindHJ) {
+        *smem = HjsPlan<2, P, T>::BYTES;
+        attr(batch_hj_kernel<T, P>);
+      } else {
+        *smem = weno_smem_bytes<P, T>(kWenoTile);
+        *threads = kWenoTile[0] * kWenoTile[1];
+        attr(batch_weno_kernel<T, P>);
+        *grid = persistent_grid(batch_weno_kernel<T, P>, *threads, *smem, n_items);
+      }
     };
-    *grid = prec == FLSP_FP64 ? g((double)0) : g((float)0);
+    if (prec == FLSP_FP64) go((double)0);
+    else go((float)0);
+    if (e != cudaSuccess) return set_error(FLSP_ERR_CUDA, std::string("batch attr: ") + cudaGetErrorString(e));
     return FLSP_OK;
   });
 }
@@ -244,9 +204,9 @@ int launch_batch_adv(cudaStream_t s, int prec, int p, const BatchProb* probs, co
   return with_degree(p, [&](auto PC) -> int {
     constexpr int P = decltype(PC)::value;
     if (prec == FLSP_FP64)
-      batch_adv_kernel<double, P><<<grid, threads, smem, s>>>(probs, items, n_items, ix, in_n, iout, stage, combine);
+      batch_adv_kernel<double, P><<<grid, threads, smem, s>>>(probs, items, ix, in_n, iout, stage, combine);
     else
-      batch_adv_kernel<float, P><<<grid, threads, smem, s>>>(probs, items, n_items, ix, in_n, iout, stage, combine);
+      batch_adv_kernel<float, P><<<grid, threads, smem, s>>>(probs, items, ix, in_n, iout, stage, combine);
     return launch_status("batch_adv_kernel");
   });
 }
@@ -256,9 +216,9 @@ int launch_batch_hj(cudaStream_t s, int prec, int p, const BatchProb* probs, con
   return with_degree(p, [&](auto PC) -> int {
     constexpr int P = decltype(PC)::value;
     if (prec == FLSP_FP64)
-      batch_hj_kernel<double, P><<<grid, threads, smem, s>>>(probs, items, n_items, isrc, iphi0, idst, mode, rk);
+      batch_hj_kernel<double, P><<<grid, threads, smem, s>>>(probs, items, isrc, iphi0, idst, mode, rk);
     else
-      batch_hj_kernel<float, P><<<grid, threads, smem, s>>>(probs, items, n_items, isrc, iphi0, idst, mode, rk);
+      batch_hj_kernel<float, P><<<grid, threads, smem, s>>>(probs, items, isrc, iphi0, idst, mode, rk);
     return launch_status("batch_hj_kernel");
   });
 }

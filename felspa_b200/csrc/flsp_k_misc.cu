@@ -106,60 +106,56 @@ int launch_fe_static_cfl(const Ctx& c, const double* u64, int pv, DevClock* clk)
   return launch_status("fe_static_cfl_kernel");
 }
 
+static long long vel_tiles(const Ctx& c) {
+  MeshArgs m = c.m;
+  const int t2[3] = {HjsTile<2>::X, HjsTile<2>::Y, 1}, t3[3] = {HjsTile<3>::X, HjsTile<3>::Y, HjsTile<3>::Z};
+  set_tile(m, c.dim, c.dim == 2 ? t2 : t3);
+  return nblocks(m);
+}
+static int vel_entries(const Ctx& c) {
+  return c.dim == 2 ? VelTabLayout<2>::entries(c.p + 2) : VelTabLayout<3>::entries(c.p + 2);
+}
+size_t vel_table_bytes(const Ctx& c) {
+  return (size_t)vel_tiles(c) * vel_entries(c) * (c.prec == FLSP_FP64 ? 8 : 4);
+}
+
 int launch_vel_tabulate(const Ctx& c, const double* vtab64, int n_terms, const int* comp, int nmax, int npt,
-                        void* tab_q, void* tab_f, const long long* foff, const long long* nf) {
+                        void* tab) {
   VelTerms vt;
   term_ranges(comp, n_terms, vt.cstart);
-  const int nq = c.p + 2;
+  const long long total = vel_tiles(c) * vel_entries(c);
   const int threads = 256;
-  auto grid = [&](long long n) { return (int)std::max<long long>(1, std::min<long long>((n + threads - 1) / threads, 148LL * 32)); };
-  const long long nqd = c.dim > 2 ? (long long)nq * nq * nq : (long long)nq * nq;
-  const long long nqf = c.dim > 2 ? (long long)nq * nq : nq;
+  const int grid = (int)std::max<long long>(1, std::min<long long>((total + threads - 1) / threads, 148LL * 32));
   auto run = [&](auto tz) -> int {
     using T = decltype(tz);
-    T* q = static_cast<T*>(tab_q);
-    T* f = static_cast<T*>(tab_f);
-    if (c.dim == 2)
-      vel_tabulate_cells<2, T><<<grid(nqd * c.m.ncell), threads, 0, c.stream>>>(c.m, vtab64, nmax, npt, vt, nq, q);
-    else
-      vel_tabulate_cells<3, T><<<grid(nqd * c.m.ncell), threads, 0, c.stream>>>(c.m, vtab64, nmax, npt, vt, nq, q);
-    for (int e = 0; e < c.dim; ++e) {
-      if (c.dim == 2)
-        vel_tabulate_faces<2, T><<<grid(nqf * nf[e]), threads, 0, c.stream>>>(c.m, vtab64, nmax, npt, vt, nq, e, nf[e],
-                                                                              f + foff[e]);
-      else
-        vel_tabulate_faces<3, T><<<grid(nqf * nf[e]), threads, 0, c.stream>>>(c.m, vtab64, nmax, npt, vt, nq, e, nf[e],
-                                                                              f + foff[e]);
-    }
+    T* t = static_cast<T*>(tab);
+    if (c.dim == 2) vel_tabulate<2, T><<<grid, threads, 0, c.stream>>>(c.m, vtab64, nmax, npt, vt, c.p + 2, total, t);
+    else vel_tabulate<3, T><<<grid, threads, 0, c.stream>>>(c.m, vtab64, nmax, npt, vt, c.p + 2, total, t);
     return launch_status("vel_tabulate");
   };
   return c.prec == FLSP_FP64 ? run(double(0)) : run(float(0));
 }
 
-int launch_fe_tabulate(const Ctx& c, const double* u64, int pv, const double (*gb)[kMaxNQ + 2], void* tab_q,
-                       void* tab_f, const long long* foff, const long long* nf) {
+int launch_fe_tabulate(const Ctx& c, const double* u64, int pv, const double (*gb)[kMaxNQ + 2], void* tab) {
   FeBasis fb;
   std::memcpy(fb.b, gb, sizeof(fb.b));
-  const int nq = c.p + 2;
-  const int threads = 256;
-  auto grid = [&](long long n) { return (int)std::max<long long>(1, std::min<long long>((n + threads - 1) / threads, 148LL * 32)); };
-  const long long nqd = c.dim > 2 ? (long long)nq * nq * nq : (long long)nq * nq;
-  const long long nqf = c.dim > 2 ? (long long)nq * nq : nq;
-  auto run = [&](auto tz) -> int {
+  return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
+    constexpr int DIM = decltype(D)::value, P = decltype(PP)::value, NQ = P + 2;
     using T = decltype(tz);
-    T* q = static_cast<T*>(tab_q);
-    T* f = static_cast<T*>(tab_f);
-    if (c.dim == 2) fe_tabulate_cells<2, T><<<grid(nqd * c.m.ncell), threads, 0, c.stream>>>(c.m, u64, pv, nq, fb, q);
-    else fe_tabulate_cells<3, T><<<grid(nqd * c.m.ncell), threads, 0, c.stream>>>(c.m, u64, pv, nq, fb, q);
-    for (int e = 0; e < c.dim; ++e) {
-      if (c.dim == 2)
-        fe_tabulate_faces<2, T><<<grid(nqf * nf[e]), threads, 0, c.stream>>>(c.m, u64, pv, nq, fb, e, nf[e], f + foff[e]);
-      else
-        fe_tabulate_faces<3, T><<<grid(nqf * nf[e]), threads, 0, c.stream>>>(c.m, u64, pv, nq, fb, e, nf[e], f + foff[e]);
-    }
-    return launch_status("fe_tabulate");
-  };
-  return c.prec == FLSP_FP64 ? run(double(0)) : run(float(0));
+    const long long tiles = vel_tiles(c);
+    const long long nc = tiles * HjsTile<DIM>::N * NQ * DIM, nf = tiles * VelTabLayout<DIM>::NFT * (DIM > 2 ? NQ : 1);
+    const int threads = 128;
+    auto grid = [&](long long n) { return (unsigned)std::min<long long>((n + threads - 1) / threads, 1LL << 20); };
+    auto go = [&](auto PVC) -> int {
+      constexpr int PV = decltype(PVC)::value;
+      fe_tabulate_cells<DIM, P, PV, T><<<grid(nc), threads, 0, c.stream>>>(c.m, u64, fb, nc, static_cast<T*>(tab));
+      fe_tabulate_faces<DIM, P, PV, T><<<grid(nf), threads, 0, c.stream>>>(c.m, u64, fb, nf, static_cast<T*>(tab));
+      return launch_status("fe_tabulate");
+    };
+    if (pv == 1) return go(std::integral_constant<int, 1>());
+    if (pv == 2) return go(std::integral_constant<int, 2>());
+    return go(std::integral_constant<int, 3>());
+  });
 }
 
 int reduce_blocks(const Ctx& c) { return (int)((c.m.ncell + 127) / 128); }

@@ -52,12 +52,8 @@ struct BatchProb {
   MeshArgs m_adv, m_hj, m_weno;   // the batch's tile shapes, no narrow band
   void* buf[3];                   // state buffers (roles are launch parameters)
   DevClock* clk;
-  const void* vtab;               // velocity table (state precision)
-  int n_terms, nmax, npt;
-  int comp[kMaxTerms];
-  const void* tab_q;              // velocity tables of the problem (VelArgs::tab_q / tab_f)
-  const void* tab_f;
-  long long tab_foff[3], tab_nf[3];
+  const void* tab;                // velocity table of the problem (VelTabLayout)
+  void* stab;                     // smooth-sign table of its reinitialisation
   int p;                          // degree 1..3
   AdvClockArgs ca;                // advection clock parameters
   double adv_scale;               // advection CFL scaling of the degree
@@ -68,10 +64,9 @@ enum BatchClockOp : int {
 };
 int upload_tables_batch();
 // shared memory one problem needs for a tile of the given kind
-int batch_smem(int kind, int p, int prec, const int* tile, int n_terms, size_t* bytes);
-// kernel attributes of the degree-p kernel for `smem` and its persistent
-// grid for n_items (every item of a launch has degree p)
-int batch_prepare(int kind, int prec, int p, size_t smem, int threads, int n_items, int* grid);
+// shared memory of the degree-p kernel of a kind, its attributes for it, and
+// the grid for n_items (every item of a launch has degree p)
+int batch_prepare(int kind, int prec, int p, int n_items, size_t* smem, int* threads, int* grid);
 int launch_batch_clock(cudaStream_t s, const BatchProb* probs, int n, int what, double cfl_max);
 int launch_batch_adv(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items, int n_items,
                      int grid, int threads, size_t smem, int ix, int in_n, int iout, int stage, int combine);
@@ -141,14 +136,10 @@ struct VelDev {
   const void* optab;   // per-axis operator rows of a sep1 velocity (T precision), or null
   int opstride;        // operator rows per (component, axis) in optab
   int* err;            // device error word (DevClock::err)
-  // velocity tables (tab): T-precision values at the cells' and faces'
-  // quadrature points (VelArgs::tab_q / tab_f), made from the terms or from
-  // the FE field of a coupled simulator (fe_pv > 0: its lattice degree)
-  bool tab;
+  // velocity table (VelTabLayout, T precision) or null, made from the terms or
+  // from the FE field of a coupled simulator (fe_pv > 0: its lattice degree)
+  const void* tab;
   int fe_pv;
-  const void* tab_q;
-  const void* tab_f;
-  long long tab_foff[3], tab_nf[3];
 };
 // stage kernel of this velocity: separable-operator kernel when optab is set
 inline bool use_sep_kernel(const VelDev& v) { return v.sep1 && v.optab != nullptr; }
@@ -191,16 +182,15 @@ int launch_static_cfl(const Ctx& c, const double* vtab64, int n_terms, const int
                       int npt, DevClock* clk);
 // static CFL part of an FE velocity lattice (FP64, degree pv), max-ed into clk->vd_static
 int launch_fe_static_cfl(const Ctx& c, const double* u64, int pv, DevClock* clk);
-// the spatial part of a sum of separable terms (FP64 term tables of
-// build_vtab, terms sorted by component) at every cell's QGauss(p+2) points
-// and every face's, in the state precision (layouts of VelArgs::tab_q / tab_f)
+// bytes of a velocity table (VelTabLayout)
+size_t vel_table_bytes(const Ctx& c);
+// the table of a sum of separable terms (FP64 term tables of build_vtab,
+// terms sorted by component), in the state precision
 int launch_vel_tabulate(const Ctx& c, const double* vtab64, int n_terms, const int* comp, int nmax, int npt,
-                        void* tab_q, void* tab_f, const long long* foff, const long long* nf);
-// the FE velocity lattice (FP64, degree pv) at every cell's QGauss(p+2)
-// points and every face's, in the state precision (layouts of VelArgs::
-// tab_q / tab_f); gb[a][q] = Lagrange basis a at Gauss point q
-int launch_fe_tabulate(const Ctx& c, const double* u64, int pv, const double (*gb)[kMaxNQ + 2], void* tab_q,
-                       void* tab_f, const long long* foff, const long long* nf);
+                        void* tab);
+// the table of the FE velocity lattice (FP64, degree pv), in the state
+// precision; gb[a][q] = Lagrange basis a at Gauss point q
+int launch_fe_tabulate(const Ctx& c, const double* u64, int pv, const double (*gb)[kMaxNQ + 2], void* tab);
 // two-level FP64 reduction; partial holds 2 * reduce_blocks(c) doubles,
 // out_dev receives two doubles (sum pair, or max)
 int launch_reduce(const Ctx& c, int which, const void* phi, const void* ref,

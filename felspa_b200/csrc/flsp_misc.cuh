@@ -254,69 +254,83 @@ __global__ void fe_static_cfl_kernel(const MeshArgs m, const double* __restrict_
   }
 }
 
-// terms of each component in a component-sorted term list
 struct VelTerms {
   int cstart[4];
 };
 
-// the spatial part of a sum of separable terms at every cell's quadrature
-// points: one thread per (point, cell), cell fastest; per term the product
-// ((coeff f0) f1) f2 of the term tables' entries, the component's terms in
-// order (the point-wise stage kernel's evaluation), in FP64, stored in T
-template <int DIM, typename T>
-__global__ void vel_tabulate_cells(const MeshArgs m, const double* __restrict__ vtab, int nmax, int npt,
-                                   const VelTerms vt, int nq, T* __restrict__ out) {
-  const int nqd = DIM > 2 ? nq * nq * nq : nq * nq;
-  const long long total = (long long)nqd * m.ncell;
-  auto row = [&](int k, int ax, int i) { return vtab + ((size_t)(k * 3 + ax) * nmax + i) * npt; };
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long cell = i % m.ncell;
-    const int q = (int)(i / m.ncell);
-    const int qx = q % nq, qy = (q / nq) % nq, qz = DIM > 2 ? q / (nq * nq) : 0;
-    const int gx = (int)(cell % m.n[0]), gy = (int)((cell / m.n[0]) % m.n[1]);
-    const int gz = DIM > 2 ? (int)(cell / ((long long)m.n[0] * m.n[1])) : 0;
-    for (int d = 0; d < DIM; ++d) {
-      double u = 0.0;
-      for (int k = vt.cstart[d]; k < vt.cstart[d + 1]; ++k) {
-        double v = row(k, 0, gx)[qx] * row(k, 1, gy)[qy];
-        if (DIM == 3) v = v * row(k, 2, gz)[qz];
-        u += v;
-      }
-      out[((size_t)d * nqd + q) * m.ncell + cell] = T(u);
-    }
+// position of entry i of a velocity table (VelTabLayout): a cell's point
+// (component d, point q, cell g) or a face's (component d = E, point q, face
+// index g over the n + e_E faces); false for entries past the mesh
+template <int DIM>
+__device__ __forceinline__ bool vel_tab_entry(const MeshArgs& m, int nq, long long i, bool& face, int& d, int& q,
+                                              int* g) {
+  using LY = VelTabLayout<DIM>;
+  using TL = HjsTile<DIM>;
+  const int nqd = DIM > 2 ? nq * nq * nq : nq * nq, per = LY::entries(nq);
+  const long long tile = i / per;
+  int r = (int)(i - tile * per);
+  const int ntx = (m.n[0] + TL::X - 1) / TL::X, nty = (m.n[1] + TL::Y - 1) / TL::Y;
+  const int o[3] = {(int)(tile % ntx) * TL::X, (int)((tile / ntx) % nty) * TL::Y,
+                    DIM > 2 ? (int)(tile / ((long long)ntx * nty)) * TL::Z : 0};
+  face = r >= DIM * nqd * TL::N;
+  int ex = TL::X, ey = TL::Y, s;
+  if (!face) {
+    s = r % TL::N;
+    q = (r / TL::N) % nqd;
+    d = r / (TL::N * nqd);
+  } else {
+    r -= DIM * nqd * TL::N;
+    s = r % LY::NFT;
+    q = r / LY::NFT;
+    d = s < LY::S0 ? 0 : (s < LY::S0 + LY::S1 ? 1 : 2);
+    s -= LY::off(d);
+    ex += d == 0;
+    ey += d == 1;
   }
+  g[0] = o[0] + s % ex;
+  g[1] = o[1] + (s / ex) % ey;
+  g[2] = DIM > 2 ? o[2] + s / (ex * ey) : 0;
+  bool in = true;
+#pragma unroll
+  for (int e = 0; e < DIM; ++e) in = in && g[e] < m.n[e] + (face && d == e);
+  return in;
 }
 
-// the normal component E at every face's points: from the lower cell's
-// upper-face entries (the first face: the upper cell's lower-face entries,
-// the same face coordinate bit for bit)
+// the table of a sum of separable terms: ((coeff f0) f1) f2 of the term
+// tables' entries, the component's terms in order, times the quadrature weight
+// over h, in FP64, stored in T; a face from its lower cell's upper-face entries
+// (the first face: the upper cell's lower-face entries, the same face
+// coordinate bit for bit)
 template <int DIM, typename T>
-__global__ void vel_tabulate_faces(const MeshArgs m, const double* __restrict__ vtab, int nmax, int npt,
-                                   const VelTerms vt, int nq, int E, long long nface, T* __restrict__ out) {
-  const int nqf = DIM > 2 ? nq * nq : nq;
-  const int nf0 = m.n[0] + (E == 0), nf1 = m.n[1] + (E == 1);
-  const int t0 = E == 0 ? 1 : 0, t1 = E == 2 ? 1 : 2;
-  const long long total = (long long)nqf * nface;
+__global__ void vel_tabulate(const MeshArgs m, const double* __restrict__ vtab, int nmax, int npt, const VelTerms vt,
+                             int nq, long long total, T* __restrict__ out) {
+  const double* wq = tab<double>(nq - 2).wq;
   auto row = [&](int k, int ax, int i) { return vtab + ((size_t)(k * 3 + ax) * nmax + i) * npt; };
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
-    const long long face = i % nface;
-    const int q = (int)(i / nface);
-    const int q0 = q % nq, q1 = DIM > 2 ? q / nq : 0;
-    const int f[3] = {(int)(face % nf0), (int)((face / nf0) % nf1), DIM > 2 ? (int)(face / ((long long)nf0 * nf1)) : 0};
-    int cidx[3] = {f[0], f[1], f[2]}, j[3] = {0, 0, 0};
-    if (f[E] > 0) { cidx[E] = f[E] - 1; j[E] = nq + 1; }
-    else j[E] = nq;
-    j[t0] = q0;
-    if (DIM > 2) j[t1] = q1;
+    bool face;
+    int d, q, g[3];
+    if (!vel_tab_entry<DIM>(m, nq, i, face, d, q, g)) continue;
+    int j[3] = {0, 0, 0};
+    double w = 1.0 / m.h[d];
+#pragma unroll
+    for (int e = 0; e < DIM; ++e) {
+      if (face && e == d) {
+        if (g[e] > 0) { g[e] -= 1; j[e] = nq + 1; }
+        else j[e] = nq;
+        continue;
+      }
+      j[e] = q % nq;
+      q /= nq;
+      w *= wq[j[e]];
+    }
     double u = 0.0;
-    for (int k = vt.cstart[E]; k < vt.cstart[E + 1]; ++k) {
-      double v = row(k, 0, cidx[0])[j[0]] * row(k, 1, cidx[1])[j[1]];
-      if (DIM == 3) v = v * row(k, 2, cidx[2])[j[2]];
+    for (int k = vt.cstart[d]; k < vt.cstart[d + 1]; ++k) {
+      double v = row(k, 0, g[0])[j[0]] * row(k, 1, g[1])[j[1]];
+      if (DIM == 3) v = v * row(k, 2, g[2])[j[2]];
       u += v;
     }
-    out[(size_t)q * nface + face] = T(u);
+    out[i] = T(u * w);
   }
 }
 
@@ -324,68 +338,112 @@ struct FeBasis {
   double b[kMaxFeVel + 1][kMaxNQ + 2];   // Lagrange basis a at Gauss point q
 };
 
-// FE velocity at every cell's quadrature points: one thread per (point,
-// cell), cell fastest; the cell's nodes times the basis products, summed x
-// fastest, in FP64, stored in T
-template <int DIM, typename T>
-__global__ void fe_tabulate_cells(const MeshArgs m, const double* __restrict__ u, int pv, int nq,
-                                  const FeBasis fb, T* __restrict__ out) {
-  const int nx = pv * m.n[0] + 1, ny = pv * m.n[1] + 1, nz = DIM > 2 ? pv * m.n[2] + 1 : 1;
+// The table of an FE velocity of degree PV, sums over the nodes factorised,
+// FP64, stored in T.  Cells: one thread per (component, plane of points,
+// cell), the plane's sum over the nodes along the last axis, then line by
+// line; a coupled run makes the table anew every outer step (48^3 Q2 FP32,
+// degree 2: 47 us for the cells; 367 us point by point).
+template <int DIM, int P, int PV, typename T>
+__global__ void fe_tabulate_cells(const MeshArgs m, const double* __restrict__ u, const FeBasis fb,
+                                  long long total, T* __restrict__ out) {
+  using LY = VelTabLayout<DIM>;
+  using TL = HjsTile<DIM>;
+  constexpr int NQ = P + 2, NQD = ipow(NQ, DIM), NQF = ipow(NQ, DIM - 1), NB = DIM > 2 ? PV + 1 : 1;
+  const double* wq = tab<double>(P).wq;
+  const int nx = PV * m.n[0] + 1, ny = PV * m.n[1] + 1, nz = DIM > 2 ? PV * m.n[2] + 1 : 1;
   const size_t nn = (size_t)nx * ny * nz;
-  const int nqd = DIM > 2 ? nq * nq * nq : nq * nq;
-  const long long total = (long long)nqd * m.ncell;
+  const int ntx = (m.n[0] + TL::X - 1) / TL::X, nty = (m.n[1] + TL::Y - 1) / TL::Y;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
-    const long long cell = i % m.ncell;
-    const int q = (int)(i / m.ncell);
-    const int qx = q % nq, qy = (q / nq) % nq, qz = DIM > 2 ? q / (nq * nq) : 0;
-    const int gx = (int)(cell % m.n[0]), gy = (int)((cell / m.n[0]) % m.n[1]);
-    const int gz = DIM > 2 ? (int)(cell / ((long long)m.n[0] * m.n[1])) : 0;
-    double acc[3] = {0.0, 0.0, 0.0};
-    for (int cz = 0; cz <= (DIM > 2 ? pv : 0); ++cz)
-      for (int cy = 0; cy <= pv; ++cy) {
-        double byz = fb.b[cy][qy];
-        if (DIM > 2) byz *= fb.b[cz][qz];
-        for (int cx = 0; cx <= pv; ++cx) {
-          const double b = fb.b[cx][qx] * byz;
-          const size_t node = ((size_t)(pv * gz + cz) * ny + pv * gy + cy) * nx + pv * gx + cx;
-          for (int d = 0; d < DIM; ++d) acc[d] += u[d * nn + node] * b;
+    const int cl = (int)(i % TL::N), k = (int)(i / TL::N % NQ), d = (int)(i / (TL::N * NQ) % DIM);
+    const long long tile = i / ((long long)TL::N * NQ * DIM);
+    const int g[3] = {(int)(tile % ntx) * TL::X + cl % TL::X, (int)(tile / ntx % nty) * TL::Y + cl / TL::X % TL::Y,
+                      DIM > 2 ? (int)(tile / ((long long)ntx * nty)) * TL::Z + cl / (TL::X * TL::Y) : 0};
+    if (g[0] >= m.n[0] || g[1] >= m.n[1] || (DIM > 2 && g[2] >= m.n[2])) continue;
+    const double* un = u + d * nn + ((size_t)(PV * g[2]) * ny + PV * g[1]) * nx + PV * g[0];
+    const size_t sl = DIM > 2 ? (size_t)ny * nx : nx;   // node stride along the last axis
+    double V[NB][PV + 1];
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int a = 0; a <= PV; ++a) {
+        double s = 0.0;
+#pragma unroll
+        for (int c = 0; c <= PV; ++c) s += un[c * sl + (size_t)b * nx + a] * fb.b[c][k];
+        V[b][a] = s;
+      }
+    const double wk = wq[k] / m.h[d];
+    T* o = out + (size_t)tile * LY::template entries<NQ>() + ((size_t)d * NQD + (size_t)k * NQF) * TL::N + cl;
+#pragma unroll
+    for (int qy = 0; qy < (DIM > 2 ? NQ : 1); ++qy) {
+      double x[PV + 1];
+#pragma unroll
+      for (int a = 0; a <= PV; ++a) {
+        x[a] = V[0][a];
+        if constexpr (DIM > 2) {
+          x[a] *= fb.b[0][qy];
+#pragma unroll
+          for (int b = 1; b < NB; ++b) x[a] += V[b][a] * fb.b[b][qy];
         }
       }
-    for (int d = 0; d < DIM; ++d) out[((size_t)d * nqd + q) * m.ncell + cell] = T(acc[d]);
+      const double w = DIM > 2 ? wk * wq[qy] : wk;
+#pragma unroll
+      for (int qx = 0; qx < NQ; ++qx) {
+        double s = 0.0;
+#pragma unroll
+        for (int a = 0; a <= PV; ++a) s += x[a] * fb.b[a][qx];
+        o[(size_t)(qx + NQ * qy) * TL::N] = T(s * (w * wq[qx]));
+      }
+    }
   }
 }
 
 // the normal component at every face's quadrature points, from the face's
-// own nodes (the basis of the others vanishes on it): one value per face
-template <int DIM, typename T>
-__global__ void fe_tabulate_faces(const MeshArgs m, const double* __restrict__ u, int pv, int nq,
-                                  const FeBasis fb, int E, long long nface, T* __restrict__ out) {
-  const int nx = pv * m.n[0] + 1, ny = pv * m.n[1] + 1, nz = DIM > 2 ? pv * m.n[2] + 1 : 1;
+// own nodes (the basis of the others vanishes on it): the same value in both
+// tiles of a face
+template <int DIM, int P, int PV, typename T>
+__global__ void fe_tabulate_faces(const MeshArgs m, const double* __restrict__ u, const FeBasis fb,
+                                  long long total, T* __restrict__ out) {
+  using LY = VelTabLayout<DIM>;
+  using TL = HjsTile<DIM>;
+  constexpr int NQ = P + 2, NQD = ipow(NQ, DIM), N1B = DIM > 2 ? PV + 1 : 1;
+  const double* wq = tab<double>(P).wq;
+  const int nx = PV * m.n[0] + 1, ny = PV * m.n[1] + 1, nz = DIM > 2 ? PV * m.n[2] + 1 : 1;
   const size_t nn = (size_t)nx * ny * nz;
-  const int nqf = DIM > 2 ? nq * nq : nq;
-  const int nf0 = m.n[0] + (E == 0), nf1 = m.n[1] + (E == 1);
-  const int t0 = E == 0 ? 1 : 0, t1 = E == 2 ? 1 : 2;
-  const long long total = (long long)nqf * nface;
+  const size_t st[3] = {1, (size_t)nx, (size_t)nx * ny};
+  const int ntx = (m.n[0] + TL::X - 1) / TL::X, nty = (m.n[1] + TL::Y - 1) / TL::Y;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
-    const long long face = i % nface;
-    const int q = (int)(i / nface);
-    const int q0 = q % nq, q1 = DIM > 2 ? q / nq : 0;
-    const int f[3] = {(int)(face % nf0), (int)((face / nf0) % nf1), DIM > 2 ? (int)(face / ((long long)nf0 * nf1)) : 0};
-    double acc = 0.0;
-    for (int c1 = 0; c1 <= (DIM > 2 ? pv : 0); ++c1)
-      for (int c0 = 0; c0 <= pv; ++c0) {
-        double b = fb.b[c0][q0];
-        if (DIM > 2) b *= fb.b[c1][q1];
-        int node[3];
-        node[E] = pv * f[E];
-        node[t0] = pv * f[t0] + c0;
-        if (DIM > 2) node[t1] = pv * f[t1] + c1;
-        else node[2] = 0;
-        acc += u[E * nn + ((size_t)node[2] * ny + node[1]) * nx + node[0]] * b;
-      }
-    out[(size_t)q * nface + face] = T(acc);
+    int s = (int)(i % LY::NFT);
+    const int q1 = (int)(i / LY::NFT % (DIM > 2 ? NQ : 1));
+    const long long tile = i / ((long long)LY::NFT * (DIM > 2 ? NQ : 1));
+    T* o = out + (size_t)tile * LY::template entries<NQ>() + (size_t)DIM * NQD * TL::N + (size_t)NQ * q1 * LY::NFT + s;
+    const int E = s < LY::S0 ? 0 : (s < LY::S0 + LY::S1 ? 1 : 2);
+    s -= LY::off(E);
+    const int ex = TL::X + (E == 0), ey = TL::Y + (E == 1);
+    const int g[3] = {(int)(tile % ntx) * TL::X + s % ex, (int)(tile / ntx % nty) * TL::Y + s / ex % ey,
+                      DIM > 2 ? (int)(tile / ((long long)ntx * nty)) * TL::Z + s / (ex * ey) : 0};
+    bool in = true;
+#pragma unroll
+    for (int e = 0; e < DIM; ++e) in = in && g[e] < m.n[e] + (E == e);
+    if (!in) continue;
+    const int t0 = E == 0 ? 1 : 0, t1 = E == 2 ? 1 : 2;
+    const double* un = u + E * nn + PV * (g[0] * st[0] + g[1] * st[1] + g[2] * st[2]);
+    const double w = DIM > 2 ? wq[q1] / m.h[E] : 1.0 / m.h[E];
+    double x[PV + 1];
+#pragma unroll
+    for (int a = 0; a <= PV; ++a) {
+      x[a] = 0.0;
+#pragma unroll
+      for (int b = 0; b < N1B; ++b) x[a] += un[a * st[t0] + b * st[t1]] * (DIM > 2 ? fb.b[b][q1] : 1.0);
+    }
+#pragma unroll
+    for (int q0 = 0; q0 < NQ; ++q0) {
+      double v = 0.0;
+#pragma unroll
+      for (int a = 0; a <= PV; ++a) v += x[a] * fb.b[a][q0];
+      o[(size_t)q0 * LY::NFT] = T(v * (w * wq[q0]));
+    }
   }
 }
 
