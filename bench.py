@@ -390,7 +390,8 @@ def run_ours(args):
                 "stage_tile": list(tile),
                 "stage_tile_ms": {"x".join(map(str, k)): v for k, v in tile_ms.items()}}
 
-    per_step_launches = REINIT_EVERY * 5 + 2 + 3 * N_PSEUDO
+    # a period: the substeps' clock, three stages each, the reinit's reset and CFL pass, its pseudo-steps
+    per_step_launches = 1 + 3 * REINIT_EVERY + 2 + N_PSEUDO
     if rank != 0:
         if dist:
             dist.destroy_process_group()

@@ -26,10 +26,10 @@ struct AdvArgs {
   const T* __restrict__ phi_s;   // stage input (read with halo)
   const T* __restrict__ phi_n;   // phi^n for the combinations
   T* __restrict__ out;
-  const DevClock* clk;
-  int stage;                      // index into clk->ct
+  const AdvStep* step;            // the substep (null: explicit)
+  int stage;                      // index into step->ct
   int combine;                    // CombineMode
-  double ct_explicit;             // time factor when clk == nullptr
+  double ct_explicit;             // time factor when step == nullptr
   double dt_explicit;
 };
 
@@ -207,9 +207,9 @@ __global__ void __launch_bounds__(256, 2) adv_stage_kernel(const AdvArgs<T> a) {
   cp_async_wait_all();
   __syncthreads();
 
-  const T ct = a.clk ? T(a.clk->ct[a.stage]) : T(a.ct_explicit);
-  const T dt = a.clk ? T(a.clk->dt) : T(a.dt_explicit);
-  const bool active = a.clk ? (a.clk->active != 0) : true;
+  const T ct = a.step ? T(a.step->ct[a.stage]) : T(a.ct_explicit);
+  const T dt = a.step ? T(a.step->dt) : T(a.dt_explicit);
+  const bool active = a.step ? (a.step->active != 0) : true;
   const int cl = tc.lx + tx * (tc.ly + ty * tc.lz);
   const int me = box_index(m, DIM, tc.lx, tc.ly, tc.lz);
   const T ih[3] = {T(1.0 / m.h[0]), T(1.0 / m.h[1]), T(DIM > 2 ? 1.0 / m.h[2] : 1.0)};

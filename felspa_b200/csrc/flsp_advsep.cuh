@@ -64,8 +64,8 @@ struct AdvSepArgs {
   const T* __restrict__ phi_s;
   const T* __restrict__ phi_n;
   T* __restrict__ out;
-  const DevClock* clk;
-  int stage;
+  const AdvStep* step;           // the substep (null: explicit)
+  int stage;                     // index into step->ct
   int combine;
   double ct_explicit;
   double dt_explicit;
@@ -297,9 +297,9 @@ __global__ void __launch_bounds__(TX * TY * TZ, sizeof(T) == 4 ? 2 : 1)
     mbar_wait(bar, 0, 1 << 22);   // give copies in flight a last chance to land
   }
 
-  const T ct = a.clk ? T(a.clk->ct[a.stage]) : T(a.ct_explicit);
-  const T dt = a.clk ? T(a.clk->dt) : T(a.dt_explicit);
-  const bool active = a.clk ? (a.clk->active != 0) : true;
+  const T ct = a.step ? T(a.step->ct[a.stage]) : T(a.ct_explicit);
+  const T dt = a.step ? T(a.step->dt) : T(a.dt_explicit);
+  const bool active = a.step ? (a.step->active != 0) : true;
   const int cl = threadIdx.x;
   const T ih[3] = {T(1.0 / m.h[0]), T(1.0 / m.h[1]), T(DIM > 2 ? 1.0 / m.h[2] : 1.0)};
   const bool work = valid && active;

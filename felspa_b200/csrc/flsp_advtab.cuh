@@ -37,10 +37,10 @@ struct AdvTabArgs {
   const T* __restrict__ phi_s;   // stage input (read with halo)
   const T* __restrict__ phi_n;   // phi^n for the combinations
   T* __restrict__ out;
-  const DevClock* clk;
-  int stage;                     // index into clk->ct
+  const AdvStep* step;           // the substep (null: explicit)
+  int stage;                     // index into step->ct
   int combine;                   // CombineMode
-  double ct_explicit, dt_explicit;   // when clk == nullptr
+  double ct_explicit, dt_explicit;   // when step == nullptr
   int* err;                      // device error word (DevClock::err) or null
 };
 
@@ -106,9 +106,9 @@ __device__ __forceinline__ void adv_tab_tile(const AdvTabArgs<T>& a, int tile) {
     const unsigned phase = ((rowcell + (unsigned)gx0) * (unsigned)NMB) & 15u;
     return reinterpret_cast<const T*>(boxb + (size_t)rr * PL::SLOT + phase + (o[0] + lx - gx0) * NMB);
   };
-  const T ct = a.clk ? T(a.clk->ct[a.stage]) : T(a.ct_explicit);
-  const T dt = a.clk ? T(a.clk->dt) : T(a.dt_explicit);
-  const bool active = a.clk ? (a.clk->active != 0) : true;
+  const T ct = a.step ? T(a.step->ct[a.stage]) : T(a.ct_explicit);
+  const T dt = a.step ? T(a.step->dt) : T(a.dt_explicit);
+  const bool active = a.step ? (a.step->active != 0) : true;
   const T* tabc = a.tab + (size_t)tile * LY::template entries<NQ>();   // the tile's cells
   const T* tabf = tabc + (size_t)DIM * NQD * NT;                       // and faces
   T Lk[N1];

@@ -137,6 +137,7 @@ struct flsp_handle {
   bool tab_ok = false;
   DevClock* clk = nullptr;
   DevClock* clk_host = nullptr;   // pinned mirror
+  AdvStep* steps = nullptr;       // the clock's next substeps (kClockSteps)
   int64_t* perm = nullptr;
   double* stage64 = nullptr;      // FP64 device staging (2 * dim * ndofs)
   double* partial = nullptr;
@@ -318,14 +319,13 @@ int other(int a, int b) {  // the buffer index that is neither a nor b
   return -1;
 }
 
-int stage(flsp_handle* h, const void* in, const void* phin, void* out, int st, int combine) {
-  return launch_adv_stage(h->ctx(), h->veldev(), in, phin, out, h->clk, st, combine, 0.0, h->adv_tile);
+int stage(flsp_handle* h, const void* in, const void* phin, void* out, const AdvStep* step, int st, int combine) {
+  return launch_adv_stage(h->ctx(), h->veldev(), in, phin, out, step, st, combine, 0.0, h->adv_tile);
 }
 
-// one SSP-RK substep on the device clock (no host synchronisation)
 // step_count: a step-count run (flsp_advance_steps, graph periods) rather
 // than a call for a time step (flsp_advance, the reference's advance_time)
-int enqueue_adv_step(flsp_handle* h, bool step_count = true) {
+AdvClockArgs clock_args(const flsp_handle* h, bool step_count) {
   AdvClockArgs ca;
   ca.cfl_max = h->cfl_max;
   ca.scale = adv_cfl_scaling(h->p);
@@ -334,25 +334,44 @@ int enqueue_adv_step(flsp_handle* h, bool step_count = true) {
   ca.tb = h->vel.tb;
   ca.rk = h->rk;
   ca.step_count = step_count ? 1 : 0;
-  ST(launch_adv_clock_begin(h->stream, h->clk, ca));
+  return ca;
+}
+
+// the stages of one SSP-RK substep
+int enqueue_adv_stages(flsp_handle* h, const AdvStep* step) {
   const int x = h->cur, y = (h->cur + 1) % 3, z = (h->cur + 2) % 3;
   void* X = h->buf[x];
   void* Y = h->buf[y];
   void* Z = h->buf[z];
   if (h->rk == 1) {
-    ST(stage(h, X, X, Y, 0, kRK1));
+    ST(stage(h, X, X, Y, step, 0, kRK1));
     h->cur = y;
   } else if (h->rk == 2) {
-    ST(stage(h, X, X, Y, 0, kRK2a));
-    ST(stage(h, Y, X, Z, 1, kRK2b));
+    ST(stage(h, X, X, Y, step, 0, kRK2a));
+    ST(stage(h, Y, X, Z, step, 1, kRK2b));
     h->cur = z;
   } else {
-    ST(stage(h, X, X, Y, 0, kRK3a));
-    ST(stage(h, Y, X, Z, 1, kRK3b));
-    ST(stage(h, Z, X, Y, 2, kRK3c));
+    ST(stage(h, X, X, Y, step, 0, kRK3a));
+    ST(stage(h, Y, X, Z, step, 1, kRK3b));
+    ST(stage(h, Z, X, Y, step, 2, kRK3c));
     h->cur = y;
   }
-  return launch_adv_clock_end(h->stream, h->clk);
+  return FLSP_OK;
+}
+
+// n SSP-RK substeps on the device clock (no host synchronisation): the clock
+// of up to kClockSteps substeps in one launch, then their stages (two clock
+// launches a substep were 4 of 22 us of a 256^2 degree-2 substep).  The
+// launch before has read its steps when the next clock launch writes them.
+int enqueue_adv_steps(flsp_handle* h, int n, bool step_count = true, double horizon = -1.0) {
+  for (int done = 0; done < n;) {
+    const int k = std::min(n - done, kClockSteps);
+    ST(launch_adv_clock_steps(h->stream, h->clk, clock_args(h, step_count), h->steps, k, true,
+                              done == 0 ? horizon : -1.0));
+    for (int i = 0; i < k; ++i) ST(enqueue_adv_stages(h, h->steps + i));
+    done += k;
+  }
+  return FLSP_OK;
 }
 
 bool reinit_limiter(const flsp_handle* h, const flsp_reinit_opts* o) {
@@ -360,10 +379,23 @@ bool reinit_limiter(const flsp_handle* h, const flsp_reinit_opts* o) {
   return o->limiter < 0 ? true : o->limiter != 0;
 }
 
-// one reinitialisation pseudo-step: reads cur and phi0, writes a free buffer
-int enqueue_hj_step(flsp_handle* h, const flsp_reinit_opts* o, int phi0_idx, bool limiter) {
-  ST(launch_hj_clock_begin(h->stream, h->clk, o->cfl_max, h->p, o->viscosity, h->m.min_diam,
-                           adv_cfl_scaling(h->p)));
+// the clock of pseudo-step k (HJSimulator::cfl_scaling, hamilton_jacobi.cc:554-580)
+HjClockArgs hj_clock_args(const flsp_handle* h, const flsp_reinit_opts* o, int k) {
+  HjClockArgs a;
+  a.cfl_max = o->cfl_max;
+  a.scale = adv_cfl_scaling(h->p);
+  a.shift = 0.0;
+  if (o->viscosity > 0.0) {
+    a.scale = std::pow((double)(h->p + 1), 2.0);
+    a.shift = o->viscosity * std::pow((double)(h->p + 1), 4.0) / std::pow(h->m.min_diam, 2.0);
+  }
+  a.k = k;
+  return a;
+}
+
+// reinitialisation pseudo-step k: reads cur and phi0, writes a free buffer
+int enqueue_hj_step(flsp_handle* h, const flsp_reinit_opts* o, int phi0_idx, bool limiter, int k) {
+  const HjClockArgs step = hj_clock_args(h, o, k);
   const int src = h->cur;
   const int dst = (src == phi0_idx) ? (phi0_idx + 1) % 3 : other(src, phi0_idx);
   const void* rdiff = nullptr;
@@ -372,7 +404,7 @@ int enqueue_hj_step(flsp_handle* h, const flsp_reinit_opts* o, int phi0_idx, boo
     ST(launch_ldg(h->ctx(), h->qbuf, h->rdiff, h->ndofs, o->viscosity, 1));
     rdiff = h->rdiff;
   }
-  ST(launch_hj(h->ctx(), h->buf[src], h->buf[phi0_idx], h->buf[dst], h->clk, kHJStep, o->rk_order, 0.0,
+  ST(launch_hj(h->ctx(), h->buf[src], h->buf[phi0_idx], h->buf[dst], h->clk, kHJStep, o->rk_order, &step,
                h->ndofs, h->hj_tile, rdiff));
   int res = dst;
   if (limiter) {
@@ -381,7 +413,7 @@ int enqueue_hj_step(flsp_handle* h, const flsp_reinit_opts* o, int phi0_idx, boo
     res = lim;
   }
   h->cur = res;
-  return launch_hj_clock_end(h->stream, h->clk);
+  return FLSP_OK;
 }
 
 int reduce_dev(flsp_handle* h, int which, const void* phi, const void* ref, bool with_ic, double* out2) {
@@ -510,11 +542,11 @@ int run_reinit(flsp_handle* h, const flsp_reinit_opts* o, int* n_iter, const Swe
   auto sweep = [&]() -> int {
     ST(launch_hj_clock_reset(h->stream, h->clk));
     // CFL estimate of the first pseudo-step: gradients of the initial state
-    ST(launch_hj(h->ctx(), h->buf[phi0], h->buf[phi0], nullptr, h->clk, kHJCflOnly, o->rk_order, 0.0,
+    ST(launch_hj(h->ctx(), h->buf[phi0], h->buf[phi0], nullptr, h->clk, kHJCflOnly, o->rk_order, nullptr,
                  h->ndofs, h->hj_tile));
     int it = 0;
     if (o->mode == FLSP_REINIT_FIXED) {
-      for (it = 0; it < o->n_pseudo_steps; ++it) ST(enqueue_hj_step(h, o, phi0, limiter));
+      for (it = 0; it < o->n_pseudo_steps; ++it) ST(enqueue_hj_step(h, o, phi0, limiter, it));
     } else {
       double horizon;
       if (o->mode == FLSP_REINIT_GLOBAL) {
@@ -526,7 +558,7 @@ int run_reinit(flsp_handle* h, const flsp_reinit_opts* o, int* n_iter, const Swe
       }
       double cum = 0.0;
       while (cum < horizon && it <= o->max_iter) {
-        ST(enqueue_hj_step(h, o, phi0, limiter));
+        ST(enqueue_hj_step(h, o, phi0, limiter, it));
         ++it;
         ST(sync_clock(h));
         cum = h->clk_host->hj_cum;
@@ -1002,6 +1034,7 @@ int flsp_create(const flsp_mesh_desc* mesh, const flsp_dg_opts* opts, flsp_handl
       return cleanup_fail(fail(FLSP_ERR_OOM, "state allocation failed"));
   if (cudaMalloc(&h->clk, sizeof(DevClock)) != cudaSuccess ||
       cudaMallocHost(&h->clk_host, sizeof(DevClock)) != cudaSuccess ||
+      cudaMalloc(&h->steps, kClockSteps * sizeof(AdvStep)) != cudaSuccess ||
       cudaMalloc(&h->stage64, sizeof(double) * (size_t)h->ndofs * 2 * h->dim) != cudaSuccess ||
       cudaMalloc(&h->red_out, 2 * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&h->ic_dev, sizeof(flsp_ic_desc)) != cudaSuccess ||
@@ -1068,6 +1101,7 @@ void flsp_destroy(flsp_handle* h) {
   if (h->lrn_ev) cudaEventDestroy(h->lrn_ev);
   if (h->clk) cudaFree(h->clk);
   if (h->clk_host) cudaFreeHost(h->clk_host);
+  if (h->steps) cudaFree(h->steps);
   if (h->perm) cudaFree(h->perm);
   if (h->curv) cudaFree(h->curv);
   if (h->bc_dev) cudaFree(h->bc_dev);
@@ -1433,11 +1467,10 @@ int flsp_advance(flsp_handle* h, double time_step, int single_cycle, double* adv
   if (!h->has_vel) return fail(FLSP_ERR_BAD_ARG, "velocity not set");
   if (!(time_step >= 0.0) || !std::isfinite(time_step)) return fail(FLSP_ERR_BAD_ARG, "bad time step");
   CU(cudaSetDevice(h->dev));
-  ST(launch_adv_clock_horizon(h->stream, h->clk, time_step));
   double cum = 0.0;
   long long guard = 0;
   do {
-    ST(enqueue_adv_step(h, false));
+    ST(enqueue_adv_steps(h, 1, false, guard == 0 ? time_step : -1.0));
     ST(sync_clock(h));
     cum = h->clk_host->scratch[1];
     if (!std::isfinite(h->clk_host->dt)) return fail(FLSP_ERR_NONFINITE, "non-finite time step");
@@ -1456,7 +1489,7 @@ int flsp_advance_steps(flsp_handle* h, int n_steps, double t_end) {
   ST(sync_clock(h));
   const double horizon = std::isfinite(t_end) ? t_end - h->clk_host->t : INFINITY;
   ST(launch_adv_clock_horizon(h->stream, h->clk, horizon));
-  for (int i = 0; i < n_steps; ++i) ST(enqueue_adv_step(h));
+  ST(enqueue_adv_steps(h, n_steps));
   CU(cudaStreamSynchronize(h->stream));
   return FLSP_OK;
 }
@@ -1475,7 +1508,7 @@ int flsp_hj_gradients(flsp_handle* h, double* grads, int64_t n) {
   CU(cudaSetDevice(h->dev));
   void* tmp = nullptr;
   CU(cudaMalloc(&tmp, (size_t)n * h->tsize));
-  int st = launch_hj(h->ctx(), h->buf[h->cur], h->buf[h->cur], tmp, nullptr, kHJGradients, 1, 0.0,
+  int st = launch_hj(h->ctx(), h->buf[h->cur], h->buf[h->cur], tmp, nullptr, kHJGradients, 1, nullptr,
                      h->ndofs, h->hj_tile);
   for (int b = 0; b < 2 * h->dim && st == FLSP_OK; ++b)
     st = launch_gather(h->ctx(), (const char*)tmp + (size_t)b * h->ndofs * h->tsize,
@@ -1531,7 +1564,7 @@ int flsp_ls_advance(flsp_handle* h, const flsp_ls_opts* o, double time_step, int
 // one reinit period on the handle's stream: `steps` advection substeps, then
 // the fixed-count reinit (graph-capturable; band buffers allocated before)
 int enqueue_period(flsp_handle* h, const flsp_reinit_opts* ro, int steps) {
-  for (int s = 0; s < steps; ++s) ST(enqueue_adv_step(h));
+  ST(enqueue_adv_steps(h, steps));
   const bool limiter = reinit_limiter(h, ro);
   const int phi0 = h->cur;
   if (ro->narrow_band) {
@@ -1543,9 +1576,9 @@ int enqueue_period(flsp_handle* h, const flsp_reinit_opts* ro, int steps) {
   }
   int st = launch_hj_clock_reset(h->stream, h->clk);
   if (st == FLSP_OK)
-    st = launch_hj(h->ctx(), h->buf[phi0], h->buf[phi0], nullptr, h->clk, kHJCflOnly, ro->rk_order, 0.0,
+    st = launch_hj(h->ctx(), h->buf[phi0], h->buf[phi0], nullptr, h->clk, kHJCflOnly, ro->rk_order, nullptr,
                    h->ndofs, h->hj_tile);
-  for (int k = 0; k < ro->n_pseudo_steps && st == FLSP_OK; ++k) st = enqueue_hj_step(h, ro, phi0, limiter);
+  for (int k = 0; k < ro->n_pseudo_steps && st == FLSP_OK; ++k) st = enqueue_hj_step(h, ro, phi0, limiter, k);
   if (ro->narrow_band) {
     const int st2 = band_end(h, phi0);
     if (st == FLSP_OK) st = st2;
@@ -1605,7 +1638,7 @@ int flsp_ls_run_steps(flsp_handle* h, const flsp_ls_opts* o, int n_steps) {
       h->n_since_reinit = 0;
     } else {
       const int k = std::min(to_reinit, n_steps - done);
-      for (int s = 0; s < k; ++s) ST(enqueue_adv_step(h));
+      ST(enqueue_adv_steps(h, k));
       done += k;
       h->n_since_reinit += k;
     }
@@ -1632,22 +1665,16 @@ int flsp_time_kernel(flsp_handle* h, int which, int reps, double* ms_per_launch)
   CU(cudaStreamSynchronize(h->stream));
   const int x = h->cur, y = (h->cur + 1) % 3, z = (h->cur + 2) % 3;
   if (which == 0) {
-    // a valid substep on the clock (idempotent: the CFL maximum is a max)
-    AdvClockArgs ca;
-    ca.cfl_max = h->cfl_max;
-    ca.scale = adv_cfl_scaling(h->p);
-    ca.tkind = h->vel.time_kind;
-    ca.ta = h->vel.ta;
-    ca.tb = h->vel.tb;
-    ca.rk = h->rk;
-    ca.step_count = 1;
-    ST(launch_adv_clock_horizon(h->stream, h->clk, INFINITY));
-    ST(launch_adv_clock_begin(h->stream, h->clk, ca));
+    // a valid substep (the clock itself stays; the CFL maximum is a max)
+    ST(launch_adv_clock_steps(h->stream, h->clk, clock_args(h, true), h->steps, 1, false, INFINITY));
   } else {
     ST(launch_hj_clock_reset(h->stream, h->clk));
     // the pseudo-steps' smooth-sign table (phi0 = the timed input)
-    ST(launch_hj(h->ctx(), h->buf[x], h->buf[x], nullptr, h->clk, kHJCflOnly, 1, 0.0, h->ndofs, h->hj_tile));
+    ST(launch_hj(h->ctx(), h->buf[x], h->buf[x], nullptr, h->clk, kHJCflOnly, 1, nullptr, h->ndofs, h->hj_tile));
   }
+  flsp_reinit_opts ro;
+  fill_reinit_defaults(&ro);
+  const HjClockArgs hs = hj_clock_args(h, &ro, 0);
   cudaEvent_t e0, e1;
   CU(cudaEventCreate(&e0));
   CU(cudaEventCreate(&e1));
@@ -1658,11 +1685,11 @@ int flsp_time_kernel(flsp_handle* h, int which, int reps, double* ms_per_launch)
     const int n = pass == 0 ? 1 : reps;
     for (int r = 0; r < n && st == FLSP_OK; ++r) {
       if (which == 0) {
-        st = stage(h, h->buf[x], h->buf[x], h->buf[y], 0, kRK3a);
-        if (st == FLSP_OK) st = stage(h, h->buf[y], h->buf[x], h->buf[z], 1, kRK3b);
-        if (st == FLSP_OK) st = stage(h, h->buf[z], h->buf[x], h->buf[y], 2, kRK3c);
+        st = stage(h, h->buf[x], h->buf[x], h->buf[y], h->steps, 0, kRK3a);
+        if (st == FLSP_OK) st = stage(h, h->buf[y], h->buf[x], h->buf[z], h->steps, 1, kRK3b);
+        if (st == FLSP_OK) st = stage(h, h->buf[z], h->buf[x], h->buf[y], h->steps, 2, kRK3c);
       } else {
-        st = launch_hj(h->ctx(), h->buf[x], h->buf[x], h->buf[y], h->clk, kHJStep, 1, 0.0, h->ndofs,
+        st = launch_hj(h->ctx(), h->buf[x], h->buf[x], h->buf[y], h->clk, kHJStep, 1, &hs, h->ndofs,
                        h->hj_tile);
       }
     }
@@ -1893,8 +1920,7 @@ int flsp_ls_run_steps_learned(flsp_handle* h, flsp_mlp* net, const flsp_learned_
         const int cur0 = h->cur;
         cudaGraph_t g = nullptr;
         CU(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        int st = FLSP_OK;
-        for (int s = 0; s < to_reinit && st == FLSP_OK; ++s) st = enqueue_adv_step(h);
+        int st = enqueue_adv_steps(h, to_reinit);
         if (st == FLSP_OK && fb) {
           st = enqueue_learned_fallback(h, net, o);
         } else if (st == FLSP_OK) {
@@ -1919,7 +1945,7 @@ int flsp_ls_run_steps_learned(flsp_handle* h, flsp_mlp* net, const flsp_learned_
       h->n_since_reinit = 0;
     } else {
       const int k = n_steps - done;
-      for (int s = 0; s < k; ++s) ST(enqueue_adv_step(h));
+      ST(enqueue_adv_steps(h, k));
       done += k;
       h->n_since_reinit += k;
     }
@@ -2014,6 +2040,7 @@ int batch_build(flsp_batch* b, const int* adv_tile, const int* hj_tile) {
     set_tile(q.m_weno, 2, kWenoTile);
     for (int k = 0; k < 3; ++k) q.buf[k] = h->buf[k];
     q.clk = h->clk;
+    q.steps = h->steps;
     if (!h->tab_ok) return fail(FLSP_ERR_BAD_ARG, "batched problem without velocity tables");
     q.tab = h->tab;
     q.stab = h->hj_stab;
@@ -2119,7 +2146,7 @@ int batch_adv_all(flsp_batch* b, int in, int pn, int out, int stage, int combine
   return batch_each_degree(b, kBatchKindAdv, [&](int p, cudaStream_t s) {
     return launch_batch_adv(s, b->prec, p, b->probs, b->items_adv + b->deg_off[kBatchKindAdv][p],
                             b->deg_cnt[kBatchKindAdv][p], b->deg_grid[kBatchKindAdv][p], b->deg_thr[kBatchKindAdv][p],
-                            b->deg_smem[kBatchKindAdv][p], in, pn, out, stage, combine);
+                            b->deg_smem[kBatchKindAdv][p], in, pn, out, 0, stage, combine);
   });
 }
 
@@ -2127,7 +2154,7 @@ int batch_hj_all(flsp_batch* b, int src, int phi0, int dst, int mode, int rk) {
   return batch_each_degree(b, kBatchKindHJ, [&](int p, cudaStream_t s) {
     return launch_batch_hj(s, b->prec, p, b->probs, b->items_hj + b->deg_off[kBatchKindHJ][p],
                            b->deg_cnt[kBatchKindHJ][p], b->deg_grid[kBatchKindHJ][p], b->deg_thr[kBatchKindHJ][p],
-                           b->deg_smem[kBatchKindHJ][p], src, phi0, dst, mode, rk);
+                           b->deg_smem[kBatchKindHJ][p], src, phi0, dst, mode, rk, 0.2, 0);
   });
 }
 
@@ -2139,41 +2166,41 @@ int batch_chain(flsp_batch* b, int p, cudaStream_t s, int steps, const flsp_rein
   const BatchProb* probs = b->probs + b->prob_off[p];
   const int np = b->prob_cnt[p];
   const int kA = kBatchKindAdv, kH = kBatchKindHJ, kW = kBatchKindWeno;
-  auto stage = [&](int in, int pn, int out, int k, int comb) {
+  auto stage = [&](int in, int pn, int out, int step, int k, int comb) {
     return launch_batch_adv(s, b->prec, p, b->probs, b->items_adv + b->deg_off[kA][p], b->deg_cnt[kA][p],
-                            b->deg_grid[kA][p], b->deg_thr[kA][p], b->deg_smem[kA][p], in, pn, out, k, comb);
+                            b->deg_grid[kA][p], b->deg_thr[kA][p], b->deg_smem[kA][p], in, pn, out, step, k, comb);
   };
   for (int k = 0; k < steps; ++k) {
-    ST(launch_batch_clock(s, probs, np, kBatchAdvBegin, 0.0));
+    const int at = k % kClockSteps;
+    if (at == 0) ST(launch_batch_clock_steps(s, probs, np, std::min(steps - k, kClockSteps), true));
     const int x = *cur, y = (x + 1) % 3, z = (x + 2) % 3;
     if (b->rk == 1) {
-      ST(stage(x, x, y, 0, kRK1));
+      ST(stage(x, x, y, at, 0, kRK1));
       *cur = y;
     } else if (b->rk == 2) {
-      ST(stage(x, x, y, 0, kRK2a));
-      ST(stage(y, x, z, 1, kRK2b));
+      ST(stage(x, x, y, at, 0, kRK2a));
+      ST(stage(y, x, z, at, 1, kRK2b));
       *cur = z;
     } else {
-      ST(stage(x, x, y, 0, kRK3a));
-      ST(stage(y, x, z, 1, kRK3b));
-      ST(stage(z, x, y, 2, kRK3c));
+      ST(stage(x, x, y, at, 0, kRK3a));
+      ST(stage(y, x, z, at, 1, kRK3b));
+      ST(stage(z, x, y, at, 2, kRK3c));
       *cur = y;
     }
-    ST(launch_batch_clock(s, probs, np, kBatchAdvEnd, 0.0));
   }
   if (!ro) return FLSP_OK;
-  auto hj = [&](int src, int phi0, int dst, int mode) {
+  auto hj = [&](int src, int phi0, int dst, int mode, int k) {
     return launch_batch_hj(s, b->prec, p, b->probs, b->items_hj + b->deg_off[kH][p], b->deg_cnt[kH][p],
-                           b->deg_grid[kH][p], b->deg_thr[kH][p], b->deg_smem[kH][p], src, phi0, dst, mode, ro->rk_order);
+                           b->deg_grid[kH][p], b->deg_thr[kH][p], b->deg_smem[kH][p], src, phi0, dst, mode, ro->rk_order, ro->cfl_max,
+                           k);
   };
   const int phi0 = *cur;
-  ST(launch_batch_clock(s, probs, np, kBatchHjReset, 0.0));
-  ST(hj(phi0, phi0, -1, kHJCflOnly));
+  ST(launch_batch_clock(s, probs, np, kBatchHjReset));
+  ST(hj(phi0, phi0, -1, kHJCflOnly, 0));
   for (int k = 0; k < ro->n_pseudo_steps; ++k) {
-    ST(launch_batch_clock(s, probs, np, kBatchHjBegin, ro->cfl_max));
     const int src = *cur;
     const int dst = (src == phi0) ? (phi0 + 1) % 3 : other(src, phi0);
-    ST(hj(src, phi0, dst, kHJStep));
+    ST(hj(src, phi0, dst, kHJStep, k));
     int res = dst;
     if (limiter) {
       const int lim = other(dst, phi0);
@@ -2183,7 +2210,6 @@ int batch_chain(flsp_batch* b, int p, cudaStream_t s, int steps, const flsp_rein
       res = lim;
     }
     *cur = res;
-    ST(launch_batch_clock(s, probs, np, kBatchHjEnd, 0.0));
   }
   return FLSP_OK;
 }
@@ -2336,7 +2362,7 @@ int flsp_batch_autotune(flsp_batch* b, flsp_batch_tuning* out) {
   int bi = 0;
   for (int c = 0; c < 1; ++c) {
     ST(batch_build(b, ca[c], ch[0]));
-    ST(launch_batch_clock(b->stream, b->probs, (int)b->h.size(), kBatchAdvBegin, 0.0));
+    ST(launch_batch_clock_steps(b->stream, b->probs, (int)b->h.size(), 1, false));
     const int x = b->cur, y = (x + 1) % 3;
     double ms = 0.0;
     ST(time_it([&]() {
@@ -2392,7 +2418,7 @@ int flsp_batch_run_steps(flsp_batch* b, const flsp_ls_opts* o, int n_steps) {
   ST(batch_sync_problems(b));
   const bool limiter = ro.limiter != 0;   // 2D: on unless switched off (reinit.cc:475-478)
   const int n = (int)b->h.size();
-  ST(launch_batch_clock(b->stream, b->probs, n, kBatchAdvHorizon, 0.0));
+  ST(launch_batch_clock(b->stream, b->probs, n, kBatchAdvHorizon));
   int done = 0;
   while (done < n_steps) {
     const int to_reinit = o->execute_reinit ? o->reinit_frequency - b->n_since_reinit : n_steps - done;
@@ -2576,7 +2602,7 @@ int group_run(flsp_group* g, const GroupMode& gm, int n_periods) {
           if (gm.net) {
             // the members' network passes share the network's buffers: they
             // follow one another on its stream (member order)
-            for (int s = 0; s < gm.freq && st == FLSP_OK; ++s) st = enqueue_adv_step(h);
+            st = enqueue_adv_steps(h, gm.freq);
             if (st == FLSP_OK && gm.fallback) {
               st = enqueue_learned_fallback(h, gm.net, gm.lo);
             } else if (st == FLSP_OK) {

@@ -221,14 +221,27 @@ struct DevClock {
   int err;           // device error word (0 = ok)
   // reinitialisation
   double hj_vd_run;  // running max of characteristic speed / diam
-  double hj_dt;      // current pseudo-step
-  double hj_cum;     // accumulated pseudo-time (before the current step)
-  unsigned long long hj_vd_bits;  // atomicMax slot for the next CFL estimate
+  double hj_dt;      // last pseudo-step
+  double hj_cum;     // accumulated pseudo-time
+  // running maxima of the CFL estimate (atomicMax on the bit patterns):
+  // pseudo-step k reads slot k % 3, accumulates slot (k + 1) % 3 and clears
+  // slot (k + 2) % 3
+  unsigned long long hj_vd[3];
   int hj_iter;
   int hj_pending;
   double band_ratio; // accumulated pseudo-time / horizon (host convenience)
   double scratch[4];
 };
+
+// one substep of the advection clock, computed ahead of its stages (the
+// velocity is known in advance, so the clock needs nothing from the field)
+struct AdvStep {
+  double ct[3];      // velocity time factor at the RK stage times
+  double dt, t;      // substep and its start time
+  int active;        // the substep is non-zero
+  int pad;
+};
+constexpr int kClockSteps = 32;   // substeps one clock launch computes at most
 
 // stage combinations of the SSP-RK schemes (time_integration.implement.h:141-234)
 enum CombineMode : int {
@@ -251,6 +264,13 @@ struct AdvClockArgs {
   double ta, tb;
   int rk;
   int step_count;   // 1: a step-count run (the horizon only caps the time)
+};
+
+// reinitialisation clock: pseudo-step k of size cfl_max / (scale vd + shift),
+// vd the running maximum of the CFL estimate
+struct HjClockArgs {
+  double cfl_max, scale, shift;
+  int k;
 };
 
 // time factor kinds (flsp_time_kind)

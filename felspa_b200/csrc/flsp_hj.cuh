@@ -36,7 +36,7 @@ struct HJArgs {
   DevClock* clk;
   int mode;
   int rk;                       // reinit RK order (all stages see the same L)
-  double dt_explicit;           // used when clk == nullptr
+  HjClockArgs step;             // pseudo-step sizes
   long long block;              // gradient block stride (ncell * nb)
   const T* __restrict__ rdiff;  // LDG diffusion RHS per unit volume (nu > 0) or null
   T* stab;                      // smooth-sign table of the tensor-product kernel (hjs_kernel)

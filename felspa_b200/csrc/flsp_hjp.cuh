@@ -38,7 +38,7 @@ struct HjpPlan {
   static constexpr int SLOT = (((TL::X + 2) * NMB + 30) + 15) / 16 * 16;
   static constexpr int NS = ipow(NQ, DIM) + (1 << DIM);
   static constexpr size_t TAB_BYTES = (size_t)NS * TL::N * sizeof(T);
-  static constexpr size_t OFF_BOX = 32;   // mbarrier, CFL maximum
+  static constexpr size_t OFF_BOX = 32;   // mbarrier, CFL maximum, pseudo-step
   static constexpr size_t OFF_GR = OFF_BOX + (size_t)NROWS * SLOT;
   // modal gradients [mean, half difference][axis][mode][cell]; the results'
   // staging at the end
@@ -116,6 +116,7 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjp_min_blocks<DIM,
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem_raw);
   MaxSlot<T>* cfl = reinterpret_cast<MaxSlot<T>*>(smem_raw + 16);
+  double* sdt = reinterpret_cast<double*>(smem_raw + 24);   // the pseudo-step
   unsigned char* boxb = smem_raw + PL::OFF_BOX;
   T* gr = reinterpret_cast<T*>(smem_raw + PL::OFF_GR);    // [2][DIM][NBG][NT]
   T* stl = reinterpret_cast<T*>(smem_raw + PL::OFF_TAB);  // table slice [NS][NT]
@@ -125,7 +126,13 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjp_min_blocks<DIM,
   // part of the launch's tile
   const int sx = m.tile[0] / TX, sy = m.tile[1] / TY, sz = DIM > 2 ? m.tile[2] / TZ : 1;
   const int slot = (int)blockIdx.x / (sx * sy * sz), part = (int)blockIdx.x % (sx * sy * sz);
-  if (tile_inactive(m, slot)) return;
+  const bool step = a.mode == kHJStep, fill = !step;
+  const bool first = blockIdx.x == 0;
+  double vd = 0.0;   // thread 0: the running CFL maximum before this step
+  if (tile_inactive(m, slot)) {
+    if (step && first && threadIdx.x == 0) hj_clock_step(a.clk, a.step, true, vd);
+    return;
+  }
   const int tile = m.tiles ? m.tiles[slot] : slot;
   int o[3];
   {
@@ -137,7 +144,6 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjp_min_blocks<DIM,
   }
   if (o[0] >= m.n[0] || o[1] >= m.n[1] || o[2] >= m.n[2]) return;   // a part past the mesh
   T* const tabp = a.stab + ((size_t)tile * (sx * sy * sz) + part) * NS * NT;
-  const bool step = a.mode == kHJStep, fill = !step;
   if (threadIdx.x == 0) {
     mbar_init(bar, 32 + (step ? 1 : 0));
     *cfl = 0;
@@ -147,6 +153,7 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjp_min_blocks<DIM,
     if (step) {
       mbar_arrive_expect_tx(bar, (unsigned)PL::TAB_BYTES);
       bulk_g2s(stl, tabp, (unsigned)PL::TAB_BYTES, bar);
+      *sdt = hj_clock_step(a.clk, a.step, first, vd);
     }
   }
   if (threadIdx.x < 32) bulk_box_rows<DIM, TX, TY, TZ, NMB, PL::SLOT>(m, a.phi, boxb, o[0], o[1], o[2], bar);
@@ -161,7 +168,6 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjp_min_blocks<DIM,
     const unsigned phase = ((rowcell + (unsigned)gx0) * (unsigned)NMB) & 15u;
     return reinterpret_cast<const T*>(boxb + (size_t)rr * PL::SLOT + phase + (o[0] + lx - gx0) * NMB);
   };
-  const T dt = a.clk ? T(a.clk->hj_dt) : T(a.dt_explicit);
   const T hmin = T(m.min_diam);
   T Lk[N1], Dk[N1];   // this thread's Gauss plane
 #pragma unroll
@@ -288,7 +294,7 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjp_min_blocks<DIM,
   slot_max(cfl, vmax);
   if (!step) {
     __syncthreads();
-    if (threadIdx.x == 0 && a.clk) atomic_max_pos(&a.clk->hj_vd_bits, slot_value(cfl) / m.diam);
+    if (threadIdx.x == 0) atomic_max_pos(&a.clk->hj_vd[0], slot_value(cfl) / m.diam);
     return;
   }
 
@@ -374,7 +380,11 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjp_min_blocks<DIM,
       for (int aa = 0; aa + b < N1; ++aa) ub[(size_t)(k * NQF + aa + N1 * b) * NT + cl] = U[b][aa];
   }
   __syncthreads();   // planes done: the gradients become the store staging
-  if (threadIdx.x == 0 && a.clk) atomic_max_pos(&a.clk->hj_vd_bits, slot_value(cfl) / m.diam);
+  if (threadIdx.x == 0) {   // the running maximum of the next step (the first block has put this one's)
+    const double bm = slot_value(cfl) / m.diam;
+    if (bm > vd) atomic_max_pos(&a.clk->hj_vd[(a.step.k + 1) % 3], bm);
+  }
+  const T dt = T(*sdt);
 
   // -------- (3) columns (a, b) of modes, dealt to the threads of a cell:
   // project over the planes, update, stage

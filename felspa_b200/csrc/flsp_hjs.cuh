@@ -33,6 +33,7 @@
 // narrow band selects among them; the tile index is the global one).
 #pragma once
 #include "flsp_device.cuh"
+#include "flsp_clock.cuh"
 #include "flsp_hj.cuh"
 
 namespace flsp {
@@ -55,7 +56,7 @@ struct HjsPlan {
   static constexpr int BY = TL::Y + 2, BZ = DIM > 2 ? TL::Z + 2 : 1, NROWS = BY * BZ;
   static constexpr int NMB = NM * (int)sizeof(T);   // bytes per cell
   static constexpr int SLOT = (((TL::X + 2) * NMB + 30) + 15) / 16 * 16;
-  static constexpr size_t OFF_BOX = 32;   // mbarrier, CFL maximum
+  static constexpr size_t OFF_BOX = 32;   // mbarrier, CFL maximum, pseudo-step
   static constexpr size_t OFF_JN = OFF_BOX + (size_t)NROWS * SLOT;
   static constexpr size_t OFF_JV = OFF_JN + (size_t)2 * DIM * NQF * TL::N * sizeof(T);
   // the tile's slice of the sign table (pseudo-steps: staged with the box);
@@ -286,11 +287,17 @@ __device__ __forceinline__ void hjs_tile(const HJArgs<T>& a, int slot) {
   T* jn = reinterpret_cast<T*>(smem_raw + PL::OFF_JN);   // [2*DIM*NQF][NT]
   T* jv = reinterpret_cast<T*>(smem_raw + PL::OFF_JV);   // [2*DIM*NC][NT]
   MaxSlot<T>* cfl = reinterpret_cast<MaxSlot<T>*>(smem_raw + 16);
+  double* sdt = reinterpret_cast<double*>(smem_raw + 24);   // the pseudo-step
   T* stl = reinterpret_cast<T*>(smem_raw + PL::OFF_UB);   // table slice [NS][NT] (pseudo-steps)
   T* ub = stl;                                            // plane projections [NQ][NQF][NT] (u < NU used)
   const MeshArgs& m = a.m;
   const Tab1D<T>& tb = tab<T>(P);
-  if (tile_inactive(m, slot)) return;
+  const bool step = a.mode == kHJStep;
+  double vd = 0.0;   // thread 0: the running CFL maximum before this step
+  if (tile_inactive(m, slot)) {
+    if (step && slot == 0 && threadIdx.x == 0) hj_clock_step(a.clk, a.step, true, vd);
+    return;
+  }
 
   auto origin = [&](int slot, int* o) {
     int b = m.tiles ? m.tiles[slot] : slot;
@@ -299,7 +306,6 @@ __device__ __forceinline__ void hjs_tile(const HJArgs<T>& a, int slot) {
     o[1] = DIM > 1 ? (b % m.ntile[1]) * TY : 0;
     o[2] = DIM > 2 ? (b / m.ntile[1]) * TZ : 0;
   };
-  const bool step = a.mode == kHJStep;
   const int cl = (int)threadIdx.x % NT, k = (int)threadIdx.x / NT;   // cell, Gauss plane
   const int l[3] = {cl % TX, (cl / TX) % TY, DIM > 2 ? cl / (TX * TY) : 0};
   const T ih[3] = {T(1.0 / m.h[0]), T(1.0 / m.h[1]), T(DIM > 2 ? 1.0 / m.h[2] : 1.0)};
@@ -313,7 +319,6 @@ __device__ __forceinline__ void hjs_tile(const HJArgs<T>& a, int slot) {
     Dk[b] = tb.Dq[b][k];
     if (step) Dk[b] *= ih[DIM - 1];   // the pseudo-steps' plane derivative, per unit length
   }
-  const T dt = a.clk ? T(a.clk->hj_dt) : T(a.dt_explicit);
   T vmax = T(0);
 
   int o[3];
@@ -330,6 +335,7 @@ __device__ __forceinline__ void hjs_tile(const HJArgs<T>& a, int slot) {
     if (step) {
       mbar_arrive_expect_tx(bar, (unsigned)PL::TAB_BYTES);
       bulk_g2s(stl, a.stab + (size_t)tile * NS * NT, (unsigned)PL::TAB_BYTES, bar);
+      *sdt = hj_clock_step(a.clk, a.step, slot == 0, vd);
     }
   }
   if (threadIdx.x < 32) bulk_box_rows<DIM, TX, TY, TZ, NMB, PL::SLOT>(m, a.phi, boxb, o[0], o[1], o[2], bar);
@@ -511,7 +517,7 @@ __device__ __forceinline__ void hjs_tile(const HJArgs<T>& a, int slot) {
   slot_max(cfl, vmax);
   if (!step) {
     __syncthreads();
-    if (threadIdx.x == 0 && a.clk) atomic_max_pos(&a.clk->hj_vd_bits, slot_value(cfl) / m.diam);
+    if (threadIdx.x == 0) atomic_max_pos(&a.clk->hj_vd[0], slot_value(cfl) / m.diam);
     return;
   }
 
@@ -630,7 +636,11 @@ __device__ __forceinline__ void hjs_tile(const HJArgs<T>& a, int slot) {
     }
   }
   __syncthreads();   // planes done: the face-jump area becomes the store staging
-  if (threadIdx.x == 0 && a.clk) atomic_max_pos(&a.clk->hj_vd_bits, slot_value(cfl) / m.diam);
+  if (threadIdx.x == 0) {   // the running maximum of the next step (the first block has put this one's)
+    const double bm = slot_value(cfl) / m.diam;
+    if (bm > vd) atomic_max_pos(&a.clk->hj_vd[(a.step.k + 1) % 3], bm);
+  }
+  const T dt = T(*sdt);
 
   // -------- columns u = k, k + NQ, ... of modes: project over the planes,
   // update, stage

@@ -17,9 +17,9 @@ int upload_tables_adv() {
 
 static int sep_unit(int what, const Ctx& c, const VelDev* v, const int* tile, size_t* bytes,
                     const void* in = nullptr, const void* phin = nullptr, void* out = nullptr,
-                    const DevClock* clk = nullptr, int stage = 0, int combine = 0, double ct = 0.0) {
-  if (c.dim == 2) return sep2_call(what, c, v, tile, bytes, in, phin, out, clk, stage, combine, ct);
-  return sep3_call(what, c, v, tile, bytes, in, phin, out, clk, stage, combine, ct);
+                    const AdvStep* step = nullptr, int stage = 0, int combine = 0, double ct = 0.0) {
+  if (c.dim == 2) return sep2_call(what, c, v, tile, bytes, in, phin, out, step, stage, combine, ct);
+  return sep3_call(what, c, v, tile, bytes, in, phin, out, step, stage, combine, ct);
 }
 
 // the table kernel's fixed tile
@@ -119,7 +119,7 @@ int adv_prepare(const Ctx& c, const VelDev& v, const int* tile) {
 }
 
 int launch_adv_stage(const Ctx& c, const VelDev& v, const void* in, const void* phin, void* out,
-                     const DevClock* clk, int stage, int combine, double ct_explicit,
+                     const AdvStep* step, int stage, int combine, double ct_explicit,
                      const int* tile) {
   if (use_sep_kernel(v)) {
     int t[3];
@@ -128,7 +128,7 @@ int launch_adv_stage(const Ctx& c, const VelDev& v, const void* in, const void* 
       const int st = adv_default_tile(c, v, t);
       if (st) return st;
     }
-    return sep_unit(2, c, &v, t, nullptr, in, phin, out, clk, stage, combine, ct_explicit);
+    return sep_unit(2, c, &v, t, nullptr, in, phin, out, step, stage, combine, ct_explicit);
   }
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
     constexpr int DIM = decltype(D)::value, P = decltype(PP)::value;
@@ -144,7 +144,7 @@ int launch_adv_stage(const Ctx& c, const VelDev& v, const void* in, const void* 
       a.phi_s = reinterpret_cast<const T*>(in);
       a.phi_n = reinterpret_cast<const T*>(phin);
       a.out = reinterpret_cast<T*>(out);
-      a.clk = clk;
+      a.step = step;
       a.stage = stage;
       a.combine = combine;
       a.ct_explicit = ct_explicit;
@@ -174,7 +174,7 @@ int launch_adv_stage(const Ctx& c, const VelDev& v, const void* in, const void* 
     a.phi_s = reinterpret_cast<const T*>(in);
     a.phi_n = reinterpret_cast<const T*>(phin);
     a.out = reinterpret_cast<T*>(out);
-    a.clk = clk;
+    a.step = step;
     a.stage = stage;
     a.combine = combine;
     a.ct_explicit = ct_explicit;

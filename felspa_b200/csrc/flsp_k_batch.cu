@@ -40,7 +40,7 @@ __device__ __forceinline__ void copy_mesh(MeshArgs* dst, const MeshArgs& src) {
 template <typename T, int P>
 __global__ void __launch_bounds__(HjsTile<2>::N * (P + 2), advtab_min_blocks<2, P, T>())
     batch_adv_kernel(const BatchProb* __restrict__ probs, const int2* __restrict__ items, int ix, int in_n, int iout,
-                     int stage, int combine) {
+                     int step, int stage, int combine) {
   __shared__ AdvTabArgs<T> a;
   const int2 w = items[blockIdx.x];
   const BatchProb& pr = probs[w.x];
@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(HjsTile<2>::N * (P + 2), advtab_min_blocks<2, 
     a.phi_s = reinterpret_cast<const T*>(pr.buf[ix]);
     a.phi_n = reinterpret_cast<const T*>(pr.buf[in_n]);
     a.out = reinterpret_cast<T*>(pr.buf[iout]);
-    a.clk = pr.clk;
+    a.step = pr.steps + step;
     a.stage = stage;
     a.combine = combine;
     a.err = &pr.clk->err;
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(HjsTile<2>::N * (P + 2), advtab_min_blocks<2, 
 template <typename T, int P>
 __global__ void __launch_bounds__(HjsTile<2>::N * (P + 2), hjs_min_blocks<2, P, T>())
     batch_hj_kernel(const BatchProb* __restrict__ probs, const int2* __restrict__ items, int isrc, int iphi0, int idst,
-                    int mode, int rk) {
+                    int mode, int rk, double cfl_max, int k) {
   __shared__ HJArgs<T> a;
   const int2 w = items[blockIdx.x];
   const BatchProb& pr = probs[w.x];
@@ -74,7 +74,10 @@ __global__ void __launch_bounds__(HjsTile<2>::N * (P + 2), hjs_min_blocks<2, P, 
     a.clk = pr.clk;
     a.mode = mode;
     a.rk = rk;
-    a.dt_explicit = 0.0;
+    a.step.cfl_max = cfl_max;
+    a.step.scale = pr.adv_scale;
+    a.step.shift = 0.0;
+    a.step.k = k;
     a.rdiff = nullptr;
     a.stab = reinterpret_cast<T*>(pr.stab);
     a.err = &pr.clk->err;
@@ -124,19 +127,18 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// clocks: one thread per problem
-__global__ void batch_clock_kernel(const BatchProb* __restrict__ probs, int n, int what, double cfl_max) {
+// clocks
+__global__ void batch_clock_kernel(const BatchProb* __restrict__ probs, int n, int what) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const BatchProb& pr = probs[i];
-  switch (what) {
-    case kBatchAdvBegin: adv_clock_begin_body(pr.clk, pr.ca); break;
-    case kBatchAdvEnd: adv_clock_end_body(pr.clk); break;
-    case kBatchAdvHorizon: adv_clock_horizon_body(pr.clk, __longlong_as_double(0x7ff0000000000000LL)); break;
-    case kBatchHjReset: hj_clock_reset_body(pr.clk); break;
-    case kBatchHjBegin: hj_clock_begin_body(pr.clk, cfl_max, pr.p, 0.0, pr.m_hj.min_diam, pr.adv_scale); break;
-    default: hj_clock_end_body(pr.clk); break;
-  }
+  if (what == kBatchAdvHorizon) adv_clock_horizon_body(pr.clk, __longlong_as_double(0x7ff0000000000000LL));
+  else hj_clock_reset_body(pr.clk);
+}
+// a warp per problem
+__global__ void batch_clock_steps_kernel(const BatchProb* __restrict__ probs, int n_steps, int commit) {
+  const BatchProb& pr = probs[blockIdx.x];
+  adv_clock_steps_body(pr.clk, pr.ca, pr.steps, n_steps, commit != 0);
 }
 
 template <typename K>
@@ -151,9 +153,14 @@ int persistent_grid(K kern, int threads, size_t smem, int n_items) {
 
 }  // namespace
 
-int launch_batch_clock(cudaStream_t s, const BatchProb* probs, int n, int what, double cfl_max) {
-  batch_clock_kernel<<<(n + 127) / 128, 128, 0, s>>>(probs, n, what, cfl_max);
+int launch_batch_clock(cudaStream_t s, const BatchProb* probs, int n, int what) {
+  batch_clock_kernel<<<(n + 127) / 128, 128, 0, s>>>(probs, n, what);
   return launch_status("batch_clock_kernel");
+}
+
+int launch_batch_clock_steps(cudaStream_t s, const BatchProb* probs, int n, int n_steps, bool commit) {
+  batch_clock_steps_kernel<<<n, 32, 0, s>>>(probs, n_steps, commit ? 1 : 0);
+  return launch_status("batch_clock_steps_kernel");
 }
 
 // f(integral_constant<int, p>) for the degree p in 1..3
@@ -200,25 +207,26 @@ int batch_prepare(int kind, int prec, int p, int n_items, size_t* smem, int* thr
 }
 
 int launch_batch_adv(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items, int n_items,
-                     int grid, int threads, size_t smem, int ix, int in_n, int iout, int stage, int combine) {
+                     int grid, int threads, size_t smem, int ix, int in_n, int iout, int step, int stage, int combine) {
   return with_degree(p, [&](auto PC) -> int {
     constexpr int P = decltype(PC)::value;
     if (prec == FLSP_FP64)
-      batch_adv_kernel<double, P><<<grid, threads, smem, s>>>(probs, items, ix, in_n, iout, stage, combine);
+      batch_adv_kernel<double, P><<<grid, threads, smem, s>>>(probs, items, ix, in_n, iout, step, stage, combine);
     else
-      batch_adv_kernel<float, P><<<grid, threads, smem, s>>>(probs, items, ix, in_n, iout, stage, combine);
+      batch_adv_kernel<float, P><<<grid, threads, smem, s>>>(probs, items, ix, in_n, iout, step, stage, combine);
     return launch_status("batch_adv_kernel");
   });
 }
 
 int launch_batch_hj(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items, int n_items,
-                    int grid, int threads, size_t smem, int isrc, int iphi0, int idst, int mode, int rk) {
+                    int grid, int threads, size_t smem, int isrc, int iphi0, int idst, int mode, int rk, double cfl_max,
+                    int k) {
   return with_degree(p, [&](auto PC) -> int {
     constexpr int P = decltype(PC)::value;
     if (prec == FLSP_FP64)
-      batch_hj_kernel<double, P><<<grid, threads, smem, s>>>(probs, items, isrc, iphi0, idst, mode, rk);
+      batch_hj_kernel<double, P><<<grid, threads, smem, s>>>(probs, items, isrc, iphi0, idst, mode, rk, cfl_max, k);
     else
-      batch_hj_kernel<float, P><<<grid, threads, smem, s>>>(probs, items, isrc, iphi0, idst, mode, rk);
+      batch_hj_kernel<float, P><<<grid, threads, smem, s>>>(probs, items, isrc, iphi0, idst, mode, rk, cfl_max, k);
     return launch_status("batch_hj_kernel");
   });
 }

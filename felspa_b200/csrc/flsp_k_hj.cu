@@ -104,7 +104,7 @@ int launch_ldg(const Ctx& c, const void* in, void* out, long long block, double 
 }
 
 int launch_hj(const Ctx& c, const void* phi, const void* phi0, void* out, DevClock* clk, int mode,
-              int rk, double dt_explicit, long long block, const int* tile, const void* rdiff) {
+              int rk, const HjClockArgs* step, long long block, const int* tile, const void* rdiff) {
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
     constexpr int DIM = decltype(D)::value, P = decltype(PP)::value;
     using T = decltype(tz);
@@ -121,7 +121,7 @@ int launch_hj(const Ctx& c, const void* phi, const void* phi0, void* out, DevClo
     a.clk = clk;
     a.mode = mode;
     a.rk = rk;
-    a.dt_explicit = dt_explicit;
+    if (step) a.step = *step;
     a.block = block;
     a.rdiff = reinterpret_cast<const T*>(rdiff);
     if (mode == kHJGradients) {   // the export, every cell
@@ -134,7 +134,8 @@ int launch_hj(const Ctx& c, const void* phi, const void* phi0, void* out, DevClo
     apply_band(c, kNbHJ, a.m);
     // the smooth-sign table is filled by the sweep's kHJCflOnly launch,
     // which evaluates phi0 as phi
-    if (!c.hj_stab) return set_error(FLSP_ERR_BAD_ARG, "reinit sign table not allocated");
+    if (!c.hj_stab || !clk || (mode == kHJStep && !step))
+      return set_error(FLSP_ERR_BAD_ARG, "reinit sign table or clock missing");
     if (mode == kHJCflOnly && phi != phi0)
       return set_error(FLSP_ERR_BAD_ARG, "the sign-table launch needs phi == phi0");
     using TL = HjsTile<DIM>;
@@ -142,7 +143,7 @@ int launch_hj(const Ctx& c, const void* phi, const void* phi0, void* out, DevClo
         (c.basis == FLSP_BASIS_Q && (a.m.tile[0] != TL::X || a.m.tile[1] != TL::Y || a.m.tile[2] != TL::Z)))
       return set_error(FLSP_ERR_BAD_ARG, "the reinit kernels have a fixed tile");
     a.stab = reinterpret_cast<T*>(c.hj_stab);
-    a.err = clk ? &clk->err : nullptr;
+    a.err = &clk->err;
     const int threads = TL::N * (P + 2);
     if (c.basis == FLSP_BASIS_Q) {
       hjs_kernel<DIM, P, T><<<(unsigned)nblocks(a.m), threads, HjsPlan<DIM, P, T>::BYTES, c.stream>>>(a);

@@ -210,13 +210,10 @@ int launch_nonfinite(const Ctx& c, const void* x, long long n, unsigned int* cou
   return launch_status("nonfinite_kernel");
 }
 
-int launch_adv_clock_begin(cudaStream_t s, DevClock* clk, const AdvClockArgs& a) {
-  adv_clock_begin<<<1, 1, 0, s>>>(clk, a);
-  return launch_status("adv_clock_begin");
-}
-int launch_adv_clock_end(cudaStream_t s, DevClock* clk) {
-  adv_clock_end<<<1, 1, 0, s>>>(clk);
-  return launch_status("adv_clock_end");
+int launch_adv_clock_steps(cudaStream_t s, DevClock* clk, const AdvClockArgs& a, AdvStep* steps, int n, bool commit,
+                           double horizon) {
+  adv_clock_steps<<<1, 32, 0, s>>>(clk, a, steps, n, commit ? 1 : 0, horizon);
+  return launch_status("adv_clock_steps");
 }
 int launch_adv_clock_horizon(cudaStream_t s, DevClock* clk, double time_step) {
   adv_clock_horizon<<<1, 1, 0, s>>>(clk, time_step);
@@ -225,15 +222,6 @@ int launch_adv_clock_horizon(cudaStream_t s, DevClock* clk, double time_step) {
 int launch_hj_clock_reset(cudaStream_t s, DevClock* clk) {
   hj_clock_reset<<<1, 1, 0, s>>>(clk);
   return launch_status("hj_clock_reset");
-}
-int launch_hj_clock_begin(cudaStream_t s, DevClock* clk, double cfl_max, int p, double nu,
-                          double min_diam, double adv_scale) {
-  hj_clock_begin<<<1, 1, 0, s>>>(clk, cfl_max, p, nu, min_diam, adv_scale);
-  return launch_status("hj_clock_begin");
-}
-int launch_hj_clock_end(cudaStream_t s, DevClock* clk) {
-  hj_clock_end<<<1, 1, 0, s>>>(clk);
-  return launch_status("hj_clock_end");
 }
 
 }  // namespace flsp

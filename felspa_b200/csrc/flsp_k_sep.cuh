@@ -33,7 +33,7 @@ int with_sep_tile(const int* t, F&& f) {
 // kernel's attributes, 2 = launch one stage
 template <int DIM>
 int sep_call(int what, const Ctx& c, const VelDev* v, const int* tile, size_t* bytes, const void* in,
-             const void* phin, void* out, const DevClock* clk, int stage, int combine, double ct_explicit) {
+             const void* phin, void* out, const AdvStep* step, int stage, int combine, double ct_explicit) {
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
     constexpr int DD = decltype(D)::value;
     if constexpr (DD != DIM) {
@@ -74,7 +74,7 @@ int sep_call(int what, const Ctx& c, const VelDev* v, const int* tile, size_t* b
           b.phi_s = reinterpret_cast<const T*>(in);
           b.phi_n = reinterpret_cast<const T*>(phin);
           b.out = reinterpret_cast<T*>(out);
-          b.clk = clk;
+          b.step = step;
           b.stage = stage;
           b.combine = combine;
           b.ct_explicit = ct_explicit;

@@ -11,8 +11,8 @@ int upload_tables_sep2() {
 }
 
 int sep2_call(int what, const Ctx& c, const VelDev* v, const int* tile, size_t* bytes, const void* in,
-              const void* phin, void* out, const DevClock* clk, int stage, int combine, double ct_explicit) {
-  return sep_call<2>(what, c, v, tile, bytes, in, phin, out, clk, stage, combine, ct_explicit);
+              const void* phin, void* out, const AdvStep* step, int stage, int combine, double ct_explicit) {
+  return sep_call<2>(what, c, v, tile, bytes, in, phin, out, step, stage, combine, ct_explicit);
 }
 
 }  // namespace flsp

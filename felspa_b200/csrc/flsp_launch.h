@@ -52,6 +52,7 @@ struct BatchProb {
   MeshArgs m_adv, m_hj, m_weno;   // the batch's tile shapes, no narrow band
   void* buf[3];                   // state buffers (roles are launch parameters)
   DevClock* clk;
+  AdvStep* steps;                 // its next substeps
   const void* tab;                // velocity table of the problem (VelTabLayout)
   void* stab;                     // smooth-sign table of its reinitialisation
   int p;                          // degree 1..3
@@ -60,18 +61,21 @@ struct BatchProb {
 };
 enum BatchKernelKind : int { kBatchKindAdv = 0, kBatchKindHJ = 1, kBatchKindWeno = 2 };
 enum BatchClockOp : int {
-  kBatchAdvBegin = 0, kBatchAdvEnd = 1, kBatchAdvHorizon = 2, kBatchHjReset = 3, kBatchHjBegin = 4, kBatchHjEnd = 5
+  kBatchAdvHorizon = 0, kBatchHjReset = 1
 };
 int upload_tables_batch();
 // shared memory one problem needs for a tile of the given kind
 // shared memory of the degree-p kernel of a kind, its attributes for it, and
 // the grid for n_items (every item of a launch has degree p)
 int batch_prepare(int kind, int prec, int p, int n_items, size_t* smem, int* threads, int* grid);
-int launch_batch_clock(cudaStream_t s, const BatchProb* probs, int n, int what, double cfl_max);
+int launch_batch_clock(cudaStream_t s, const BatchProb* probs, int n, int what);
+// the next n_steps substeps of every problem (its steps array); commit as in
+// launch_adv_clock_steps
+int launch_batch_clock_steps(cudaStream_t s, const BatchProb* probs, int n, int n_steps, bool commit);
 int launch_batch_adv(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items, int n_items,
-                     int grid, int threads, size_t smem, int ix, int in_n, int iout, int stage, int combine);
+                     int grid, int threads, size_t smem, int ix, int in_n, int iout, int step, int stage, int combine);
 int launch_batch_hj(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items, int n_items,
-                    int grid, int threads, size_t smem, int isrc, int iphi0, int idst, int mode, int rk);
+                    int grid, int threads, size_t smem, int isrc, int iphi0, int idst, int mode, int rk, double cfl_max, int k);
 int launch_batch_weno(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items, int n_items,
                       int grid, int threads, size_t smem, int iin, int iout, int2* list, unsigned int* list_n,
                       long long n_cells);
@@ -146,16 +150,16 @@ inline bool use_sep_kernel(const VelDev& v) { return v.sep1 && v.optab != nullpt
 // separable stage kernel units: what = 0 shared-memory bytes of the tile,
 // 1 kernel attributes, 2 launch (flsp_k_sep.cuh)
 int sep2_call(int what, const Ctx& c, const VelDev* v, const int* tile, size_t* bytes, const void* in,
-              const void* phin, void* out, const DevClock* clk, int stage, int combine, double ct_explicit);
+              const void* phin, void* out, const AdvStep* step, int stage, int combine, double ct_explicit);
 int sep3_call(int what, const Ctx& c, const VelDev* v, const int* tile, size_t* bytes, const void* in,
-              const void* phin, void* out, const DevClock* clk, int stage, int combine, double ct_explicit);
+              const void* phin, void* out, const AdvStep* step, int stage, int combine, double ct_explicit);
 // tile: cells per CTA (nullptr = default); smem attribute is set on first use
 int adv_default_tile(const Ctx& c, const VelDev& v, int* tile);
 int adv_prepare(const Ctx& c, const VelDev& v, const int* tile);
 // the tile shapes the stage kernel for this velocity is built with (at most 8)
 int adv_tile_candidates(const Ctx& c, const VelDev& v, int (*out)[3], int* n);
 int launch_adv_stage(const Ctx& c, const VelDev& v, const void* in, const void* phin, void* out,
-                     const DevClock* clk, int stage, int combine, double ct_explicit,
+                     const AdvStep* step, int stage, int combine, double ct_explicit,
                      const int* tile);
 
 // ---------------- reinitialisation (flsp_k_hj.cu) ----------------
@@ -164,7 +168,7 @@ int hj_prepare(const Ctx& c, const int* tile);
 // bytes of the tensor-product reinit kernel's smooth-sign table for `tile`
 int hj_table_bytes(const Ctx& c, const int* tile, size_t* bytes);
 int launch_hj(const Ctx& c, const void* phi, const void* phi0, void* out, DevClock* clk, int mode,
-              int rk, double dt_explicit, long long block, const int* tile,
+              int rk, const HjClockArgs* step, long long block, const int* tile,
               const void* rdiff = nullptr);
 // LDG artificial viscosity: mode 0 = alternating gradient q (DIM blocks)
 // from phi, mode 1 = diffusion RHS (per unit volume) from q
@@ -200,13 +204,12 @@ int launch_scatter(const Ctx& c, const double* src, void* dst, const int64_t* pe
 int launch_gather(const Ctx& c, const void* src, double* dst, const int64_t* perm);
 int launch_nonfinite(const Ctx& c, const void* x, long long n, unsigned int* count);
 
-int launch_adv_clock_begin(cudaStream_t s, DevClock* clk, const AdvClockArgs& a);
-int launch_adv_clock_end(cudaStream_t s, DevClock* clk);
+// the next n <= kClockSteps substeps into steps; commit: the clock moves past
+// them; horizon >= 0: an advance call of that length starts
+int launch_adv_clock_steps(cudaStream_t s, DevClock* clk, const AdvClockArgs& a, AdvStep* steps, int n, bool commit,
+                           double horizon = -1.0);
 int launch_adv_clock_horizon(cudaStream_t s, DevClock* clk, double time_step);
 int launch_hj_clock_reset(cudaStream_t s, DevClock* clk);
-int launch_hj_clock_begin(cudaStream_t s, DevClock* clk, double cfl_max, int p, double nu,
-                          double min_diam, double adv_scale);
-int launch_hj_clock_end(cudaStream_t s, DevClock* clk);
 
 // ---------------- output (flsp_io.cu) ----------------
 // out[k * (n_sub+1)^dim + j] = the state of host cell k at its patch vertex j

@@ -15,14 +15,12 @@ constexpr double kEpsD = 2.220446049250313e-16;
 // clocks
 // ---------------------------------------------------------------------
 
-// clock kernels: one thread (the updates are in flsp_clock.cuh)
-__global__ void adv_clock_begin(DevClock* c, const AdvClockArgs a) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  adv_clock_begin_body(c, a);
-}
-__global__ void adv_clock_end(DevClock* c) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  adv_clock_end_body(c);
+// clock kernels (the updates are in flsp_clock.cuh)
+// the next n substeps (one warp); horizon >= 0 starts an advance call of that
+// length first
+__global__ void adv_clock_steps(DevClock* c, const AdvClockArgs a, AdvStep* st, int n, int commit, double horizon) {
+  if (horizon >= 0.0 && threadIdx.x == 0) adv_clock_horizon_body(c, horizon);
+  adv_clock_steps_body(c, a, st, n, commit != 0);
 }
 __global__ void adv_clock_horizon(DevClock* c, double time_step) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
@@ -32,15 +30,6 @@ __global__ void hj_clock_reset(DevClock* c) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   hj_clock_reset_body(c);
 }
-__global__ void hj_clock_begin(DevClock* c, double cfl_max, int p, double nu, double min_diam, double adv_scale) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  hj_clock_begin_body(c, cfl_max, p, nu, min_diam, adv_scale);
-}
-__global__ void hj_clock_end(DevClock* c) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  hj_clock_end_body(c);
-}
-
 // ---------------------------------------------------------------------
 // host DoF order <-> device layout (optional cell permutation)
 // ---------------------------------------------------------------------
