@@ -78,6 +78,7 @@ struct Tab1D {
   T D0[kMaxN1], D1[kMaxN1];             // L_a'(0), L_a'(1)
   T H0[kMaxN1], H1[kMaxN1];             // L_a''(0), L_a''(1)
   T A[kMaxN1][kMaxN1];                  // int_0^1 L_a' L_b
+  T S[kMaxN1][kMaxN1];                  // int_0^1 L_a(x) L_b(x + 1)
   T xl[kMaxN1], wl[kMaxN1];             // Gauss (p+1) points/weights
   T Ll[kMaxN1][kMaxN1];                 // L_a(xl)
   T Dl[kMaxN1][kMaxN1];                 // L_a'(xl)

@@ -3,11 +3,8 @@
 // in ONE launch per RK stage (and one per reinit pseudo-step and limiter pass)
 // per degree.  A block serves a work item (problem, tile) of one degree with
 // the same per-tile bodies as the single-problem kernels (adv_tab_tile,
-// hjs_tile; the limiter's detection, weno_tile, walks its items persistently);
-// each degree has its own instantiation, so its registers, shared memory and
+// hjs_tile, weno_tile); each degree has its own instantiation, so its registers, shared memory and
 // occupancy are its own, not those of the most demanding degree in the batch.
-#include <algorithm>
-#include <cstring>
 #include <string>
 #include <type_traits>
 
@@ -86,45 +83,22 @@ __global__ void __launch_bounds__(HjsTile<2>::N * (P + 2), hjs_min_blocks<2, P, 
   hjs_tile<2, P, T>(a, w.y);
 }
 
+// two blocks per (problem, tile)
 template <typename T, int P>
-__global__ void __launch_bounds__(256, 2)
-    batch_weno_kernel(const BatchProb* __restrict__ probs, const int2* __restrict__ items, int n_items, int iin,
-                      int iout, int2* list, unsigned int* list_n) {
+__global__ void __launch_bounds__(WenoBlock::N)
+    batch_weno_kernel(const BatchProb* __restrict__ probs, const int2* __restrict__ items, int iin, int iout) {
   __shared__ WenoArgs<T> a;
-  for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-    const int2 w = items[it];
-    if (threadIdx.x == 0) {
-      const BatchProb& pr = probs[w.x];
-      a.m = pr.m_weno;
-      a.in = reinterpret_cast<const T*>(pr.buf[iin]);
-      a.out = reinterpret_cast<T*>(pr.buf[iout]);
-      a.count = nullptr;
-      a.list = list;
-      a.list_n = list_n;
-      a.problem = w.x;
-    }
-    __syncthreads();
-    weno_tile<P, T>(a, w.y);
-    __syncthreads();
+  const int2 w = items[blockIdx.x / 2];
+  const BatchProb& pr = probs[w.x];
+  copy_mesh(&a.m, pr.m_weno);
+  if (threadIdx.x == 0) {
+    a.in = reinterpret_cast<const T*>(pr.buf[iin]);
+    a.out = reinterpret_cast<T*>(pr.buf[iout]);
+    a.count = nullptr;
+    a.err = &pr.clk->err;
   }
-}
-
-// the troubled cells of every problem of the launch's degree: a warp each
-template <typename T, int P>
-__global__ void __launch_bounds__(256)
-    batch_weno_fix_kernel(const BatchProb* __restrict__ probs, const int2* __restrict__ list,
-                          const unsigned int* __restrict__ list_n, int iin, int iout) {
-  constexpr int NM = (P + 1) * (P + 1);
-  __shared__ T sh[8][5 * NM];
-  const int wl = threadIdx.x >> 5;
-  const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), nwarps = (int)((gridDim.x * blockDim.x) >> 5);
-  const unsigned int n = *list_n;
-  for (unsigned int i = warp; i < n; i += nwarps) {
-    const int2 e = list[i];
-    const BatchProb& pr = probs[e.x];
-    weno_fix<P, T>(pr.m_weno, reinterpret_cast<const T*>(pr.buf[iin]), reinterpret_cast<T*>(pr.buf[iout]), e.y,
-                   sh[wl]);
-  }
+  __syncthreads();
+  weno_tile<P, false, T>(a, w.y, (int)blockIdx.x % 2);
 }
 
 // clocks
@@ -139,16 +113,6 @@ __global__ void batch_clock_kernel(const BatchProb* __restrict__ probs, int n, i
 __global__ void batch_clock_steps_kernel(const BatchProb* __restrict__ probs, int n_steps, int commit) {
   const BatchProb& pr = probs[blockIdx.x];
   adv_clock_steps_body(pr.clk, pr.ca, pr.steps, n_steps, commit != 0);
-}
-
-template <typename K>
-int persistent_grid(K kern, int threads, size_t smem, int n_items) {
-  int per_sm = 0, dev = 0, nsm = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  return std::max(1, std::min(n_items, nsm * per_sm));
 }
 
 }  // namespace
@@ -193,10 +157,10 @@ int batch_prepare(int kind, int prec, int p, int n_items, size_t* smem, int* thr
         *smem = HjsPlan<2, P, T>::BYTES;
         attr(batch_hj_kernel<T, P>);
       } else {
-        *smem = weno_smem_bytes<P, T>(kWenoTile);
-        *threads = kWenoTile[0] * kWenoTile[1];
+        *smem = WenoPlan<P, false, T>::BYTES;
+        *threads = WenoBlock::N;
+        *grid = 2 * n_items;
         attr(batch_weno_kernel<T, P>);
-        *grid = persistent_grid(batch_weno_kernel<T, P>, *threads, *smem, n_items);
       }
     };
     if (prec == FLSP_FP64) go((double)0);
@@ -232,20 +196,11 @@ int launch_batch_hj(cudaStream_t s, int prec, int p, const BatchProb* probs, con
 }
 
 int launch_batch_weno(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items, int n_items,
-                      int grid, int threads, size_t smem, int iin, int iout, int2* list, unsigned int* list_n,
-                      long long n_cells) {
-  cudaError_t e = cudaMemsetAsync(list_n, 0, sizeof(unsigned int), s);
-  if (e != cudaSuccess) return set_error(FLSP_ERR_CUDA, std::string("batch weno list: ") + cudaGetErrorString(e));
-  const int fix_grid = (int)std::max<long long>(1, std::min<long long>((n_cells + 7) / 8, 148LL * 4));
+                      int grid, int threads, size_t smem, int iin, int iout) {
   return with_degree(p, [&](auto PC) -> int {
     constexpr int P = decltype(PC)::value;
-    if (prec == FLSP_FP64) {
-      batch_weno_kernel<double, P><<<grid, threads, smem, s>>>(probs, items, n_items, iin, iout, list, list_n);
-      batch_weno_fix_kernel<double, P><<<fix_grid, 256, 0, s>>>(probs, list, list_n, iin, iout);
-    } else {
-      batch_weno_kernel<float, P><<<grid, threads, smem, s>>>(probs, items, n_items, iin, iout, list, list_n);
-      batch_weno_fix_kernel<float, P><<<fix_grid, 256, 0, s>>>(probs, list, list_n, iin, iout);
-    }
+    if (prec == FLSP_FP64) batch_weno_kernel<double, P><<<grid, threads, smem, s>>>(probs, items, iin, iout);
+    else batch_weno_kernel<float, P><<<grid, threads, smem, s>>>(probs, items, iin, iout);
     return launch_status("batch_weno_kernel");
   });
 }

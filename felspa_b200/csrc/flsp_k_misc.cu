@@ -30,15 +30,18 @@ int weno_prepare(const Ctx& c) {
     if constexpr (decltype(D)::value != 2) {
       return set_error(FLSP_ERR_UNSUPPORTED, "WENO limiter is 2D only");
     } else {
-      const size_t smem = weno_smem_bytes<P, T>(kWenoTile);
-      cudaError_t e = cudaFuncSetAttribute(weno_kernel<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      static_assert(kWenoTile[0] == WenoBlock::X && kWenoTile[1] == 2 * WenoBlock::Y, "two blocks per tile");
+      const bool q = c.basis == FLSP_BASIS_Q;
+      cudaError_t e = cudaFuncSetAttribute(q ? weno_kernel<P, false, T> : weno_kernel<P, true, T>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(q ? WenoPlan<P, false, T>::BYTES : WenoPlan<P, true, T>::BYTES));
       if (e != cudaSuccess) return set_error(FLSP_ERR_CUDA, std::string("weno attr: ") + cudaGetErrorString(e));
       return FLSP_OK;
     }
   });
 }
 
-int launch_weno(const Ctx& c, const void* in, void* out, unsigned int* count, int2* list, unsigned int* list_n) {
+int launch_weno(const Ctx& c, const void* in, void* out, unsigned int* count, int* err) {
   if (c.dim != 2) return set_error(FLSP_ERR_UNSUPPORTED, "WENO limiter is 2D only (reinit.cc:475-478)");
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
     constexpr int P = decltype(PP)::value;
@@ -54,17 +57,12 @@ int launch_weno(const Ctx& c, const void* in, void* out, unsigned int* count, in
       a.in = reinterpret_cast<const T*>(in);
       a.out = reinterpret_cast<T*>(out);
       a.count = count;
-      a.list = list;
-      a.list_n = list_n;
-      a.problem = 0;
-      cudaError_t e = cudaMemsetAsync(list_n, 0, sizeof(unsigned int), c.stream);
-      if (e != cudaSuccess) return set_error(FLSP_ERR_CUDA, std::string("weno list: ") + cudaGetErrorString(e));
-      const size_t smem = weno_smem_bytes<P, T>(a.m.tile);
-      weno_kernel<P, T><<<(unsigned)nblocks(a.m), kWenoTile[0] * kWenoTile[1], smem, c.stream>>>(a);
-      // the troubled cells: a warp each, at most one warp per cell
-      const long long want = (c.m.ncell + 7) / 8;
-      const int grid = (int)std::max<long long>(1, std::min<long long>(want, 148LL * 4));
-      weno_fix_kernel<P, T><<<grid, 256, 0, c.stream>>>(a);
+      a.err = err;
+      const unsigned grid = 2u * (unsigned)nblocks(a.m);
+      if (c.basis == FLSP_BASIS_Q)
+        weno_kernel<P, false, T><<<grid, WenoBlock::N, WenoPlan<P, false, T>::BYTES, c.stream>>>(a);
+      else
+        weno_kernel<P, true, T><<<grid, WenoBlock::N, WenoPlan<P, true, T>::BYTES, c.stream>>>(a);
       return launch_status("weno_kernel");
     }
   });

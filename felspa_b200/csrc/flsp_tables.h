@@ -77,6 +77,18 @@ inline void fill_tab(Tab1D<T>& tb, int p) {
       }
       tb.A[a][b] = T((double)s);
     }
+  // S_ab = int_0^1 L_a(x) L_b(x + 1) (degree 2p, exact likewise)
+  for (int a = 0; a < n1; ++a)
+    for (int b = 0; b < n1; ++b) {
+      long double s = 0;
+      for (int q = 0; q < nq; ++q) {
+        double va[8], vb[8], t1[8], t2[8];
+        leg_all(n1, x[q], va, t1, t2);
+        leg_all(n1, x[q] + 1.0, vb, t1, t2);
+        s += (long double)w[q] * va[a] * vb[b];
+      }
+      tb.S[a][b] = T((double)s);
+    }
   {
     double l0[8], l1[8], tmp1[8], tmp2[8];
     leg_all(n1, 0.0, l0, tmp1, tmp2);
