@@ -94,6 +94,7 @@ __device__ __forceinline__ void adv_tab_tile(const AdvTabArgs<T>& a, int tile) {
   }
   if (threadIdx.x == 0) mbar_init(bar, 32);
   __syncthreads();
+  chain_wait();
   if (threadIdx.x < 32) bulk_box_rows<DIM, TX, TY, TZ, NMB, PL::SLOT>(m, a.phi_s, boxb, o[0], o[1], o[2], bar);
   const int cl = (int)threadIdx.x % NT, k = (int)threadIdx.x / NT;   // cell, Gauss plane
   const int l[3] = {cl % TX, (cl / TX) % TY, DIM > 2 ? cl / (TX * TY) : 0};
@@ -370,6 +371,7 @@ __device__ __forceinline__ void adv_tab_tile(const AdvTabArgs<T>& a, int tile) {
       }
   }
   __syncthreads();
+  chain_release();
   combine_rows<DIM, TX, TY, TZ, NBG, NT * NQ / 32, T>(m, cellp, sb, a.phi_n, a.out, a.combine, dt, active, o[0], o[1],
                                                       o[2]);
 }

@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjp_min_blocks<DIM,
   const bool step = a.mode == kHJStep, fill = !step;
   const bool first = blockIdx.x == 0;
   double vd = 0.0;   // thread 0: the running CFL maximum before this step
+  chain_wait();
   if (tile_inactive(m, slot)) {
     if (step && first && threadIdx.x == 0) hj_clock_step(a.clk, a.step, true, vd);
     return;
@@ -414,6 +415,7 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjp_min_blocks<DIM,
       }
   }
   __syncthreads();
+  chain_release();
   store_cells<DIM, TX, TY, TZ, NBG, T>(m, sb, a.out, o[0], o[1], o[2]);
 }
 

@@ -294,6 +294,7 @@ __device__ __forceinline__ void hjs_tile(const HJArgs<T>& a, int slot) {
   const Tab1D<T>& tb = tab<T>(P);
   const bool step = a.mode == kHJStep;
   double vd = 0.0;   // thread 0: the running CFL maximum before this step
+  chain_wait();
   if (tile_inactive(m, slot)) {
     if (step && slot == 0 && threadIdx.x == 0) hj_clock_step(a.clk, a.step, true, vd);
     return;
@@ -669,6 +670,7 @@ __device__ __forceinline__ void hjs_tile(const HJArgs<T>& a, int slot) {
     }
   }
   __syncthreads();
+  chain_release();
   store_cells<DIM, TX, TY, TZ, NM, T>(m, sb, a.out, o[0], o[1], o[2]);
   }
 }

@@ -150,13 +150,10 @@ int launch_adv_stage(const Ctx& c, const VelDev& v, const void* in, const void* 
       a.ct_explicit = ct_explicit;
       a.err = v.err;
       const int threads = HjsTile<DIM>::N * (P + 2);
-      if (c.basis == FLSP_BASIS_Q)
-        adv_tab_kernel<DIM, P, false, T>
-            <<<(unsigned)nblocks(a.m), threads, AdvTabPlan<DIM, P, false, T>::BYTES, c.stream>>>(a);
-      else
-        adv_tab_kernel<DIM, P, true, T>
-            <<<(unsigned)nblocks(a.m), threads, AdvTabPlan<DIM, P, true, T>::BYTES, c.stream>>>(a);
-      return launch_status("adv_tab_kernel");
+      const bool q = c.basis == FLSP_BASIS_Q;
+      return launch_chained("adv_tab_kernel", q ? adv_tab_kernel<DIM, P, false, T> : adv_tab_kernel<DIM, P, true, T>,
+                            (unsigned)nblocks(a.m), threads,
+                            q ? AdvTabPlan<DIM, P, false, T>::BYTES : AdvTabPlan<DIM, P, true, T>::BYTES, c.stream, a);
     }
     AdvArgs<T> a;
     std::memset(&a, 0, sizeof(a));

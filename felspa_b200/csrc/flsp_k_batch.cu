@@ -103,6 +103,7 @@ __global__ void __launch_bounds__(WenoBlock::N)
 
 // clocks
 __global__ void batch_clock_kernel(const BatchProb* __restrict__ probs, int n, int what) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const BatchProb& pr = probs[i];
@@ -111,6 +112,7 @@ __global__ void batch_clock_kernel(const BatchProb* __restrict__ probs, int n, i
 }
 // a warp per problem
 __global__ void batch_clock_steps_kernel(const BatchProb* __restrict__ probs, int n_steps, int commit) {
+  chain_wait();
   const BatchProb& pr = probs[blockIdx.x];
   adv_clock_steps_body(pr.clk, pr.ca, pr.steps, n_steps, commit != 0);
 }
@@ -118,13 +120,12 @@ __global__ void batch_clock_steps_kernel(const BatchProb* __restrict__ probs, in
 }  // namespace
 
 int launch_batch_clock(cudaStream_t s, const BatchProb* probs, int n, int what) {
-  batch_clock_kernel<<<(n + 127) / 128, 128, 0, s>>>(probs, n, what);
-  return launch_status("batch_clock_kernel");
+  return launch_chained("batch_clock_kernel", batch_clock_kernel, (unsigned)(n + 127) / 128, 128, 0, s, probs, n, what);
 }
 
 int launch_batch_clock_steps(cudaStream_t s, const BatchProb* probs, int n, int n_steps, bool commit) {
-  batch_clock_steps_kernel<<<n, 32, 0, s>>>(probs, n_steps, commit ? 1 : 0);
-  return launch_status("batch_clock_steps_kernel");
+  return launch_chained("batch_clock_steps_kernel", batch_clock_steps_kernel, (unsigned)n, 32, 0, s, probs, n_steps,
+                        commit ? 1 : 0);
 }
 
 // f(integral_constant<int, p>) for the degree p in 1..3
@@ -174,11 +175,8 @@ int launch_batch_adv(cudaStream_t s, int prec, int p, const BatchProb* probs, co
                      int grid, int threads, size_t smem, int ix, int in_n, int iout, int step, int stage, int combine) {
   return with_degree(p, [&](auto PC) -> int {
     constexpr int P = decltype(PC)::value;
-    if (prec == FLSP_FP64)
-      batch_adv_kernel<double, P><<<grid, threads, smem, s>>>(probs, items, ix, in_n, iout, step, stage, combine);
-    else
-      batch_adv_kernel<float, P><<<grid, threads, smem, s>>>(probs, items, ix, in_n, iout, step, stage, combine);
-    return launch_status("batch_adv_kernel");
+    return launch_chained("batch_adv_kernel", prec == FLSP_FP64 ? batch_adv_kernel<double, P> : batch_adv_kernel<float, P>,
+                          (unsigned)grid, threads, smem, s, probs, items, ix, in_n, iout, step, stage, combine);
   });
 }
 
@@ -187,11 +185,8 @@ int launch_batch_hj(cudaStream_t s, int prec, int p, const BatchProb* probs, con
                     int k) {
   return with_degree(p, [&](auto PC) -> int {
     constexpr int P = decltype(PC)::value;
-    if (prec == FLSP_FP64)
-      batch_hj_kernel<double, P><<<grid, threads, smem, s>>>(probs, items, isrc, iphi0, idst, mode, rk, cfl_max, k);
-    else
-      batch_hj_kernel<float, P><<<grid, threads, smem, s>>>(probs, items, isrc, iphi0, idst, mode, rk, cfl_max, k);
-    return launch_status("batch_hj_kernel");
+    return launch_chained("batch_hj_kernel", prec == FLSP_FP64 ? batch_hj_kernel<double, P> : batch_hj_kernel<float, P>,
+                          (unsigned)grid, threads, smem, s, probs, items, isrc, iphi0, idst, mode, rk, cfl_max, k);
   });
 }
 
@@ -199,9 +194,9 @@ int launch_batch_weno(cudaStream_t s, int prec, int p, const BatchProb* probs, c
                       int grid, int threads, size_t smem, int iin, int iout) {
   return with_degree(p, [&](auto PC) -> int {
     constexpr int P = decltype(PC)::value;
-    if (prec == FLSP_FP64) batch_weno_kernel<double, P><<<grid, threads, smem, s>>>(probs, items, iin, iout);
-    else batch_weno_kernel<float, P><<<grid, threads, smem, s>>>(probs, items, iin, iout);
-    return launch_status("batch_weno_kernel");
+    return launch_chained("batch_weno_kernel",
+                          prec == FLSP_FP64 ? batch_weno_kernel<double, P> : batch_weno_kernel<float, P>, (unsigned)grid,
+                          threads, smem, s, probs, items, iin, iout);
   });
 }
 

@@ -98,8 +98,8 @@ int launch_ldg(const Ctx& c, const void* in, void* out, long long block, double 
     a.block = block;
     a.nu = nu;
     const size_t smem = ldg_smem_bytes<DIM, P, T>(a.m.tile);
-    ldg_kernel<DIM, P, T><<<(unsigned)nblocks(a.m), t[0] * t[1] * t[2], smem, c.stream>>>(a, mode);
-    return launch_status("ldg_kernel");
+    return launch_chained("ldg_kernel", ldg_kernel<DIM, P, T>, (unsigned)nblocks(a.m), t[0] * t[1] * t[2], smem, c.stream,
+                          a, mode);
   });
 }
 
@@ -146,13 +146,12 @@ int launch_hj(const Ctx& c, const void* phi, const void* phi0, void* out, DevClo
     a.err = &clk->err;
     const int threads = TL::N * (P + 2);
     if (c.basis == FLSP_BASIS_Q) {
-      hjs_kernel<DIM, P, T><<<(unsigned)nblocks(a.m), threads, HjsPlan<DIM, P, T>::BYTES, c.stream>>>(a);
-      return launch_status("hjs_kernel");
+      return launch_chained("hjs_kernel", hjs_kernel<DIM, P, T>, (unsigned)nblocks(a.m), threads,
+                            HjsPlan<DIM, P, T>::BYTES, c.stream, a);
     }
     const long long parts = (long long)(a.m.tile[0] / TL::X) * (a.m.tile[1] / TL::Y) * (a.m.tile[2] / TL::Z);
-    hjp_kernel<DIM, P, T>
-        <<<(unsigned)(nblocks(a.m) * parts), threads, HjpPlan<DIM, P, T>::BYTES, c.stream>>>(a);
-    return launch_status("hjp_kernel");
+    return launch_chained("hjp_kernel", hjp_kernel<DIM, P, T>, (unsigned)(nblocks(a.m) * parts), threads,
+                          HjpPlan<DIM, P, T>::BYTES, c.stream, a);
   });
 }
 

@@ -59,11 +59,9 @@ int launch_weno(const Ctx& c, const void* in, void* out, unsigned int* count, in
       a.count = count;
       a.err = err;
       const unsigned grid = 2u * (unsigned)nblocks(a.m);
-      if (c.basis == FLSP_BASIS_Q)
-        weno_kernel<P, false, T><<<grid, WenoBlock::N, WenoPlan<P, false, T>::BYTES, c.stream>>>(a);
-      else
-        weno_kernel<P, true, T><<<grid, WenoBlock::N, WenoPlan<P, true, T>::BYTES, c.stream>>>(a);
-      return launch_status("weno_kernel");
+      const bool q = c.basis == FLSP_BASIS_Q;
+      return launch_chained("weno_kernel", q ? weno_kernel<P, false, T> : weno_kernel<P, true, T>, grid, WenoBlock::N,
+                            q ? WenoPlan<P, false, T>::BYTES : WenoPlan<P, true, T>::BYTES, c.stream, a);
     }
   });
 }
@@ -210,16 +208,14 @@ int launch_nonfinite(const Ctx& c, const void* x, long long n, unsigned int* cou
 
 int launch_adv_clock_steps(cudaStream_t s, DevClock* clk, const AdvClockArgs& a, AdvStep* steps, int n, bool commit,
                            double horizon) {
-  adv_clock_steps<<<1, 32, 0, s>>>(clk, a, steps, n, commit ? 1 : 0, horizon);
-  return launch_status("adv_clock_steps");
+  return launch_chained("adv_clock_steps", adv_clock_steps, 1, 32, 0, s, clk, a, steps, n, commit ? 1 : 0, horizon);
 }
 int launch_adv_clock_horizon(cudaStream_t s, DevClock* clk, double time_step) {
   adv_clock_horizon<<<1, 1, 0, s>>>(clk, time_step);
   return launch_status("adv_clock_horizon");
 }
 int launch_hj_clock_reset(cudaStream_t s, DevClock* clk) {
-  hj_clock_reset<<<1, 1, 0, s>>>(clk);
-  return launch_status("hj_clock_reset");
+  return launch_chained("hj_clock_reset", hj_clock_reset, 1, 1, 0, s, clk);
 }
 
 }  // namespace flsp

@@ -78,8 +78,7 @@ int sep_call(int what, const Ctx& c, const VelDev* v, const int* tile, size_t* b
           b.stage = stage;
           b.combine = combine;
           b.ct_explicit = ct_explicit;
-          kern<<<(unsigned)nblocks(b.m), TX * TY * TZ, PL::BYTES, c.stream>>>(b);
-          return launch_status("adv_sep_kernel");
+          return launch_chained("adv_sep_kernel", kern, (unsigned)nblocks(b.m), TX * TY * TZ, PL::BYTES, c.stream, b);
         });
       };
       if (c.basis == FLSP_BASIS_P) return body(std::true_type());

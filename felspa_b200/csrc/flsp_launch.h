@@ -121,6 +121,29 @@ inline int launch_status(const char* what) {
   return FLSP_OK;
 }
 
+// Launch of a kernel that follows the chain's protocol (chain_release /
+// chain_wait): its blocks may start while the kernel before it on the stream
+// drains.
+template <typename... KA, typename... A>
+int launch_chained(const char* what, void (*kern)(KA...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s,
+                   A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, KA(args)...);
+  const cudaError_t last = cudaGetLastError();
+  if (e == cudaSuccess) e = last;
+  if (e != cudaSuccess) return set_error(FLSP_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+  return FLSP_OK;
+}
+
 // ---------------- tables (one per unit) ----------------
 int upload_tables_adv();
 int upload_tables_hj();

@@ -19,6 +19,7 @@ constexpr double kEpsD = 2.220446049250313e-16;
 // the next n substeps (one warp); horizon >= 0 starts an advance call of that
 // length first
 __global__ void adv_clock_steps(DevClock* c, const AdvClockArgs a, AdvStep* st, int n, int commit, double horizon) {
+  chain_wait();
   if (horizon >= 0.0 && threadIdx.x == 0) adv_clock_horizon_body(c, horizon);
   adv_clock_steps_body(c, a, st, n, commit != 0);
 }
@@ -27,6 +28,7 @@ __global__ void adv_clock_horizon(DevClock* c, double time_step) {
   adv_clock_horizon_body(c, time_step);
 }
 __global__ void hj_clock_reset(DevClock* c) {
+  chain_wait();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   hj_clock_reset_body(c);
 }

@@ -135,12 +135,13 @@ __device__ __forceinline__ void weno_tile(const WenoArgs<T>& a, int slot, int pa
   T* sb = reinterpret_cast<T*>(smem_raw + PL::OFF_SB);
   const MeshArgs& m = a.m;
   const Tab1D<T>& tb = tab<T>(P);
+  if (threadIdx.x == 0) mbar_init(bar, 32);
+  __syncthreads();
+  chain_wait();
   if (tile_inactive(m, slot)) return;
   const int tile = m.tiles ? m.tiles[slot] : slot;
   const int ox = (tile % m.ntile[0]) * m.tile[0], oy = (tile / m.ntile[0]) * m.tile[1] + part * TY;
   if (oy >= m.n[1]) return;
-  if (threadIdx.x == 0) mbar_init(bar, 32);
-  __syncthreads();
   if (threadIdx.x < 32) bulk_box_rows<2, TX, TY, 1, NMB, PL::SLOT>(m, a.in, boxb, ox, oy, 0, bar);
   const int lx = (int)threadIdx.x % TX, ly = (int)threadIdx.x / TX;
   const int gx = ox + lx, gy = oy + ly, gx0 = max(ox - 1, 0);
@@ -241,6 +242,7 @@ __device__ __forceinline__ void weno_tile(const WenoArgs<T>& a, int slot, int pa
   } else {
     __syncthreads();
   }
+  chain_release();
   store_cells<2, TX, TY, 1, NBG, T>(m, sb, a.out, ox, oy, 0);
 }
 
