@@ -130,6 +130,8 @@ struct flsp_handle {
   // velocity of a coupled FE simulator (fe_pv > 0): the nodal lattice (FP64)
   int fe_pv = 0;
   double* fe_u64 = nullptr;
+  double* fe_next = nullptr;      // the next lattice, until it has been checked
+  int64_t fe_next_n = 0;
   // velocity table at the cells' and faces' quadrature points (state
   // precision, VelTabLayout): the FE field, or a velocity of several terms per
   // component; tab_ok when it holds the current velocity
@@ -138,6 +140,8 @@ struct flsp_handle {
   DevClock* clk = nullptr;
   DevClock* clk_host = nullptr;   // pinned mirror
   AdvStep* steps = nullptr;       // the clock's next substeps (kClockSteps)
+  double* pin = nullptr;          // pinned: small results on their way to the host
+  double* grad64 = nullptr;       // gradient export before the cell permutation
   int64_t* perm = nullptr;
   double* stage64 = nullptr;      // FP64 device staging (2 * dim * ndofs)
   double* partial = nullptr;
@@ -418,18 +422,30 @@ int reduce_dev(flsp_handle* h, int which, const void* phi, const void* ref, bool
   Ctx c = h->ctx();
   ST(ensure_partial(h, reduce_blocks(c)));
   ST(launch_reduce(c, which, phi, ref, with_ic ? h->ic_dev : nullptr, h->partial, h->red_out));
-  CU(cudaMemcpyAsync(out2, h->red_out, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  CU(cudaMemcpyAsync(h->pin, h->red_out, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   CU(cudaStreamSynchronize(h->stream));
+  out2[0] = h->pin[0];
+  out2[1] = h->pin[1];
   return FLSP_OK;
 }
 
-int check_finite(flsp_handle* h, const void* x) {
-  CU(cudaMemsetAsync(h->flag_dev, 0, sizeof(unsigned int), h->stream));
-  ST(launch_nonfinite(h->ctx(), x, h->ndofs, h->flag_dev));
-  unsigned int cnt = 0;
-  CU(cudaMemcpyAsync(&cnt, h->flag_dev, sizeof(cnt), cudaMemcpyDeviceToHost, h->stream));
+// the count of non-finite values a launch left in flag_dev (waits for it)
+int read_flag(flsp_handle* h, unsigned int* n) {
+  CU(cudaMemcpyAsync(h->pin, h->flag_dev, sizeof(*n), cudaMemcpyDeviceToHost, h->stream));
   CU(cudaStreamSynchronize(h->stream));
-  if (cnt) return fail(FLSP_ERR_NONFINITE, std::to_string(cnt) + " non-finite coefficients");
+  std::memcpy(n, h->pin, sizeof(*n));
+  return FLSP_OK;
+}
+
+// a device vector as n host coefficients
+int read_coeffs(flsp_handle* h, const void* src, double* out, int64_t n) {
+  const void* from = src;
+  if (h->prec != FLSP_FP64 || h->perm) {   // else the device's layout is the host's
+    ST(launch_gather(h->ctx(), src, h->stage64, h->perm));
+    from = h->stage64;
+  }
+  CU(cudaMemcpyAsync(out, from, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream));
+  CU(cudaStreamSynchronize(h->stream));
   return FLSP_OK;
 }
 
@@ -1032,6 +1048,7 @@ int flsp_create(const flsp_mesh_desc* mesh, const flsp_dg_opts* opts, flsp_handl
       return cleanup_fail(fail(FLSP_ERR_OOM, "state allocation failed"));
   if (cudaMalloc(&h->clk, sizeof(DevClock)) != cudaSuccess ||
       cudaMallocHost(&h->clk_host, sizeof(DevClock)) != cudaSuccess ||
+      cudaMallocHost(&h->pin, 64) != cudaSuccess ||
       cudaMalloc(&h->steps, kClockSteps * sizeof(AdvStep)) != cudaSuccess ||
       cudaMalloc(&h->stage64, sizeof(double) * (size_t)h->ndofs * 2 * h->dim) != cudaSuccess ||
       cudaMalloc(&h->red_out, 2 * sizeof(double)) != cudaSuccess ||
@@ -1097,6 +1114,9 @@ void flsp_destroy(flsp_handle* h) {
   if (h->clk) cudaFree(h->clk);
   if (h->clk_host) cudaFreeHost(h->clk_host);
   if (h->steps) cudaFree(h->steps);
+  if (h->pin) cudaFreeHost(h->pin);
+  if (h->grad64) cudaFree(h->grad64);
+  if (h->fe_next) cudaFree(h->fe_next);
   if (h->perm) cudaFree(h->perm);
   if (h->curv) cudaFree(h->curv);
   if (h->bc_dev) cudaFree(h->bc_dev);
@@ -1148,9 +1168,22 @@ int flsp_set_velocity_fe(flsp_handle* h, int degree, const double* values, int64
   long long nn = 1;
   for (int d = 0; d < h->dim; ++d) nn *= (long long)degree * h->m.n[d] + 1;
   if (n != (int64_t)h->dim * nn) return fail(FLSP_ERR_BAD_ARG, "FE velocity size mismatch");
-  for (int64_t i = 0; i < n; ++i)
-    if (!std::isfinite(values[i])) return fail(FLSP_ERR_BAD_ARG, "non-finite FE velocity value");
   CU(cudaSetDevice(h->dev));
+  // checked on the device (48^3, degree 2: 2.7 M values took the host 2.5 ms)
+  // in a lattice of its own: the velocity in force stays as it is until then
+  if (h->fe_next_n != n) {
+    if (h->fe_next) cudaFree(h->fe_next);
+    h->fe_next = nullptr;
+    h->fe_next_n = 0;
+    CU(cudaMalloc(&h->fe_next, (size_t)n * sizeof(double)));
+    h->fe_next_n = n;
+  }
+  CU(cudaMemsetAsync(h->flag_dev, 0, sizeof(unsigned int), h->stream));
+  CU(cudaMemcpyAsync(h->fe_next, values, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  ST(launch_nonfinite(h->stream, h->fe_next, n, h->flag_dev));
+  unsigned int bad = 0;
+  ST(read_flag(h, &bad));
+  if (bad) return fail(FLSP_ERR_BAD_ARG, "non-finite FE velocity value");
   const bool same = h->fe_pv == degree && h->fe_u64 != nullptr;
   if (!same) {
     // an FE field has no analytic terms: zero tables, time factor 1
@@ -1169,8 +1202,7 @@ int flsp_set_velocity_fe(flsp_handle* h, int degree, const double* values, int64
   std::memset(gb, 0, sizeof(gb));
   for (int a = 0; a <= degree; ++a)
     for (int j = 0; j < h->p + 2; ++j) gb[a][j] = lagrange(degree, gl, a, xq[j]);
-  // in place: ordered after the work already queued on the problem's stream
-  CU(cudaMemcpyAsync(h->fe_u64, values, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  std::swap(h->fe_u64, h->fe_next);
   Ctx c = h->ctx();
   ST(launch_fe_tabulate(c, h->fe_u64, degree, gb, h->tab));
   CU(cudaMemsetAsync(&h->clk->vd_static, 0, sizeof(double), h->stream));
@@ -1187,20 +1219,26 @@ int flsp_set_state(flsp_handle* h, const double* coeffs, int64_t n) {
   if (!h || !coeffs) return fail(FLSP_ERR_BAD_ARG, "null argument");
   if (n != h->ndofs) return fail(FLSP_ERR_BAD_ARG, "size mismatch");
   CU(cudaSetDevice(h->dev));
-  CU(cudaMemcpyAsync(h->stage64, coeffs, sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
-  ST(launch_scatter(h->ctx(), h->stage64, h->buf[h->cur], h->perm));
-  CU(cudaStreamSynchronize(h->stream));
-  return check_finite(h, h->buf[h->cur]);
+  CU(cudaMemsetAsync(h->flag_dev, 0, sizeof(unsigned int), h->stream));
+  if (h->prec == FLSP_FP64 && !h->perm) {   // the host's layout is the device's
+    double* dst = static_cast<double*>(h->buf[h->cur]);
+    CU(cudaMemcpyAsync(dst, coeffs, sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
+    ST(launch_nonfinite(h->stream, dst, n, h->flag_dev));
+  } else {
+    CU(cudaMemcpyAsync(h->stage64, coeffs, sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
+    ST(launch_scatter(h->ctx(), h->stage64, h->buf[h->cur], h->perm, h->flag_dev));
+  }
+  unsigned int bad = 0;
+  ST(read_flag(h, &bad));
+  if (bad) return fail(FLSP_ERR_NONFINITE, std::to_string(bad) + " non-finite coefficients");
+  return FLSP_OK;
 }
 
 int flsp_get_state(flsp_handle* h, double* coeffs, int64_t n) {
   if (!h || !coeffs) return fail(FLSP_ERR_BAD_ARG, "null argument");
   if (n != h->ndofs) return fail(FLSP_ERR_BAD_ARG, "size mismatch");
   CU(cudaSetDevice(h->dev));
-  ST(launch_gather(h->ctx(), h->buf[h->cur], h->stage64, h->perm));
-  CU(cudaMemcpyAsync(coeffs, h->stage64, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream));
-  CU(cudaStreamSynchronize(h->stream));
-  return FLSP_OK;
+  return read_coeffs(h, h->buf[h->cur], coeffs, n);
 }
 
 int flsp_eval_patches(flsp_handle* h, int n_sub, double* values, int64_t n) {
@@ -1369,11 +1407,9 @@ int flsp_export_solutions(flsp_handle* h, const char* path, const char* label) {
 int flsp_set_time(flsp_handle* h, double t) {
   if (!h) return fail(FLSP_ERR_BAD_ARG, "null handle");
   CU(cudaSetDevice(h->dev));
-  ST(sync_clock(h));
-  h->clk_host->t = t;
-  CU(cudaMemcpyAsync(h->clk, h->clk_host, sizeof(DevClock), cudaMemcpyHostToDevice, h->stream));
-  CU(cudaStreamSynchronize(h->stream));
-  return FLSP_OK;
+  h->pin[0] = t;
+  CU(cudaMemcpyAsync(&h->clk->t, h->pin, sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  return sync_clock(h);
 }
 
 int flsp_get_time(const flsp_handle* hc, double* t) {
@@ -1448,10 +1484,7 @@ int flsp_advect_rhs(flsp_handle* h, double t, double* phidot, int64_t n) {
   const int tmp = (h->cur + 1) % 3;
   ST(launch_adv_stage(h->ctx(), h->veldev(), h->buf[h->cur], h->buf[h->cur], h->buf[tmp], nullptr, 0,
                       kRhsOnly, host_time_factor(h->vel, t), h->adv_tile));
-  ST(launch_gather(h->ctx(), h->buf[tmp], h->stage64, h->perm));
-  CU(cudaMemcpyAsync(phidot, h->stage64, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream));
-  CU(cudaStreamSynchronize(h->stream));
-  return FLSP_OK;
+  return read_coeffs(h, h->buf[tmp], phidot, n);
 }
 
 // AdvectSimulator::advance_time(time_step, compute_single_cycle)
@@ -1479,12 +1512,14 @@ int flsp_advance_steps(flsp_handle* h, int n_steps, double t_end) {
   if (!h->has_vel) return fail(FLSP_ERR_BAD_ARG, "velocity not set");
   if (n_steps < 0) return fail(FLSP_ERR_BAD_ARG, "negative step count");
   CU(cudaSetDevice(h->dev));
-  ST(sync_clock(h));
-  const double horizon = std::isfinite(t_end) ? t_end - h->clk_host->t : INFINITY;
+  double horizon = INFINITY;
+  if (std::isfinite(t_end)) {
+    ST(sync_clock(h));
+    horizon = t_end - h->clk_host->t;
+  }
   ST(launch_adv_clock_horizon(h->stream, h->clk, horizon));
   ST(enqueue_adv_steps(h, n_steps));
-  CU(cudaStreamSynchronize(h->stream));
-  return FLSP_OK;
+  return sync_clock(h);
 }
 
 int flsp_reinit(flsp_handle* h, const flsp_reinit_opts* o, int* n_iter) {
@@ -1499,19 +1534,20 @@ int flsp_hj_gradients(flsp_handle* h, double* grads, int64_t n) {
   if (!h || !grads) return fail(FLSP_ERR_BAD_ARG, "null argument");
   if (n != 2 * h->dim * h->ndofs) return fail(FLSP_ERR_BAD_ARG, "size mismatch (2*dim*n_dofs)");
   CU(cudaSetDevice(h->dev));
-  void* tmp = nullptr;
-  CU(cudaMalloc(&tmp, (size_t)n * h->tsize));
-  int st = launch_hj(h->ctx(), h->buf[h->cur], h->buf[h->cur], tmp, nullptr, kHJGradients, 1, nullptr,
-                     h->ndofs, h->hj_tile);
-  for (int b = 0; b < 2 * h->dim && st == FLSP_OK; ++b)
-    st = launch_gather(h->ctx(), (const char*)tmp + (size_t)b * h->ndofs * h->tsize,
-                       h->stage64 + b * h->ndofs, h->perm);
-  if (st == FLSP_OK) {
-    cudaMemcpyAsync(grads, h->stage64, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream);
-    if (cudaStreamSynchronize(h->stream) != cudaSuccess) st = fail(FLSP_ERR_CUDA, "sync failed");
+  // straight into the staging buffer, or through a kept one where the cells
+  // are permuted
+  if (h->perm && !h->grad64) CU(cudaMalloc(&h->grad64, (size_t)n * sizeof(double)));
+  double* dst = h->perm ? h->grad64 : h->stage64;
+  ST(launch_hj(h->ctx(), h->buf[h->cur], h->buf[h->cur], dst, nullptr, kHJGradients, 1, nullptr, h->ndofs, h->hj_tile));
+  if (h->perm) {
+    Ctx c = h->ctx();
+    c.prec = FLSP_FP64;
+    for (int b = 0; b < 2 * h->dim; ++b)
+      ST(launch_gather(c, h->grad64 + (size_t)b * h->ndofs, h->stage64 + (size_t)b * h->ndofs, h->perm));
   }
-  cudaFree(tmp);
-  return st;
+  CU(cudaMemcpyAsync(grads, h->stage64, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream));
+  CU(cudaStreamSynchronize(h->stream));
+  return FLSP_OK;
 }
 
 int flsp_weno_limit(flsp_handle* h, int* n_troubled) {
@@ -1521,8 +1557,7 @@ int flsp_weno_limit(flsp_handle* h, int* n_troubled) {
   const int dst = (h->cur + 1) % 3;
   ST(launch_weno(h->ctx(), h->buf[h->cur], h->buf[dst], h->flag_dev, &h->clk->err));
   unsigned int cnt = 0;
-  CU(cudaMemcpyAsync(&cnt, h->flag_dev, sizeof(cnt), cudaMemcpyDeviceToHost, h->stream));
-  CU(cudaStreamSynchronize(h->stream));
+  ST(read_flag(h, &cnt));
   h->cur = dst;
   if (n_troubled) *n_troubled = (int)cnt;
   return FLSP_OK;

@@ -32,7 +32,8 @@ struct HJArgs {
   MeshArgs m;
   const T* __restrict__ phi;    // phi^k (read with halo)
   const T* __restrict__ phi0;   // phi at reinit start
-  T* __restrict__ out;          // phi^{k+1} or gradient blocks
+  T* __restrict__ out;          // phi^{k+1}
+  double* __restrict__ grad;    // gradient blocks (the export)
   DevClock* clk;
   int mode;
   int rk;                       // reinit RK order (all stages see the same L)
@@ -138,8 +139,8 @@ __global__ void __launch_bounds__(256) hj_gradient_kernel(const HJArgs<T> a) {
         T bs = T(0);
 #pragma unroll
         for (int b = 0; b < N1; ++b) bs -= tb.A[aa][b] * c[base + b * st[e]];
-        a.out[(long long)e * a.block + cell * m.nb + k] = (bs + tb.L1[aa] * tup - tb.L0[aa] * tnl) * ih;
-        a.out[(long long)(DIM + e) * a.block + cell * m.nb + k] = (bs + tb.L1[aa] * tnu - tb.L0[aa] * tlo) * ih;
+        a.grad[(long long)e * a.block + cell * m.nb + k] = (bs + tb.L1[aa] * tup - tb.L0[aa] * tnl) * ih;
+        a.grad[(long long)(DIM + e) * a.block + cell * m.nb + k] = (bs + tb.L1[aa] * tnu - tb.L0[aa] * tlo) * ih;
       }
     }
   }

@@ -127,6 +127,7 @@ int launch_hj(const Ctx& c, const void* phi, const void* phi0, void* out, DevClo
     if (mode == kHJGradients) {   // the export, every cell
       static const int tg[3] = {HjgTile<DIM>::X, HjgTile<DIM>::Y, HjgTile<DIM>::Z};
       set_tile(a.m, DIM, tg);
+      a.grad = reinterpret_cast<double*>(out);
       hj_gradient_kernel<DIM, P, T>
           <<<(unsigned)nblocks(a.m), tg[0] * tg[1] * tg[2], hjg_smem_bytes<DIM, P, T>(), c.stream>>>(a);
       return launch_status("hj_gradient_kernel");

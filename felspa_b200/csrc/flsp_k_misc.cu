@@ -180,12 +180,12 @@ int launch_reduce(const Ctx& c, int which, const void* phi, const void* ref,
 
 static int grid_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 148 * 16); }
 
-int launch_scatter(const Ctx& c, const double* src, void* dst, const int64_t* perm) {
+int launch_scatter(const Ctx& c, const double* src, void* dst, const int64_t* perm, unsigned int* count) {
   const long long n = c.m.ncell * c.m.nb;
   if (c.prec == FLSP_FP64)
-    scatter_state<double><<<grid_for(n), 256, 0, c.stream>>>(src, (double*)dst, perm, c.m.ncell, c.m.nb);
+    scatter_state<double><<<grid_for(n), 256, 0, c.stream>>>(src, (double*)dst, perm, c.m.ncell, c.m.nb, count);
   else
-    scatter_state<float><<<grid_for(n), 256, 0, c.stream>>>(src, (float*)dst, perm, c.m.ncell, c.m.nb);
+    scatter_state<float><<<grid_for(n), 256, 0, c.stream>>>(src, (float*)dst, perm, c.m.ncell, c.m.nb, count);
   return launch_status("scatter_state");
 }
 
@@ -198,11 +198,8 @@ int launch_gather(const Ctx& c, const void* src, double* dst, const int64_t* per
   return launch_status("gather_state");
 }
 
-int launch_nonfinite(const Ctx& c, const void* x, long long n, unsigned int* count) {
-  if (c.prec == FLSP_FP64)
-    nonfinite_kernel<double><<<grid_for(n), 256, 0, c.stream>>>((const double*)x, n, count);
-  else
-    nonfinite_kernel<float><<<grid_for(n), 256, 0, c.stream>>>((const float*)x, n, count);
+int launch_nonfinite(cudaStream_t s, const double* x, long long n, unsigned int* count) {
+  nonfinite_kernel<double><<<grid_for(n), 256, 0, s>>>(x, n, count);
   return launch_status("nonfinite_kernel");
 }
 

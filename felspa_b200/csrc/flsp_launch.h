@@ -221,9 +221,10 @@ int launch_fe_tabulate(const Ctx& c, const double* u64, int pv, const double (*g
 int launch_reduce(const Ctx& c, int which, const void* phi, const void* ref,
                   const flsp_ic_desc* ic_dev, double* partial, double* out_dev);
 int reduce_blocks(const Ctx& c);
-int launch_scatter(const Ctx& c, const double* src, void* dst, const int64_t* perm);
+// *count += the non-finite values written
+int launch_scatter(const Ctx& c, const double* src, void* dst, const int64_t* perm, unsigned int* count);
 int launch_gather(const Ctx& c, const void* src, double* dst, const int64_t* perm);
-int launch_nonfinite(const Ctx& c, const void* x, long long n, unsigned int* count);
+int launch_nonfinite(cudaStream_t s, const double* x, long long n, unsigned int* count);
 
 // the next n <= kClockSteps substeps into steps; commit: the clock moves past
 // them; horizon >= 0: an advance call of that length starts

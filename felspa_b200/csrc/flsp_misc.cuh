@@ -35,16 +35,24 @@ __global__ void hj_clock_reset(DevClock* c) {
 // ---------------------------------------------------------------------
 // host DoF order <-> device layout (optional cell permutation)
 // ---------------------------------------------------------------------
+// count: the non-finite values written
 template <typename T>
 __global__ void scatter_state(const double* __restrict__ src, T* __restrict__ dst,
-                              const int64_t* __restrict__ perm, long long ncell, int nb) {
+                              const int64_t* __restrict__ perm, long long ncell, int nb, unsigned int* count) {
   const long long n = ncell * nb;
+  unsigned int bad = 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    const long long k = i / nb, j = i - k * nb;
-    const long long cell = perm ? perm[k] : k;
-    dst[cell * nb + j] = T(src[i]);
+    long long o = i;
+    if (perm) {
+      const long long k = i / nb;
+      o = perm[k] * nb + (i - k * nb);
+    }
+    const T v = T(src[i]);
+    if (!isfinite((double)v)) ++bad;
+    dst[o] = v;
   }
+  if (bad) atomicAdd(count, bad);
 }
 
 template <typename T>
@@ -53,9 +61,12 @@ __global__ void gather_state(const T* __restrict__ src, double* __restrict__ dst
   const long long n = ncell * nb;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    const long long k = i / nb, j = i - k * nb;
-    const long long cell = perm ? perm[k] : k;
-    dst[i] = double(src[cell * nb + j]);
+    long long o = i;
+    if (perm) {
+      const long long k = i / nb;
+      o = perm[k] * nb + (i - k * nb);
+    }
+    dst[i] = double(src[o]);
   }
 }
 

@@ -73,6 +73,8 @@ struct flsp_mlp {
   int* err = nullptr;                  // device error word
   float* hbuf = nullptr;               // host staging (pinned)
   size_t hbuf_bytes = 0;
+  float* io = nullptr;                 // device side of it
+  size_t io_bytes = 0;
   // training pairs (device): features n x n_in, targets n x n_out
   int64_t n_pairs = 0, pair_cap = 0;
   float* feat = nullptr;
