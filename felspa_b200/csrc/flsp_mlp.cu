@@ -132,12 +132,19 @@ __global__ void k_out_grad(const float* __restrict__ y, int ldy, const float* __
   }
 }
 
-// out[n] = sum_p part[p * ld + n] in a fixed order, n < n_valid
+// out[n] = sum_p part[p * ld + n] in a fixed order, n < n_valid: a block of
+// 32 columns x 8 slices of the rows, the slices' sums then added in order (one
+// thread per column: 11 us for 256 rows)
 __global__ void k_colsum(const float* __restrict__ part, int P, int ld, int n_valid, float* __restrict__ out) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= n_valid) return;
+  __shared__ double sl[8][32];
+  const int n = blockIdx.x * 32 + (threadIdx.x & 31), k = threadIdx.x >> 5;
   double s = 0.0;
-  for (int p = 0; p < P; ++p) s += part[(long long)p * ld + n];
+  if (n < n_valid)
+    for (int p = (int)((long long)P * k / 8); p < (int)((long long)P * (k + 1) / 8); ++p) s += part[(long long)p * ld + n];
+  sl[k][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (k > 0 || n >= n_valid) return;
+  for (int i = 1; i < 8; ++i) s += sl[i][threadIdx.x];
   out[n] = (float)s;
 }
 
@@ -338,7 +345,7 @@ static int gemm(cudaStream_t st, const TcGemmArgs& a, int ksplit = 1) {
     return set_error(FLSP_ERR_BAD_ARG, "tensor-core GEMM: bad K split");
   const size_t smem = tc_gemm_smem(a.N);
   MST(gemm_attr<EPI>());
-  tc_gemm_kernel<EPI><<<dim3(a.M / kTcBM, ksplit), 128, smem, st>>>(a);
+  tc_gemm_kernel<EPI><<<dim3(a.M / kTcBM, ksplit), kTcThreads, smem, st>>>(a);
   return launch_status("tc_gemm_kernel");
 }
 
@@ -537,7 +544,7 @@ static int mlp_backward_dev(flsp_mlp* net, int64_t n) {
     b.colsum = net->colsum;
     b.err = net->err;
     MST(gemm<kEpiBackAct>(st, b));
-    k_colsum<<<1, 256, 0, st>>>(net->colsum, R / 32, 256, net->L[l - 1].n_out, net->g + net->L[l - 1].b_off);
+    k_colsum<<<8, 256, 0, st>>>(net->colsum, R / 32, 256, net->L[l - 1].n_out, net->g + net->L[l - 1].b_off);
     MST(launch_status("k_colsum"));
     G = net->gh[cur];
     gk = 256;
@@ -562,7 +569,7 @@ static int output_grad(flsp_mlp* net, int64_t n, const float* dy_dev, const int*
   const int nblk = R / 256 + 1;
   out_grad_launch(net, nblk, dy_dev, net->targ, idx, (int)n, R);
   MST(launch_status("k_out_grad"));
-  k_colsum<<<1, 32, 0, net->stream>>>(net->colsum, nblk, net->y_ld, net->n_out, net->g + net->L[4].b_off);
+  k_colsum<<<(net->n_out + 31) / 32, 256, 0, net->stream>>>(net->colsum, nblk, net->y_ld, net->n_out, net->g + net->L[4].b_off);
   MST(launch_status("k_colsum"));
   k_sum_double<<<1, 1, 0, net->stream>>>(net->loss_part, nblk, net->loss_dev);
   return launch_status("k_sum_double");

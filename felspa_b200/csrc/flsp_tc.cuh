@@ -18,9 +18,11 @@
 // One CTA computes a 128 x N tile (N <= 256, N % 16 == 0): warp 0 issues
 // the bulk copies of a 3-stage pipeline, one thread of warp 1 issues the
 // MMAs (K = 16 per instruction) and commits each stage back to the
-// producer through an mbarrier, and all four warps read the accumulator
-// out of TMEM (warp w owns lanes 32w..32w+31 = tile rows) for the
-// epilogue.  Every wait is bounded; a timeout sets a bit in the error word.
+// producer through an mbarrier, and all sixteen warps read the accumulator
+// out of TMEM (warp w owns lanes 32 (w % 4).. = tile rows, and every fourth
+// block of 16 columns) for the epilogue, which bounds these shapes (K <= 768:
+// the erf of 32,768 elements per tile against 17 MFLOP): 8192 x 256 x 256 with
+// GELU and its derivative 40 us with four warps, 14 so.  Every wait is bounded; a timeout sets a bit in the error word.
 #pragma once
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -32,6 +34,7 @@ namespace flsp {
 constexpr int kTcBM = 128;      // rows per CTA tile (MMA M)
 constexpr int kTcBK = 64;       // K per pipeline stage
 constexpr int kTcStages = 3;
+constexpr int kTcThreads = 512; // four warps per 32 rows of the epilogue
 constexpr int kErrTcTimeout = 2;   // error-word bit: a tensor-core pipeline wait ran out
 
 // offset (elements) of (r, k) in a packed R x K operand
@@ -132,7 +135,7 @@ __device__ __forceinline__ float gelu_d_f(float x) {
 }
 
 template <int EPI>
-__global__ void __launch_bounds__(128, 1) tc_gemm_kernel(const TcGemmArgs a) {
+__global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const TcGemmArgs a) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // layout: [stages][A chunk 16 KB][B chunk N*128 B] | barriers | TMEM slot
   const int N = a.N;
@@ -206,10 +209,11 @@ __global__ void __launch_bounds__(128, 1) tc_gemm_kernel(const TcGemmArgs a) {
   if (!ok && a.err && lane == 0) atomicOr(a.err, kErrTcTimeout);
   tc_fence_after();
 
-  const int r = m0 + warp * 32 + lane;   // tile row owned by this thread
-  const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
+  const int wr = warp & 3;             // a warp reads the TMEM lanes of its place in the warpgroup
+  const int r = m0 + wr * 32 + lane;   // tile row owned by this thread
+  const uint32_t trow = tmem + ((uint32_t)(wr * 32) << 16);
   float csum[16];
-  for (int c0 = 0; c0 < N; c0 += 16) {
+  for (int c0 = (warp >> 2) * 16; c0 < N; c0 += kTcThreads / 8) {
     float v[16];
     tmem_ld16(trow + (uint32_t)c0, v);
     if (!ok) continue;
@@ -219,7 +223,12 @@ __global__ void __launch_bounds__(128, 1) tc_gemm_kernel(const TcGemmArgs a) {
       for (int i = 0; i < 16; ++i) {
         const float z = v[i] + a.bias[c0 + i];
         o[i] = __float2bfloat16_rn(gelu_f(z));
-        if (a.gd_out) a.gd_out[(long long)r * N + c0 + i] = gelu_d_f(z);
+        if (a.gd_out) v[i] = gelu_d_f(z);
+      }
+      if (a.gd_out) {
+        float4* gd = reinterpret_cast<float4*>(a.gd_out + (long long)r * N + c0);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) gd[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
       }
       uint4* dst0 = reinterpret_cast<uint4*>(a.out_bf16 + packed_off(r, c0, a.M));
       uint4* dst1 = reinterpret_cast<uint4*>(a.out_bf16 + packed_off(r, c0 + 8, a.M));
@@ -231,9 +240,13 @@ __global__ void __launch_bounds__(128, 1) tc_gemm_kernel(const TcGemmArgs a) {
         if (c0 + i < a.n_valid && r < a.m_valid) a.y[(long long)r * a.ldy + c0 + i] = v[i] + a.bias[c0 + i];
     } else if constexpr (EPI == kEpiBackAct) {
       __align__(16) __nv_bfloat16 o[16];
+      __align__(16) float gd[16];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        reinterpret_cast<float4*>(gd)[i] = *reinterpret_cast<const float4*>(a.gd_in + (long long)r * N + c0 + 4 * i);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const float g = v[i] * a.gd_in[(long long)r * N + c0 + i];
+        const float g = v[i] * gd[i];
         o[i] = __float2bfloat16_rn(g);
         csum[i] = g;
       }
@@ -255,7 +268,7 @@ __global__ void __launch_bounds__(128, 1) tc_gemm_kernel(const TcGemmArgs a) {
         if (lane == 0) {
 #pragma unroll
           for (int i = 0; i < 16; ++i)
-            a.colsum[((long long)blockIdx.x * 4 + warp) * N + c0 + i] = csum[i];
+            a.colsum[((long long)blockIdx.x * 4 + wr) * N + c0 + i] = csum[i];
         }
       }
     } else {
