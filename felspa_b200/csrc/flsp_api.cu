@@ -137,10 +137,11 @@ struct flsp_handle {
   // component; tab_ok when it holds the current velocity
   void* tab = nullptr;
   bool tab_ok = false;
+  char* small = nullptr;          // the small device blocks: clk, steps, red_out, flag_dev, ic_dev
   DevClock* clk = nullptr;
   DevClock* clk_host = nullptr;   // pinned mirror
   AdvStep* steps = nullptr;       // the clock's next substeps (kClockSteps)
-  double* pin = nullptr;          // pinned: small results on their way to the host
+  double* pin = nullptr;          // pinned, behind clk_host: small results on their way to the host
   double* grad64 = nullptr;       // gradient export before the cell permutation
   int64_t* perm = nullptr;
   double* stage64 = nullptr;      // FP64 device staging (2 * dim * ndofs)
@@ -1046,15 +1047,20 @@ int flsp_create(const flsp_mesh_desc* mesh, const flsp_dg_opts* opts, flsp_handl
     // padded: the stage kernel's bulk row copies round their ends up to 16 bytes
     if (cudaMalloc(&h->buf[i], h->ndofs * h->tsize + kStatePad) != cudaSuccess)
       return cleanup_fail(fail(FLSP_ERR_OOM, "state allocation failed"));
-  if (cudaMalloc(&h->clk, sizeof(DevClock)) != cudaSuccess ||
-      cudaMallocHost(&h->clk_host, sizeof(DevClock)) != cudaSuccess ||
-      cudaMallocHost(&h->pin, 64) != cudaSuccess ||
-      cudaMalloc(&h->steps, kClockSteps * sizeof(AdvStep)) != cudaSuccess ||
-      cudaMalloc(&h->stage64, sizeof(double) * (size_t)h->ndofs * 2 * h->dim) != cudaSuccess ||
-      cudaMalloc(&h->red_out, 2 * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&h->ic_dev, sizeof(flsp_ic_desc)) != cudaSuccess ||
-      cudaMalloc(&h->flag_dev, sizeof(unsigned int)) != cudaSuccess)
+  // the small blocks in one device and one pinned allocation
+  constexpr size_t at_steps = 512, at_red = at_steps + kClockSteps * sizeof(AdvStep), at_flag = at_red + 64,
+                   at_ic = at_flag + 64;
+  static_assert(sizeof(DevClock) <= at_steps && at_red % 16 == 0, "offsets of the small blocks");
+  if (cudaMalloc(&h->small, at_ic + sizeof(flsp_ic_desc)) != cudaSuccess ||
+      cudaMallocHost(&h->clk_host, at_steps + 64) != cudaSuccess ||
+      cudaMalloc(&h->stage64, sizeof(double) * (size_t)h->ndofs * 2 * h->dim) != cudaSuccess)
     return cleanup_fail(fail(FLSP_ERR_OOM, "allocation failed"));
+  h->clk = reinterpret_cast<DevClock*>(h->small);
+  h->steps = reinterpret_cast<AdvStep*>(h->small + at_steps);
+  h->red_out = reinterpret_cast<double*>(h->small + at_red);
+  h->flag_dev = reinterpret_cast<unsigned int*>(h->small + at_flag);
+  h->ic_dev = reinterpret_cast<flsp_ic_desc*>(h->small + at_ic);
+  h->pin = reinterpret_cast<double*>(reinterpret_cast<char*>(h->clk_host) + at_steps);
   cudaMemset(h->clk, 0, sizeof(DevClock));
   cudaMemset(h->buf[0], 0, h->ndofs * h->tsize);
   if (mesh->host_cell_order) {
@@ -1111,10 +1117,8 @@ void flsp_destroy(flsp_handle* h) {
     if (q) cudaFree(q);
   if (h->lrn_count_host) cudaFreeHost(h->lrn_count_host);
   if (h->lrn_ev) cudaEventDestroy(h->lrn_ev);
-  if (h->clk) cudaFree(h->clk);
+  if (h->small) cudaFree(h->small);
   if (h->clk_host) cudaFreeHost(h->clk_host);
-  if (h->steps) cudaFree(h->steps);
-  if (h->pin) cudaFreeHost(h->pin);
   if (h->grad64) cudaFree(h->grad64);
   if (h->fe_next) cudaFree(h->fe_next);
   if (h->perm) cudaFree(h->perm);
@@ -1122,9 +1126,6 @@ void flsp_destroy(flsp_handle* h) {
   if (h->bc_dev) cudaFree(h->bc_dev);
   if (h->stage64) cudaFree(h->stage64);
   if (h->partial) cudaFree(h->partial);
-  if (h->red_out) cudaFree(h->red_out);
-  if (h->ic_dev) cudaFree(h->ic_dev);
-  if (h->flag_dev) cudaFree(h->flag_dev);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
 }
