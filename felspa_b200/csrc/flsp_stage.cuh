@@ -74,7 +74,9 @@ __device__ __forceinline__ void combine_rows(const MeshArgs& m, const CellP& cel
                                              bool active, int ox, int oy, int oz) {
   // ---- RK combination fused into the coalesced store: one warp per row of
   // cells along x; stage input from the box, phi^n from HBM, all of a
-  // lane's phi^n loads issued before the first use
+  // lane's phi^n loads issued before the first use.  Plain loads: the kernel
+  // before may still write phi^n when this one starts (chain_wait), which the
+  // read-only path does not allow for
   const Combine<T> comb(combine, dt);
   const bool need_n = combine == kRK2b || combine == kRK3b || combine == kRK3c;
   constexpr int NROW = TY * TZ, ROWE = TX * NBG;
@@ -104,7 +106,7 @@ __device__ __forceinline__ void combine_rows(const MeshArgs& m, const CellP& cel
 #pragma unroll
         for (int k = 0; k < KV; ++k) {
           const int e = lane + 32 * k;
-          pn[jj][k] = (need_n && active && rok && e < RV) ? __ldg(src + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+          pn[jj][k] = (need_n && active && rok && e < RV) ? src[e] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
       }
 #pragma unroll
@@ -150,7 +152,7 @@ __device__ __forceinline__ void combine_rows(const MeshArgs& m, const CellP& cel
 #pragma unroll
         for (int k = 0; k < KPR; ++k) {
           const int e = lane + 32 * k;
-          pn[jj][k] = (need_n && active && rok && e < nx * NBG) ? __ldg(phi_n + gbase + e) : T(0);
+          pn[jj][k] = (need_n && active && rok && e < nx * NBG) ? phi_n[gbase + e] : T(0);
         }
       }
 #pragma unroll
