@@ -608,6 +608,12 @@ static int ensure_staging(flsp_mlp* net, size_t bytes) {
   return FLSP_OK;
 }
 
+// one size for a batch's forward and backward calls: the second of them finds
+// its buffers there
+static int ensure_call_staging(flsp_mlp* net, size_t n) {
+  return ensure_staging(net, (std::max(n, (size_t)net->n_params) + 1) * 4);
+}
+
 // the device staging of a very large batch is not kept
 static void release_staging(flsp_mlp* net) {
   if (net->io_bytes <= 4 * kPinnedMax) return;
@@ -803,7 +809,7 @@ int flsp_mlp_forward(flsp_mlp* net, const float* x, int64_t batch, float* y) {
   MCU(cudaSetDevice(net->dev));
   MST(mlp_ensure_cap(net, batch));
   const size_t nx = (size_t)batch * net->n_in, ny = (size_t)batch * net->n_out;
-  MST(ensure_staging(net, (std::max(nx, ny) + 1) * 4));
+  MST(ensure_call_staging(net, nx + ny));
   MST(stage_in(net, x, 0, nx));
   MST(mlp_pack_input(net, net->io, nullptr, batch, nullptr));
   MST(mlp_forward_dev(net, batch, false, nullptr));
@@ -821,7 +827,7 @@ int flsp_mlp_backward(flsp_mlp* net, const float* x, const float* dy, int64_t ba
   MCU(cudaSetDevice(net->dev));
   MST(mlp_ensure_cap(net, batch));
   const size_t nx = (size_t)batch * net->n_in, ny = (size_t)batch * net->n_out;
-  MST(ensure_staging(net, (std::max(nx + ny, (size_t)net->n_params) + 1) * 4));
+  MST(ensure_call_staging(net, nx + ny));
   MST(stage_in(net, x, 0, nx));
   MST(stage_in(net, dy, nx, ny));
   MST(mlp_pack_input(net, net->io, nullptr, batch, nullptr));
