@@ -20,10 +20,15 @@
 // [comp][point][cell], then w_q u_E / h_E at the tile's faces [point][slot]
 // (faces of two tiles twice), so every load of a warp is contiguous and the
 // weights cost nothing.
-// What bounds it: the table, 1.06 KB per cell and stage (3D Q2 FP32), from
-// L2 or HBM, and latency.  Against one thread per cell with every point
-// summed from all modes (128 registers, 16 warps per SM): 48^3 Q2 FP32
-// 131 -> 43 us a stage, 256^2 11.6 -> 8.2.
+// In 2D the tile's slice comes to shared memory by one bulk copy, issued before
+// the kernel before has finished; in 3D (64 KB at Q2 FP32) it would cost the
+// CTAs that hide its latency, and the threads read it from L2 or HBM.
+// What bounds it: in 3D the table, 1.06 KB per cell and stage (Q2 FP32), and
+// latency; in 2D latency.  Against one thread per cell with every point summed
+// from all modes (128 registers, 16 warps per SM): 48^3 Q2 FP32 131 -> 43 us a
+// stage, 256^2 11.6 -> 8.2.  A batched stage of 16 degree-3 problems (248,000
+// cells, FP32), where the long-scoreboard stall was the largest: 85 us with the
+// table read by the threads, 20 warps per SM; see advtab_min_blocks.
 #pragma once
 #include "flsp_hjs.cuh"
 #include "flsp_stage.cuh"
@@ -58,13 +63,24 @@ struct AdvTabPlan {
   static constexpr size_t OFF_FL = OFF_BOX + (size_t)NROWS * SLOT;                          // [NF][NFT]
   static constexpr size_t OFF_UB = (OFF_FL + (size_t)NF * LY::NFT * sizeof(T) + 15) / 16 * 16;   // [NQ][2][NU][N]
   static constexpr size_t OFF_SB = OFF_UB + (size_t)NQ * 2 * NU * TL::N * sizeof(T);        // [N][NBG]
-  static constexpr size_t BYTES = OFF_SB + (size_t)TL::N * NBG * sizeof(T);
+  static constexpr size_t OFF_TB = (OFF_SB + (size_t)TL::N * NBG * sizeof(T) + 15) / 16 * 16;
+  // 2D: the tile's table slice (15.7 KB at Q3 FP32) is brought into shared memory
+  static constexpr bool STAGED = DIM == 2;
+  static constexpr unsigned TBYTES = LY::entries(NQ) * sizeof(T);
+  static_assert(TBYTES % 16 == 0, "bulk copies move 16-byte pieces");
+  static constexpr size_t BYTES = OFF_TB + (STAGED ? TBYTES : 0);
 };
 
-// CTAs per SM the registers are held to: FP32 3D three (24 warps)
+// CTAs per SM the registers are held to.  3D FP32: three (24 warps).  2D: as
+// many as cost no spills worth the name (P = 3 FP32: 64 -> 48 registers with 8
+// bytes spilled, 20 -> 40 warps per SM; P = 2: 52 -> 40, 32 -> 48 warps; FP64
+// P = 3: 106 -> 96, 10 -> 20 warps, P = 2: 76 -> 64, 24 -> 32 warps): with the
+// table in shared memory 48 uneven problems of degrees 1..3 took 22.4 ms without
+// the bounds, 20.7 with them, in FP64 (20 steps) 26.8 and 23.3.
 template <int DIM, int P, typename T>
 constexpr int advtab_min_blocks() {
-  return DIM == 3 && sizeof(T) == 4 ? 3 : 1;
+  if (DIM == 3) return sizeof(T) == 4 ? 3 : 1;
+  return sizeof(T) == 4 ? (P == 3 ? 4 : P == 2 ? 6 : 8) : (P == 3 ? 2 : P == 2 ? 4 : 1);
 }
 
 // one tile of a stage; every thread of the block calls it
@@ -92,8 +108,14 @@ __device__ __forceinline__ void adv_tab_tile(const AdvTabArgs<T>& a, int tile) {
     o[1] = (b % m.ntile[1]) * TY;
     o[2] = DIM > 2 ? (b / m.ntile[1]) * TZ : 0;
   }
-  if (threadIdx.x == 0) mbar_init(bar, 32);
+  if (threadIdx.x == 0) mbar_init(bar, 32 + (PL::STAGED ? 1 : 0));
   __syncthreads();
+  // the table does not change during a run; the field does
+  const T* tabg = a.tab + (size_t)tile * LY::template entries<NQ>();
+  if (PL::STAGED && threadIdx.x == 0) {
+    mbar_arrive_expect_tx(bar, PL::TBYTES);
+    bulk_g2s(smem_raw + PL::OFF_TB, tabg, PL::TBYTES, bar);
+  }
   chain_wait();
   if (threadIdx.x < 32) bulk_box_rows<DIM, TX, TY, TZ, NMB, PL::SLOT>(m, a.phi_s, boxb, o[0], o[1], o[2], bar);
   const int cl = (int)threadIdx.x % NT, k = (int)threadIdx.x / NT;   // cell, Gauss plane
@@ -110,8 +132,12 @@ __device__ __forceinline__ void adv_tab_tile(const AdvTabArgs<T>& a, int tile) {
   const T ct = a.step ? T(a.step->ct[a.stage]) : T(a.ct_explicit);
   const T dt = a.step ? T(a.step->dt) : T(a.dt_explicit);
   const bool active = a.step ? (a.step->active != 0) : true;
-  const T* tabc = a.tab + (size_t)tile * LY::template entries<NQ>();   // the tile's cells
-  const T* tabf = tabc + (size_t)DIM * NQD * NT;                       // and faces
+  const T* tabc = PL::STAGED ? reinterpret_cast<const T*>(smem_raw + PL::OFF_TB) : tabg;   // the tile's cells
+  const T* tabf = tabc + (size_t)DIM * NQD * NT;                                           // and faces
+  auto entry = [](const T* p) -> T {
+    if constexpr (PL::STAGED) return *p;
+    else return __ldg(p);
+  };
   T Lk[N1];
 #pragma unroll
   for (int b = 0; b < N1; ++b) Lk[b] = tb.Lq[b][k];
@@ -133,7 +159,7 @@ __device__ __forceinline__ void adv_tab_tile(const AdvTabArgs<T>& a, int tile) {
     T u[NQF];
     const T* uf = tabf + LY::off(E) + r;
 #pragma unroll
-    for (int q = 0; q < NQF; ++q) u[q] = __ldg(uf + (size_t)q * LY::NFT);
+    for (int q = 0; q < NQF; ++q) u[q] = entry(uf + (size_t)q * LY::NFT);
     // which side is upwind at the points (the time factor's sign with it)
     bool some_m = false, some_p = false;
 #pragma unroll
@@ -269,9 +295,9 @@ __device__ __forceinline__ void adv_tab_tile(const AdvTabArgs<T>& a, int tile) {
       const T* tq = tabc + (size_t)((DIM > 2 ? NQ * qy + NQF * k : NQ * k)) * NT + cl;
 #pragma unroll
       for (int qx = 0; qx < NQ; ++qx) {
-        f0[qx] = __ldg(tq + (size_t)qx * NT);
-        f1[qx] = __ldg(tq + (size_t)(NQD + qx) * NT);
-        if constexpr (DIM > 2) f2[qx] = __ldg(tq + (size_t)(2 * NQD + qx) * NT);
+        f0[qx] = entry(tq + (size_t)qx * NT);
+        f1[qx] = entry(tq + (size_t)(NQD + qx) * NT);
+        if constexpr (DIM > 2) f2[qx] = entry(tq + (size_t)(2 * NQD + qx) * NT);
       }
 #pragma unroll
       for (int aa = 0; aa < N1; ++aa) {
