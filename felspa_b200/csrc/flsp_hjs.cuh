@@ -71,10 +71,14 @@ struct HjsPlan {
 // CTAs per SM the registers are held to: FP32 3D, as many as the shared
 // memory admits (80 registers, 24 warps: left to itself the compiler takes
 // 105 and two CTAs, and the kernel is no faster than before it lost a third
-// of its instructions)
+// of its instructions).  2D P = 3 one more than its registers would allow
+// (FP32 72 -> 64 registers, 20 -> 30 warps; FP64 116 -> 96, 10 -> 20 warps:
+// inviscid 233x190 run 4.07 -> 3.89 ms, band reinit of 256x240 6.4 -> 5.7);
+// P = 2 spills when held (256^2 run 3.00 -> 3.02 ms) and is left alone.
 template <int DIM, int P, typename T>
 constexpr int hjs_min_blocks() {
-  return DIM == 3 && sizeof(T) == 4 ? (P == 1 ? 4 : 3) : 1;
+  if (DIM == 2) return P == 3 ? (sizeof(T) == 4 ? 3 : 2) : 1;
+  return sizeof(T) == 4 ? (P == 1 ? 4 : 3) : 1;
 }
 
 // smooth sign from phi0's value and (scaled) gradient at a point, with the
