@@ -151,7 +151,6 @@ struct flsp_handle {
   flsp_ic_desc* ic_dev = nullptr;
   unsigned int* flag_dev = nullptr;
   int n_since_reinit = 0;
-  void* qbuf = nullptr;     // LDG alternating gradient (dim blocks)
   void* rdiff = nullptr;    // LDG diffusion RHS
   int adv_tile[3] = {0, 0, 0};
   int hj_tile[3] = {0, 0, 0};
@@ -170,7 +169,7 @@ struct flsp_handle {
   cudaEvent_t lrn_ev = nullptr;   // orders the network's stream with the handle's
   // compute-restricted narrow band of the reinitialisation
   int* nb_flags = nullptr;    // ncell band flags
-  int* nb_lists = nullptr;    // 3 tile lists of ncell entries (HJ, LDG, WENO)
+  int* nb_lists = nullptr;    // 3 tile lists of ncell entries (HJ, LDG, WENO), then a flag per LDG tile
   int* nb_counts = nullptr;   // their device counts
   bool nb_use[3] = {false, false, false};   // lists in force for the launches
   std::map<unsigned long long, GraphEntry> graphs;
@@ -203,6 +202,7 @@ struct flsp_handle {
       c.nb_tiles[k] = nb_use[k] ? nb_lists + (size_t)k * m.ncell : nullptr;
       c.nb_count[k] = nb_use[k] ? nb_counts + k : nullptr;
     }
+    c.nb_ldg_listed = nb_use[kNbLdg] ? nb_lists + 3 * (size_t)m.ncell : nullptr;
     c.hj_stab = hj_stab;
     return c;
   }
@@ -309,9 +309,8 @@ int prepare_kernels(flsp_handle* h) {
   return FLSP_OK;
 }
 
-// LDG viscosity buffers (allocated outside any stream capture)
+// LDG viscosity buffer (allocated outside any stream capture)
 int ensure_ldg_buffers(flsp_handle* h) {
-  if (!h->qbuf) CU(cudaMalloc(&h->qbuf, (size_t)h->dim * h->ndofs * h->tsize));
   if (!h->rdiff) CU(cudaMalloc(&h->rdiff, (size_t)h->ndofs * h->tsize));
   return FLSP_OK;
 }
@@ -403,8 +402,7 @@ int enqueue_hj_step(flsp_handle* h, const flsp_reinit_opts* o, int phi0_idx, boo
   const int dst = (src == phi0_idx) ? (phi0_idx + 1) % 3 : other(src, phi0_idx);
   const void* rdiff = nullptr;
   if (o->viscosity > 0.0) {   // LDGDiffusionTerm of the current solution (ldg.cc:249-298)
-    ST(launch_ldg(h->ctx(), h->buf[src], h->qbuf, h->ndofs, o->viscosity, 0));
-    ST(launch_ldg(h->ctx(), h->qbuf, h->rdiff, h->ndofs, o->viscosity, 1));
+    ST(launch_ldg(h->ctx(), h->buf[src], h->rdiff, o->viscosity, &h->clk->err));
     rdiff = h->rdiff;
   }
   ST(launch_hj(h->ctx(), h->buf[src], h->buf[phi0_idx], h->buf[dst], h->clk, kHJStep, o->rk_order, &step,
@@ -489,7 +487,7 @@ int validate_reinit(const flsp_handle* h, const flsp_reinit_opts* o) {
 int ensure_band_buffers(flsp_handle* h) {
   if (!h->nb_flags) {
     CU(cudaMalloc(&h->nb_flags, (size_t)h->m.ncell * sizeof(int)));
-    CU(cudaMalloc(&h->nb_lists, 3 * (size_t)h->m.ncell * sizeof(int)));
+    CU(cudaMalloc(&h->nb_lists, 4 * (size_t)h->m.ncell * sizeof(int)));
     CU(cudaMalloc(&h->nb_counts, 3 * sizeof(int)));
   }
   return FLSP_OK;
@@ -517,9 +515,9 @@ int band_begin(flsp_handle* h, const flsp_reinit_opts* o, int phi0, bool limiter
   h->nb_use[kNbHJ] = true;
   if (o->viscosity > 0.0) {
     ST(launch_band_tiles(c, h->nb_flags, h->dim == 2 ? kLdgTile2 : kLdgTile3, margin,
-                         h->nb_lists + (size_t)kNbLdg * h->m.ncell, h->nb_counts + kNbLdg));
+                         h->nb_lists + (size_t)kNbLdg * h->m.ncell, h->nb_counts + kNbLdg,
+                         h->nb_lists + 3 * (size_t)h->m.ncell));
     h->nb_use[kNbLdg] = true;
-    CU(cudaMemsetAsync(h->qbuf, 0, (size_t)h->dim * h->ndofs * h->tsize, h->stream));
     CU(cudaMemsetAsync(h->rdiff, 0, (size_t)h->ndofs * h->tsize, h->stream));
   }
   if (limiter) {
@@ -1103,7 +1101,6 @@ void flsp_destroy(flsp_handle* h) {
   clear_graphs(h);
   for (int i = 0; i < 3; ++i) if (h->buf[i]) cudaFree(h->buf[i]);
   if (h->snap) cudaFree(h->snap);
-  if (h->qbuf) cudaFree(h->qbuf);
   if (h->rdiff) cudaFree(h->rdiff);
   if (h->hj_stab) cudaFree(h->hj_stab);
   if (h->vtab) cudaFree(h->vtab);

@@ -519,11 +519,6 @@ __device__ __forceinline__ void cp_async_elem(T* smem, const T* gmem) {
   else
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
 }
-// 16 bytes, both addresses 16-byte aligned (past the L1: read once per CTA)
-__device__ __forceinline__ void cp_async_16(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // Load of the tile and its face halo (no edges/corners) from a cell-major
@@ -633,33 +628,6 @@ __device__ __forceinline__ void store_tile(const MeshArgs& m, const T* __restric
   }
 }
 
-// Halo box of the TX x TY x TZ tile at (ox, oy, oz) as rows of cells along x:
-// row (ly, lz) holds cells [max(ox - 1, 0), min(ox + TX + 1, n)) of NMB bytes
-// from the 16-byte aligned address at or below the first, in slot
-// (ly + 1) + BY (lz + 1) of SLOT bytes; rows outside the mesh and edge rows
-// are left out.  One warp per row, 16 bytes per lane: against one bulk copy
-// per row (36 rows of 0.7 KB for a 4x4x4 tile) it spreads the requests over
-// the load units.  Completes with cp_async_wait_all() and a barrier.
-template <int DIM, int TX, int TY, int TZ, int NMB, int SLOT>
-__device__ __forceinline__ void load_box_rows(const MeshArgs& m, const void* g, unsigned char* box, int ox, int oy,
-                                              int oz, int warp, int nw) {
-  constexpr int BY = TY + 2, NROWS = BY * (DIM > 2 ? TZ + 2 : 1);
-  const int lane = threadIdx.x & 31;
-  const char* src = reinterpret_cast<const char*>(g);
-  const int hx0 = max(ox - 1, 0), hx1 = min(ox + TX + 1, m.n[0]);
-  for (int rr = warp; rr < NROWS; rr += nw) {
-    const int ly = rr % BY - 1, lz = DIM > 2 ? rr / BY - 1 : 0;
-    const bool yout = ly < 0 || ly >= TY, zout = DIM > 2 && (lz < 0 || lz >= TZ);
-    if (yout && zout) continue;
-    const int gy = oy + ly, gz = oz + lz;
-    if (gy < 0 || gy >= m.n[1] || (DIM > 2 && (gz < 0 || gz >= m.n[2]))) continue;
-    const long long rowcell = (long long)m.n[0] * (gy + (long long)m.n[1] * (DIM > 2 ? gz : 0));
-    const long long a0 = ((rowcell + hx0) * NMB) & ~15LL;
-    const int n16 = (int)(((rowcell + hx1) * NMB + 15 - a0) >> 4);
-    for (int c = lane; c < n16; c += 32) cp_async_16(box + (size_t)rr * SLOT + 16 * c, src + a0 + 16 * c);
-  }
-}
-
 // ---------------------------------------------------------------------
 // Bulk asynchronous copies (TMA engine, cp.async.bulk) completing on a
 // shared-memory mbarrier.  Copies are plain global -> own-CTA shared
@@ -689,17 +657,21 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
       "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
 }
-// The rows of load_box_rows by one bulk copy each, issued by the lanes of one
-// warp: 32 arrivals on the barrier, each announcing its lane's bytes.
-template <int DIM, int TX, int TY, int TZ, int NMB, int SLOT>
+// Halo box of the TX x TY x TZ tile at (ox, oy, oz), HL cells wide, as rows of
+// cells along x: row (ly, lz) holds cells [max(ox - HL, 0), min(ox + TX + HL, n))
+// of NMB bytes from the 16-byte aligned address at or below the first, in slot
+// (ly + HL) + BY (lz + HL) of SLOT bytes; rows outside the mesh and edge rows
+// are left out.  One bulk copy per row, issued by the lanes of one warp: 32
+// arrivals on the barrier, each announcing its lane's bytes.
+template <int DIM, int TX, int TY, int TZ, int NMB, int SLOT, int HL = 1>
 __device__ __forceinline__ void bulk_box_rows(const MeshArgs& m, const void* g, unsigned char* box, int ox, int oy,
                                               int oz, unsigned long long* bar) {
-  constexpr int BY = TY + 2, NROWS = BY * (DIM > 2 ? TZ + 2 : 1);
+  constexpr int BY = TY + 2 * HL, NROWS = BY * (DIM > 2 ? TZ + 2 * HL : 1);
   const char* src = reinterpret_cast<const char*>(g);
-  const int hx0 = max(ox - 1, 0), hx1 = min(ox + TX + 1, m.n[0]);
+  const int hx0 = max(ox - HL, 0), hx1 = min(ox + TX + HL, m.n[0]);
   unsigned bytes = 0;
   for (int rr = threadIdx.x & 31; rr < NROWS; rr += 32) {
-    const int ly = rr % BY - 1, lz = DIM > 2 ? rr / BY - 1 : 0;
+    const int ly = rr % BY - HL, lz = DIM > 2 ? rr / BY - HL : 0;
     const bool yout = ly < 0 || ly >= TY, zout = DIM > 2 && (lz < 0 || lz >= TZ);
     if (yout && zout) continue;
     const int gy = oy + ly, gz = oz + lz;

@@ -329,8 +329,8 @@ __device__ __forceinline__ void hjs_tile(const HJArgs<T>& a, int slot) {
   int o[3];
   origin(slot, o);
   const int tile = m.tiles ? m.tiles[slot] : slot;
-  // the tile's slice of the sign table by one bulk copy, the halo box by
-  // 16-byte copies of every warp
+  // the tile's slice of the sign table by one bulk copy, the halo box by row
+  // copies of the first warp's lanes
   if (threadIdx.x == 0) {
     mbar_init(bar, 32 + (step ? 1 : 0));
     *cfl = 0;

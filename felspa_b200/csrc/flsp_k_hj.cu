@@ -75,31 +75,43 @@ int ldg_prepare(const Ctx& c) {
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
     constexpr int DIM = decltype(D)::value, P = decltype(PP)::value;
     using T = decltype(tz);
-    const size_t smem = ldg_smem_bytes<DIM, P, T>(DIM == 2 ? kLdgTile2 : kLdgTile3);
-    cudaError_t e = cudaFuncSetAttribute(ldg_kernel<DIM, P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = cudaSuccess;
+    auto attr = [&](auto k, size_t smem) {
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    };
+    if (c.basis == FLSP_BASIS_Q) attr(ldg_kernel<DIM, P, false, T>, LdgPlan<DIM, P, false, T>::BYTES);
+    else attr(ldg_kernel<DIM, P, true, T>, LdgPlan<DIM, P, true, T>::BYTES);
     if (e != cudaSuccess) return set_error(FLSP_ERR_CUDA, std::string("ldg attr: ") + cudaGetErrorString(e));
     return FLSP_OK;
   });
 }
 
-int launch_ldg(const Ctx& c, const void* in, void* out, long long block, double nu, int mode) {
+int launch_ldg(const Ctx& c, const void* in, void* out, double nu, int* err) {
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
     constexpr int DIM = decltype(D)::value, P = decltype(PP)::value;
     using T = decltype(tz);
+    using TL = LdgTile<DIM>;
     LdgArgs<T> a;
     std::memset(&a, 0, sizeof(a));
     a.m = c.m;
     const int* t = DIM == 2 ? kLdgTile2 : kLdgTile3;
+    static_assert(kLdgTile2[0] % LdgTile<2>::X == 0 && kLdgTile2[1] % LdgTile<2>::Y == 0 &&
+                      kLdgTile3[0] % LdgTile<3>::X == 0 && kLdgTile3[1] % LdgTile<3>::Y == 0 &&
+                      kLdgTile3[2] % LdgTile<3>::Z == 0,
+                  "the band's unit is whole blocks");
     set_tile(a.m, DIM, t);
     apply_band(c, kNbLdg, a.m);
+    a.listed = a.m.tiles ? c.nb_ldg_listed : nullptr;
     a.in = reinterpret_cast<const T*>(in);
     a.out = reinterpret_cast<T*>(out);
-    a.block = block;
     a.nu = nu;
-    const size_t smem = ldg_smem_bytes<DIM, P, T>(a.m.tile);
-    return launch_chained("ldg_kernel", ldg_kernel<DIM, P, T>, (unsigned)nblocks(a.m), t[0] * t[1] * t[2], smem, c.stream,
-                          a, mode);
+    a.err = err;
+    const long long blocks = nblocks(a.m) * (t[0] / TL::X) * (t[1] / TL::Y) * (t[2] / TL::Z);
+    const bool q = c.basis == FLSP_BASIS_Q;
+    return launch_chained("ldg_kernel", q ? ldg_kernel<DIM, P, false, T> : ldg_kernel<DIM, P, true, T>, (unsigned)blocks,
+                          TL::N * DIM, q ? LdgPlan<DIM, P, false, T>::BYTES : LdgPlan<DIM, P, true, T>::BYTES, c.stream,
+                          a);
   });
 }
 

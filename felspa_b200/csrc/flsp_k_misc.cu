@@ -416,7 +416,7 @@ __global__ void band_flags_kernel(const T* __restrict__ phi0, long long ncell, i
 
 // one thread per tile: any flagged cell in the tile grown by `margin`?
 __global__ void band_tiles_kernel(const int* __restrict__ flags, MeshArgs m, int dim, int margin,
-                                  int* __restrict__ list, int* __restrict__ count) {
+                                  int* __restrict__ list, int* __restrict__ count, int* __restrict__ listed) {
   const long long ntiles = (long long)m.ntile[0] * m.ntile[1] * m.ntile[2];
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < ntiles;
        t += (long long)gridDim.x * blockDim.x) {
@@ -434,6 +434,7 @@ __global__ void band_tiles_kernel(const int* __restrict__ flags, MeshArgs m, int
             break;
           }
     if (any) list[atomicAdd(count, 1)] = (int)t;
+    if (listed) listed[t] = any ? 1 : 0;
   }
 }
 
@@ -457,14 +458,15 @@ int launch_band_flags(const Ctx& c, const void* phi0, double thr, int* flags) {
   return launch_status("band_flags_kernel");
 }
 
-int launch_band_tiles(const Ctx& c, const int* flags, const int* tile, int margin, int* list, int* count) {
+int launch_band_tiles(const Ctx& c, const int* flags, const int* tile, int margin, int* list, int* count,
+                      int* listed) {
   MeshArgs m = c.m;
   m.tiles = nullptr;
   m.n_tiles = nullptr;
   set_tile(m, c.dim, tile);
   cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int), c.stream);
   if (e != cudaSuccess) return set_error(FLSP_ERR_CUDA, std::string("band tiles: ") + cudaGetErrorString(e));
-  band_tiles_kernel<<<grid_for(nblocks(m)), 256, 0, c.stream>>>(flags, m, c.dim, margin, list, count);
+  band_tiles_kernel<<<grid_for(nblocks(m)), 256, 0, c.stream>>>(flags, m, c.dim, margin, list, count, listed);
   return launch_status("band_tiles_kernel");
 }
 

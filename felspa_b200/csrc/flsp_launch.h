@@ -23,6 +23,7 @@ struct Ctx {
   cudaStream_t stream;
   const int* nb_tiles[3];   // active tile lists (null: every tile)
   const int* nb_count[3];   // device counts of the lists
+  const int* nb_ldg_listed; // narrow band: per LDG tile, 1 if it is listed
   void* hj_stab;            // smooth-sign table of the tensor-product reinit kernel
 };
 
@@ -34,9 +35,11 @@ inline constexpr int kWenoTile[3] = {16, 16, 1};
 // narrow band: flags[c] = 1 for cells with |mean phi0| <= thr; then the
 // list of tiles of shape `tile` that hold a flagged cell within `margin`
 // cells of the tile (device count in *count, order of the list arbitrary:
-// each tile is computed independently)
+// each tile is computed independently); listed (may be null): per tile, 1 if
+// it is in the list
 int launch_band_flags(const Ctx& c, const void* phi0, double thr, int* flags);
-int launch_band_tiles(const Ctx& c, const int* flags, const int* tile, int margin, int* list, int* count);
+int launch_band_tiles(const Ctx& c, const int* flags, const int* tile, int margin, int* list, int* count,
+                      int* listed = nullptr);
 // out[c] = phi0[c] for cells with flags[c] == 0
 int launch_band_restore(const Ctx& c, const void* phi0, void* out, const int* flags);
 // band flags of the listed cells whose list flag is set (all others 0); the
@@ -195,7 +198,7 @@ int launch_hj(const Ctx& c, const void* phi, const void* phi0, void* out, DevClo
 // LDG artificial viscosity: mode 0 = alternating gradient q (DIM blocks)
 // from phi, mode 1 = diffusion RHS (per unit volume) from q
 int ldg_prepare(const Ctx& c);
-int launch_ldg(const Ctx& c, const void* in, void* out, long long block, double nu, int mode);
+int launch_ldg(const Ctx& c, const void* in, void* out, double nu, int* err);
 
 // ---------------- misc (flsp_k_misc.cu) ----------------
 int weno_prepare(const Ctx& c);

@@ -98,6 +98,24 @@ def test_sweep(oracle, flsp, p, basis, n):
     assert rel(sim.get_solution_vector(), phi) <= 1e-11
 
 
+@pytest.mark.parametrize("p,basis,n", [c for c in CASES if len(c[2]) == 3] + [(2, Q, (1, 5)), (2, P, (18, 2)),
+                                                                          (3, Q, (35, 9))])
+def test_viscous_sweep(oracle, flsp, p, basis, n):
+    """the diffusion term reads two cells to each side: axes of one, two and
+    more cells, blocks (16 x 8, 4 x 4 x 4) that end in the mesh"""
+    dim = len(n)
+    orc = oracle.Problem(dim, n, p, basis)
+    phi = orc.project(F.sphere((0.47, 0.56, 0.52)[:dim], 0.31))
+    pb = Problem(Mesh(dim, n), p, basis=basis, precision=abi.FP64)
+    pb.set_state(phi)
+    o = abi.default_reinit_opts(mode=abi.REINIT_FIXED, n_pseudo_steps=3, limiter=0, viscosity=5e-3, cfl_max=0.1)
+    ReinitSimulatorLDG(pb).run_iteration(o)
+    st, _ = orc.reinit(phi, o)
+    assert st == 0
+    assert rel(pb.get_state(), phi) <= 1e-11
+    pb.close()
+
+
 @pytest.mark.parametrize("p,basis,n", [c for c in CASES if len(c[2]) == 2])
 def test_limiter(oracle, flsp, p, basis, n):
     """the rough field: nearly every cell is troubled"""
