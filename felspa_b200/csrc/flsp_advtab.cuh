@@ -67,6 +67,10 @@ struct AdvTabPlan {
   // 2D: the tile's table slice (15.7 KB at Q3 FP32) is brought into shared memory
   static constexpr bool STAGED = DIM == 2;
   static constexpr unsigned TBYTES = LY::entries(NQ) * sizeof(T);
+  // 3D FP64, one CTA per SM: the slice (129 KB at Q2) asked into the L2 ahead, 48^3
+  // Q2 110.8 -> 102.9 us a stage, 32^3 31.1 -> 31.0; with FP32's three CTAs it
+  // takes their bandwidth (48^3 42.2 -> 44.8)
+  static constexpr bool PREFETCH = DIM == 3 && sizeof(T) == 8;
   static_assert(TBYTES % 16 == 0, "bulk copies move 16-byte pieces");
   static constexpr size_t BYTES = OFF_TB + (STAGED ? TBYTES : 0);
 };
@@ -116,6 +120,7 @@ __device__ __forceinline__ void adv_tab_tile(const AdvTabArgs<T>& a, int tile) {
     mbar_arrive_expect_tx(bar, PL::TBYTES);
     bulk_g2s(smem_raw + PL::OFF_TB, tabg, PL::TBYTES, bar);
   }
+  if (PL::PREFETCH && threadIdx.x == 0) bulk_prefetch_l2(tabg, PL::TBYTES);
   chain_wait();
   if (threadIdx.x < 32) bulk_box_rows<DIM, TX, TY, TZ, NMB, PL::SLOT>(m, a.phi_s, boxb, o[0], o[1], o[2], bar);
   const int cl = (int)threadIdx.x % NT, k = (int)threadIdx.x / NT;   // cell, Gauss plane

@@ -657,6 +657,10 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
       "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
 }
+// 16-byte aligned address, size a multiple of 16
+__device__ __forceinline__ void bulk_prefetch_l2(const void* src, unsigned bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(src), "r"(bytes) : "memory");
+}
 // Halo box of the TX x TY x TZ tile at (ox, oy, oz), HL cells wide, as rows of
 // cells along x: row (ly, lz) holds cells [max(ox - HL, 0), min(ox + TX + HL, n))
 // of NMB bytes from the 16-byte aligned address at or below the first, in slot
