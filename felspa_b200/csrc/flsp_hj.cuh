@@ -1,9 +1,9 @@
 // flsp_hj.cuh — what the Hamilton-Jacobi reinitialisation kernels share, and
 // the export of the LDG one-sided gradients.
 //
-// The pseudo-step kernels (hjs_kernel, flsp_hjs.cuh: tensor-product basis;
-// hjp_kernel, flsp_hjp.cuh: total-degree basis; hjq_tile, flsp_hjq.cuh: the
-// batched problems) replace, per pseudo-step
+// The pseudo-step kernels (hjs_kernel, flsp_hjs.cuh: tensor-product basis, the
+// batched problems too; hjp_kernel, flsp_hjp.cuh: total-degree basis) replace,
+// per pseudo-step
 // (src/pde/hamilton_jacobi.cc:514-551):
 //   local_left_right_gradients  (hamilton_jacobi.cc:462-511; LDG integrators
 //                                src/pde/ldg.cc:355-376, 510-740)

@@ -2,9 +2,8 @@
 // product (FE_DGQLegendre) basis, with the work of a cell split over its
 // Gauss planes.
 //
-// Same operator and operation order as hjq_tile (flsp_hjq.cuh; the
-// reference functions it replaces are listed in flsp_hj.cuh), restated for
-// throughput:
+// The point-wise operator (the reference functions it replaces are listed in
+// flsp_hj.cuh), restated for throughput:
 //  * the smooth sign S(phi0) (src/level_set/reinit.cc:121-133) depends on
 //    phi0 alone, which stays fixed through a reinitialisation sweep.  The
 //    sweep's first launch (mode kHJCflOnly, phi == phi0) evaluates it at the
@@ -20,8 +19,8 @@
 //    neighbours), the Hamiltonian takes the mean and half the difference of
 //    the one-sided gradients, and the plane projections overwrite the sign
 //    table entries of the thread's own plane.
-// What bounds it: issue and latency (64^3 Q2 FP32: 68 M warp instructions,
-// 57 % issue active, 24 warps per SM; the loads, barriers and store alone take
+// What bounds it: issue and latency (64^3 Q2 FP32: 61.5 M warp instructions,
+// 58 % issue active, 24 warps per SM; the loads, barriers and store alone take
 // 47 us).  64^3 Q2 FP32 135 -> 98 us, 128^3 996 -> 708, 45x37x50 Q2 FP64
 // 129 -> 101, 256^2 Q2 FP32 14.4 -> 10.3 against the kernel with plain sums
 // and a two-pass copy issue.
