@@ -143,6 +143,21 @@ def test_band_over_everything_p_basis(flsp, n):
     assert np.array_equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("p,basis,n", [(2, P, (33, 20)), (3, Q, (17, 9)), (1, P, (9, 7, 10)), (2, Q, (9, 7, 10))])
+def test_viscous_band_over_everything(flsp, p, basis, n):
+    """the diffusion term with every band tile listed is the full sweep's"""
+    dim = len(n)
+    outs = []
+    for kw in ({}, {"narrow_band": 1, "band_cells": 1e9}):
+        pb = Problem(Mesh(dim, n), p, basis=basis, precision=abi.FP64)
+        pb.project(F.sphere((0.47, 0.56, 0.52)[:dim], 0.31))
+        ReinitSimulatorLDG(pb).run_iteration(abi.default_reinit_opts(
+            mode=abi.REINIT_FIXED, n_pseudo_steps=3, viscosity=5e-3, cfl_max=0.1, limiter=0, **kw))
+        outs.append(pb.get_state())
+        pb.close()
+    assert np.array_equal(outs[0], outs[1])
+
+
 @pytest.mark.parametrize("steps", [1, 31, 32, 33, 70])
 def test_substeps_ahead(flsp, steps):
     """substeps computed up to 32 ahead equal substeps computed one by one"""
