@@ -2008,6 +2008,7 @@ struct flsp_batch {
   int deg_thr[3][4] = {};
   int deg_grid[3][4] = {};
   bool built = false;
+  unsigned long long plan_gen = 0;   // the members' generations the descriptors were made at
   std::map<unsigned long long, GraphEntry> graphs;
   // the degrees' launches of a stage run side by side: one stream per
   // degree, forked from and joined back into the batch stream
@@ -2029,6 +2030,13 @@ void batch_free_plan(flsp_batch* b) {
   for (auto& kv : b->graphs)
     if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
   b->graphs.clear();
+}
+
+// grows whenever a member's velocity changes: the descriptors hold its time factor
+unsigned long long batch_gen(const flsp_batch* b) {
+  unsigned long long g = 0;
+  for (const flsp_handle* h : b->h) g += h->gen;
+  return g;
 }
 
 // descriptors and work lists of every problem for tiles (adv, hj)
@@ -2120,6 +2128,7 @@ int batch_build(flsp_batch* b, const int* adv_tile, const int* hj_tile) {
     b->adv_tile[d] = adv_tile[d];
     b->hj_tile[d] = hj_tile[d];
   }
+  b->plan_gen = batch_gen(b);
   b->built = true;
   return FLSP_OK;
 }
@@ -2425,6 +2434,11 @@ int flsp_batch_run_steps(flsp_batch* b, const flsp_ls_opts* o, int n_steps) {
   CU(cudaSetDevice(b->dev));
   if (!b->tuned) ST(flsp_batch_autotune(b, nullptr));
   ST(batch_sync_problems(b));
+  if (!b->built || b->plan_gen != batch_gen(b)) {
+    CU(cudaStreamSynchronize(b->stream));   // launches that read the descriptors in force
+    const int ta[3] = {b->adv_tile[0], b->adv_tile[1], 1}, th[3] = {b->hj_tile[0], b->hj_tile[1], 1};
+    ST(batch_build(b, ta, th));
+  }
   const bool limiter = ro.limiter != 0;   // 2D: on unless switched off (reinit.cc:475-478)
   const int n = (int)b->h.size();
   ST(launch_batch_clock(b->stream, b->probs, n, kBatchAdvHorizon));
