@@ -1,7 +1,6 @@
 """Batched problems: many independent 2D level-set problems advanced by one
-persistent launch per RK stage / reinit pseudo-step, periods replayed from
-captured CUDA graphs, tile shapes from the batch autotuner
-(flsp_batch_* in include/flsp_dg.h).  Not in the reference, where a
+launch per degree and RK stage / reinit pseudo-step, periods replayed from
+captured CUDA graphs (flsp_batch_* in include/flsp_dg.h).  Not in the reference, where a
 simulator object holds one problem."""
 import ctypes as C
 
@@ -102,7 +101,7 @@ def uneven_batch_benchmark(n_problems=256, steps=500, reinit_every=10, n_pseudo=
                            compare_steps=100):
     """Batched configuration: DoF-steps/s of the whole batch (device time of
     `steps` steps with a reinit every `reinit_every`, CUDA events on the batch
-    stream) and the autotuner's report; for comparison, on `compare_problems`
+    stream) and the batched launches' times; for comparison, on `compare_problems`
     of the problems (all of them by default), the same problems issued one
     after the other, each in its own graph-replayed run on its own stream (so
     that they overlap on the GPU), and as one group (one graph per period, a

@@ -1981,8 +1981,8 @@ int flsp_ls_run_steps_learned(flsp_handle* h, flsp_mlp* net, const flsp_learned_
 
 // ---- batched problems (no counterpart in the reference: one problem per
 // simulator object there).  Many independent 2D problems advance in one
-// persistent launch per RK stage and per reinit pseudo-step, periods
-// replayed from captured CUDA graphs, tile shapes from the autotuner.
+// launch per degree, RK stage and reinit pseudo-step, periods replayed from
+// captured CUDA graphs.
 }  // extern "C"
 
 struct flsp_batch {
@@ -1991,17 +1991,14 @@ struct flsp_batch {
   std::vector<flsp_handle*> h;
   int cur = 0;             // common buffer role of every problem
   int n_since_reinit = 0;
-  bool tuned = false;
-  int adv_tile[3] = {16, 16, 1}, hj_tile[3] = {16, 8, 1};
-  flsp_batch_tuning tuning;
-  // device descriptors and work lists for the current tiles
+  // device descriptors and work lists
   BatchProb* probs = nullptr;
   int2* items_adv = nullptr;
   int2* items_hj = nullptr;
   int2* items_weno = nullptr;
   int n_adv = 0, n_hj = 0, n_weno = 0;
   // per kernel kind (adv, hj, weno) and degree 1..3: the items' range in the
-  // kind's list (sorted by degree), shared memory, persistent grid
+  // kind's list (sorted by degree), shared memory, threads and grid
   int deg_off[3][4] = {}, deg_cnt[3][4] = {};
   int prob_off[4] = {}, prob_cnt[4] = {};   // per degree: its range of the descriptors
   size_t deg_smem[3][4] = {};
@@ -2039,8 +2036,12 @@ unsigned long long batch_gen(const flsp_batch* b) {
   return g;
 }
 
-// descriptors and work lists of every problem for tiles (adv, hj)
-int batch_build(flsp_batch* b, const int* adv_tile, const int* hj_tile) {
+// the stage's and the pseudo-step's tile: the kernels give a cell a thread per
+// Gauss plane and fix it at compile time
+constexpr int kBatchTile[3] = {HjsTile<2>::X, HjsTile<2>::Y, HjsTile<2>::Z};
+
+// descriptors and work lists of every problem
+int batch_build(flsp_batch* b) {
   batch_free_plan(b);
   const int n = (int)b->h.size();
   std::vector<BatchProb> pr((size_t)n);
@@ -2064,8 +2065,8 @@ int batch_build(flsp_batch* b, const int* adv_tile, const int* hj_tile) {
     q.m_adv.n_tiles = nullptr;
     q.m_hj = q.m_adv;
     q.m_weno = q.m_adv;
-    set_tile(q.m_adv, 2, adv_tile);
-    set_tile(q.m_hj, 2, hj_tile);
+    set_tile(q.m_adv, 2, kBatchTile);
+    set_tile(q.m_hj, 2, kBatchTile);
     set_tile(q.m_weno, 2, kWenoTile);
     for (int k = 0; k < 3; ++k) q.buf[k] = h->buf[k];
     q.clk = h->clk;
@@ -2124,10 +2125,6 @@ int batch_build(flsp_batch* b, const int* adv_tile, const int* hj_tile) {
       if (b->deg_cnt[k][p] > 0)
         ST(batch_prepare(k, b->prec, p, b->deg_cnt[k][p], &b->deg_smem[k][p], &b->deg_thr[k][p], &b->deg_grid[k][p]));
   }
-  for (int d = 0; d < 3; ++d) {
-    b->adv_tile[d] = adv_tile[d];
-    b->hj_tile[d] = hj_tile[d];
-  }
   b->plan_gen = batch_gen(b);
   b->built = true;
   return FLSP_OK;
@@ -2142,6 +2139,17 @@ int batch_sync_problems(flsp_batch* b) {
       h->cur = b->cur;
     }
   return FLSP_OK;
+}
+
+// ready to launch: the members' own work done, one buffer role, descriptors of
+// the velocities in force
+int batch_ready(flsp_batch* b) {
+  for (flsp_handle* h : b->h)
+    if (!h->has_vel) return fail(FLSP_ERR_BAD_ARG, "velocity not set for every problem");
+  ST(batch_sync_problems(b));
+  if (b->built && b->plan_gen == batch_gen(b)) return FLSP_OK;
+  CU(cudaStreamSynchronize(b->stream));   // launches that read the descriptors in force
+  return batch_build(b);
 }
 
 // the stage / reinit step / limiter of every problem: one launch per degree
@@ -2306,7 +2314,6 @@ int flsp_batch_create(int n, const flsp_mesh_desc* meshes, const flsp_dg_opts* o
       return fail(FLSP_ERR_BAD_ARG, "batched problems share precision, RK order and device");
   }
   flsp_batch* b = new flsp_batch();
-  std::memset(&b->tuning, 0, sizeof(b->tuning));
   b->dev = opts[0].device;
   b->prec = opts[0].precision;
   b->rk = opts[0].rk_order;
@@ -2347,19 +2354,15 @@ int flsp_batch_problem(flsp_batch* b, int i, flsp_handle** h) {
   return FLSP_OK;
 }
 
+// times the batched launches as they are (no choice is left: kBatchTile)
 int flsp_batch_autotune(flsp_batch* b, flsp_batch_tuning* out) {
   if (!b) return fail(FLSP_ERR_BAD_ARG, "null argument");
   CU(cudaSetDevice(b->dev));
-  for (flsp_handle* h : b->h)
-    if (!h->has_vel) return fail(FLSP_ERR_BAD_ARG, "velocity not set for every problem");
-  ST(batch_sync_problems(b));
-  // one tile each: the kernels give a cell a thread per Gauss plane and fix the
-  // tile at compile time
-  static const int ca[][3] = {{HjsTile<2>::X, HjsTile<2>::Y, 1}};
-  static const int ch[][3] = {{HjsTile<2>::X, HjsTile<2>::Y, 1}};
+  ST(batch_ready(b));
+  if (!out) return FLSP_OK;
   flsp_batch_tuning t;
   std::memset(&t, 0, sizeof(t));
-  cudaEvent_t e0, e1;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
   CU(cudaEventCreate(&e0));
   CU(cudaEventCreate(&e1));
   auto time_it = [&](auto&& launch, double* ms) -> int {
@@ -2374,51 +2377,20 @@ int flsp_batch_autotune(flsp_batch* b, flsp_batch_tuning* out) {
     *ms = f / reps;
     return FLSP_OK;
   };
-  // the stage: clock set-up at the current time (harmless: the step's own
-  // set-up recomputes it), the first RK stage into a free buffer
-  double best = 1e300;
-  int bi = 0;
-  for (int c = 0; c < 1; ++c) {
-    ST(batch_build(b, ca[c], ch[0]));
-    ST(launch_batch_clock_steps(b->stream, b->probs, (int)b->h.size(), 1, false));
-    const int x = b->cur, y = (x + 1) % 3;
-    double ms = 0.0;
-    ST(time_it([&]() {
-      return batch_adv_all(b, x, x, y, 0, kRK3a);
-    }, &ms));
-    t.adv_cand[c][0] = ca[c][0];
-    t.adv_cand[c][1] = ca[c][1];
-    t.adv_ms[c] = ms;
-    if (ms < best) { best = ms; bi = c; }
-  }
-  t.n_adv = 1;
-  // the reinit step: the CFL pass (reads the state, writes only the clock's
-  // CFL slot, which every reinit resets)
-  best = 1e300;
-  int bj = 0;
-  for (int c = 0; c < 1; ++c) {
-    ST(batch_build(b, ca[bi], ch[c]));
-    const int x = b->cur;
-    double ms = 0.0;
-    ST(time_it([&]() {
-      return batch_hj_all(b, x, x, -1, kHJCflOnly, 1);
-    }, &ms));
-    t.hj_cand[c][0] = ch[c][0];
-    t.hj_cand[c][1] = ch[c][1];
-    t.hj_ms[c] = ms;
-    if (ms < best) { best = ms; bj = c; }
-  }
-  t.n_hj = 1;
+  // the stage: clock set-up at the current time (harmless: the step's own set-up
+  // recomputes it), the first RK stage into a free buffer; the reinit step: the
+  // CFL pass, which writes the sign tables and the clocks' CFL slots (every
+  // reinit writes both anew)
+  const int x = b->cur, y = (x + 1) % 3;
+  int st = launch_batch_clock_steps(b->stream, b->probs, (int)b->h.size(), 1, false);
+  if (st == FLSP_OK) st = time_it([&]() { return batch_adv_all(b, x, x, y, 0, kRK3a); }, &t.adv_ms[0]);
+  if (st == FLSP_OK) st = time_it([&]() { return batch_hj_all(b, x, x, -1, kHJCflOnly, 1); }, &t.hj_ms[0]);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  ST(batch_build(b, ca[bi], ch[bj]));
-  t.adv_tile[0] = ca[bi][0];
-  t.adv_tile[1] = ca[bi][1];
-  t.hj_tile[0] = ch[bj][0];
-  t.hj_tile[1] = ch[bj][1];
-  b->tuning = t;
-  b->tuned = true;
-  if (out) *out = t;
+  ST(st);
+  t.n_adv = t.n_hj = 1;
+  for (int d = 0; d < 2; ++d) t.adv_tile[d] = t.hj_tile[d] = t.adv_cand[0][d] = t.hj_cand[0][d] = kBatchTile[d];
+  *out = t;
   return FLSP_OK;
 }
 
@@ -2432,13 +2404,7 @@ int flsp_batch_run_steps(flsp_batch* b, const flsp_ls_opts* o, int n_steps) {
     ST(validate_reinit(b->h[0], &ro));
   }
   CU(cudaSetDevice(b->dev));
-  if (!b->tuned) ST(flsp_batch_autotune(b, nullptr));
-  ST(batch_sync_problems(b));
-  if (!b->built || b->plan_gen != batch_gen(b)) {
-    CU(cudaStreamSynchronize(b->stream));   // launches that read the descriptors in force
-    const int ta[3] = {b->adv_tile[0], b->adv_tile[1], 1}, th[3] = {b->hj_tile[0], b->hj_tile[1], 1};
-    ST(batch_build(b, ta, th));
-  }
+  ST(batch_ready(b));
   const bool limiter = ro.limiter != 0;   // 2D: on unless switched off (reinit.cc:475-478)
   const int n = (int)b->h.size();
   ST(launch_batch_clock(b->stream, b->probs, n, kBatchAdvHorizon));

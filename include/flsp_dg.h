@@ -580,10 +580,9 @@ void flsp_default_learned_opts(flsp_learned_opts* o);
    Batched problems (no counterpart in the reference, where one simulator
    object holds one problem).  Many independent 2D Q-basis problems (own
    meshes, degrees 1..3, velocities, ICs and clocks; one precision and RK
-   order) advance together: one persistent launch per RK stage and per
-   reinit pseudo-step covers every problem, a reinit period is replayed from
-   a captured CUDA graph, and the tile shapes come from flsp_batch_autotune
-   (run on first use if not called).  Problem i is a regular handle
+   order) advance together: one launch per RK stage and per reinit
+   pseudo-step covers every problem of a degree, and a reinit period is
+   replayed from a captured CUDA graph.  Problem i is a regular handle
    (flsp_batch_problem) for set-up, state exchange and reductions; the
    batch owns it.
    ------------------------------------------------------------------ */
@@ -604,6 +603,8 @@ int flsp_batch_create(int n, const flsp_mesh_desc* meshes, const flsp_dg_opts* o
 void flsp_batch_destroy(flsp_batch* b);
 int flsp_batch_size(const flsp_batch* b, int* n);
 int flsp_batch_problem(flsp_batch* b, int i, flsp_handle** h);
+/* times the batched stage and pseudo-step launches; their tile is fixed, so
+   one candidate of each is reported and nothing changes (never needed)   */
 int flsp_batch_autotune(flsp_batch* b, flsp_batch_tuning* out);
 /* n_steps substeps of every problem with a fixed-count reinit every
    reinit_frequency steps (no viscosity, no narrow band); enqueued, returns
