@@ -60,7 +60,7 @@ struct AdvSepArgs {
   const T* __restrict__ optab;   // [(d*3 + e) * nmax + i][OPW]
   int nmax;                      // row stride per (d, e): >= n[e] + kOpRowPad (a tile's
                                  // bulk copy of its rows never leaves the table)
-  int* err;                      // device error word (DevClock::err)
+  int* err;                      // the problem's error word
   const T* __restrict__ phi_s;
   const T* __restrict__ phi_n;
   T* __restrict__ out;

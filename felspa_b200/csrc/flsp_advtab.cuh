@@ -46,7 +46,7 @@ struct AdvTabArgs {
   int stage;                     // index into step->ct
   int combine;                   // CombineMode
   double ct_explicit, dt_explicit;   // when step == nullptr
-  int* err;                      // device error word (DevClock::err) or null
+  int* err;                      // the problem's error word
 };
 
 template <int DIM, int P, bool PB, typename T>

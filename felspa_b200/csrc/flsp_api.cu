@@ -142,6 +142,7 @@ struct flsp_handle {
   DevClock* clk_host = nullptr;   // pinned mirror
   AdvStep* steps = nullptr;       // the clock's next substeps (kClockSteps)
   double* pin = nullptr;          // pinned, behind clk_host: small results on their way to the host
+  int* err = nullptr;             // pinned, behind them: the error word, written by kernels (no copy to read it)
   double* grad64 = nullptr;       // gradient export before the cell permutation
   int64_t* perm = nullptr;
   double* stage64 = nullptr;      // FP64 device staging (2 * dim * ndofs)
@@ -204,6 +205,7 @@ struct flsp_handle {
     }
     c.nb_ldg_listed = nb_use[kNbLdg] ? nb_lists + 3 * (size_t)m.ncell : nullptr;
     c.hj_stab = hj_stab;
+    c.err = err;
     return c;
   }
   flsp_velocity_desc vel_dev;   // terms as laid out in the device tables
@@ -219,7 +221,7 @@ struct flsp_handle {
     for (int k = 0; k < vel_dev.n_terms; ++k) v.sep1 = v.sep1 && vel_dev.terms[k].comp == k;
     v.optab = v.sep1 ? optab : nullptr;
     v.opstride = opstride;
-    v.err = clk ? &clk->err : nullptr;
+    v.err = err;
     if (fe_pv > 0) {
       v.sep1 = false;
       v.optab = nullptr;
@@ -275,8 +277,9 @@ int ensure_partial(flsp_handle* h, int n) {
   return FLSP_OK;
 }
 
-int device_error(int err) {
-  if (err & kErrCopyTimeout)
+// after a wait for the stream: what its kernels left in the error word
+int device_error(const flsp_handle* h) {
+  if (*static_cast<const volatile int*>(h->err) & kErrCopyTimeout)
     return fail(FLSP_ERR_TIMEOUT, "a kernel's wait for its bulk copies ran out (results invalid)");
   return FLSP_OK;
 }
@@ -284,7 +287,7 @@ int device_error(int err) {
 int sync_clock(flsp_handle* h) {
   CU(cudaMemcpyAsync(h->clk_host, h->clk, sizeof(DevClock), cudaMemcpyDeviceToHost, h->stream));
   CU(cudaStreamSynchronize(h->stream));
-  return device_error(h->clk_host->err);
+  return device_error(h);
 }
 
 // kernel configuration of this handle (tiles, shared-memory attributes);
@@ -402,7 +405,7 @@ int enqueue_hj_step(flsp_handle* h, const flsp_reinit_opts* o, int phi0_idx, boo
   const int dst = (src == phi0_idx) ? (phi0_idx + 1) % 3 : other(src, phi0_idx);
   const void* rdiff = nullptr;
   if (o->viscosity > 0.0) {   // LDGDiffusionTerm of the current solution (ldg.cc:249-298)
-    ST(launch_ldg(h->ctx(), h->buf[src], h->rdiff, o->viscosity, &h->clk->err));
+    ST(launch_ldg(h->ctx(), h->buf[src], h->rdiff, o->viscosity));
     rdiff = h->rdiff;
   }
   ST(launch_hj(h->ctx(), h->buf[src], h->buf[phi0_idx], h->buf[dst], h->clk, kHJStep, o->rk_order, &step,
@@ -410,7 +413,7 @@ int enqueue_hj_step(flsp_handle* h, const flsp_reinit_opts* o, int phi0_idx, boo
   int res = dst;
   if (limiter) {
     const int lim = other(dst, phi0_idx);
-    ST(launch_weno(h->ctx(), h->buf[dst], h->buf[lim], nullptr, &h->clk->err));
+    ST(launch_weno(h->ctx(), h->buf[dst], h->buf[lim], nullptr));
     res = lim;
   }
   h->cur = res;
@@ -1059,6 +1062,8 @@ int flsp_create(const flsp_mesh_desc* mesh, const flsp_dg_opts* opts, flsp_handl
   h->flag_dev = reinterpret_cast<unsigned int*>(h->small + at_flag);
   h->ic_dev = reinterpret_cast<flsp_ic_desc*>(h->small + at_ic);
   h->pin = reinterpret_cast<double*>(reinterpret_cast<char*>(h->clk_host) + at_steps);
+  h->err = reinterpret_cast<int*>(h->pin + 4);
+  *h->err = 0;
   cudaMemset(h->clk, 0, sizeof(DevClock));
   cudaMemset(h->buf[0], 0, h->ndofs * h->tsize);
   if (mesh->host_cell_order) {
@@ -1482,7 +1487,8 @@ int flsp_advect_rhs(flsp_handle* h, double t, double* phidot, int64_t n) {
   const int tmp = (h->cur + 1) % 3;
   ST(launch_adv_stage(h->ctx(), h->veldev(), h->buf[h->cur], h->buf[h->cur], h->buf[tmp], nullptr, 0,
                       kRhsOnly, host_time_factor(h->vel, t), h->adv_tile));
-  return read_coeffs(h, h->buf[tmp], phidot, n);
+  ST(read_coeffs(h, h->buf[tmp], phidot, n));
+  return device_error(h);
 }
 
 // AdvectSimulator::advance_time(time_step, compute_single_cycle)
@@ -1523,9 +1529,9 @@ int flsp_advance_steps(flsp_handle* h, int n_steps, double t_end) {
 int flsp_reinit(flsp_handle* h, const flsp_reinit_opts* o, int* n_iter) {
   if (!h) return fail(FLSP_ERR_BAD_ARG, "null handle");
   CU(cudaSetDevice(h->dev));
-  int st = run_reinit(h, o, n_iter);
+  const int st = run_reinit(h, o, n_iter);
   cudaStreamSynchronize(h->stream);
-  return st;
+  return st ? st : device_error(h);
 }
 
 int flsp_hj_gradients(flsp_handle* h, double* grads, int64_t n) {
@@ -1553,9 +1559,10 @@ int flsp_weno_limit(flsp_handle* h, int* n_troubled) {
   CU(cudaSetDevice(h->dev));
   CU(cudaMemsetAsync(h->flag_dev, 0, sizeof(unsigned int), h->stream));
   const int dst = (h->cur + 1) % 3;
-  ST(launch_weno(h->ctx(), h->buf[h->cur], h->buf[dst], h->flag_dev, &h->clk->err));
+  ST(launch_weno(h->ctx(), h->buf[h->cur], h->buf[dst], h->flag_dev));
   unsigned int cnt = 0;
   ST(read_flag(h, &cnt));
+  ST(device_error(h));
   h->cur = dst;
   if (n_troubled) *n_troubled = (int)cnt;
   return FLSP_OK;
@@ -1676,6 +1683,14 @@ int flsp_sync(flsp_handle* h) {
   if (!h) return fail(FLSP_ERR_BAD_ARG, "null handle");
   CU(cudaSetDevice(h->dev));
   return sync_clock(h);
+}
+
+int flsp_set_device_error(flsp_handle* h, int err) {
+  if (!h) return fail(FLSP_ERR_BAD_ARG, "null handle");
+  CU(cudaSetDevice(h->dev));
+  CU(cudaStreamSynchronize(h->stream));
+  *h->err = err;
+  return FLSP_OK;
 }
 
 int flsp_stream(const flsp_handle* h, void** stream) {
@@ -1825,6 +1840,7 @@ int flsp_mlp_collect(flsp_mlp* net, flsp_handle* h, double band_cells, const fls
   ST(launch_patch_targets(h->stream, h->prec, h->m.nb, h->lrn_save, h->buf[h->cur], hh, h->lrn_cells, n,
                           net->targ + net->n_pairs * net->n_out));
   CU(cudaStreamSynchronize(h->stream));
+  ST(device_error(h));
   net->n_pairs += n;
   if (n_added) *n_added = n;
   return FLSP_OK;
@@ -1883,6 +1899,7 @@ int flsp_reinit_learned(flsp_handle* h, flsp_mlp* net, const flsp_learned_opts* 
     h->cur = res;
     stl.hj_ran = 1;
     CU(cudaStreamSynchronize(h->stream));
+    ST(device_error(h));
   } else {
     h->cur = out;
   }
@@ -2071,6 +2088,7 @@ int batch_build(flsp_batch* b) {
     for (int k = 0; k < 3; ++k) q.buf[k] = h->buf[k];
     q.clk = h->clk;
     q.steps = h->steps;
+    q.err = h->err;
     if (!h->tab_ok) return fail(FLSP_ERR_BAD_ARG, "batched problem without velocity tables");
     q.tab = h->tab;
     q.stab = h->hj_stab;

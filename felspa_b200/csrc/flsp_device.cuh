@@ -232,7 +232,6 @@ struct DevClock {
   int active;        // current substep is non-zero
   int pending;       // dt still to be added to t
   int n_substeps;    // executed substeps
-  int err;           // device error word (0 = ok)
   // reinitialisation
   double hj_vd_run;  // running max of characteristic speed / diam
   double hj_dt;      // last pseudo-step
@@ -634,7 +633,7 @@ __device__ __forceinline__ void store_tile(const MeshArgs& m, const T* __restric
 // memory: no cluster multicast.  Both addresses 16-byte aligned, size a
 // multiple of 16.
 // ---------------------------------------------------------------------
-constexpr int kErrCopyTimeout = 1;   // DevClock::err bit: a bulk-copy wait ran out
+constexpr int kErrCopyTimeout = 1;   // bit of a problem's error word: a bulk-copy wait ran out
 constexpr int kOpRowPad = 32;        // operator-table rows past the mesh per (d, e) block
 constexpr int kStatePad = 256;       // bytes past the end of every state buffer
 

@@ -178,6 +178,7 @@ __global__ void __launch_bounds__(HjsTile<DIM>::N * (P + 2), hjp_min_blocks<DIM,
   }
   if (!mbar_wait(bar, 0u, 1 << 22)) {
     if (threadIdx.x == 0 && a.err) atomicOr(a.err, kErrCopyTimeout);
+    mbar_wait(bar, 0u, 1 << 22);   // give copies in flight a last chance to land
   }
 
   // -------- (1) modal gradients: axis k of the thread's cell (whole warps per axis)

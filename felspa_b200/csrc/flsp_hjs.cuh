@@ -355,6 +355,7 @@ __device__ __forceinline__ void hjs_tile(const HJArgs<T>& a, int slot) {
   };
   if (!mbar_wait(bar, 0u, 1 << 22)) {
     if (threadIdx.x == 0 && a.err) atomicOr(a.err, kErrCopyTimeout);
+    mbar_wait(bar, 0u, 1 << 22);   // give copies in flight a last chance to land
   }
 
   // -------- face jumps, one work item per face of the tile

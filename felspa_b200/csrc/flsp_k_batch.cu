@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(HjsTile<2>::N * (P + 2), advtab_min_blocks<2, 
     a.step = pr.steps + step;
     a.stage = stage;
     a.combine = combine;
-    a.err = &pr.clk->err;
+    a.err = pr.err;
   }
   __syncthreads();
   adv_tab_tile<2, P, false, T>(a, w.y);
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(HjsTile<2>::N * (P + 2), hjs_min_blocks<2, P, 
     a.step.k = k;
     a.rdiff = nullptr;
     a.stab = reinterpret_cast<T*>(pr.stab);
-    a.err = &pr.clk->err;
+    a.err = pr.err;
   }
   __syncthreads();
   hjs_tile<2, P, T>(a, w.y);
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(WenoBlock::N)
     a.in = reinterpret_cast<const T*>(pr.buf[iin]);
     a.out = reinterpret_cast<T*>(pr.buf[iout]);
     a.count = nullptr;
-    a.err = &pr.clk->err;
+    a.err = pr.err;
   }
   __syncthreads();
   weno_tile<P, false, T>(a, w.y, (int)blockIdx.x % 2);

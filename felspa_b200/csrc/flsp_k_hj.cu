@@ -87,7 +87,7 @@ int ldg_prepare(const Ctx& c) {
   });
 }
 
-int launch_ldg(const Ctx& c, const void* in, void* out, double nu, int* err) {
+int launch_ldg(const Ctx& c, const void* in, void* out, double nu) {
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
     constexpr int DIM = decltype(D)::value, P = decltype(PP)::value;
     using T = decltype(tz);
@@ -106,7 +106,7 @@ int launch_ldg(const Ctx& c, const void* in, void* out, double nu, int* err) {
     a.in = reinterpret_cast<const T*>(in);
     a.out = reinterpret_cast<T*>(out);
     a.nu = nu;
-    a.err = err;
+    a.err = c.err;
     const long long blocks = nblocks(a.m) * (t[0] / TL::X) * (t[1] / TL::Y) * (t[2] / TL::Z);
     const bool q = c.basis == FLSP_BASIS_Q;
     return launch_chained("ldg_kernel", q ? ldg_kernel<DIM, P, false, T> : ldg_kernel<DIM, P, true, T>, (unsigned)blocks,
@@ -156,7 +156,7 @@ int launch_hj(const Ctx& c, const void* phi, const void* phi0, void* out, DevClo
         (c.basis == FLSP_BASIS_Q && (a.m.tile[0] != TL::X || a.m.tile[1] != TL::Y || a.m.tile[2] != TL::Z)))
       return set_error(FLSP_ERR_BAD_ARG, "the reinit kernels have a fixed tile");
     a.stab = reinterpret_cast<T*>(c.hj_stab);
-    a.err = &clk->err;
+    a.err = c.err;
     const int threads = TL::N * (P + 2);
     if (c.basis == FLSP_BASIS_Q) {
       return launch_chained("hjs_kernel", hjs_kernel<DIM, P, T>, (unsigned)nblocks(a.m), threads,

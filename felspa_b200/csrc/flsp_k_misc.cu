@@ -41,7 +41,7 @@ int weno_prepare(const Ctx& c) {
   });
 }
 
-int launch_weno(const Ctx& c, const void* in, void* out, unsigned int* count, int* err) {
+int launch_weno(const Ctx& c, const void* in, void* out, unsigned int* count) {
   if (c.dim != 2) return set_error(FLSP_ERR_UNSUPPORTED, "WENO limiter is 2D only (reinit.cc:475-478)");
   return dispatch(c, [&](auto D, auto PP, auto tz) -> int {
     constexpr int P = decltype(PP)::value;
@@ -57,7 +57,7 @@ int launch_weno(const Ctx& c, const void* in, void* out, unsigned int* count, in
       a.in = reinterpret_cast<const T*>(in);
       a.out = reinterpret_cast<T*>(out);
       a.count = count;
-      a.err = err;
+      a.err = c.err;
       const unsigned grid = 2u * (unsigned)nblocks(a.m);
       const bool q = c.basis == FLSP_BASIS_Q;
       return launch_chained("weno_kernel", q ? weno_kernel<P, false, T> : weno_kernel<P, true, T>, grid, WenoBlock::N,

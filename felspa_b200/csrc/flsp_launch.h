@@ -24,7 +24,8 @@ struct Ctx {
   const int* nb_tiles[3];   // active tile lists (null: every tile)
   const int* nb_count[3];   // device counts of the lists
   const int* nb_ldg_listed; // narrow band: per LDG tile, 1 if it is listed
-  void* hj_stab;            // smooth-sign table of the tensor-product reinit kernel
+  void* hj_stab;            // smooth-sign table of the reinit kernels
+  int* err;                 // the problem's error word (pinned host memory; 0 = ok)
 };
 
 // tile shapes of the LDG viscosity and WENO limiter kernels
@@ -56,6 +57,7 @@ struct BatchProb {
   void* buf[3];                   // state buffers (roles are launch parameters)
   DevClock* clk;
   AdvStep* steps;                 // its next substeps
+  int* err;                       // its error word
   const void* tab;                // velocity table of the problem (VelTabLayout)
   void* stab;                     // smooth-sign table of its reinitialisation
   int p;                          // degree 1..3
@@ -164,7 +166,7 @@ struct VelDev {
   bool sep1;           // term k is the only term of component k
   const void* optab;   // per-axis operator rows of a sep1 velocity (T precision), or null
   int opstride;        // operator rows per (component, axis) in optab
-  int* err;            // device error word (DevClock::err)
+  int* err;            // the problem's error word
   // velocity table (VelTabLayout, T precision) or null, made from the terms or
   // from the FE field of a coupled simulator (fe_pv > 0: its lattice degree)
   const void* tab;
@@ -198,13 +200,13 @@ int launch_hj(const Ctx& c, const void* phi, const void* phi0, void* out, DevClo
 // LDG artificial viscosity: mode 0 = alternating gradient q (DIM blocks)
 // from phi, mode 1 = diffusion RHS (per unit volume) from q
 int ldg_prepare(const Ctx& c);
-int launch_ldg(const Ctx& c, const void* in, void* out, double nu, int* err);
+int launch_ldg(const Ctx& c, const void* in, void* out, double nu);
 
 // ---------------- misc (flsp_k_misc.cu) ----------------
 int weno_prepare(const Ctx& c);
 // the 2D limiter: detection and reconstruction in one pass; count (or null)
-// receives the number of troubled cells, err a failed wait
-int launch_weno(const Ctx& c, const void* in, void* out, unsigned int* count, int* err);
+// receives the number of troubled cells
+int launch_weno(const Ctx& c, const void* in, void* out, unsigned int* count);
 int launch_project_ic(const Ctx& c, const flsp_ic_desc* ic_dev, void* out);
 int launch_static_cfl(const Ctx& c, const double* vtab64, int n_terms, const int* comp, int nmax,
                       int npt, DevClock* clk);

@@ -41,7 +41,7 @@ struct LdgArgs {
   T* __restrict__ out;         // R_diff
   const int* listed;       // narrow band: 1 for each tile that is listed (else null)
   double nu;
-  int* err;                // device error word (DevClock::err)
+  int* err;                // the problem's error word
 };
 
 // block of cells

@@ -34,7 +34,7 @@ struct WenoArgs {
   const T* __restrict__ in;
   T* __restrict__ out;
   unsigned int* count;   // troubled-cell counter (may be null)
-  int* err;              // device error word (DevClock::err) or null
+  int* err;              // the problem's error word
 };
 
 // a CTA's cells: half of a limiter tile (kWenoTile; the unit the narrow band

@@ -49,6 +49,7 @@ PROTOTYPES = {
     "flsp_ls_advance": (C.c_int, [_vp, C.POINTER(abi.LSOpts), C.c_double, C.c_int, _dp]),
     "flsp_ls_run_steps": (C.c_int, [_vp, C.POINTER(abi.LSOpts), C.c_int]),
     "flsp_sync": (C.c_int, [_vp]),
+    "flsp_set_device_error": (C.c_int, [_vp, C.c_int]),
     "flsp_stream": (C.c_int, [_vp, C.POINTER(_vp)]),
     "flsp_time_kernel": (C.c_int, [_vp, C.c_int, C.c_int, _dp]),
     "flsp_reduce": (C.c_int, [_vp, C.c_int, C.POINTER(abi.ICDesc), _dp]),

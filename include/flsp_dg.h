@@ -334,6 +334,13 @@ int flsp_ls_advance(flsp_handle* h, const flsp_ls_opts* o, double time_step,
    (flsp_get_state and the reductions synchronise by themselves).        */
 int flsp_ls_run_steps(flsp_handle* h, const flsp_ls_opts* o, int n_steps);
 int flsp_sync(flsp_handle* h);
+/* Failure injection for tests: sets the problem's device error word (1: a
+   kernel's bulk copies did not arrive in time; 0: none), as a kernel whose
+   bounded wait runs out does.  Every call that steps, reinitialises, limits
+   or evaluates the rate then fails with FLSP_ERR_TIMEOUT once it has waited
+   for its work (flsp_ls_run_steps and the learned and group periods, which
+   do not wait: the sync call after them).                                 */
+int flsp_set_device_error(flsp_handle* h, int err);
 /* the handle's cudaStream_t (for callers that order their own work or
    record CUDA events against the library's work)                       */
 int flsp_stream(const flsp_handle* h, void** stream);
