@@ -1172,22 +1172,31 @@ int flsp_set_velocity_fe(flsp_handle* h, int degree, const double* values, int64
   for (int d = 0; d < h->dim; ++d) nn *= (long long)degree * h->m.n[d] + 1;
   if (n != (int64_t)h->dim * nn) return fail(FLSP_ERR_BAD_ARG, "FE velocity size mismatch");
   CU(cudaSetDevice(h->dev));
-  // checked on the device (48^3, degree 2: 2.7 M values took the host 2.5 ms)
-  // in a lattice of its own: the velocity in force stays as it is until then
-  if (h->fe_next_n != n) {
-    if (h->fe_next) cudaFree(h->fe_next);
-    h->fe_next = nullptr;
-    h->fe_next_n = 0;
-    CU(cudaMalloc(&h->fe_next, (size_t)n * sizeof(double)));
-    h->fe_next_n = n;
-  }
-  CU(cudaMemsetAsync(h->flag_dev, 0, sizeof(unsigned int), h->stream));
-  CU(cudaMemcpyAsync(h->fe_next, values, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  ST(launch_nonfinite(h->stream, h->fe_next, n, h->flag_dev));
-  unsigned int bad = 0;
-  ST(read_flag(h, &bad));
-  if (bad) return fail(FLSP_ERR_BAD_ARG, "non-finite FE velocity value");
   const bool same = h->fe_pv == degree && h->fe_u64 != nullptr;
+  // checked before the velocity in force is touched, on the device (48^3, degree 2:
+  // 2.7 M values took the host 2.5 ms): in the staging buffer, or in a lattice of
+  // its own where that is too small; on the host where there is no room for one
+  double* next = h->stage64;
+  if (n > 2 * h->dim * h->ndofs) {
+    if (h->fe_next_n != n) {
+      if (h->fe_next) cudaFree(h->fe_next);
+      h->fe_next = nullptr;
+      h->fe_next_n = 0;
+      if (cudaMalloc(&h->fe_next, (size_t)n * sizeof(double)) == cudaSuccess) h->fe_next_n = n;
+      else cudaGetLastError();
+    }
+    next = h->fe_next;
+  }
+  unsigned int bad = 0;
+  if (next) {
+    CU(cudaMemsetAsync(h->flag_dev, 0, sizeof(unsigned int), h->stream));
+    CU(cudaMemcpyAsync(next, values, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    ST(launch_nonfinite(h->stream, next, n, h->flag_dev));
+    ST(read_flag(h, &bad));
+  } else {
+    for (int64_t i = 0; i < n; ++i) bad += !std::isfinite(values[i]);
+  }
+  if (bad) return fail(FLSP_ERR_BAD_ARG, "non-finite FE velocity value");
   if (!same) {
     // an FE field has no analytic terms: zero tables, time factor 1
     CU(cudaStreamSynchronize(h->stream));
@@ -1195,17 +1204,25 @@ int flsp_set_velocity_fe(flsp_handle* h, int degree, const double* values, int64
     std::memset(&h->vel, 0, sizeof(h->vel));
     h->vel.time_kind = FLSP_T_ONE;
     ST(build_vtab(h, false));
-    CU(cudaMalloc(&h->fe_u64, (size_t)n * sizeof(double)));
+    if (next && next == h->fe_next) {
+      std::swap(h->fe_u64, h->fe_next);
+      h->fe_next_n = 0;
+    } else {
+      CU(cudaMalloc(&h->fe_u64, (size_t)n * sizeof(double)));
+    }
     ST(ensure_vel_table(h));
     h->fe_pv = degree;
+  } else if (next && next == h->fe_next) {
+    std::swap(h->fe_u64, h->fe_next);
   }
+  if (next != h->fe_u64)   // from the staging buffer or, checked there, from the host
+    CU(cudaMemcpyAsync(h->fe_u64, next ? next : values, (size_t)n * sizeof(double), cudaMemcpyDefault, h->stream));
   double gl[kMaxFeVel + 1], xq[8], wq[8], gb[kMaxFeVel + 1][kMaxNQ + 2];
   gauss_lobatto01(degree, gl);
   gauss_rule(h->p + 2, xq, wq);
   std::memset(gb, 0, sizeof(gb));
   for (int a = 0; a <= degree; ++a)
     for (int j = 0; j < h->p + 2; ++j) gb[a][j] = lagrange(degree, gl, a, xq[j]);
-  std::swap(h->fe_u64, h->fe_next);
   Ctx c = h->ctx();
   ST(launch_fe_tabulate(c, h->fe_u64, degree, gb, h->tab));
   CU(cudaMemsetAsync(&h->clk->vd_static, 0, sizeof(double), h->stream));

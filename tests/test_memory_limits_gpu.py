@@ -1,0 +1,85 @@
+"""What a problem needs on the device, and what it does where there is no room for
+more: the rest of the GPU is held by one allocation meanwhile."""
+import numpy as np
+import pytest
+
+from felspa_b200 import abi, fields as F
+from felspa_b200.level_set import AdvectSimulator, Mesh
+from felspa_b200.lib import FlspError
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+def free():
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.cuda.mem_get_info()[0]
+
+
+class Rest:
+    """holds all of the device's memory but `leave` bytes"""
+
+    def __init__(self, leave):
+        n = free() - int(leave)
+        self.t = torch.empty(max(n, 1), dtype=torch.uint8, device="cuda:0")
+
+    def give_back(self):
+        self.t = None
+        free()
+
+
+def rate(sim):
+    return sim.explicit_time_derivative(0.0)
+
+
+def table_bytes(n, p):
+    """a velocity table of a 3D FP32 problem: 4 x 4 x 4 tiles, 64 (p+2)^3 points of
+    three components and 240 faces of (p+2)^2 points each"""
+    tiles = np.prod([(v + 3) // 4 for v in n])
+    return int(tiles) * 4 * (3 * 64 * (p + 2) ** 3 + 240 * (p + 2) ** 2)
+
+
+def test_lattice_is_checked_without_a_second_one(flsp):
+    n = (40, 40, 40)
+    sim = AdvectSimulator(Mesh(3, n), 2, basis=abi.BASIS_Q, precision=abi.FP32)
+    lattice = F.random_fe_lattice(n, 2, seed=1)
+    had = free()
+    sim.problem.set_velocity_fe(2, lattice)
+    took = had - free()
+    assert took <= table_bytes(n, 2) + lattice.nbytes + 8 * MB
+    sim.problem.set_velocity_fe(2, -lattice)
+    assert had - free() <= took + 2 * MB
+
+
+def test_lattice_without_room_for_another(flsp):
+    """degree 3 on degree-1 cells: the lattice is larger than the staging buffer,
+    and there is room for one lattice and the table only"""
+    n = (64, 64, 64)
+    warm = AdvectSimulator(Mesh(3, (8, 8, 8)), 1, basis=abi.BASIS_P, precision=abi.FP32)
+    warm.problem.project(F.sphere((0.5, 0.5, 0.5), 0.3))
+    warm.problem.set_velocity_fe(3, F.random_fe_lattice((8, 8, 8), 3, seed=1))
+    rate(warm)
+    a, b = (F.random_fe_lattice(n, 3, seed=s) for s in (2, 3))
+    sim = AdvectSimulator(Mesh(3, n), 1, basis=abi.BASIS_P, precision=abi.FP32)
+    sim.problem.project(F.sphere((0.5, 0.5, 0.5), 0.3))
+    assert a.nbytes > 100 * MB
+    rest = Rest(a.nbytes + table_bytes(n, 1) + 60 * MB)
+    try:
+        sim.problem.set_velocity_fe(3, a)
+        first = rate(sim)
+        sim.problem.set_velocity_fe(3, b)
+        second = rate(sim)
+        bad = a.copy()
+        bad.ravel()[-1] = np.inf
+        with pytest.raises(FlspError, match="non-finite"):
+            sim.problem.set_velocity_fe(3, bad)
+        assert np.array_equal(rate(sim), second)
+    finally:
+        rest.give_back()
+    for lattice, want in ((a, first), (b, second)):
+        sim.problem.set_velocity_fe(3, lattice)
+        assert np.array_equal(rate(sim), want)
+    assert not np.array_equal(first, second)
