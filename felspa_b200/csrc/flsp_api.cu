@@ -290,6 +290,23 @@ int sync_clock(flsp_handle* h) {
   return device_error(h);
 }
 
+// the reinitialisation's smooth-sign table
+int ensure_sign_table(flsp_handle* h) {
+  size_t bytes = 0;
+  ST(hj_table_bytes(h->ctx(), h->hj_tile, &bytes));
+  if (bytes == h->hj_stab_bytes) return FLSP_OK;
+  if (h->hj_stab) cudaFree(h->hj_stab);
+  h->hj_stab = nullptr;
+  h->hj_stab_bytes = 0;
+  if (cudaMalloc(&h->hj_stab, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    h->hj_stab = nullptr;
+    return fail(FLSP_ERR_OOM, "no room for the reinitialisation's sign table");
+  }
+  h->hj_stab_bytes = bytes;
+  return FLSP_OK;
+}
+
 // kernel configuration of this handle (tiles, shared-memory attributes);
 // done outside any stream capture
 int prepare_kernels(flsp_handle* h) {
@@ -298,15 +315,10 @@ int prepare_kernels(flsp_handle* h) {
   ST(adv_prepare(c, h->veldev(), h->adv_tile));
   ST(hj_default_tile(c, h->hj_tile));
   ST(hj_prepare(c, h->hj_tile));
-  size_t bytes = 0;
-  ST(hj_table_bytes(c, h->hj_tile, &bytes));
-  if (bytes != h->hj_stab_bytes) {
-    if (h->hj_stab) cudaFree(h->hj_stab);
-    h->hj_stab = nullptr;
-    h->hj_stab_bytes = 0;
-    CU(cudaMalloc(&h->hj_stab, bytes));
-    h->hj_stab_bytes = bytes;
-  }
+  // a problem in the P basis whose sign table finds no room can still advect: a
+  // reinitialisation asks again (batches hold Q problems and their tables)
+  const int st = ensure_sign_table(h);
+  if (st && h->basis == FLSP_BASIS_Q) return st;
   ST(ldg_prepare(c));
   if (h->dim == 2) ST(weno_prepare(c));
   return FLSP_OK;
@@ -464,7 +476,8 @@ void fill_reinit_defaults(flsp_reinit_opts* o) {
   o->band_cells = 6.0;
 }
 
-int validate_reinit(const flsp_handle* h, const flsp_reinit_opts* o) {
+// options as a reinitialisation takes them, and its table (before any capture)
+int validate_reinit(flsp_handle* h, const flsp_reinit_opts* o) {
   if (!o) return fail(FLSP_ERR_BAD_ARG, "null reinit options");
   if (o->mode < 0 || o->mode > 2) return fail(FLSP_ERR_BAD_ARG, "bad reinit mode");
   if (!(o->cfl_max > 0.0)) return fail(FLSP_ERR_BAD_ARG, "reinit cfl_max must be positive");
@@ -476,8 +489,8 @@ int validate_reinit(const flsp_handle* h, const flsp_reinit_opts* o) {
   if (o->viscosity < 0.0) return fail(FLSP_ERR_BAD_ARG, "negative viscosity");
   if (o->rk_order < 1 || o->rk_order > 3) return fail(FLSP_ERR_BAD_ARG, "reinit rk_order must be 1..3");
   if (o->narrow_band && !(o->band_cells > 0.0)) return fail(FLSP_ERR_BAD_ARG, "narrow band needs band_cells > 0");
-  (void)h;
-  return FLSP_OK;
+  CU(cudaSetDevice(h->dev));
+  return ensure_sign_table(h);
 }
 
 // Compute-restricted narrow band (flsp_reinit_opts::narrow_band): only the

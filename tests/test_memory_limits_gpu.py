@@ -4,8 +4,8 @@ import numpy as np
 import pytest
 
 from felspa_b200 import abi, fields as F
-from felspa_b200.level_set import AdvectSimulator, Mesh
-from felspa_b200.lib import FlspError
+from felspa_b200.level_set import AdvectSimulator, Mesh, Problem, ReinitSimulatorLDG
+from felspa_b200.lib import FlspError, check, load
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -83,3 +83,33 @@ def test_lattice_without_room_for_another(flsp):
         sim.problem.set_velocity_fe(3, lattice)
         assert np.array_equal(rate(sim), want)
     assert not np.array_equal(first, second)
+
+
+def test_advection_without_room_for_the_sign_table(flsp):
+    """P basis: the table of a reinitialisation (288 bytes a cell at 3D degree 2)
+    is no condition for a problem that only advects"""
+    n = (72, 72, 72)
+    for warm in (True, False):
+        if not warm:
+            ndofs = 10 * int(np.prod(n))
+            rest = Rest(ndofs * (3 * 4 + 6 * 8) + 60 * MB)
+        try:
+            pb = Problem(Mesh(3, (8, 8, 8) if warm else n), 2, basis=abi.BASIS_P, precision=abi.FP32, cfl_max=0.1)
+            pb.set_velocity(F.deformation_3d())
+            pb.project(F.sphere((0.4, 0.4, 0.4), 0.2))
+            check(load().flsp_advance_steps(pb.h, 2, float("inf")))
+            o = abi.default_reinit_opts(mode=abi.REINIT_FIXED, n_pseudo_steps=1)
+            if warm:
+                ReinitSimulatorLDG(pb).run_iteration(o)
+                pb.close()
+                continue
+            before = pb.get_state()
+            with pytest.raises(FlspError, match="sign table"):
+                ReinitSimulatorLDG(pb).run_iteration(o)
+            assert np.array_equal(pb.get_state(), before)
+        finally:
+            if not warm:
+                rest.give_back()
+    ReinitSimulatorLDG(pb).run_iteration(o)
+    assert not np.array_equal(pb.get_state(), before)
+    pb.close()
