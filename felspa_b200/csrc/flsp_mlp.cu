@@ -656,6 +656,16 @@ static int stage_out(flsp_mlp* net, const float* src, float* dst, size_t n) {
   return FLSP_OK;
 }
 
+// a host call's work between its staging buffers: after a failure nothing of it is
+// in flight when the next call writes them or they are freed
+template <typename F>
+static int staged_call(flsp_mlp* net, F&& body) {
+  const int st = body();
+  if (st != FLSP_OK) cudaStreamSynchronize(net->stream);
+  release_staging(net);
+  return st;
+}
+
 }  // namespace flsp
 
 using namespace flsp;
@@ -810,15 +820,15 @@ int flsp_mlp_forward(flsp_mlp* net, const float* x, int64_t batch, float* y) {
   MST(mlp_ensure_cap(net, batch));
   const size_t nx = (size_t)batch * net->n_in, ny = (size_t)batch * net->n_out;
   MST(ensure_call_staging(net, nx + ny));
-  MST(stage_in(net, x, 0, nx));
-  MST(mlp_pack_input(net, net->io, nullptr, batch, nullptr));
-  MST(mlp_forward_dev(net, batch, false, nullptr));
-  k_pack_output<<<(unsigned)std::min<size_t>((ny + 255) / 256, 4096), 256, 0, net->stream>>>(
-      net->y, net->y_ld, net->n_out, (long long)ny, net->io);
-  MST(launch_status("k_pack_output"));
-  const int st = stage_out(net, net->io, y, ny);
-  release_staging(net);
-  return st;
+  return staged_call(net, [&]() -> int {
+    MST(stage_in(net, x, 0, nx));
+    MST(mlp_pack_input(net, net->io, nullptr, batch, nullptr));
+    MST(mlp_forward_dev(net, batch, false, nullptr));
+    k_pack_output<<<(unsigned)std::min<size_t>((ny + 255) / 256, 4096), 256, 0, net->stream>>>(
+        net->y, net->y_ld, net->n_out, (long long)ny, net->io);
+    MST(launch_status("k_pack_output"));
+    return stage_out(net, net->io, y, ny);
+  });
 }
 
 int flsp_mlp_backward(flsp_mlp* net, const float* x, const float* dy, int64_t batch, float* grad) {
@@ -828,15 +838,15 @@ int flsp_mlp_backward(flsp_mlp* net, const float* x, const float* dy, int64_t ba
   MST(mlp_ensure_cap(net, batch));
   const size_t nx = (size_t)batch * net->n_in, ny = (size_t)batch * net->n_out;
   MST(ensure_call_staging(net, nx + ny));
-  MST(stage_in(net, x, 0, nx));
-  MST(stage_in(net, dy, nx, ny));
-  MST(mlp_pack_input(net, net->io, nullptr, batch, nullptr));
-  MST(mlp_forward_dev(net, batch, true, nullptr));
-  MST(output_grad(net, batch, net->io + nx, nullptr));
-  MST(mlp_backward_dev(net, batch));
-  const int st = stage_out(net, net->g, grad, (size_t)net->n_params);
-  release_staging(net);
-  return st;
+  return staged_call(net, [&]() -> int {
+    MST(stage_in(net, x, 0, nx));
+    MST(stage_in(net, dy, nx, ny));
+    MST(mlp_pack_input(net, net->io, nullptr, batch, nullptr));
+    MST(mlp_forward_dev(net, batch, true, nullptr));
+    MST(output_grad(net, batch, net->io + nx, nullptr));
+    MST(mlp_backward_dev(net, batch));
+    return stage_out(net, net->g, grad, (size_t)net->n_params);
+  });
 }
 
 int flsp_mlp_n_pairs(const flsp_mlp* net, int64_t* n) {
