@@ -585,8 +585,11 @@ static int check_err(flsp_mlp* net) {
 
 // Device staging of `bytes`, and pinned host staging of at most kPinnedMax,
 // kept for the next call (an allocation per call, freed at its end, cost most
-// of a call's time: 8192 2D patches forward and backward took 4.7 ms, 1.28 with
-// the buffers kept)
+// of a call's time: 8192 2D patches forward and backward took 4.0 ms, 1.0 with
+// the buffers kept).  The device side comes from the stream's memory pool and the
+// pinned side is the call's inputs and outputs, for the first call's sake: room for
+// the parameter gradient there (pageable without) made a fresh network's first two
+// passes over 130 3D patches 3.9 ms instead of 1.5, and later ones no faster.
 constexpr size_t kPinnedMax = (size_t)64 << 20;
 static int ensure_staging(flsp_mlp* net, size_t bytes) {
   const size_t host = std::min(bytes, kPinnedMax);
@@ -598,26 +601,19 @@ static int ensure_staging(flsp_mlp* net, size_t bytes) {
     net->hbuf_bytes = host;
   }
   if (net->io_bytes < bytes) {
-    MCU(cudaStreamSynchronize(net->stream));
-    if (net->io) cudaFree(net->io);
+    if (net->io) cudaFreeAsync(net->io, net->stream);
     net->io = nullptr;
     net->io_bytes = 0;
-    MCU(cudaMalloc(&net->io, bytes));
+    MCU(cudaMallocAsync(&net->io, bytes, net->stream));
     net->io_bytes = bytes;
   }
   return FLSP_OK;
 }
 
-// one size for a batch's forward and backward calls: the second of them finds
-// its buffers there
-static int ensure_call_staging(flsp_mlp* net, size_t n) {
-  return ensure_staging(net, (std::max(n, (size_t)net->n_params) + 1) * 4);
-}
-
 // the device staging of a very large batch is not kept
 static void release_staging(flsp_mlp* net) {
   if (net->io_bytes <= 4 * kPinnedMax) return;
-  cudaFree(net->io);
+  cudaFreeAsync(net->io, net->stream);
   net->io = nullptr;
   net->io_bytes = 0;
 }
@@ -819,7 +815,7 @@ int flsp_mlp_forward(flsp_mlp* net, const float* x, int64_t batch, float* y) {
   MCU(cudaSetDevice(net->dev));
   MST(mlp_ensure_cap(net, batch));
   const size_t nx = (size_t)batch * net->n_in, ny = (size_t)batch * net->n_out;
-  MST(ensure_call_staging(net, nx + ny));
+  MST(ensure_staging(net, (nx + ny + 1) * 4));
   return staged_call(net, [&]() -> int {
     MST(stage_in(net, x, 0, nx));
     MST(mlp_pack_input(net, net->io, nullptr, batch, nullptr));
@@ -837,7 +833,7 @@ int flsp_mlp_backward(flsp_mlp* net, const float* x, const float* dy, int64_t ba
   MCU(cudaSetDevice(net->dev));
   MST(mlp_ensure_cap(net, batch));
   const size_t nx = (size_t)batch * net->n_in, ny = (size_t)batch * net->n_out;
-  MST(ensure_call_staging(net, nx + ny));
+  MST(ensure_staging(net, (nx + ny + 1) * 4));
   return staged_call(net, [&]() -> int {
     MST(stage_in(net, x, 0, nx));
     MST(stage_in(net, dy, nx, ny));
