@@ -302,8 +302,11 @@ __device__ __forceinline__ void atomic_max_pos(unsigned long long* slot, double 
   atomicMax(slot, (unsigned long long)__double_as_longlong(v));
 }
 
-// rsqrtf of a normal number (rsqrtf's own instruction without the scaling
-// around it for subnormal inputs)
+// 1 / sqrt(x) for x >= 1e-30 by the PTX instruction rsqrt.approx.ftz.f32: relative
+// error at most 2^-22.9 over the positive finite numbers (PTX ISA, rsqrt); .ftz takes
+// a subnormal input as zero, which the caller's range excludes.  rsqrtf gave the same
+// bits in every run compared and took longer: 64^3 Q2 FP32 run 22.97 against 22.81 ms,
+// band reinitialisation of 56 x 64 x 48 6.84 against 6.77.
 __device__ __forceinline__ float rsqrt_normal(float x) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
