@@ -48,7 +48,7 @@ def parse():
                     choices=["headline", "fe", "batched"],
                     help="short run for ncu, no timing loops: headline = the 64^3 workload's set-up and 2 reinit "
                          "periods; fe = the same with the deformation field at t = 0 as a degree-2 FE velocity "
-                         "lattice; batched = the 256-problem batch, autotuned, 2 reinit periods")
+                         "lattice; batched = the 256-problem batch, 2 reinit periods")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-fp64-check", action="store_true",
                     help="skip the FP64 run of the same periods (accuracy of the FP32 mode)")
@@ -253,7 +253,6 @@ def run_ours(args):
     if args.profile == "batched":
         from felspa_b200.batch import make_batch, uneven_batch_instances
         b = make_batch(uneven_batch_instances(256), precision=abi.FP32)
-        b.autotune()
         ctl = abi.default_ls_opts(reinit_frequency=REINIT_EVERY,
                                   reinit=abi.default_reinit_opts(mode=abi.REINIT_FIXED, n_pseudo_steps=N_PSEUDO))
         b.run_steps(2 * REINIT_EVERY, ctl)
@@ -386,9 +385,7 @@ def run_ours(args):
                 "kernel": "adv_sep_kernel<3,2,float>", "ms_per_launch": ms_stage,
                 "algorithmic_bytes_per_launch": alg_bytes_per_launch, "peak_source": peak_kind,
                 "hj_ms_per_launch": ms_hj, "hj_algorithmic_bytes_per_launch": 3.0 * s * n_dofs,
-                "hj_frac": 3.0 * s * n_dofs / (ms_hj * 1e-3) / 1e9 / peak,
-                "stage_tile": list(tile),
-                "stage_tile_ms": {"x".join(map(str, k)): v for k, v in tile_ms.items()}}
+                "hj_frac": 3.0 * s * n_dofs / (ms_hj * 1e-3) / 1e9 / peak}
 
     # a period: the substeps' clock, three stages each, the reinit's reset and CFL pass, its pseudo-steps
     per_step_launches = 1 + 3 * REINIT_EVERY + 2 + N_PSEUDO
@@ -416,19 +413,24 @@ def run_ours(args):
                 "d2h_bytes_per_step": 8 * n_dofs, "ms_per_step": e2e_total / args.steps},
         "gpu_launches": per_step_launches * args.steps,
         "clocks": clocks,
+    }
+    # the side measurements go to stderr, a JSON line of their own: the result's
+    # line stays short enough for a reader that keeps the end of stdout
+    detail = {
         "fp64": fp64,
         "accuracy": {"area_rel_change": (area1 - area0) / area0,
                      "fp32_vs_fp64": (fp64 or {}).get("fp32_vs_fp64")},
+        "stage_tile": list(tile), "stage_tile_ms": {"x".join(map(str, k)): v for k, v in tile_ms.items()},
     }
     if world == 1 and not args.no_oracle_checks:
-        line["accuracy"]["sphere_64cubed_vs_oracle"] = sphere_vs_oracle(local)
-        line["accuracy"]["zalesak_128"] = zalesak_accuracy(local)
+        detail["accuracy"]["sphere_64cubed_vs_oracle"] = sphere_vs_oracle(local)
+        detail["accuracy"]["zalesak_128"] = zalesak_accuracy(local)
     if world == 1 and not args.no_learned:
-        line["learned_vs_plain"] = learned_comparison()
-        line["learned_vs_plain_3d"] = learned_comparison_3d()
+        detail["learned_vs_plain"] = learned_comparison()
+        detail["learned_vs_plain_3d"] = learned_comparison_3d()
     if world == 1 and not args.no_variants:
         from felspa_b200 import fields as F
-        line["variants"] = {
+        detail["variants"] = {
             "narrow_band_64cubed": {
                 "what": "the headline workload with the compute-restricted narrow band (6 cells) in the reinit",
                 **variant_rate(abi.FP32, local, N_CELLS, F.deformation_3d(), F.sphere((0.35, 0.35, 0.35), 0.15), 10,
@@ -439,30 +441,31 @@ def run_ours(args):
                         "16 cosine modes; plain full-sweep reinit",
                 **variant_rate(abi.FP32, local, 128, F.plume_3d(), F.perturbed_plane(seed=5), 4)},
         }
-        line["variants"]["fe_velocity_64cubed"] = {
+        detail["variants"]["fe_velocity_64cubed"] = {
             "what": "the headline workload with the velocity of a coupled FE simulator: the deformation field at "
                     "t = 0 as a continuous Q2 nodal field on the Gauss-Lobatto lattice (flsp_set_velocity_fe, "
                     "constant in time), evaluated per cell at the quadrature points by the point-wise stage kernel",
             **variant_rate(abi.FP32, local, N_CELLS, F.deformation_3d(), F.sphere((0.35, 0.35, 0.35), 0.15), 10,
                            fe_degree=2)}
         from felspa_b200.batch import plume_group
-        line["variants"]["plume_group"] = {
+        detail["variants"]["plume_group"] = {
             "what": "a large 3D run with side problems: the 128^3 Q2 FP32 plume problem and 8 side 64^3 problems (perturbed "
                     "planes, seeds 5..13) advanced together, each reinit period (5 SSP-RK3 substeps + a fixed "
                     "5-pseudo-step plain reinit) of all 9 problems replayed from ONE CUDA graph (one branch per "
                     "problem); compared with the same periods replayed problem by problem",
             **plume_group(periods=40)}
         if not args.no_learned:
-            line["variants"]["plume_group_learned"] = plume_group_learned()
+            detail["variants"]["plume_group_learned"] = plume_group_learned()
     if world == 1 and not args.no_batched:
         from felspa_b200.batch import uneven_batch_benchmark
         r = uneven_batch_benchmark()
-        line["batched"] = {
+        detail["batched"] = {
             "workload": "256 independent 2D Q problems, meshes log-uniform 32^2..256^2, degree U{1,2,3}, union of 1-4 "
                         "circles, 8-mode Fourier stream-function velocity (seeds default_rng(1000+i)), 500 SSP-RK3 "
-                        "steps, fixed 5-pseudo-step reinit every 10, FP32; one persistent launch per RK stage / "
-                        "pseudo-step, periods replayed from CUDA graphs, tiles from the autotuner",
+                        "steps, fixed 5-pseudo-step reinit every 10, FP32; one launch per degree and RK stage / "
+                        "pseudo-step, periods replayed from CUDA graphs",
             **{k: (round(v, 6) if isinstance(v, float) else v) for k, v in r.items()}}
+    print(json.dumps({"detail": detail}), file=sys.stderr, flush=True)
     print(json.dumps(line), flush=True)
     if dist:
         dist.destroy_process_group()
