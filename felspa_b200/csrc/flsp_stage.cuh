@@ -5,28 +5,40 @@
 
 namespace flsp {
 
-// stage combination: v = phi + dt L (L itself for kRhsOnly), then the weighted
-// sum (v + b phi^n) f with phi^n, its products and sums in the order CombineMode
-// states (kRK3c as (v + phi^n / 2) (2/3): the same bits, both factors moved by a
-// power of two).  A narrow band and a learned reinitialisation compare cell means
-// with a threshold, so the last bits decide which cells they take: the order is
-// part of the result.  v + w (phi^n - v) leaves out the FP32 constant's scaling by
-// up to 1 + 3e-8 a step and ends 3 to 5 times nearer the 64-bit field, but it moved
-// the means at the edge of a 6-cell band by 1.3e-7 in 60 steps (this order: 9e-9, an
-// ulp), and 2 of 26 FP32 band runs by 5.8e-4 and 1.3e-3 of the field in the cells
-// that changed sides.  The two cost the same (64^3 Q2 FP32 run 22.8 and 22.9 ms).
+// stage combination: v = phi + dt L (L itself for kRhsOnly), then phi^n's share.
+// FP32: the weighted sum (v + b phi^n) f, its products and sums in the order
+// CombineMode states (kRK3c as (v + phi^n / 2) (2/3): the same bits, both factors
+// moved by a power of two).  A narrow band and a learned reinitialisation compare
+// cell means with a threshold, so the last bits decide which cells they take, and an
+// FP32 mean is near enough to it for that to happen: the order is part of the
+// result.  v + w (phi^n - v) leaves out the constant's scaling by up to 1 + 3e-8 a
+// step and ends 3 to 5 times nearer the 64-bit field, but it moved the means at the
+// edge of a 6-cell band by 1.3e-7 in 60 steps (this order: 9e-9, an ulp), and 2 of 26
+// band runs by 5.8e-4 and 1.3e-3 of the field in the cells that changed sides.  The
+// two cost the same (64^3 Q2 run 22.9 and 22.8 ms).
+// FP64: v + w (phi^n - v); 120 steps of a rotation end 7e-16 from extended
+// precision, with the weighted sum 6.5e-15.
 template <typename T>
 struct Combine {
-  T dt, b, f;
+  static constexpr bool SUM = sizeof(T) == 4;
+  T dt, w, f;
   bool rhs;
-  __device__ __forceinline__ Combine(int mode, T step)
-      : dt(mode == kRhsOnly ? T(1) : step),
-        b(mode == kRK2b ? T(1) : mode == kRK3b ? T(3) : mode == kRK3c ? T(0.5) : T(0)),
-        f(mode == kRK2b ? T(0.5) : mode == kRK3b ? T(0.25) : T(2) * (T(1) / T(3))),
-        rhs(mode == kRhsOnly) {}
+  __device__ __forceinline__ Combine(int mode, T step) : dt(mode == kRhsOnly ? T(1) : step), rhs(mode == kRhsOnly) {
+    if constexpr (SUM) {
+      w = mode == kRK2b ? T(1) : mode == kRK3b ? T(3) : mode == kRK3c ? T(0.5) : T(0);
+      f = mode == kRK2b ? T(0.5) : mode == kRK3b ? T(0.25) : T(2) * (T(1) / T(3));
+    } else {
+      w = mode == kRK2b ? T(0.5) : mode == kRK3b ? T(0.75) : mode == kRK3c ? T(1) / T(3) : T(0);
+    }
+  }
   __device__ __forceinline__ T operator()(T phi, T phin, T L) const {
-    const T v = fma(dt, L, rhs ? T(0) : phi);
-    return b != T(0) ? fma(b, phin, v) * f : v;
+    if constexpr (SUM) {
+      const T v = fma(dt, L, rhs ? T(0) : phi);
+      return w != T(0) ? fma(w, phin, v) * f : v;
+    } else {
+      const T v = (rhs ? T(0) : phi) + dt * L;
+      return w != T(0) ? v + w * (phin - v) : v;
+    }
   }
 };
 
