@@ -349,7 +349,6 @@ AdvClockArgs clock_args(const flsp_handle* h, bool step_count) {
   ca.tkind = h->vel.time_kind;
   ca.ta = h->vel.ta;
   ca.tb = h->vel.tb;
-  ca.rk = h->rk;
   ca.step_count = step_count ? 1 : 0;
   return ca;
 }
@@ -2128,7 +2127,6 @@ int batch_build(flsp_batch* b) {
     q.ca.tkind = h->vel.time_kind;
     q.ca.ta = h->vel.ta;
     q.ca.tb = h->vel.tb;
-    q.ca.rk = h->rk;
     q.ca.step_count = 1;
     q.adv_scale = adv_cfl_scaling(h->p);
     auto add = [&](const MeshArgs& m, std::vector<int2>& it) {
@@ -2200,8 +2198,7 @@ int batch_ready(flsp_batch* b) {
   return batch_build(b);
 }
 
-// the stage / reinit step / limiter of every problem: one launch per degree
-// one launch per degree present, side by side when there are several:
+// the stage or reinit step of every problem: one launch per degree present, side by side when there are several:
 // each degree's launch on its own stream forked from the batch stream and
 // joined back (graph branches under capture), so that one degree's tail
 // overlaps the others' work
@@ -2231,16 +2228,16 @@ int batch_each_degree(flsp_batch* b, int kind, F&& launch) {
 int batch_adv_all(flsp_batch* b, int in, int pn, int out, int stage, int combine) {
   return batch_each_degree(b, kBatchKindAdv, [&](int p, cudaStream_t s) {
     return launch_batch_adv(s, b->prec, p, b->probs, b->items_adv + b->deg_off[kBatchKindAdv][p],
-                            b->deg_cnt[kBatchKindAdv][p], b->deg_grid[kBatchKindAdv][p], b->deg_thr[kBatchKindAdv][p],
+                            b->deg_grid[kBatchKindAdv][p], b->deg_thr[kBatchKindAdv][p],
                             b->deg_smem[kBatchKindAdv][p], in, pn, out, 0, stage, combine);
   });
 }
 
-int batch_hj_all(flsp_batch* b, int src, int phi0, int dst, int mode, int rk) {
+int batch_hj_all(flsp_batch* b, int src, int dst, int mode, int rk) {
   return batch_each_degree(b, kBatchKindHJ, [&](int p, cudaStream_t s) {
     return launch_batch_hj(s, b->prec, p, b->probs, b->items_hj + b->deg_off[kBatchKindHJ][p],
-                           b->deg_cnt[kBatchKindHJ][p], b->deg_grid[kBatchKindHJ][p], b->deg_thr[kBatchKindHJ][p],
-                           b->deg_smem[kBatchKindHJ][p], src, phi0, dst, mode, rk, 0.2, 0);
+                           b->deg_grid[kBatchKindHJ][p], b->deg_thr[kBatchKindHJ][p],
+                           b->deg_smem[kBatchKindHJ][p], src, dst, mode, rk, 0.2, 0);
   });
 }
 
@@ -2253,7 +2250,7 @@ int batch_chain(flsp_batch* b, int p, cudaStream_t s, int steps, const flsp_rein
   const int np = b->prob_cnt[p];
   const int kA = kBatchKindAdv, kH = kBatchKindHJ, kW = kBatchKindWeno;
   auto stage = [&](int in, int pn, int out, int step, int k, int comb) {
-    return launch_batch_adv(s, b->prec, p, b->probs, b->items_adv + b->deg_off[kA][p], b->deg_cnt[kA][p],
+    return launch_batch_adv(s, b->prec, p, b->probs, b->items_adv + b->deg_off[kA][p],
                             b->deg_grid[kA][p], b->deg_thr[kA][p], b->deg_smem[kA][p], in, pn, out, step, k, comb);
   };
   for (int k = 0; k < steps; ++k) {
@@ -2275,22 +2272,22 @@ int batch_chain(flsp_batch* b, int p, cudaStream_t s, int steps, const flsp_rein
     }
   }
   if (!ro) return FLSP_OK;
-  auto hj = [&](int src, int phi0, int dst, int mode, int k) {
-    return launch_batch_hj(s, b->prec, p, b->probs, b->items_hj + b->deg_off[kH][p], b->deg_cnt[kH][p],
-                           b->deg_grid[kH][p], b->deg_thr[kH][p], b->deg_smem[kH][p], src, phi0, dst, mode, ro->rk_order, ro->cfl_max,
-                           k);
+  auto hj = [&](int src, int dst, int mode, int k) {
+    return launch_batch_hj(s, b->prec, p, b->probs, b->items_hj + b->deg_off[kH][p],
+                           b->deg_grid[kH][p], b->deg_thr[kH][p], b->deg_smem[kH][p], src, dst, mode, ro->rk_order,
+                           ro->cfl_max, k);
   };
   const int phi0 = *cur;
   ST(launch_batch_clock(s, probs, np, kBatchHjReset));
-  ST(hj(phi0, phi0, -1, kHJCflOnly, 0));
+  ST(hj(phi0, -1, kHJCflOnly, 0));
   for (int k = 0; k < ro->n_pseudo_steps; ++k) {
     const int src = *cur;
     const int dst = (src == phi0) ? (phi0 + 1) % 3 : other(src, phi0);
-    ST(hj(src, phi0, dst, kHJStep, k));
+    ST(hj(src, dst, kHJStep, k));
     int res = dst;
     if (limiter) {
       const int lim = other(dst, phi0);
-      ST(launch_batch_weno(s, b->prec, p, b->probs, b->items_weno + b->deg_off[kW][p], b->deg_cnt[kW][p],
+      ST(launch_batch_weno(s, b->prec, p, b->probs, b->items_weno + b->deg_off[kW][p],
                            b->deg_grid[kW][p], b->deg_thr[kW][p], b->deg_smem[kW][p], dst, lim));
       res = lim;
     }
@@ -2432,7 +2429,7 @@ int flsp_batch_autotune(flsp_batch* b, flsp_batch_tuning* out) {
   const int x = b->cur, y = (x + 1) % 3;
   int st = launch_batch_clock_steps(b->stream, b->probs, (int)b->h.size(), 1, false);
   if (st == FLSP_OK) st = time_it([&]() { return batch_adv_all(b, x, x, y, 0, kRK3a); }, &t.adv_ms[0]);
-  if (st == FLSP_OK) st = time_it([&]() { return batch_hj_all(b, x, x, -1, kHJCflOnly, 1); }, &t.hj_ms[0]);
+  if (st == FLSP_OK) st = time_it([&]() { return batch_hj_all(b, x, -1, kHJCflOnly, 1); }, &t.hj_ms[0]);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   ST(st);

@@ -65,11 +65,9 @@ __device__ __forceinline__ void adv_clock_horizon_body(DevClock* c, double time_
 }
 
 __device__ __forceinline__ void hj_clock_reset_body(DevClock* c) {
-  c->hj_vd_run = 0.0;
   c->hj_dt = 0.0;
   c->hj_cum = 0.0;
   for (int k = 0; k < 3; ++k) c->hj_vd[k] = 0ull;
-  c->hj_iter = 0;
 }
 
 // Size of pseudo-step a.k (ReinitSimulatorLDG::advance_time, reinit.cc:396-408,
@@ -80,10 +78,8 @@ __device__ __forceinline__ double hj_clock_step(DevClock* c, const HjClockArgs& 
   vd = __longlong_as_double((long long)c->hj_vd[a.k % 3]);
   const double dt = a.cfl_max / (a.scale * vd + a.shift);
   if (first) {
-    c->hj_vd_run = vd;
     c->hj_dt = dt;
     c->hj_cum += dt;
-    c->hj_iter += 1;
     c->hj_vd[(a.k + 2) % 3] = 0ull;
     atomic_max_pos(&c->hj_vd[(a.k + 1) % 3], vd);
   }

@@ -226,24 +226,16 @@ struct DevClock {
   double dt;         // current substep
   double vd_run;     // running max of (max vertex |u|)/diam (never reset:
                      // the reference CFLEstimator keeps its maximum)
-  double t_end;      // clamp for the substep (time_step - cumulative)
-  double ct[3];      // velocity time factor at the RK stage times
   double vd_static;  // max over vertices of |u_spatial| / diam
-  int active;        // current substep is non-zero
-  int pending;       // dt still to be added to t
   int n_substeps;    // executed substeps
   // reinitialisation
-  double hj_vd_run;  // running max of characteristic speed / diam
   double hj_dt;      // last pseudo-step
   double hj_cum;     // accumulated pseudo-time
   // running maxima of the CFL estimate (atomicMax on the bit patterns):
   // pseudo-step k reads slot k % 3, accumulates slot (k + 1) % 3 and clears
   // slot (k + 2) % 3
   unsigned long long hj_vd[3];
-  int hj_iter;
-  int hj_pending;
-  double band_ratio; // accumulated pseudo-time / horizon (host convenience)
-  double scratch[4];
+  double scratch[2]; // length of the advance call, cumulative time in it
 };
 
 // one substep of the advection clock, computed ahead of its stages (the
@@ -275,7 +267,6 @@ struct AdvClockArgs {
   double cfl_max, scale;
   int tkind;
   double ta, tb;
-  int rk;
   int step_count;   // 1: a step-count run (the horizon only caps the time)
 };
 

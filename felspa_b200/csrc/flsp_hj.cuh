@@ -26,12 +26,10 @@
 
 namespace flsp {
 
-
 template <typename T>
 struct HJArgs {
   MeshArgs m;
   const T* __restrict__ phi;    // phi^k (read with halo)
-  const T* __restrict__ phi0;   // phi at reinit start
   T* __restrict__ out;          // phi^{k+1}
   double* __restrict__ grad;    // gradient blocks (the export)
   DevClock* clk;
@@ -43,18 +41,6 @@ struct HJArgs {
   T* stab;                      // smooth-sign table of the tensor-product kernel (hjs_kernel)
   int* err;                     // the problem's error word
 };
-
-// add the cell's LDG diffusion RHS (HBM layout) to R (Q layout)
-template <int NM, typename T>
-__device__ __forceinline__ void add_rdiff(const MeshArgs& m, const T* rdiff, long long cell, T* R) {
-  if (!rdiff) return;
-  for (int k = 0; k < m.nb; ++k) {
-    const T v = rdiff[cell * m.nb + k];
-#pragma unroll
-    for (int q = 0; q < NM; ++q)
-      if (q == m.g2q[k]) R[q] += v;
-  }
-}
 
 // tile of the gradient export
 template <int DIM>

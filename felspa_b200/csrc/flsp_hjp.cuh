@@ -22,7 +22,7 @@
 // The launch's tiles (m.tile) may hold several HjsTile blocks of cells: block
 // b serves part b % NS of tile b / NS.  The narrow band lists whole tiles,
 // and which cells it sweeps is part of its result, so the tiles keep their
-// shapes (band_tile in flsp_k_hj.cu).
+// shapes (hj_default_tile, flsp_k_hj.cu).
 #pragma once
 #include "flsp_hjs.cuh"
 

@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(HjsTile<2>::N * (P + 2), advtab_min_blocks<2, 
 
 template <typename T, int P>
 __global__ void __launch_bounds__(HjsTile<2>::N * (P + 2), hjs_min_blocks<2, P, T>())
-    batch_hj_kernel(const BatchProb* __restrict__ probs, const int2* __restrict__ items, int isrc, int iphi0, int idst,
+    batch_hj_kernel(const BatchProb* __restrict__ probs, const int2* __restrict__ items, int isrc, int idst,
                     int mode, int rk, double cfl_max, int k) {
   __shared__ HJArgs<T> a;
   const int2 w = items[blockIdx.x];
@@ -66,7 +66,6 @@ __global__ void __launch_bounds__(HjsTile<2>::N * (P + 2), hjs_min_blocks<2, P, 
   copy_mesh(&a.m, pr.m_hj);
   if (threadIdx.x == 0) {
     a.phi = reinterpret_cast<const T*>(pr.buf[isrc]);
-    a.phi0 = reinterpret_cast<const T*>(pr.buf[iphi0]);
     a.out = idst >= 0 ? reinterpret_cast<T*>(pr.buf[idst]) : nullptr;
     a.clk = pr.clk;
     a.mode = mode;
@@ -171,7 +170,7 @@ int batch_prepare(int kind, int prec, int p, int n_items, size_t* smem, int* thr
   });
 }
 
-int launch_batch_adv(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items, int n_items,
+int launch_batch_adv(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items,
                      int grid, int threads, size_t smem, int ix, int in_n, int iout, int step, int stage, int combine) {
   return with_degree(p, [&](auto PC) -> int {
     constexpr int P = decltype(PC)::value;
@@ -180,17 +179,16 @@ int launch_batch_adv(cudaStream_t s, int prec, int p, const BatchProb* probs, co
   });
 }
 
-int launch_batch_hj(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items, int n_items,
-                    int grid, int threads, size_t smem, int isrc, int iphi0, int idst, int mode, int rk, double cfl_max,
-                    int k) {
+int launch_batch_hj(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items,
+                    int grid, int threads, size_t smem, int isrc, int idst, int mode, int rk, double cfl_max, int k) {
   return with_degree(p, [&](auto PC) -> int {
     constexpr int P = decltype(PC)::value;
     return launch_chained("batch_hj_kernel", prec == FLSP_FP64 ? batch_hj_kernel<double, P> : batch_hj_kernel<float, P>,
-                          (unsigned)grid, threads, smem, s, probs, items, isrc, iphi0, idst, mode, rk, cfl_max, k);
+                          (unsigned)grid, threads, smem, s, probs, items, isrc, idst, mode, rk, cfl_max, k);
   });
 }
 
-int launch_batch_weno(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items, int n_items,
+int launch_batch_weno(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items,
                       int grid, int threads, size_t smem, int iin, int iout) {
   return with_degree(p, [&](auto PC) -> int {
     constexpr int P = decltype(PC)::value;

@@ -128,7 +128,6 @@ int launch_hj(const Ctx& c, const void* phi, const void* phi0, void* out, DevClo
     else hj_default_tile(c, t);
     set_tile(a.m, DIM, t);
     a.phi = reinterpret_cast<const T*>(phi);
-    a.phi0 = reinterpret_cast<const T*>(phi0);
     a.out = reinterpret_cast<T*>(out);
     a.clk = clk;
     a.mode = mode;

@@ -69,7 +69,6 @@ enum BatchClockOp : int {
   kBatchAdvHorizon = 0, kBatchHjReset = 1
 };
 int upload_tables_batch();
-// shared memory one problem needs for a tile of the given kind
 // shared memory of the degree-p kernel of a kind, its attributes for it, and
 // the grid for n_items (every item of a launch has degree p)
 int batch_prepare(int kind, int prec, int p, int n_items, size_t* smem, int* threads, int* grid);
@@ -77,11 +76,11 @@ int launch_batch_clock(cudaStream_t s, const BatchProb* probs, int n, int what);
 // the next n_steps substeps of every problem (its steps array); commit as in
 // launch_adv_clock_steps
 int launch_batch_clock_steps(cudaStream_t s, const BatchProb* probs, int n, int n_steps, bool commit);
-int launch_batch_adv(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items, int n_items,
+int launch_batch_adv(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items,
                      int grid, int threads, size_t smem, int ix, int in_n, int iout, int step, int stage, int combine);
-int launch_batch_hj(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items, int n_items,
-                    int grid, int threads, size_t smem, int isrc, int iphi0, int idst, int mode, int rk, double cfl_max, int k);
-int launch_batch_weno(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items, int n_items,
+int launch_batch_hj(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items,
+                    int grid, int threads, size_t smem, int isrc, int idst, int mode, int rk, double cfl_max, int k);
+int launch_batch_weno(cudaStream_t s, int prec, int p, const BatchProb* probs, const int2* items,
                       int grid, int threads, size_t smem, int iin, int iout);
 
 // restrict a launch's MeshArgs to the narrow-band tile list of `kind`
@@ -197,8 +196,7 @@ int hj_table_bytes(const Ctx& c, const int* tile, size_t* bytes);
 int launch_hj(const Ctx& c, const void* phi, const void* phi0, void* out, DevClock* clk, int mode,
               int rk, const HjClockArgs* step, long long block, const int* tile,
               const void* rdiff = nullptr);
-// LDG artificial viscosity: mode 0 = alternating gradient q (DIM blocks)
-// from phi, mode 1 = diffusion RHS (per unit volume) from q
+// LDG artificial viscosity: the diffusion RHS (per unit volume) of `in`
 int ldg_prepare(const Ctx& c);
 int launch_ldg(const Ctx& c, const void* in, void* out, double nu);
 
