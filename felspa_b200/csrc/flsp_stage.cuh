@@ -14,8 +14,8 @@ namespace flsp {
 // result.  v + w (phi^n - v) leaves out the constant's scaling by up to 1 + 3e-8 a
 // step and ends 3 to 5 times nearer the 64-bit field, but it moved the means at the
 // edge of a 6-cell band by 1.3e-7 in 60 steps (this order: 9e-9, an ulp), and 2 of 26
-// band runs by 5.8e-4 and 1.3e-3 of the field in the cells that changed sides.  The
-// two cost the same (64^3 Q2 run 22.9 and 22.8 ms).
+// band runs by 5.8e-4 and 1.3e-3 of the field in the cells that changed sides.  They
+// cost the same in 3D (64^3 Q2 run 22.95 and 22.97 ms), the sum 0.7 % of a 256^2 run.
 // FP64: v + w (phi^n - v); 120 steps of a rotation end 7e-16 from extended
 // precision, with the weighted sum 6.5e-15.
 template <typename T>
