@@ -1,5 +1,7 @@
 """What a problem needs on the device, and what it does where there is no room for
 more: the rest of the GPU is held by one allocation meanwhile."""
+import gc
+
 import numpy as np
 import pytest
 
@@ -14,6 +16,7 @@ MB = 1 << 20
 
 
 def free():
+    gc.collect()   # problems that earlier tests left
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     return torch.cuda.mem_get_info()[0]
